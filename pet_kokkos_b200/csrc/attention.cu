@@ -13,6 +13,7 @@
 // the backward) rows are staged once in shared memory with 16-byte loads, then a
 // thread per token walks them (all threads read the same shared row: a broadcast).
 #include "attention.h"
+#include "gemm.h"
 
 namespace petb {
 
@@ -219,16 +220,7 @@ void bwd_hd(Stream& st, const AttnArgs& p) {
   launch(st, k_attn_bwd<HD>, p, sizeof(float) * (4 * size_t(p.S) * HD + 4 * size_t(p.S)), opted);
 }
 
-}  // namespace
-
-void attention_forward(Stream& st, const AttnArgs& p) {
-  if (p.N == 0) return;
-  // The reference's own count (tools/roofline.py:188-202): 4 sum(cnt^2) D flops forward, 10 backward;
-  // qkv read and the output written once.
-  const double D = double(p.H) * p.hd;
-  const ProfScope ps(st, PC_ATTN_FWD, 4.0 * p.pairs * D, 4.0 * p.T * (4.0 * D + 2.0 * p.H));
-  if (p.mode != ATTN_NATIVE && attention_forward_mma(st, p)) return;
-  if (attention_forward_tiled(st, p)) return;
+void forward_streaming(Stream& st, const AttnArgs& p) {
   switch (p.hd) {
     case 16: return fwd_hd<16>(st, p);
     case 32: return fwd_hd<32>(st, p);
@@ -239,13 +231,7 @@ void attention_forward(Stream& st, const AttnArgs& p) {
     default: throw Error(1, "attention: head_dim " + std::to_string(p.hd) + " is not one of 16, 32, 48, 64, 80, 128");
   }
 }
-
-void attention_backward(Stream& st, const AttnArgs& p) {
-  if (p.N == 0) return;
-  const double D = double(p.H) * p.hd;
-  const ProfScope ps(st, PC_ATTN_BWD, 10.0 * p.pairs * D, 4.0 * p.T * (8.0 * D + 3.0 * p.H));
-  if (p.mode != ATTN_NATIVE && attention_backward_mma(st, p)) return;
-  if (attention_backward_tiled(st, p)) return;
+void backward_streaming(Stream& st, const AttnArgs& p) {
   switch (p.hd) {
     case 16: return bwd_hd<16>(st, p);
     case 32: return bwd_hd<32>(st, p);
@@ -255,6 +241,29 @@ void attention_backward(Stream& st, const AttnArgs& p) {
     case 128: return bwd_hd<128>(st, p);
     default: throw Error(1, "attention: head_dim " + std::to_string(p.hd) + " is not one of 16, 32, 48, 64, 80, 128");
   }
+}
+
+}  // namespace
+
+void attention_forward(Stream& st, const AttnArgs& p) {
+  if (p.N == 0) return;
+  // The reference's own count (tools/roofline.py:188-202): 4 sum(cnt^2) D flops forward, 10 backward;
+  // qkv read and the output written once.
+  const double D = double(p.H) * p.hd;
+  const ProfScope ps(st, PC_ATTN_FWD, 4.0 * p.pairs * D, 4.0 * p.T * (4.0 * D + 2.0 * p.H));
+  if (p.mode != ATTN_NATIVE && attention_forward_mma(st, p)) return;
+  if (!attention_forward_tiled(st, p)) forward_streaming(st, p);
+  // the CUDA-core kernels leave the rows' maxima to a pass of its own
+  if (p.merged_max) row_max(st, p.merged_max, p.merged, int(D), int(p.T), int(D));
+}
+
+void attention_backward(Stream& st, const AttnArgs& p) {
+  if (p.N == 0) return;
+  const double D = double(p.H) * p.hd;
+  const ProfScope ps(st, PC_ATTN_BWD, 10.0 * p.pairs * D, 4.0 * p.T * (8.0 * D + 3.0 * p.H));
+  if (p.mode != ATTN_NATIVE && attention_backward_mma(st, p)) return;
+  if (!attention_backward_tiled(st, p)) backward_streaming(st, p);
+  if (p.qkv_adj_max) row_max(st, p.qkv_adj_max, p.qkv_adj, int(3 * D), int(p.T), int(3 * D));
 }
 
 }  // namespace petb

@@ -20,10 +20,12 @@ struct AttnArgs {
   const float* cut = nullptr;       // [E] cutoff factor of each edge token
   const float* qkv = nullptr;       // [T,3D] columns Q | K | V
   float* merged = nullptr;          // [T,D] attention output before the output projection
+  uint32_t* merged_max = nullptr;   // [T] unless null, each row's largest |merged| is raised into it (zeroed by the caller)
   float* ml = nullptr;              // [T,H,2] each query's running max and 1/sum (null: not saved)
   // backward
   const float* dmerged = nullptr;   // [T,D]
   float* qkv_adj = nullptr;         // [T,3D]
+  uint32_t* qkv_adj_max = nullptr;  // [T] unless null, each row's largest |qkv_adj| likewise
   float* cfh = nullptr;             // [T,H] each key's score adjoint summed over its queries
 };
 

@@ -36,6 +36,17 @@ __device__ __forceinline__ float warp_sum(float v) {
   return v;
 }
 
+// The largest magnitude of one row's values, held by the four lanes of a quad as KS pairs (c0, c1) of an accumulator,
+// raised into mx[row] (the GEMM that reads the rows scales them by it).
+template <int KS>
+__device__ __forceinline__ void raise_row(uint32_t* mx, size_t row, bool live, const float (*acc)[4], int c, float scale, int t) {
+  float m = 0.f;
+#pragma unroll
+  for (int db = 0; db < KS; ++db) m = fmaxf(m, fmaxf(fabsf(acc[db][c] * scale), fabsf(acc[db][c + 1] * scale)));
+  m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1)), m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
+  if (live && t == 0) atomicMax(mx + row, __float_as_uint(m));
+}
+
 struct Frag {
   uint32_t hi, lo;
 };
@@ -240,6 +251,10 @@ __global__ void __launch_bounds__(32 * ((MAXKB + 1) / 2), MAXKB <= 10 ? 4 : 1) k
     if (q0 < cnt) *reinterpret_cast<float2*>(p.merged + g0 * D + h * HD + 8 * db + 2 * t) = make_float2(o[db][0], o[db][1]);
     if (q1 < cnt) *reinterpret_cast<float2*>(p.merged + g1 * D + h * HD + 8 * db + 2 * t) = make_float2(o[db][2], o[db][3]);
   }
+  if (p.merged_max) {
+    raise_row<KS>(p.merged_max, g0, q0 < cnt, o, 0, 1.f, t);
+    raise_row<KS>(p.merged_max, g1, q1 < cnt, o, 2, 1.f, t);
+  }
   if (t == 0 && p.ml) {
     if (q0 < cnt) p.ml[(g0 * p.H + h) * 2] = dead0 ? kOff : m0, p.ml[(g0 * p.H + h) * 2 + 1] = il0;
     if (q1 < cnt) p.ml[(g1 * p.H + h) * 2] = dead1 ? kOff : m1, p.ml[(g1 * p.H + h) * 2 + 1] = il1;
@@ -346,6 +361,10 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 320 ? 2 : 1) k_attn_bwd_mma(Attn
       if (i1 < cnt)
         *reinterpret_cast<float2*>(p.qkv_adj + g1 * 3 * D + h * HD + 8 * db + 2 * t) = make_float2(dq[db][2] * p.sc, dq[db][3] * p.sc);
     }
+    if (p.qkv_adj_max) {
+      raise_row<KS>(p.qkv_adj_max, g0, i0 < cnt, dq, 0, p.sc, t);
+      raise_row<KS>(p.qkv_adj_max, g1, i1 < cnt, dq, 2, p.sc, t);
+    }
   } else {
     // transposed: rows are keys. S^T = K Q^T and dP^T = V dO^T per block of 8 queries; the accumulator
     // fragment of dS^T (and P^T) is the A operand of dK = dS^T Q (and dV = P^T dO).
@@ -409,6 +428,12 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 320 ? 2 : 1) k_attn_bwd_mma(Attn
         *reinterpret_cast<float2*>(p.qkv_adj + g1 * 3 * D + D + c) = make_float2(dk[db][2] * p.sc, dk[db][3] * p.sc);
         *reinterpret_cast<float2*>(p.qkv_adj + g1 * 3 * D + 2 * D + c) = make_float2(dv[db][2], dv[db][3]);
       }
+    }
+    if (p.qkv_adj_max) {
+      raise_row<KS>(p.qkv_adj_max, g0, i0 < cnt, dk, 0, p.sc, t);
+      raise_row<KS>(p.qkv_adj_max, g1, i1 < cnt, dk, 2, p.sc, t);
+      raise_row<KS>(p.qkv_adj_max, g0, i0 < cnt, dv, 0, 1.f, t);
+      raise_row<KS>(p.qkv_adj_max, g1, i1 < cnt, dv, 2, 1.f, t);
     }
     if (t == 0) {  // each key's dS summed over its queries: the cutoff factor's share from this head
       if (i0 < cnt) p.cfh[g0 * p.H + h] = cf0;

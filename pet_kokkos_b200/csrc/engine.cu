@@ -197,7 +197,7 @@ Engine::Engine(const std::string& json, const std::string& weights, const pet_op
   PETB_CUDA(cudaEventCreate(&ev0));
   PETB_CUDA(cudaEventCreate(&ev1));
   PETB_CUDA(cudaMallocHost(&pinned, 64 * sizeof(int)));
-  model.reset(new Model(ckpt));
+  model.reset(new Model(ckpt, gemm_mode));
 }
 
 Engine::~Engine() {
@@ -686,7 +686,7 @@ void Engine::fetch(pet_results* out) {
   PETB_CUDA(cudaStreamSynchronize(st.s));
   float ms = 0.f;
   if (cudaEventElapsedTime(&ms, ev0, ev1) == cudaSuccess) last_ms = ms;
-  if (gemm_mode != GEMM_NATIVE && gemm_tensor_error(st))
+  if (gemm_tensor_error(st))
     throw Error(5, "pet: a tensor-core GEMM gave up waiting on its pipeline; the results of this evaluation are invalid");
 }
 
@@ -1117,7 +1117,7 @@ void Engine::compute_step_device(const pet_device_arrays* a, const double* cell,
     if (skip) PETB_CUDA(cudaMemcpyAsync(pinned + 8, md.overflow, sizeof(int), cudaMemcpyDeviceToHost, st.s));
     PETB_CUDA(cudaStreamSynchronize(st.s));
     // a tensor-core GEMM that gave up on a wait left garbage behind, and the adds above have put it into the caller's arrays
-    if (gemm_mode != GEMM_NATIVE && gemm_tensor_error(st))
+    if (gemm_tensor_error(st))
       throw Error(5, "pet: a tensor-core GEMM gave up waiting on its pipeline; the arrays this step added into are invalid");
     if (skip && pinned[8] != 0) {  // outgrown: drop the capacities and run the step again, read back and resized
       md.caps_valid = false;
@@ -1281,7 +1281,7 @@ void Engine::compute_pairs(const pet_pair_list* v, const double* positions, cons
   }
   session_step(*this, positions, true, cell, forces);
   if (fixed_step_overflowed(*this)) session_step(*this, positions, true, cell, forces);
-  if (gemm_mode != GEMM_NATIVE && gemm_tensor_error(st))  // synchronizes the stream
+  if (gemm_tensor_error(st))  // synchronizes the stream
     throw Error(5, "pet: a tensor-core GEMM gave up waiting on its pipeline; the results of this evaluation are invalid");
   if (out) {
     *out = pet_device_results{};
@@ -1312,55 +1312,22 @@ void Engine::gemm_host(int mode, bool w_transposed, int m, int n, int k, const f
   PETB_CUDA(cudaStreamSynchronize(st.s));
   tmp_arena.reset();
   float* dA = tmp_arena.alloc<float>(size_t(m) * k);
-  float* dW = tmp_arena.alloc<float>(2 * size_t(n) * k);  // and, for the 3xTF32 mode, the low parts of its split behind it
+  float* dW = tmp_arena.alloc<float>(size_t(n) * k);
   float* dC = tmp_arena.alloc<float>(size_t(m) * n);
   PETB_CUDA(cudaMemcpyAsync(dA, A, 4 * size_t(m) * k, cudaMemcpyHostToDevice, st.s));
-  // The kernels take the weight K-major, [n, k]; the other orientation is transposed here, as a
-  // loaded weight is kept in both.
-  std::vector<float> wt;
-  const float* hw = W;
-  if (!w_transposed) {
-    wt.resize(size_t(n) * k);
-    for (int p = 0; p < k; ++p)
-      for (int j = 0; j < n; ++j) wt[size_t(j) * k + p] = W[size_t(p) * n + j];
-    hw = wt.data();
-  }
-  PETB_CUDA(cudaMemcpyAsync(dW, hw, 4 * size_t(n) * k, cudaMemcpyHostToDevice, st.s));
+  PETB_CUDA(cudaMemcpyAsync(dW, W, 4 * size_t(n) * k, cudaMemcpyHostToDevice, st.s));
   GemmArgs a;
-  a.A = dA, a.lda = k, a.B = dW, a.ldb = k, a.C = dC, a.ldc = n, a.M = m, a.N = n, a.K = k;
-  std::vector<float> wlo;
-  if (mode == GEMM_TF32X3) {  // the weight's low parts, made once as for a loaded weight (x minus its leading 11 bits, rounded)
-    wlo.resize(size_t(n) * k);
-    for (size_t i = 0; i < wlo.size(); ++i) {
-      uint32_t bits, lo;
-      std::memcpy(&bits, &hw[i], 4);
-      bits &= 0xFFFFE000u;
-      float hi;
-      std::memcpy(&hi, &bits, 4);
-      const float r = hw[i] - hi;
-      std::memcpy(&lo, &r, 4);
-      lo += 0x1000u;
-      std::memcpy(&wlo[i], &lo, 4);
-    }
-    PETB_CUDA(cudaMemcpyAsync(dW + size_t(n) * k, wlo.data(), 4 * wlo.size(), cudaMemcpyHostToDevice, st.s));
-    a.b_lo_offset = size_t(n) * k;
-  }
-  std::vector<uint16_t> w16;
-  if (mode == GEMM_BF16) {  // the weight again as bf16, round to nearest even, as a loaded weight is kept
-    w16.resize(size_t(n) * k);
-    for (size_t i = 0; i < w16.size(); ++i) {
-      uint32_t u;
-      std::memcpy(&u, &hw[i], 4);
-      w16[i] = uint16_t((u + 0x7FFFu + ((u >> 16) & 1u)) >> 16);
-    }
-    uint16_t* d16 = tmp_arena.alloc<uint16_t>(w16.size());
-    PETB_CUDA(cudaMemcpyAsync(d16, w16.data(), 2 * w16.size(), cudaMemcpyHostToDevice, st.s));
-    a.B16 = d16;
-  }
-  gemm(st, tmp_arena, a, mode);
+  a.A = dA, a.lda = k, a.C = dC, a.ldc = n, a.M = m, a.N = n, a.K = k;
+  // the weight packed from either orientation, as a loaded one is
+  auto pack = [&](Format fmt) {
+    uint16_t* out = tmp_arena.alloc<uint16_t>(packed_halves(fmt, n, k));
+    return pack_weight(st.s, fmt, dW, w_transposed ? k : 1, w_transposed ? 1 : n, n, k, out, tmp_arena.alloc<uint32_t>(1));
+  };
+  a.nat = pack(FMT_F16X3), a.fast = pack(format_of(mode));
+  gemm(st, tmp_arena, a);
   PETB_CUDA(cudaMemcpyAsync(C, dC, 4 * size_t(m) * n, cudaMemcpyDeviceToHost, st.s));
   PETB_CUDA(cudaStreamSynchronize(st.s));
-  if (mode != GEMM_NATIVE && gemm_tensor_error(st)) throw Error(5, "pet: a tensor-core GEMM gave up waiting on its pipeline");
+  if (gemm_tensor_error(st)) throw Error(5, "pet: a tensor-core GEMM gave up waiting on its pipeline");
 }
 
 }  // namespace petb

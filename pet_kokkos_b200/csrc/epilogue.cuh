@@ -25,6 +25,10 @@ struct EpiLoad {
   float e0, e1, e2, e3;  // compress: the edge's (v, |v|) in float
 };
 
+__device__ __forceinline__ float max_abs4(float a, float b, float c, float d) {
+  return fmaxf(fmaxf(fabsf(a), fabsf(b)), fmaxf(fabsf(c), fabsf(d)));
+}
+
 template <int EPI>
 __device__ __forceinline__ EpiLoad epilogue_load4(const GemmArgs& p, int row, int col) {
   const size_t r = size_t(row);
@@ -46,8 +50,9 @@ __device__ __forceinline__ EpiLoad epilogue_load4(const GemmArgs& p, int row, in
 }
 
 // acc[0..3] are the accumulators of C(row, col..col+3); col % 4 == 0 and col + 3 < N.
+// Returns the largest magnitude it put into C.
 template <int EPI>
-__device__ __forceinline__ void epilogue_apply4(const GemmArgs& p, int row, int col, const float* acc, const EpiLoad& l) {
+__device__ __forceinline__ float epilogue_apply4(const GemmArgs& p, int row, int col, const float* acc, const EpiLoad& l) {
   const size_t r = size_t(row);
   float z[4] = {acc[0], acc[1], acc[2], acc[3]};
   if (EPI == EPI_PLAIN || EPI == EPI_SILU || EPI == EPI_SWIGLU || EPI == EPI_COMPRESS) {
@@ -59,16 +64,23 @@ __device__ __forceinline__ void epilogue_apply4(const GemmArgs& p, int row, int 
   if (EPI == EPI_PLAIN) {
     if (p.res && row >= p.res_row0) z[0] += l.a.x, z[1] += l.a.y, z[2] += l.a.z, z[3] += l.a.w;
     st4(p.C + r * p.ldc + col, make_float4(z[0], z[1], z[2], z[3]));
+    return max_abs4(z[0], z[1], z[2], z[3]);
   } else if (EPI == EPI_SILU) {
     if (p.pre) st4(p.pre + r * p.ldp + col, make_float4(z[0], z[1], z[2], z[3]));
-    st4(p.C + r * p.ldc + col, make_float4(silu_f(z[0]), silu_f(z[1]), silu_f(z[2]), silu_f(z[3])));
+    const float4 o = make_float4(silu_f(z[0]), silu_f(z[1]), silu_f(z[2]), silu_f(z[3]));
+    st4(p.C + r * p.ldc + col, o);
+    return max_abs4(o.x, o.y, o.z, o.w);
   } else if (EPI == EPI_SWIGLU) {
     if (p.pre) st4(p.pre + r * p.ldp + col, make_float4(z[0], z[1], z[2], z[3]));
-    if (p.C)
-      *reinterpret_cast<float2*>(p.C + r * p.ldc + col / 2) = make_float2(z[0] * sigmoid_f(z[1]), z[2] * sigmoid_f(z[3]));
+    if (!p.C) return 0.f;
+    const float2 o = make_float2(z[0] * sigmoid_f(z[1]), z[2] * sigmoid_f(z[3]));
+    *reinterpret_cast<float2*>(p.C + r * p.ldc + col / 2) = o;
+    return fmaxf(fabsf(o.x), fabsf(o.y));
   } else if (EPI == EPI_SILU_BWD) {
     const float4 x = l.a;
-    st4(p.C + r * p.ldc + col, make_float4(z[0] * dsilu_f(x.x), z[1] * dsilu_f(x.y), z[2] * dsilu_f(x.z), z[3] * dsilu_f(x.w)));
+    const float4 o = make_float4(z[0] * dsilu_f(x.x), z[1] * dsilu_f(x.y), z[2] * dsilu_f(x.z), z[3] * dsilu_f(x.w));
+    st4(p.C + r * p.ldc + col, o);
+    return max_abs4(o.x, o.y, o.z, o.w);
   } else if (EPI == EPI_SWIGLU_BWD) {
     const float4 xa = l.a, xb = l.b;
     const float v[4] = {xa.x, xa.z, xb.x, xb.z}, g[4] = {xa.y, xa.w, xb.y, xb.w};
@@ -81,6 +93,7 @@ __device__ __forceinline__ void epilogue_apply4(const GemmArgs& p, int row, int 
     }
     st4(p.C + r * p.ldc + 2 * col, make_float4(o[0], o[1], o[2], o[3]));
     st4(p.C + r * p.ldc + 2 * col + 4, make_float4(o[4], o[5], o[6], o[7]));
+    return fmaxf(max_abs4(o[0], o[1], o[2], o[3]), max_abs4(o[4], o[5], o[6], o[7]));
   } else if (EPI == EPI_COMPRESS) {
     const float tt[4] = {l.a.x, l.a.y, l.a.z, l.a.w};
 #pragma unroll
@@ -89,14 +102,17 @@ __device__ __forceinline__ void epilogue_apply4(const GemmArgs& p, int row, int 
       z[j] = z[j] + tt[j] + w.x * l.e0 + w.y * l.e1 + w.z * l.e2 + w.w * l.e3;
     }
     if (p.pre) st4(p.pre + r * p.ldp + col, make_float4(z[0], z[1], z[2], z[3]));
-    st4(p.C + r * p.ldc + col, make_float4(silu_f(z[0]), silu_f(z[1]), silu_f(z[2]), silu_f(z[3])));
+    const float4 o = make_float4(silu_f(z[0]), silu_f(z[1]), silu_f(z[2]), silu_f(z[3]));
+    st4(p.C + r * p.ldc + col, o);
+    return max_abs4(o.x, o.y, o.z, o.w);
   }
+  return 0.f;
 }
 
 template <int EPI>
-__device__ __forceinline__ void epilogue_run4(const GemmArgs& p, int row, int col, const float* acc) {
+__device__ __forceinline__ float epilogue_run4(const GemmArgs& p, int row, int col, const float* acc) {
   const EpiLoad l = epilogue_load4<EPI>(p, row, col);
-  epilogue_apply4<EPI>(p, row, col, acc, l);
+  return epilogue_apply4<EPI>(p, row, col, acc, l);
 }
 
 }  // namespace petb

@@ -9,10 +9,12 @@
 // (src/ops.cpp:326-365).
 //
 // Two kernel families share the epilogue code:
-//   * native: fp32 FMA on the CUDA cores, one accumulation chain per output in k
-//     order, so a row's bits do not depend on how many rows the GEMM has;
-//   * tensor: tcgen05.mma (kind::tf32 or kind::f16 with bf16 operands) with TMA-fed
-//     shared-memory tiles and the accumulator in tensor memory.
+//   * tensor (gemm_tc.cu): tcgen05.mma kind::f16 with TMA-fed shared-memory tiles and the accumulator in tensor memory.
+//     Operands wider than 16 bits are split into 16-bit parts whose products are summed in fp32; the formats below say
+//     into which, for each mode;
+//   * fp32 FMA on the CUDA cores (gemm_simt.cu): one accumulation chain per output in k order, for operands that have
+//     no packed weight (pet_gemm_host_static) or that TMA cannot address.
+// A row's bits depend on that row and the weight alone, in both: not on how many rows share its launch.
 #pragma once
 
 #include "common.h"
@@ -30,17 +32,59 @@ enum Epilogue {
 
 enum GemmMode { GEMM_NATIVE = 0, GEMM_TF32 = 1, GEMM_BF16 = 2, GEMM_TF32X3 = 3 };
 
+// How an fp32 operand is handed to the 16-bit tensor cores. The fp16 formats scale it by a power of two first: s brings the
+// largest value of the row (of the matrix, for a weight) to [2^14, 2^15).
+//   FMT_F16X3 (native)   s x = h + m + l: h is s x rounded to a multiple of 2^8, eight bits of the row's largest value; what
+//                        remains goes into two fp16 parts. Every value is represented to its last bit, or to 2^-23 of
+//                        itself where it is below 2^-6 of the row's largest. Six products; h.h on its own accumulator,
+//                        where 1024 columns of K sum without any rounding; the rest (hm mh mm hl lh, 2^-8 of it and less;
+//                        what is left out is below 2^-27) on another. The two meet in one fp32 addition.
+//   FMT_F16X2 (3xTF32)   s x = h + l, two fp16 parts: 22 bits or more for every value down to 2^-18 of the row's largest, an
+//                        error of 2^-40 of the largest below that. Three products (hl lh hh), one accumulator.
+//   FMT_TF32X2 (3xTF32)  x = h + l, two tf32 parts: h is x as the tensor core reads it (its leading 11 bits, truncated), l the
+//                        rest rounded to tf32. Three products of 8 columns of K each, one accumulator: twice FMT_F16X2's
+//                        operand bytes and twice its instructions.
+//   FMT_F16 (tf32)       x's leading 11 bits, truncated: the value a tf32 tensor core reads of x, as one fp16.
+//   FMT_TF32 (tf32)      x as it is, read by a tf32 tensor core: the same operand value as FMT_F16's for twice the bytes.
+//   FMT_BF16 (bf16)      x rounded to bf16.
+enum Format { FMT_F16X3 = 0, FMT_F16X2 = 1, FMT_F16 = 2, FMT_BF16 = 3, FMT_TF32X2 = 4, FMT_TF32 = 5 };
+inline Format format_of(int mode) {
+  return mode == GEMM_TF32X3 ? FMT_F16X2 : mode == GEMM_TF32 ? FMT_F16 : mode == GEMM_BF16 ? FMT_BF16 : FMT_F16X3;
+}
+constexpr bool scales_rows(int fmt) { return fmt == FMT_F16X3 || fmt == FMT_F16X2 || fmt == FMT_F16; }
+
+// A weight [rows, K] in one format, made once when it was loaded. K is padded with zeros to a multiple of 32.
+//   FMT_F16X3   main [rows][Kp/32][h 32 | m 32], low [rows][Kp] the l parts; `amax` the bits of the matrix's largest |x|
+//   FMT_F16X2   main [rows][Kp/32][h 32 | l 32]; `amax`
+//   FMT_F16     main [rows][Kp]; `amax`
+//   FMT_BF16    main [rows][Kp]
+//   FMT_TF32X2  main [rows][Kp] and low [rows][Kp], fp32 words; FMT_TF32 main alone
+struct PackedB {
+  Format fmt = FMT_F16X3;
+  const uint16_t* main = nullptr;
+  const uint16_t* low = nullptr;
+  const uint32_t* amax = nullptr;
+  int Kp = 0;
+};
+inline int packed_k(int K) { return (K + 31) / 32 * 32; }
+// 16-bit values and bytes a packed weight takes (main and low together), rows padded apart to 16 bytes.
+inline size_t packed_halves(int fmt, int rows, int K) {
+  return size_t(rows) * packed_k(K) * (fmt == FMT_F16X3 ? 3 : fmt == FMT_F16X2 || fmt == FMT_TF32 ? 2 : fmt == FMT_TF32X2 ? 4 : 1);
+}
+// Packs W [rows, K] (element (r, k) at W[r * ld_r + k * ld_k]) into `out`; `amax` is one device word, written here.
+PackedB pack_weight(cudaStream_t s, Format fmt, const float* W, size_t ld_r, size_t ld_k, int rows, int K, uint16_t* out, uint32_t* amax);
+
 struct GemmArgs {
   const float* A = nullptr;  // [M,K]
   int lda = 0;
-  const float* B = nullptr;  // [N,K]
+  const float* B = nullptr;  // [N,K] fp32: read by the CUDA-core kernel alone
   int ldb = 0;
-  // Non-zero: B + b_lo_offset holds the low parts of B's 3xTF32 split, computed once when the weights were loaded
-  // (same shape and pitch); the tensor-core kernel then loads them instead of splitting every B tile it stages.
-  size_t b_lo_offset = 0;
-  // B again as bf16 [N,K] with the same pitch in elements (round to nearest even, made when the weights were loaded):
-  // what the bf16 mode's tensor-core kernel reads. Null: the bf16 mode runs this GEMM as tf32.
-  const uint16_t* B16 = nullptr;
+  PackedB nat, fast;         // B in the native format, and in the one this GEMM runs in
+  // The fp16 formats scale each row of A: the bits of the row's largest |value| (0 for a row of zeros),
+  // kept up to date by whatever wrote A. Null: found by a pass over A.
+  const uint32_t* a_max = nullptr;
+  // Unless null, each row's largest |C| is raised into c_max (atomicMax on the bits; the caller zeroed it).
+  uint32_t* c_max = nullptr;
   float* C = nullptr;        // [M, N] (EPI_SWIGLU: [M,N/2]; EPI_SWIGLU_BWD: [M,2N])
   int ldc = 0;
   int M = 0, N = 0, K = 0;
@@ -59,12 +103,14 @@ struct GemmArgs {
   int epi = EPI_PLAIN;
 };
 
-// Runs the GEMM in `mode`. The tensor modes need K % 8 == 0 (tf32) or K % 16 == 0
-// (bf16), N % 8 == 0 and 16-byte aligned rows; anything else takes the native kernel.
-void gemm(Stream& st, Arena& arena, const GemmArgs& a, int mode);
+// Runs the GEMM in the format of `fast`, or of `nat` where it has fewer than 64 rows.
+void gemm(Stream& st, Arena& arena, const GemmArgs& a);
 
 // out[M] = A[M,K] . w[K] + b (a one-column linear layer), one warp per row.
 void gemv_rows(Stream& st, const float* A, int lda, const float* w, const float* bias, float* out, int M, int K);
+
+// mx[r] = bits of the largest |x(r, :)|.
+void row_max(Stream& st, uint32_t* mx, const float* x, int ld, int R, int D);
 
 // Non-zero if a tensor-core kernel launched on this stream gave up on a bounded wait since the
 // last call (synchronizes the stream; clears the flag).

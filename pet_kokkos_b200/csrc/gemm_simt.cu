@@ -1,16 +1,18 @@
-// The fp32 (native) GEMM on the CUDA cores and the GEMM dispatcher: see gemm.h.
+// The fp32 GEMM on the CUDA cores and the GEMM dispatcher: see gemm.h.
 //
 // 128 x 128 x 16 tiles, 256 threads, 8 x 8 outputs per thread, operands staged in
 // shared memory (transposed, so the inner loop reads float4s) with the next tile's
 // global loads issued before the current tile's arithmetic. Each output is one
 // chain of fused multiply-adds over k in increasing order, whatever the tile or
-// the row count: a row's result depends on that row alone.
+// the row count: a row's result depends on that row alone. It serves callers whose
+// weight has no packed form (pet_gemm_host_static): with the weight's parts at hand
+// the tensor cores are four times faster and no less exact.
 #include "epilogue.cuh"
 
 namespace petb {
 
-void gemm_tensor(Stream& st, Arena& arena, const GemmArgs& a, int mode);  // gemm_tc.cu
-bool gemm_tensor_usable(const GemmArgs& a, int mode);
+void gemm_tensor(Stream& st, Arena& arena, const GemmArgs& a, const PackedB& w);  // gemm_tc.cu
+bool gemm_tensor_usable(const GemmArgs& a, const PackedB& w);
 
 namespace {
 
@@ -130,9 +132,9 @@ void launch_native(Stream& st, const GemmArgs& a) {
 
 }  // namespace
 
-void gemm(Stream& st, Arena& arena, const GemmArgs& a, int mode) {
+void gemm(Stream& st, Arena& arena, const GemmArgs& a) {
   if (a.M <= 0 || a.N <= 0) return;
-  if (a.N % 4 || a.K % 4 || a.lda % 4 || a.ldb % 4 || a.ldc % 2)
+  if (a.N % 4 || a.K % 4 || a.lda % 4 || (a.B && a.ldb % 4) || a.ldc % 2)
     throw Error(2, "gemm: widths must be multiples of 4 (N=" + std::to_string(a.N) + ", K=" + std::to_string(a.K) + ")");
   // Algorithmic work: 2MNK flops; A, B, C once each, plus what the epilogue reads and writes.
   double bytes = 4.0 * (double(a.M) * a.K + double(a.N) * a.K + double(a.M) * a.N);
@@ -141,7 +143,10 @@ void gemm(Stream& st, Arena& arena, const GemmArgs& a, int mode) {
   if (a.epi == EPI_SWIGLU) bytes -= 2.0 * a.M * a.N;      // h is half as wide as the product
   if (a.epi == EPI_SWIGLU_BWD) bytes += 4.0 * a.M * a.N;  // pre_adj is twice as wide
   const ProfScope ps(st, PC_GEMM, 2.0 * a.M * a.N * a.K, bytes);
-  if (mode != GEMM_NATIVE && gemm_tensor_usable(a, mode)) return gemm_tensor(st, arena, a, mode);
+  // Fewer than half a tile of rows: the speed modes' products would not be felt there, so they run at full precision.
+  const PackedB& w = a.M < 64 || a.N < 32 ? a.nat : a.fast;
+  if (gemm_tensor_usable(a, w)) return gemm_tensor(st, arena, a, w);
+  if (!a.B) throw Error(3, "gemm: this weight has no fp32 copy for the CUDA cores");
   switch (a.epi) {
     case EPI_PLAIN: return launch_native<EPI_PLAIN>(st, a);
     case EPI_SILU: return launch_native<EPI_SILU>(st, a);

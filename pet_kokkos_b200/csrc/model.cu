@@ -16,7 +16,7 @@ using Taps = std::map<std::string, std::pair<const float*, size_t>>;
 // ---- weights -----------------------------------------------------------------
 //
 // A checkpoint tensor is uploaded once as it is stored (doubles) and every layout the kernels read is made from it
-// on the device: both orientations in fp32, the low parts of their 3xTF32 split, and bf16 copies of both. The
+// on the device: fp32, and both orientations packed in the formats the calculator's GEMM mode reads (gemm.h). The
 // SwiGLU row pairing and the fold of compress.0 are index maps and short fp64 sums over the uploaded tensors, so
 // the host never loops over a weight.
 
@@ -27,26 +27,12 @@ namespace {
 // thread's run of columns (the reference does the same at load, src/model.cpp:211-222).
 __device__ __forceinline__ int stored_row(int a, int rows, int paired) { return paired ? (a & 1) * (rows / 2) + (a >> 1) : a; }
 
-__device__ __forceinline__ uint16_t bf16_bits(float x) {  // round to nearest even; weights are finite
-  const uint32_t u = __float_as_uint(x);
-  return uint16_t((u + 0x7FFFu + ((u >> 16) & 1u)) >> 16);
-}
-// x minus its leading 11 significant bits, with half of the last bit the tensor core keeps added so that its
-// truncation of this part rounds.
-__device__ __forceinline__ float tf32_low_part(float x) {
-  return __uint_as_float(__float_as_uint(x - __uint_as_float(__float_as_uint(x) & 0xFFFFE000u)) + 0x1000u);
-}
-
-// src [rows, ld] doubles (the first `cols` columns of each row) -> [w | wt | w_lo | wt_lo] floats, then bf16 w, wt.
-__global__ void k_weight_layouts(const double* src, int ld, int rows, int cols, int paired, float* out, uint16_t* out16) {
+// src [rows, ld] doubles (the first `cols` columns of each row) -> [rows, cols] floats.
+__global__ void k_weight_rows(const double* src, int ld, int rows, int cols, int paired, float* out) {
   const size_t n = size_t(rows) * cols, i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int a = int(i / cols), b = int(i % cols);
-  const float v = float(src[size_t(stored_row(a, rows, paired)) * ld + b]);
-  const size_t t = size_t(b) * rows + a;
-  out[i] = v, out[n + t] = v;
-  out[2 * n + i] = out[3 * n + t] = tf32_low_part(v);
-  out16[i] = out16[n + t] = bf16_bits(v);
+  out[i] = float(src[size_t(stored_row(a, rows, paired)) * ld + b]);
 }
 __global__ void k_weight_vector(const double* src, int len, int paired, float* out) {
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
@@ -97,7 +83,7 @@ struct Staged {
 };
 
 // What the network reads from a checkpoint, as (tensor name, how it is prepared).
-enum class Prep { Matrix, Vector, PairedMatrix, PairedVector, CompressFold };
+enum class Prep { Table, Matrix, Vector, PairedMatrix, PairedVector, CompressFold };  // Table: read row by row, never a GEMM operand
 struct PlanItem {
   std::string name;
   Prep prep;
@@ -115,7 +101,7 @@ std::vector<PlanItem> weight_plan(const Hypers& h) {
     plan.push_back({stem + ".weight", Prep::Vector});
     if (h.layernorm) plan.push_back({stem + ".bias", Prep::Vector});
   };
-  plan.push_back({"edge_embedder.weight", Prep::Matrix});
+  plan.push_back({"edge_embedder.weight", Prep::Table});
   for (int L = 0; L < h.num_gnn_layers; ++L) {
     const std::string layer = "gnn_layers." + std::to_string(L);
     plan.push_back({layer + ".compress.0", Prep::CompressFold, L});
@@ -138,10 +124,11 @@ std::vector<PlanItem> weight_plan(const Hypers& h) {
   }
   for (int i = 0; i < h.num_readout_layers; ++i) {
     const std::string r = std::to_string(i);
-    plan.push_back({"node_embedders." + r + ".weight", Prep::Matrix});
+    plan.push_back({"node_embedders." + r + ".weight", Prep::Table});
     for (const char* side : {"node", "edge"}) {
       dense(std::string(side) + "_heads.energy." + r + ".0"), dense(std::string(side) + "_heads.energy." + r + ".2");
-      dense(std::string(side) + "_last_layers.energy." + r + ".energy___0");
+      const std::string last = std::string(side) + "_last_layers.energy." + r + ".energy___0";
+      plan.push_back({last + ".weight", Prep::Table}), plan.push_back({last + ".bias", Prep::Vector});
     }
   }
   return plan;
@@ -149,16 +136,37 @@ std::vector<PlanItem> weight_plan(const Hypers& h) {
 
 }  // namespace
 
-void Model::put_mat(const std::string& name, const double* src, int ld, int rows, int cols, bool paired) {
+void Model::put_mat(const std::string& name, const double* src, int ld, int rows, int cols, bool paired, bool operand) {
   const size_t n = size_t(rows) * cols;
   float* dev = nullptr;
-  PETB_CUDA(cudaMalloc(&dev, (4 * n + n + 8) * sizeof(float)));  // four fp32 layouts, then two bf16 ones (2n halves)
+  PETB_CUDA(cudaMalloc(&dev, (n + 4) * sizeof(float)));
   owned_.push_back(dev);
-  uint16_t* dev16 = reinterpret_cast<uint16_t*>(dev + 4 * n);
-  if (n) k_weight_layouts<<<cdiv((long long) n, 256), 256>>>(src, ld, rows, cols, paired ? 1 : 0, dev, dev16);
+  if (n) k_weight_rows<<<cdiv((long long) n, 256), 256>>>(src, ld, rows, cols, paired ? 1 : 0, dev);
   PETB_CUDA(cudaGetLastError());
   Mat m;
-  m.w = dev, m.wt = dev + n, m.rows = rows, m.cols = cols, m.lo_off = 2 * n, m.w16 = dev16, m.wt16 = dev16 + n;
+  m.w = dev, m.rows = rows, m.cols = cols;
+  if (operand) {  // both orientations in the native format (every mode runs its smallest GEMMs in it) and in the mode's own
+    auto pack = [&](Format f, bool transposed) {
+      const int r = transposed ? cols : rows, k = transposed ? rows : cols;
+      uint16_t* out = nullptr;
+      const size_t bytes = (packed_halves(f, r, k) * 2 + 15) & ~size_t(15);
+      PETB_CUDA(cudaMalloc(&out, bytes + 16));
+      owned_.push_back(out);
+      return pack_weight(nullptr, f, dev, transposed ? 1 : cols, transposed ? cols : 1, r, k, out,
+                         reinterpret_cast<uint32_t*>(reinterpret_cast<char*>(out) + bytes));
+    };
+    // At widths past 256 the forward of the 3xTF32 and tf32 modes keeps the tf32 instructions. The accumulator's
+    // truncations pull every product sum toward zero by a factor that goes with their number, one per 8 columns of K and
+    // product there, one per 16 in fp16; and where activations are truncated to 11 bits, the last bit of a sum decides some
+    // of them. Up to 256 columns energies agree between the two to 1e-6 (3xTF32) and 2e-4 (tf32); at 512, where a network
+    // energy of 2.6 eV per atom stood against -2.6 of composition energy, to 2e-4 and 2e-3 of their sum: there the modes'
+    // energies stay what they were. Forces feel neither, so the backward runs in fp16 parts at every width.
+    const Format fmt = format_of(mode_), wide_forward = fmt == FMT_F16X2 ? FMT_TF32X2 : fmt == FMT_F16 ? FMT_TF32 : fmt;
+    const Format forward = h_.d_pet > 256 ? wide_forward : fmt;
+    m.nat = pack(FMT_F16X3, false), m.nat_t = pack(FMT_F16X3, true);
+    m.fast = forward == FMT_F16X3 ? m.nat : pack(forward, false);
+    m.fast_t = fmt == FMT_F16X3 ? m.nat_t : pack(fmt, true);
+  }
   mat_[name] = m;
 }
 
@@ -197,14 +205,14 @@ void Model::fold_compress(const Checkpoint& ck, const std::string& c0, int L) {
   k_fold_geometry<<<cdiv(D, 128), 128>>>(W.p, K, We.p, be.p, b0.p, D, wx.p, b.p);
   k_fold_species<<<cdiv((long long) ns * D, 128), 128>>>(W.p, K, T.p, ns, D, tab.p);
   PETB_CUDA(cudaGetLastError());
-  put_mat(c0 + "@x4", wx.p, 4, D, 4, false);
+  put_mat(c0 + "@x4", wx.p, 4, D, 4, false, false);
   put_vec(c0 + "@b", b.p, D, false);
-  put_mat(c0 + "@tab", tab.p, D, ns, D, false);
-  if (L > 0) put_mat(c0 + "@in", W.p + 2 * D, K, D, D, false);
+  put_mat(c0 + "@tab", tab.p, D, ns, D, false, false);
+  if (L > 0) put_mat(c0 + "@in", W.p + 2 * D, K, D, D, false, true);
   PETB_CUDA(cudaDeviceSynchronize());  // the staged tensors are freed on return
 }
 
-Model::Model(const Checkpoint& ck) : h_(ck.hypers), scale_(ck.energy_scale) {
+Model::Model(const Checkpoint& ck, int gemm_mode) : h_(ck.hypers), scale_(ck.energy_scale), mode_(gemm_mode) {
   const bool ff = h_.feedforward, ln = h_.layernorm, expanded = h_.expanded_node(), swiglu = h_.swiglu;
 
   // The two families the reference implements (src/model.cpp:314-334); anything else is refused by name.
@@ -223,11 +231,11 @@ Model::Model(const Checkpoint& ck) : h_(ck.hypers), scale_(ck.energy_scale) {
       continue;
     }
     const Tensor& t = ck.at(it.name);
-    const bool matrix = it.prep == Prep::Matrix || it.prep == Prep::PairedMatrix;
+    const bool matrix = it.prep == Prep::Table || it.prep == Prep::Matrix || it.prep == Prep::PairedMatrix;
     const bool paired = it.prep == Prep::PairedMatrix || it.prep == Prep::PairedVector;
     if (matrix && t.shape.size() != 2) throw Error(1, "model: expected a 2-D tensor '" + it.name + "'");
     const Staged dev(t);
-    if (matrix) put_mat(it.name, dev.p, dev.cols, dev.rows, dev.cols, paired);
+    if (matrix) put_mat(it.name, dev.p, dev.cols, dev.rows, dev.cols, paired, it.prep != Prep::Table);
     else put_vec(it.name, dev.p, int(t.numel()), paired);
     PETB_CUDA(cudaDeviceSynchronize());
   }
@@ -270,54 +278,93 @@ int attention_mode_for(int gemm_mode) {
   return gemm_mode == GEMM_NATIVE ? ATTN_NATIVE : gemm_mode == GEMM_TF32X3 ? ATTN_TF32X3 : ATTN_TF32;
 }
 
+// Rows of an activation or adjoint, with the bits of each row's largest magnitude where the mode's operand format wants
+// them (gemm.h); whatever writes the rows keeps them.
+struct Rows {
+  float* p = nullptr;
+  uint32_t* mx = nullptr;
+  Rows from(size_t row, int ld) const { return {p + row * ld, mx ? mx + row : nullptr}; }
+};
+
+// The arrays of row maxima of one pass: one zeroed block from `save`, a fresh part of it for every tensor written (a GEMM
+// raises its rows' maxima atomically, so they start from zero). Modes that need none get null pointers; so does whatever
+// the block has no room left for (an edge MLP in very small chunks), whose GEMM then looks for the maxima itself.
+class RowMaxima {
+ public:
+  RowMaxima(Stream& st, Arena& save, size_t words) : size_(words) {
+    if (!words) return;
+    base_ = save.alloc<uint32_t>(words);
+    PETB_CUDA(cudaMemsetAsync(base_, 0, words * sizeof(uint32_t), st.s));
+  }
+  uint32_t* take(size_t rows) {
+    rows = (rows + 31) & ~size_t(31);
+    if (used_ + rows > size_) return nullptr;
+    uint32_t* p = base_ + used_;
+    used_ += rows;
+    return p;
+  }
+  Rows fresh(float* p, size_t rows) { return {p, take(rows)}; }
+
+ private:
+  uint32_t* base_ = nullptr;
+  size_t size_ = 0, used_ = 0;
+};
+
 struct Gemms {
   Stream& st;
   Arena& tmp;
-  int mode;
 
-  // out[M, W.rows] = in[M, W.cols] . W^T + bias (+ res for rows >= res_row0)
-  void linear(float* out, const float* in, const Mat& W, const float* bias, int M, const float* res = nullptr,
-              int res_row0 = 0) const {
+  static GemmArgs args(const Rows& out, const Rows& in, const Mat& W, bool transposed, int M) {
     GemmArgs a;
-    a.A = in, a.lda = W.cols, a.B = W.w, a.ldb = W.cols, a.b_lo_offset = W.lo_off, a.B16 = W.w16, a.C = out, a.ldc = W.rows;
-    a.M = M, a.N = W.rows, a.K = W.cols, a.bias = bias, a.res = res, a.ldr = W.rows, a.res_row0 = res_row0;
-    gemm(st, tmp, a, mode);
+    a.A = in.p, a.a_max = in.mx, a.C = out.p, a.c_max = out.mx, a.M = M;
+    a.N = transposed ? W.cols : W.rows, a.K = transposed ? W.rows : W.cols;
+    a.lda = a.K, a.ldc = a.ldr = a.ldp = a.N;
+    a.nat = transposed ? W.nat_t : W.nat, a.fast = transposed ? W.fast_t : W.fast;
+    return a;
+  }
+  // out[M, W.rows] = in[M, W.cols] . W^T + bias (+ res for rows >= res_row0)
+  void linear(const Rows& out, const Rows& in, const Mat& W, const float* bias, int M, const float* res = nullptr,
+              int res_row0 = 0) const {
+    GemmArgs a = args(out, in, W, false, M);
+    a.bias = bias, a.res = res, a.res_row0 = res_row0;
+    gemm(st, tmp, a);
   }
   // out = silu(pre), pre = in . W^T + bias, kept when `pre` is given
-  void linear_silu(float* out, float* pre, const float* in, const Mat& W, const float* bias, int M) const {
-    GemmArgs a;
-    a.A = in, a.lda = W.cols, a.B = W.w, a.ldb = W.cols, a.b_lo_offset = W.lo_off, a.B16 = W.w16, a.C = out, a.ldc = W.rows;
-    a.M = M, a.N = W.rows, a.K = W.cols, a.bias = bias, a.pre = pre, a.ldp = W.rows, a.epi = EPI_SILU;
-    gemm(st, tmp, a, mode);
+  void linear_silu(const Rows& out, float* pre, const Rows& in, const Mat& W, const float* bias, int M) const {
+    GemmArgs a = args(out, in, W, false, M);
+    a.bias = bias, a.pre = pre, a.epi = EPI_SILU;
+    gemm(st, tmp, a);
   }
   // pre[M, 2F] = in . W^T + bias (interleaved v, g); h[M, F] = v * sigmoid(g)
-  void swiglu_in(float* h, float* pre, const float* in, const Mat& W, const float* bias, int M) const {
-    GemmArgs a;
-    a.A = in, a.lda = W.cols, a.B = W.w, a.ldb = W.cols, a.b_lo_offset = W.lo_off, a.B16 = W.w16, a.C = h, a.ldc = W.rows / 2;
-    a.M = M, a.N = W.rows, a.K = W.cols, a.bias = bias, a.pre = pre, a.ldp = W.rows, a.epi = EPI_SWIGLU;
-    gemm(st, tmp, a, mode);
+  void swiglu_in(const Rows& h, float* pre, const Rows& in, const Mat& W, const float* bias, int M) const {
+    GemmArgs a = args(h, in, W, false, M);
+    a.ldc = W.rows / 2, a.bias = bias, a.pre = pre, a.epi = EPI_SWIGLU;
+    gemm(st, tmp, a);
   }
   // in_adj[M, W.cols] (+)= out_adj[M, W.rows] . W
-  void linear_bwd(float* in_adj, const float* out_adj, const Mat& W, int M, bool acc) const {
-    GemmArgs a;
-    a.A = out_adj, a.lda = W.rows, a.B = W.wt, a.ldb = W.rows, a.b_lo_offset = W.lo_off, a.B16 = W.wt16, a.C = in_adj, a.ldc = W.cols;
-    a.M = M, a.N = W.cols, a.K = W.rows, a.res = acc ? in_adj : nullptr, a.ldr = W.cols;
-    gemm(st, tmp, a, mode);
+  void linear_bwd(const Rows& in_adj, const Rows& out_adj, const Mat& W, int M, bool acc) const {
+    GemmArgs a = args(in_adj, out_adj, W, true, M);
+    a.res = acc ? in_adj.p : nullptr;
+    gemm(st, tmp, a);
   }
   // grad[M, W.cols] = (out_adj . W) * silu'(pre)
-  void linear_silu_bwd(float* grad, const float* out_adj, const Mat& W, const float* pre, int M) const {
-    GemmArgs a;
-    a.A = out_adj, a.lda = W.rows, a.B = W.wt, a.ldb = W.rows, a.b_lo_offset = W.lo_off, a.B16 = W.wt16, a.C = grad, a.ldc = W.cols;
-    a.M = M, a.N = W.cols, a.K = W.rows, a.pre = const_cast<float*>(pre), a.ldp = W.cols, a.epi = EPI_SILU_BWD;
-    gemm(st, tmp, a, mode);
+  void linear_silu_bwd(const Rows& grad, const Rows& out_adj, const Mat& W, const float* pre, int M) const {
+    GemmArgs a = args(grad, out_adj, W, true, M);
+    a.pre = const_cast<float*>(pre), a.epi = EPI_SILU_BWD;
+    gemm(st, tmp, a);
   }
   // pre_adj[M, 2F] from h_adj = out_adj . W_out and the saved pre
-  void swiglu_out_bwd(float* pre_adj, const float* out_adj, const Mat& w_out, const float* pre, int M) const {
-    GemmArgs a;
-    a.A = out_adj, a.lda = w_out.rows, a.B = w_out.wt, a.ldb = w_out.rows, a.b_lo_offset = w_out.lo_off, a.B16 = w_out.wt16, a.C = pre_adj, a.ldc = 2 * w_out.cols;
-    a.M = M, a.N = w_out.cols, a.K = w_out.rows, a.pre = const_cast<float*>(pre), a.ldp = 2 * w_out.cols;
-    a.epi = EPI_SWIGLU_BWD;
-    gemm(st, tmp, a, mode);
+  void swiglu_out_bwd(const Rows& pre_adj, const Rows& out_adj, const Mat& w_out, const float* pre, int M) const {
+    GemmArgs a = args(pre_adj, out_adj, w_out, true, M);
+    a.ldc = a.ldp = 2 * w_out.cols, a.pre = const_cast<float*>(pre), a.epi = EPI_SWIGLU_BWD;
+    gemm(st, tmp, a);
+  }
+  // act = silu(pre), pre = in . W_in^T + b + tab[species] + wx . (v, |v|): compress.0 past the first layer
+  void compress(const Rows& act, float* pre, const Rows& in, const Mat& W, const float* b, const Mat& tab, const Mat& x4,
+                const PackedEdges& pk) const {
+    GemmArgs a = args(act, in, W, false, pk.E);
+    a.bias = b, a.pre = pre, a.tab = tab.w, a.sp = pk.species, a.wx = x4.w, a.vec = pk.vec, a.dist = pk.dist, a.epi = EPI_COMPRESS;
+    gemm(st, tmp, a);
   }
 };
 
@@ -406,6 +453,7 @@ MemoryNeed Model::memory_need(int tier, int N, int E, int n_live) const {
   save += (relayer ? 1.0 : G) * layer;
   save += 2 * n * Dh + 2 * e * Dh + 2 * n + e + 2 * n;              // readout
   save += 5 * e + n * Dn + e * D + T * D + 6 * e + 30 * n;          // adjoints, edge gradients (doubles), forces, virials
+  save += double(row_maxima_words(N, E)) * (relayer ? 2 : 1);       // (a layer run again takes its own)
   // tmp: the fullest scope
   const double attention_bwd = T * (5 * D + H) + (keep ? 0.0 : T * 4 * D);
   const double attention_fwd = T * D + (keep ? 0.0 : T * 3 * D);
@@ -417,6 +465,13 @@ MemoryNeed Model::memory_need(int tier, int N, int E, int n_live) const {
   need.save = size_t(save * 4.0 * 1.03) + (size_t(8) << 20);
   need.tmp = size_t(tmp * 4.0 * 1.03) + (size_t(8) << 20);
   return need;
+}
+
+// Rows whose maxima a pass keeps (class RowMaxima): what each layer, block and readout writes for a GEMM to read.
+size_t Model::row_maxima_words(int N, int E) const {
+  if (!scales_rows(format_of(mode_))) return 0;
+  const size_t G = h_.num_gnn_layers, A = h_.num_attention_layers, T = size_t(N) + E + 64, n = size_t(N) + 64;
+  return G * ((11 * A + 8) * T + 6 * A * n) + 4 * T + 6 * n;
 }
 
 size_t Model::memory_estimate(int tier, int N, int E) const {
@@ -436,7 +491,7 @@ PassOut Model::run_feedforward(Stream& st, Arena& save, Arena& tmp, const Packed
   const int N = pk.N, E = pk.E, T = N + E, S = pk.M + 1;
   const int D = h_.d_pet, Dn = h_.d_node, Dh = h_.d_head, H = h_.num_heads, hd = h_.head_dim;
   const int G = h_.num_gnn_layers, A = h_.num_attention_layers;
-  const Gemms gm{st, tmp, mode};
+  const Gemms gm{st, tmp};
   const float sc = float(1.0 / (std::sqrt(double(hd)) * h_.attention_temperature));
   const size_t Ea = E > 0 ? E : 1, Ta = T > 0 ? T : 1, Na = N > 0 ? N : 1;
 
@@ -445,9 +500,11 @@ PassOut Model::run_feedforward(Stream& st, Arena& save, Arena& tmp, const Packed
   last_tier_ = tier, last_estimate_ = memory_estimate(tier, N, E);
   const bool keep_wide = tier == RECOMPUTE_NEVER, relayer = grad && tier == RECOMPUTE_LAYERS;
   const int chunk = keep_wide ? 0 : edge_chunk_rows(E);
+  RowMaxima maxima(st, save, row_maxima_words(N, E) * (relayer ? 2 : 1));  // a layer run again takes its own
 
   struct Block {
-    float *tok, *qkv, *merged, *ml, *eps, *node_res, *pre_c, *pre_e;
+    float *tok, *qkv, *ml, *node_res, *pre_c, *pre_e;
+    Rows merged, eps;
   };
   struct Layer {
     float *cpre, *cph_pre, *out_edge;
@@ -458,27 +515,27 @@ PassOut Model::run_feedforward(Stream& st, Arena& save, Arena& tmp, const Packed
     at.N = N, at.H = H, at.hd = hd, at.S = S, at.sc = sc, at.off = pk.off, at.cut = pk.cut;
     at.mode = attention_mode_for(mode);
     at.pairs = pk.pairs, at.T = T;
-    at.qkv = qkv, at.merged = b.merged, at.ml = b.ml;
+    at.qkv = qkv, at.merged = b.merged.p, at.ml = b.ml;
     return at;
   };
   // qkv = W_in . norm(tokens) + b
   auto make_qkv = [&](float* qkv, const std::string& tl, float* tok) {
     Scope s(tmp);
-    float* attn_in = tmp.alloc<float>(Ta * D);
-    norm_fwd(st, attn_in, tok, nullptr, vec(tl + ".norm_attention.weight"), nullptr, T, D);
-    gm.linear(qkv, attn_in, mat(tl + ".attention.input_linear.weight"), vec(tl + ".attention.input_linear.bias"), T);
+    const Rows attn_in = maxima.fresh(tmp.alloc<float>(Ta * D), Ta);
+    norm_fwd(st, attn_in.p, tok, nullptr, vec(tl + ".norm_attention.weight"), nullptr, T, D, attn_in.mx);
+    gm.linear({qkv}, attn_in, mat(tl + ".attention.input_linear.weight"), vec(tl + ".attention.input_linear.bias"), T);
   };
   // The edge MLP's first half on rows [r0, r0 + nr): pre = W_in . norm(eps) + b and, with `he`, v * sigmoid(g).
-  auto edge_mlp_in = [&](float* he, float* pre, const float* eps_rows, const std::string& tl, int nr) {
-    float* edge_norm = tmp.alloc<float>(size_t(nr) * D);
-    norm_fwd(st, edge_norm, const_cast<float*>(eps_rows), nullptr, vec(tl + ".norm_mlp.weight"), nullptr, nr, D);
+  auto edge_mlp_in = [&](const Rows& he, float* pre, const float* eps_rows, const std::string& tl, int nr) {
+    const Rows edge_norm = maxima.fresh(tmp.alloc<float>(size_t(nr) * D), nr);
+    norm_fwd(st, edge_norm.p, const_cast<float*>(eps_rows), nullptr, vec(tl + ".norm_mlp.weight"), nullptr, nr, D, edge_norm.mx);
     gm.swiglu_in(he, pre, edge_norm, mat(tl + ".mlp.w_in.weight"), vec(tl + ".mlp.w_in.bias"), nr);
   };
 
   // One message-passing layer forward: node_in [N,Dn] -> node_out, input_edge [E,D] updated in place, saves in `sl`
   // (from `save`; the wide ones only with keep). `remote_in` [n_live, D] holds the partner rows of an exchanged list:
   // asked for from the other ranks when `ask`, else the rows a first run of this layer received.
-  auto layer_forward = [&](int L, const float* node_in, float* node_out, float* input_edge, Layer& sl, bool keep,
+  auto layer_forward = [&](int L, const Rows& node_in, Rows& node_out, Rows& input_edge, Layer& sl, bool keep,
                            float* remote_in, bool ask) {
     const std::string g = "gnn_layers." + std::to_string(L), ls = std::to_string(L), c0 = g + ".compress.0";
     sl.blk.resize(A);
@@ -489,56 +546,53 @@ PassOut Model::run_feedforward(Stream& st, Arena& save, Arena& tmp, const Packed
     sl.cpre = save.alloc<float>(Ea * D);
     {
       Scope s0(tmp);
-      float* cact = tmp.alloc<float>(Ea * D);
+      const Rows cact = maxima.fresh(tmp.alloc<float>(Ea * D), Ea);
       if (L == 0) {
-        compress0(st, cact, sl.cpre, vec(c0 + "@b"), mat(c0 + "@tab").w, mat(c0 + "@x4").w, pk, D);
+        compress0(st, cact.p, sl.cpre, vec(c0 + "@b"), mat(c0 + "@tab").w, mat(c0 + "@x4").w, pk, D, cact.mx);
       } else {
-        const Mat& wi = mat(c0 + "@in");
-        GemmArgs a;
-        a.A = input_edge, a.lda = D, a.B = wi.w, a.ldb = D, a.b_lo_offset = wi.lo_off, a.B16 = wi.w16, a.C = cact, a.ldc = D;
-        a.M = E, a.N = D, a.K = D;
-        a.bias = vec(c0 + "@b"), a.pre = sl.cpre, a.ldp = D, a.tab = mat(c0 + "@tab").w, a.sp = pk.species;
-        a.wx = mat(c0 + "@x4").w, a.vec = pk.vec, a.dist = pk.dist, a.epi = EPI_COMPRESS;
-        gemm(st, tmp, a, mode);
+        gm.compress(cact, sl.cpre, input_edge, mat(c0 + "@in"), vec(c0 + "@b"), mat(c0 + "@tab"), mat(c0 + "@x4"), pk);
       }
-      gm.linear(tokbuf[0] + size_t(N) * D, cact, mat(g + ".compress.2.weight"), vec(g + ".compress.2.bias"), E);
+      gm.linear({tokbuf[0] + size_t(N) * D}, cact, mat(g + ".compress.2.weight"), vec(g + ".compress.2.bias"), E);
     }
     tap(taps, "et" + ls, tokbuf[0] + size_t(N) * D, size_t(E) * D);
 
-    const float* node_cur = node_in;
+    Rows node_cur = node_in;
     for (int a = 0; a < A; ++a) {
       const std::string tl = g + ".trans.layers." + std::to_string(a), tag = ls + "_" + std::to_string(a);
       Block& b = sl.blk[a];
       const Mat &w_cin = mat(tl + ".center_mlp.w_in.weight"), &w_ein = mat(tl + ".mlp.w_in.weight");
       b.tok = tokbuf[a];
-      b.merged = save.alloc<float>(Ta * D);
+      b.merged = maxima.fresh(save.alloc<float>(Ta * D), Ta);
       b.ml = save.alloc<float>(Ta * H * 2);
-      b.eps = save.alloc<float>(Ta * D);  // rows < N: the attention output's atom rows; rows >= N: eps
+      b.eps = maxima.fresh(save.alloc<float>(Ta * D), Ta);  // rows < N: the attention output's atom rows; rows >= N: eps
       b.node_res = save.alloc<float>(Na * Dn);
       b.pre_c = save.alloc<float>(Na * w_cin.rows);
       b.qkv = keep ? save.alloc<float>(Ta * 3 * D) : nullptr;
       b.pre_e = keep ? save.alloc<float>(Ea * w_ein.rows) : nullptr;
-      float* node_next = a + 1 == A ? node_out : save.alloc<float>(Na * Dn);
+      const Rows node_next = maxima.fresh(a + 1 == A ? node_out.p : save.alloc<float>(Na * Dn), Na);
+      if (a + 1 == A) node_out = node_next;
       float* edge_next = tokbuf[a + 1] + size_t(N) * D;
 
-      gm.linear(b.tok, node_cur, mat(tl + ".center_contraction.weight"), vec(tl + ".center_contraction.bias"), N);
+      gm.linear({b.tok}, node_cur, mat(tl + ".center_contraction.weight"), vec(tl + ".center_contraction.bias"), N);
       {
         Scope s1(tmp);
         float* qkv = keep ? b.qkv : tmp.alloc<float>(Ta * 3 * D);
         make_qkv(qkv, tl, b.tok);
-        attention_forward(st, attention_args(b, qkv));
+        AttnArgs at = attention_args(b, qkv);
+        at.merged_max = b.merged.mx;
+        attention_forward(st, at);
       }
-      tap(taps, "merged" + tag, b.merged, size_t(T) * D);
+      tap(taps, "merged" + tag, b.merged.p, size_t(T) * D);
       // attn_out = merged W_out^T + b; its edge rows take the residual: eps = attn_out + edge_cur.
       gm.linear(b.eps, b.merged, mat(tl + ".attention.output_linear.weight"), vec(tl + ".attention.output_linear.bias"), T,
                 b.tok, N);
       // node_res = node_cur + expansion(atom rows of attn_out)
-      gm.linear(b.node_res, b.eps, mat(tl + ".center_expansion.weight"), vec(tl + ".center_expansion.bias"), N, node_cur, 0);
+      gm.linear({b.node_res}, b.eps, mat(tl + ".center_expansion.weight"), vec(tl + ".center_expansion.bias"), N, node_cur.p, 0);
       {
         Scope s2(tmp);
-        float* node_norm = tmp.alloc<float>(Na * Dn);
-        float* hc = tmp.alloc<float>(Na * (w_cin.rows / 2));
-        norm_fwd(st, node_norm, b.node_res, nullptr, vec(tl + ".norm_center_features.weight"), nullptr, N, Dn);
+        const Rows node_norm = maxima.fresh(tmp.alloc<float>(Na * Dn), Na);
+        const Rows hc = maxima.fresh(tmp.alloc<float>(Na * (w_cin.rows / 2)), Na);
+        norm_fwd(st, node_norm.p, b.node_res, nullptr, vec(tl + ".norm_center_features.weight"), nullptr, N, Dn, node_norm.mx);
         gm.swiglu_in(hc, b.pre_c, node_norm, w_cin, vec(tl + ".center_mlp.w_in.bias"), N);
         gm.linear(node_next, hc, mat(tl + ".center_mlp.w_out.weight"), vec(tl + ".center_mlp.w_out.bias"), N, b.node_res, 0);
       }
@@ -546,22 +600,21 @@ PassOut Model::run_feedforward(Stream& st, Arena& save, Arena& tmp, const Packed
       for (int r0 = 0; r0 < E; r0 += rows) {
         const int nr = std::min(rows, E - r0);
         Scope s3(tmp);
-        float* eps_rows = b.eps + (size_t(N) + r0) * D;
-        float* he = tmp.alloc<float>(size_t(nr) * (w_ein.rows / 2));
+        float* eps_rows = b.eps.p + (size_t(N) + r0) * D;
+        const Rows he = maxima.fresh(tmp.alloc<float>(size_t(nr) * (w_ein.rows / 2)), nr);
         float* pre = keep ? b.pre_e + size_t(r0) * w_ein.rows : tmp.alloc<float>(size_t(nr) * w_ein.rows);
         edge_mlp_in(he, pre, eps_rows, tl, nr);
-        gm.linear(edge_next + size_t(r0) * D, he, mat(tl + ".mlp.w_out.weight"), vec(tl + ".mlp.w_out.bias"), nr, eps_rows, 0);
+        gm.linear({edge_next + size_t(r0) * D}, he, mat(tl + ".mlp.w_out.weight"), vec(tl + ".mlp.w_out.bias"), nr, eps_rows, 0);
       }
       node_cur = node_next;
-      tap(taps, "node" + tag, node_cur, size_t(N) * Dn);
+      tap(taps, "node" + tag, node_cur.p, size_t(N) * Dn);
       tap(taps, "edge" + tag, edge_next, size_t(E) * D);
     }
     sl.out_edge = tokbuf[A] + size_t(N) * D;
     sl.cph_pre = save.alloc<float>(Ea * 2 * D);
     {
       Scope s4(tmp);
-      float* comb = tmp.alloc<float>(Ea * 2 * D);
-      float* cph = tmp.alloc<float>(Ea * 2 * D);
+      const Rows comb = maxima.fresh(tmp.alloc<float>(Ea * 2 * D), Ea), cph = maxima.fresh(tmp.alloc<float>(Ea * 2 * D), Ea);
       RemoteRows remote;
       if (pk.exchange) {  // edges to ghosts read their partners' rows from the ghosts' ranks (src/feedforward.cpp:171-179)
         if (ask) {
@@ -571,36 +624,40 @@ PassOut Model::run_feedforward(Stream& st, Arena& save, Arena& tmp, const Packed
         }
         remote = RemoteRows{pk.remote_of, remote_in};
       }
-      concat_norm_fwd(st, comb, sl.out_edge, pk.reverse, input_edge, vec("combination_norms." + ls + ".weight"),
-                      vec("combination_norms." + ls + ".bias"), E, D, remote);
+      concat_norm_fwd(st, comb.p, sl.out_edge, pk.reverse, input_edge.p, vec("combination_norms." + ls + ".weight"),
+                      vec("combination_norms." + ls + ".bias"), E, D, remote, comb.mx);
       gm.linear_silu(cph, sl.cph_pre, comb, mat("combination_mlps." + ls + ".0.weight"), vec("combination_mlps." + ls + ".0.bias"), E);
+      input_edge.mx = maxima.take(Ea);
       gm.linear(input_edge, cph, mat("combination_mlps." + ls + ".2.weight"), vec("combination_mlps." + ls + ".2.bias"), E,
-                input_edge, 0);
+                input_edge.p, 0);
     }
-    tap(taps, "input_edge" + ls, input_edge, size_t(E) * D);
+    tap(taps, "input_edge" + ls, input_edge.p, size_t(E) * D);
   };
 
   // ---- forward ----
   std::vector<Layer> sav(G);
-  std::vector<float*> node_at(G + 1), ie_at(G, nullptr), remote_in(G, nullptr);
-  for (int L = 0; L <= G; ++L) node_at[L] = save.alloc<float>(Na * Dn);  // the nodes entering layer L; [G]: the readout's
-  float* input_edge = save.alloc<float>(Ea * D);
+  std::vector<Rows> node_at(G + 1), ie_at(G);
+  std::vector<float*> remote_in(G, nullptr);
+  for (int L = 0; L <= G; ++L) node_at[L] = {save.alloc<float>(Na * Dn)};  // the nodes entering layer L; [G]: the readout's
+  Rows input_edge = {save.alloc<float>(Ea * D)};  // layer 0 does not multiply it: its rows' maxima come with layer 0's output
   if (pk.exchange)
     for (int L = 0; L < G; ++L) remote_in[L] = save.alloc<float>(size_t(pk.n_live > 0 ? pk.n_live : 1) * D);
   if (relayer)
-    for (int L = 0; L < G; ++L) ie_at[L] = save.alloc<float>(Ea * D);  // input_edge as it entered layer L
-  gather_rows(st, node_at[0], mat("node_embedders.0.weight").w, pk.atom_species, N, Dn);
-  gather_rows(st, input_edge, mat("edge_embedder.weight").w, pk.species, E, D);
+    for (int L = 0; L < G; ++L) ie_at[L] = {save.alloc<float>(Ea * D)};  // input_edge as it entered layer L
+  node_at[0].mx = maxima.take(Na);
+  gather_rows(st, node_at[0].p, mat("node_embedders.0.weight").w, pk.atom_species, N, Dn, node_at[0].mx);
+  gather_rows(st, input_edge.p, mat("edge_embedder.weight").w, pk.species, E, D);
   for (int L = 0; L < G; ++L) {
     if (relayer) {
-      PETB_CUDA(cudaMemcpyAsync(ie_at[L], input_edge, sizeof(float) * size_t(E) * D, cudaMemcpyDeviceToDevice, st.s));
+      ie_at[L].mx = input_edge.mx;
+      PETB_CUDA(cudaMemcpyAsync(ie_at[L].p, input_edge.p, sizeof(float) * size_t(E) * D, cudaMemcpyDeviceToDevice, st.s));
       Scope layer_saves(save);  // nothing of the layer is kept: the backward runs it again
       layer_forward(L, node_at[L], node_at[L + 1], input_edge, sav[L], false, remote_in[L], true);
     } else {
       layer_forward(L, node_at[L], node_at[L + 1], input_edge, sav[L], grad && keep_wide, remote_in[L], true);
     }
   }
-  float* node = node_at[G];
+  const Rows node = node_at[G];
 
   // ---- readout (src/model.cpp:656-691) ----
   float* nh0_pre = save.alloc<float>(Na * Dh);
@@ -613,16 +670,15 @@ PassOut Model::run_feedforward(Stream& st, Arena& save, Arena& tmp, const Packed
   double* per_atom = save.alloc<double>(pk.n_atoms > 0 ? pk.n_atoms : 1);
   {
     Scope s5(tmp);
-    float* nh0 = tmp.alloc<float>(Na * Dh);
+    const Rows nh0 = maxima.fresh(tmp.alloc<float>(Na * Dh), Na), eh0 = maxima.fresh(tmp.alloc<float>(Ea * Dh), Ea);
     float* nh1 = tmp.alloc<float>(Na * Dh);
-    float* eh0 = tmp.alloc<float>(Ea * Dh);
     float* eh1 = tmp.alloc<float>(Ea * Dh);
     gm.linear_silu(nh0, nh0_pre, node, mat("node_heads.energy.0.0.weight"), vec("node_heads.energy.0.0.bias"), N);
-    gm.linear_silu(nh1, nh1_pre, nh0, mat("node_heads.energy.0.2.weight"), vec("node_heads.energy.0.2.bias"), N);
+    gm.linear_silu({nh1}, nh1_pre, nh0, mat("node_heads.energy.0.2.weight"), vec("node_heads.energy.0.2.bias"), N);
     gemv_rows(st, nh1, Dh, mat("node_last_layers.energy.0.energy___0.weight").w, vec("node_last_layers.energy.0.energy___0.bias"),
               node_pred, N, Dh);
     gm.linear_silu(eh0, eh0_pre, input_edge, mat("edge_heads.energy.0.0.weight"), vec("edge_heads.energy.0.0.bias"), E);
-    gm.linear_silu(eh1, eh1_pre, eh0, mat("edge_heads.energy.0.2.weight"), vec("edge_heads.energy.0.2.bias"), E);
+    gm.linear_silu({eh1}, eh1_pre, eh0, mat("edge_heads.energy.0.2.weight"), vec("edge_heads.energy.0.2.bias"), E);
     gemv_rows(st, eh1, Dh, mat("edge_last_layers.energy.0.energy___0.weight").w, vec("edge_last_layers.energy.0.energy___0.bias"),
               edge_pred, E, Dh);
   }
@@ -637,38 +693,38 @@ PassOut Model::run_feedforward(Stream& st, Arena& save, Arena& tmp, const Packed
   float* cf_adj = save.alloc<float>(Ea);
   PETB_CUDA(cudaMemsetAsync(x4_adj, 0, sizeof(float) * Ea * 4, st.s));
   PETB_CUDA(cudaMemsetAsync(cf_adj, 0, sizeof(float) * Ea, st.s));
-  float* node_adj = save.alloc<float>(Na * Dn);
-  float* ie_adj = save.alloc<float>(Ea * D);
-  float* tok_adj = save.alloc<float>(Ta * D);
-  float* edge_adj = tok_adj + size_t(N) * D;
+  Rows node_adj = maxima.fresh(save.alloc<float>(Na * Dn), Na), ie_adj = maxima.fresh(save.alloc<float>(Ea * D), Ea);
+  Rows tok_adj = {save.alloc<float>(Ta * D)};
   {
     Scope s6(tmp);
-    float* nh1_adj = tmp.alloc<float>(Na * Dh);
-    float* nh0_adj = tmp.alloc<float>(Na * Dh);
-    float* eh1_adj = tmp.alloc<float>(Ea * Dh);
-    float* eh0_adj = tmp.alloc<float>(Ea * Dh);
-    readout_seed_bwd(st, nh1_adj, mat("node_last_layers.energy.0.energy___0.weight").w, nh1_pre, nullptr, nullptr, pk.n_local, N, Dh);
+    const Rows nh1_adj = maxima.fresh(tmp.alloc<float>(Na * Dh), Na), nh0_adj = maxima.fresh(tmp.alloc<float>(Na * Dh), Na);
+    const Rows eh1_adj = maxima.fresh(tmp.alloc<float>(Ea * Dh), Ea), eh0_adj = maxima.fresh(tmp.alloc<float>(Ea * Dh), Ea);
+    readout_seed_bwd(st, nh1_adj.p, mat("node_last_layers.energy.0.energy___0.weight").w, nh1_pre, nullptr, nullptr, pk.n_local, N, Dh,
+                     nh1_adj.mx);
     gm.linear_silu_bwd(nh0_adj, nh1_adj, mat("node_heads.energy.0.2.weight"), nh0_pre, N);
     gm.linear_bwd(node_adj, nh0_adj, mat("node_heads.energy.0.0.weight"), N, false);
-    readout_seed_bwd(st, eh1_adj, mat("edge_last_layers.energy.0.energy___0.weight").w, eh1_pre, pk.cut, pk.center, pk.n_local, E, Dh);
+    readout_seed_bwd(st, eh1_adj.p, mat("edge_last_layers.energy.0.energy___0.weight").w, eh1_pre, pk.cut, pk.center, pk.n_local, E, Dh,
+                     eh1_adj.mx);
     gm.linear_silu_bwd(eh0_adj, eh1_adj, mat("edge_heads.energy.0.2.weight"), eh0_pre, E);
     gm.linear_bwd(ie_adj, eh0_adj, mat("edge_heads.energy.0.0.weight"), E, false);
   }
+  // The adjoint of a layer's tokens is one buffer written again and again: each writer of its edge rows or of all of it
+  // takes fresh maxima.
   for (int L = G - 1; L >= 0; --L) {
     const std::string g = "gnn_layers." + std::to_string(L), ls = std::to_string(L), c0 = g + ".compress.0";
     Scope relayered(save);  // under Layers: this layer's saves, made again below and dropped after its backward
     Layer again;
     if (relayer) {
-      float* scratch_node = save.alloc<float>(Na * Dn);
+      Rows scratch_node = {save.alloc<float>(Na * Dn)};
       layer_forward(L, node_at[L], scratch_node, ie_at[L], again, false, remote_in[L], false);
     }
     const Layer& sl = relayer ? again : sav[L];
     {
       Scope s7(tmp);
-      float* cph_adj = tmp.alloc<float>(Ea * 2 * D);
+      const Rows cph_adj = maxima.fresh(tmp.alloc<float>(Ea * 2 * D), Ea);
       float* cnorm_adj = tmp.alloc<float>(Ea * 2 * D);
       gm.linear_silu_bwd(cph_adj, ie_adj, mat("combination_mlps." + ls + ".2.weight"), sl.cph_pre, E);
-      gm.linear_bwd(cnorm_adj, cph_adj, mat("combination_mlps." + ls + ".0.weight"), E, false);
+      gm.linear_bwd({cnorm_adj}, cph_adj, mat("combination_mlps." + ls + ".0.weight"), E, false);
       RemoteRows remote;
       float* remote_adj = nullptr;
       if (pk.exchange) {  // the partner's rank wants the adjoint of the row this edge read (src/feedforward.cpp:241-255)
@@ -680,44 +736,50 @@ PassOut Model::run_feedforward(Stream& st, Arena& save, Arena& tmp, const Packed
                                pk.n_live, D, remote);
         exchange_rows(st, pk, send, remote_adj, D);
       }
-      concat_norm_bwd(st, edge_adj, cnorm_adj, sl.out_edge, pk.reverse, ie_adj, vec("combination_norms." + ls + ".weight"), E, D,
-                      remote, remote_adj);
+      tok_adj.mx = maxima.take(Ta);
+      const Rows edge_adj = tok_adj.from(N, D);
+      concat_norm_bwd(st, edge_adj.p, cnorm_adj, sl.out_edge, pk.reverse, ie_adj.p, vec("combination_norms." + ls + ".weight"), E, D,
+                      remote, remote_adj, edge_adj.mx);
     }
     for (int a = A - 1; a >= 0; --a) {
       const std::string tl = g + ".trans.layers." + std::to_string(a);
       const Block& b = sl.blk[a];
       const Mat &w_cin = mat(tl + ".center_mlp.w_in.weight"), &w_ein = mat(tl + ".mlp.w_in.weight");
       // the two MLPs: afterwards edge_adj and node_adj are eps's and node_res's
+      const Rows edge_adj = tok_adj.from(N, D);  // of the MLP's output
+      tok_adj.mx = maxima.take(Ta);
+      const Rows eps_adj = tok_adj.from(N, D);   // the same rows once the MLP's backward has added to them
       const int rows = b.pre_e || chunk <= 0 ? (E > 0 ? E : 1) : chunk;
       for (int r0 = 0; r0 < E; r0 += rows) {
         const int nr = std::min(rows, E - r0);
         Scope s8(tmp);
-        const float* eps_rows = b.eps + (size_t(N) + r0) * D;
-        float* adj_rows = edge_adj + size_t(r0) * D;
+        const float* eps_rows = b.eps.p + (size_t(N) + r0) * D;
+        const Rows adj_rows = edge_adj.from(r0, D);
         const float* pre = b.pre_e ? b.pre_e + size_t(r0) * w_ein.rows : nullptr;
         if (!pre) {  // the pre-activation was not kept: these rows' again
           float* again_pre = tmp.alloc<float>(size_t(nr) * w_ein.rows);
-          edge_mlp_in(nullptr, again_pre, eps_rows, tl, nr);
+          edge_mlp_in({}, again_pre, eps_rows, tl, nr);
           pre = again_pre;
         }
-        float* pre_adj = tmp.alloc<float>(size_t(nr) * w_ein.rows);
+        const Rows pre_adj = maxima.fresh(tmp.alloc<float>(size_t(nr) * w_ein.rows), nr);
         float* enorm_adj = tmp.alloc<float>(size_t(nr) * D);
         gm.swiglu_out_bwd(pre_adj, adj_rows, mat(tl + ".mlp.w_out.weight"), pre, nr);
-        gm.linear_bwd(enorm_adj, pre_adj, w_ein, nr, false);
-        norm_bwd(st, adj_rows, enorm_adj, eps_rows, vec(tl + ".norm_mlp.weight"), false, nr, D, 0);
+        gm.linear_bwd({enorm_adj}, pre_adj, w_ein, nr, false);
+        norm_bwd(st, adj_rows.p, enorm_adj, eps_rows, vec(tl + ".norm_mlp.weight"), false, nr, D, 0, nullptr, eps_adj.from(r0, D).mx);
       }
       {
         Scope s9(tmp);
-        float* prec_adj = tmp.alloc<float>(Na * w_cin.rows);
+        const Rows prec_adj = maxima.fresh(tmp.alloc<float>(Na * w_cin.rows), Na);
         float* cnorm_adj = tmp.alloc<float>(Na * Dn);
         gm.swiglu_out_bwd(prec_adj, node_adj, mat(tl + ".center_mlp.w_out.weight"), b.pre_c, N);
-        gm.linear_bwd(cnorm_adj, prec_adj, w_cin, N, false);
-        norm_bwd(st, node_adj, cnorm_adj, b.node_res, vec(tl + ".norm_center_features.weight"), false, N, Dn, 0);
+        gm.linear_bwd({cnorm_adj}, prec_adj, w_cin, N, false);
+        node_adj.mx = maxima.take(Na);
+        norm_bwd(st, node_adj.p, cnorm_adj, b.node_res, vec(tl + ".norm_center_features.weight"), false, N, Dn, 0, nullptr, node_adj.mx);
       }
       {  // attention: the output adjoint is [expansion's input adjoint ; eps adjoint] = tok_adj
         Scope s10(tmp);
         float* dmerged = tmp.alloc<float>(Ta * D);
-        float* qkv_adj = tmp.alloc<float>(Ta * 3 * D);
+        const Rows qkv_adj = maxima.fresh(tmp.alloc<float>(Ta * 3 * D), Ta);
         float* cfh = tmp.alloc<float>(Ta * H);
         float* attn_in_adj = tmp.alloc<float>(Ta * D);
         const float* qkv = b.qkv;
@@ -727,23 +789,26 @@ PassOut Model::run_feedforward(Stream& st, Arena& save, Arena& tmp, const Packed
           qkv = again_qkv;
         }
         gm.linear_bwd(tok_adj, node_adj, mat(tl + ".center_expansion.weight"), N, false);
-        gm.linear_bwd(dmerged, tok_adj, mat(tl + ".attention.output_linear.weight"), T, false);
+        gm.linear_bwd({dmerged}, tok_adj, mat(tl + ".attention.output_linear.weight"), T, false);
         AttnArgs at = attention_args(b, qkv);
-        at.dmerged = dmerged, at.qkv_adj = qkv_adj, at.cfh = cfh;
+        at.dmerged = dmerged, at.qkv_adj = qkv_adj.p, at.qkv_adj_max = qkv_adj.mx, at.cfh = cfh;
         attention_backward(st, at);
         cutoff_share(st, cf_adj, cfh, pk.cut, N, E, H);
-        gm.linear_bwd(attn_in_adj, qkv_adj, mat(tl + ".attention.input_linear.weight"), T, false);
+        gm.linear_bwd({attn_in_adj}, qkv_adj, mat(tl + ".attention.input_linear.weight"), T, false);
         // through the norm, back to where the tokens came from: atom rows to the contraction's
         // output adjoint (written), edge rows onto the edge residual (accumulated)
-        norm_bwd(st, tok_adj, attn_in_adj, b.tok, vec(tl + ".norm_attention.weight"), false, T, D, N);
+        tok_adj.mx = maxima.take(Ta);
+        norm_bwd(st, tok_adj.p, attn_in_adj, b.tok, vec(tl + ".norm_attention.weight"), false, T, D, N, nullptr, tok_adj.mx);
       }
+      node_adj.mx = maxima.take(Na);
       gm.linear_bwd(node_adj, tok_adj, mat(tl + ".center_contraction.weight"), N, true);
     }
-    {  // edge_adj is now et's
+    {  // the edge rows are now et's
       Scope s11(tmp);
-      float* gz = tmp.alloc<float>(Ea * D);
-      gm.linear_silu_bwd(gz, edge_adj, mat(g + ".compress.2.weight"), sl.cpre, E);
-      compress_geometry_bwd(st, x4_adj, gz, mat(c0 + "@x4").w, E, D);
+      const Rows gz = maxima.fresh(tmp.alloc<float>(Ea * D), Ea);
+      gm.linear_silu_bwd(gz, tok_adj.from(N, D), mat(g + ".compress.2.weight"), sl.cpre, E);
+      compress_geometry_bwd(st, x4_adj, gz.p, mat(c0 + "@x4").w, E, D);
+      ie_adj.mx = maxima.take(Ea);
       if (L > 0) gm.linear_bwd(ie_adj, gz, mat(c0 + "@in"), E, true);
     }
   }
@@ -762,22 +827,23 @@ PassOut Model::run_residual(Stream& st, Arena& save, Arena& tmp, const PackedEdg
   const int N = pk.N, E = pk.E, T = N + E, S = pk.M + 1;
   const int D = h_.d_pet, Dh = h_.d_head, H = h_.num_heads, hd = h_.head_dim;
   const int G = h_.num_gnn_layers, A = h_.num_attention_layers;
-  const Gemms gm{st, tmp, mode};
+  const Gemms gm{st, tmp};
   const float sc = float(1.0 / (std::sqrt(double(hd)) * h_.attention_temperature));
   const size_t Ea = E > 0 ? E : 1, Ta = T > 0 ? T : 1, Na = N > 0 ? N : 1;
+  RowMaxima maxima(st, save, row_maxima_words(N, E));
 
   struct Block {
     float *qkv, *merged, *ml, *s1, *s2, *pre;
   };
   struct Layer {
-    float *cpre, *tokens;
+    float* cpre;
     float *nh0_pre, *nh1_pre, *eh0_pre, *eh1_pre, *edge_pred;
     std::vector<Block> blk;
   };
   std::vector<Layer> sav(G);
 
-  float* input_edge = save.alloc<float>(Ea * D);
-  gather_rows(st, input_edge, mat("edge_embedder.weight").w, pk.species, E, D);
+  Rows input_edge = {save.alloc<float>(Ea * D)};  // layer 0 does not multiply it
+  gather_rows(st, input_edge.p, mat("edge_embedder.weight").w, pk.species, E, D);
   float* net = save.alloc<float>(Na);
   float* node_pred = save.alloc<float>(Na);
   double* per_atom = save.alloc<double>(pk.n_atoms > 0 ? pk.n_atoms : 1);
@@ -787,24 +853,18 @@ PassOut Model::run_residual(Stream& st, Arena& save, Arena& tmp, const PackedEdg
     const std::string g = "gnn_layers." + std::to_string(L), ls = std::to_string(L), c0 = g + ".compress.0";
     Layer& sl = sav[L];
     sl.blk.resize(A);
-    sl.tokens = save.alloc<float>(Ta * D);
+    Rows tokens = maxima.fresh(save.alloc<float>(Ta * D), Ta);
     sl.cpre = save.alloc<float>(Ea * D);
-    float* tokens = sl.tokens;
-    gather_rows(st, tokens, mat("node_embedders." + ls + ".weight").w, pk.atom_species, N, D);
+    gather_rows(st, tokens.p, mat("node_embedders." + ls + ".weight").w, pk.atom_species, N, D, tokens.mx);
     {
       Scope s0(tmp);
-      float* cact = tmp.alloc<float>(Ea * D);
+      const Rows cact = maxima.fresh(tmp.alloc<float>(Ea * D), Ea);
       if (L == 0) {
-        compress0(st, cact, sl.cpre, vec(c0 + "@b"), mat(c0 + "@tab").w, mat(c0 + "@x4").w, pk, D);
+        compress0(st, cact.p, sl.cpre, vec(c0 + "@b"), mat(c0 + "@tab").w, mat(c0 + "@x4").w, pk, D, cact.mx);
       } else {
-        const Mat& wi = mat(c0 + "@in");
-        GemmArgs a;
-        a.A = input_edge, a.lda = D, a.B = wi.w, a.ldb = D, a.b_lo_offset = wi.lo_off, a.B16 = wi.w16, a.C = cact, a.ldc = D, a.M = E, a.N = D, a.K = D;
-        a.bias = vec(c0 + "@b"), a.pre = sl.cpre, a.ldp = D, a.tab = mat(c0 + "@tab").w, a.sp = pk.species;
-        a.wx = mat(c0 + "@x4").w, a.vec = pk.vec, a.dist = pk.dist, a.epi = EPI_COMPRESS;
-        gemm(st, tmp, a, mode);
+        gm.compress(cact, sl.cpre, input_edge, mat(c0 + "@in"), vec(c0 + "@b"), mat(c0 + "@tab"), mat(c0 + "@x4"), pk);
       }
-      gm.linear(tokens + size_t(N) * D, cact, mat(g + ".compress.2.weight"), vec(g + ".compress.2.bias"), E);
+      gm.linear(tokens.from(N, D), cact, mat(g + ".compress.2.weight"), vec(g + ".compress.2.bias"), E);
     }
     for (int a = 0; a < A; ++a) {
       const std::string tl = g + ".trans.layers." + std::to_string(a);
@@ -816,43 +876,43 @@ PassOut Model::run_residual(Stream& st, Arena& save, Arena& tmp, const PackedEdg
       b.s1 = save.alloc<float>(Ta * D);
       b.s2 = save.alloc<float>(Ta * D);
       b.pre = save.alloc<float>(Ta * w_in.rows);
-      gm.linear(b.qkv, tokens, mat(tl + ".attention.input_linear.weight"), vec(tl + ".attention.input_linear.bias"), T);
+      gm.linear({b.qkv}, tokens, mat(tl + ".attention.input_linear.weight"), vec(tl + ".attention.input_linear.bias"), T);
       AttnArgs at;
       at.N = N, at.H = H, at.hd = hd, at.S = S, at.sc = sc, at.off = pk.off, at.cut = pk.cut;
       at.mode = attention_mode_for(mode);
       at.pairs = pk.pairs, at.T = T;
-      at.qkv = b.qkv, at.merged = b.merged, at.ml = b.ml;
+      const Rows merged = maxima.fresh(b.merged, Ta);
+      at.qkv = b.qkv, at.merged = b.merged, at.ml = b.ml, at.merged_max = merged.mx;
       attention_forward(st, at);
       // s1 = attention(tokens) + tokens
-      gm.linear(b.s1, b.merged, mat(tl + ".attention.output_linear.weight"), vec(tl + ".attention.output_linear.bias"), T,
-                tokens, 0);
+      gm.linear({b.s1}, merged, mat(tl + ".attention.output_linear.weight"), vec(tl + ".attention.output_linear.bias"), T,
+                tokens.p, 0);
       Scope s1(tmp);
-      float* tok_a = tmp.alloc<float>(Ta * D);
-      float* hmid = tmp.alloc<float>(Ta * w_in.rows);
-      norm_fwd(st, tok_a, b.s1, nullptr, vec(tl + ".norm_attention.weight"), vec(tl + ".norm_attention.bias"), T, D);
+      const Rows tok_a = maxima.fresh(tmp.alloc<float>(Ta * D), Ta), hmid = maxima.fresh(tmp.alloc<float>(Ta * w_in.rows), Ta);
+      norm_fwd(st, tok_a.p, b.s1, nullptr, vec(tl + ".norm_attention.weight"), vec(tl + ".norm_attention.bias"), T, D, tok_a.mx);
       gm.linear_silu(hmid, b.pre, tok_a, w_in, vec(tl + ".mlp.w_in.bias"), T);
       // s2 = mlp(tok_a) + tok_a; tokens = LN(s2)
-      gm.linear(b.s2, hmid, mat(tl + ".mlp.w_out.weight"), vec(tl + ".mlp.w_out.bias"), T, tok_a, 0);
-      norm_fwd(st, tokens, b.s2, nullptr, vec(tl + ".norm_mlp.weight"), vec(tl + ".norm_mlp.bias"), T, D);
+      gm.linear({b.s2}, hmid, mat(tl + ".mlp.w_out.weight"), vec(tl + ".mlp.w_out.bias"), T, tok_a.p, 0);
+      tokens.mx = maxima.take(Ta);
+      norm_fwd(st, tokens.p, b.s2, nullptr, vec(tl + ".norm_mlp.weight"), vec(tl + ".norm_mlp.bias"), T, D, tokens.mx);
     }
-    tap(taps, "tokens" + ls, tokens, size_t(T) * D);
+    tap(taps, "tokens" + ls, tokens.p, size_t(T) * D);
     // this layer's readout, summed onto the earlier layers' (src/model.cpp:656-691)
     sl.nh0_pre = save.alloc<float>(Na * Dh), sl.nh1_pre = save.alloc<float>(Na * Dh);
     sl.eh0_pre = save.alloc<float>(Ea * Dh), sl.eh1_pre = save.alloc<float>(Ea * Dh);
     sl.edge_pred = save.alloc<float>(Ea);
     {
       Scope s2(tmp);
-      float* nh0 = tmp.alloc<float>(Na * Dh);
+      const Rows nh0 = maxima.fresh(tmp.alloc<float>(Na * Dh), Na), eh0 = maxima.fresh(tmp.alloc<float>(Ea * Dh), Ea);
       float* nh1 = tmp.alloc<float>(Na * Dh);
-      float* eh0 = tmp.alloc<float>(Ea * Dh);
       float* eh1 = tmp.alloc<float>(Ea * Dh);
       const std::string nh = "node_heads.energy." + ls, eh = "edge_heads.energy." + ls;
       const std::string nl = "node_last_layers.energy." + ls + ".energy___0", el = "edge_last_layers.energy." + ls + ".energy___0";
       gm.linear_silu(nh0, sl.nh0_pre, tokens, mat(nh + ".0.weight"), vec(nh + ".0.bias"), N);
-      gm.linear_silu(nh1, sl.nh1_pre, nh0, mat(nh + ".2.weight"), vec(nh + ".2.bias"), N);
+      gm.linear_silu({nh1}, sl.nh1_pre, nh0, mat(nh + ".2.weight"), vec(nh + ".2.bias"), N);
       gemv_rows(st, nh1, Dh, mat(nl + ".weight").w, vec(nl + ".bias"), node_pred, N, Dh);
-      gm.linear_silu(eh0, sl.eh0_pre, tokens + size_t(N) * D, mat(eh + ".0.weight"), vec(eh + ".0.bias"), E);
-      gm.linear_silu(eh1, sl.eh1_pre, eh0, mat(eh + ".2.weight"), vec(eh + ".2.bias"), E);
+      gm.linear_silu(eh0, sl.eh0_pre, tokens.from(N, D), mat(eh + ".0.weight"), vec(eh + ".0.bias"), E);
+      gm.linear_silu({eh1}, sl.eh1_pre, eh0, mat(eh + ".2.weight"), vec(eh + ".2.bias"), E);
       gemv_rows(st, eh1, Dh, mat(el + ".weight").w, vec(el + ".bias"), sl.edge_pred, E, Dh);
       readout_energy(st, net, per_atom, node_pred, sl.edge_pred, pk, comp_, scale_, L > 0, L + 1 == G);
       tap(taps, "node_pred" + ls, node_pred, N);
@@ -865,11 +925,12 @@ PassOut Model::run_residual(Stream& st, Arena& save, Arena& tmp, const PackedEdg
         const size_t La = size_t(pk.n_live > 0 ? pk.n_live : 1) * D;
         float* send = tmp.alloc<float>(La);
         float* recv = tmp.alloc<float>(La);
-        gather_live(st, send, tokens + size_t(N) * D, D, 0, pk.live_packed, pk.n_live, D);
+        gather_live(st, send, tokens.p + size_t(N) * D, D, 0, pk.live_packed, pk.n_live, D);
         exchange_rows(st, pk, send, recv, D);
         remote = RemoteRows{pk.remote_of, recv};
       }
-      message_average(st, input_edge, tokens + size_t(N) * D, pk.reverse, E, D, remote);
+      input_edge.mx = maxima.take(Ea);
+      message_average(st, input_edge.p, tokens.p + size_t(N) * D, pk.reverse, E, D, remote, input_edge.mx);
     }
   }
   if (!grad) return finish(st, save, pk, false, nullptr, nullptr, nullptr, per_atom);
@@ -889,22 +950,20 @@ PassOut Model::run_residual(Stream& st, Arena& save, Arena& tmp, const PackedEdg
     const std::string g = "gnn_layers." + std::to_string(L), ls = std::to_string(L), c0 = g + ".compress.0";
     const Layer& sl = sav[L];
     Scope layer_scope(tmp);
-    float* tokens_adj = tmp.alloc<float>(Ta * D);
+    Rows tokens_adj = {tmp.alloc<float>(Ta * D)};
     float* alt = tmp.alloc<float>(Ta * D);
     {  // the readout's adjoint of this layer's tokens
       Scope s3(tmp);
-      float* nh1_adj = tmp.alloc<float>(Na * Dh);
-      float* nh0_adj = tmp.alloc<float>(Na * Dh);
-      float* eh1_adj = tmp.alloc<float>(Ea * Dh);
-      float* eh0_adj = tmp.alloc<float>(Ea * Dh);
+      const Rows nh1_adj = maxima.fresh(tmp.alloc<float>(Na * Dh), Na), nh0_adj = maxima.fresh(tmp.alloc<float>(Na * Dh), Na);
+      const Rows eh1_adj = maxima.fresh(tmp.alloc<float>(Ea * Dh), Ea), eh0_adj = maxima.fresh(tmp.alloc<float>(Ea * Dh), Ea);
       const std::string nh = "node_heads.energy." + ls, eh = "edge_heads.energy." + ls;
       const std::string nl = "node_last_layers.energy." + ls + ".energy___0", el = "edge_last_layers.energy." + ls + ".energy___0";
-      readout_seed_bwd(st, nh1_adj, mat(nl + ".weight").w, sl.nh1_pre, nullptr, nullptr, pk.n_local, N, Dh);
+      readout_seed_bwd(st, nh1_adj.p, mat(nl + ".weight").w, sl.nh1_pre, nullptr, nullptr, pk.n_local, N, Dh, nh1_adj.mx);
       gm.linear_silu_bwd(nh0_adj, nh1_adj, mat(nh + ".2.weight"), sl.nh0_pre, N);
       gm.linear_bwd(tokens_adj, nh0_adj, mat(nh + ".0.weight"), N, false);
-      readout_seed_bwd(st, eh1_adj, mat(el + ".weight").w, sl.eh1_pre, pk.cut, pk.center, pk.n_local, E, Dh);
+      readout_seed_bwd(st, eh1_adj.p, mat(el + ".weight").w, sl.eh1_pre, pk.cut, pk.center, pk.n_local, E, Dh, eh1_adj.mx);
       gm.linear_silu_bwd(eh0_adj, eh1_adj, mat(eh + ".2.weight"), sl.eh0_pre, E);
-      gm.linear_bwd(tokens_adj + size_t(N) * D, eh0_adj, mat(eh + ".0.weight"), E, false);
+      gm.linear_bwd(tokens_adj.from(N, D), eh0_adj, mat(eh + ".0.weight"), E, false);
     }
     float* ie_next = ie_adj == ie_a ? ie_b : ie_a;
     if (L + 1 < G) {
@@ -917,7 +976,7 @@ PassOut Model::run_residual(Stream& st, Arena& save, Arena& tmp, const PackedEdg
         exchange_rows(st, pk, send, recv, D);
         remote = RemoteRows{pk.remote_of, recv};
       }
-      message_average_bwd(st, ie_next, tokens_adj + size_t(N) * D, ie_adj, pk.reverse, E, D, remote);
+      message_average_bwd(st, ie_next, tokens_adj.p + size_t(N) * D, ie_adj, pk.reverse, E, D, remote);
     }
     else PETB_CUDA(cudaMemsetAsync(ie_next, 0, sizeof(float) * Ea * D, st.s));
     for (int a = A - 1; a >= 0; --a) {
@@ -925,43 +984,45 @@ PassOut Model::run_residual(Stream& st, Arena& save, Arena& tmp, const PackedEdg
       const Block& b = sl.blk[a];
       const Mat& w_in = mat(tl + ".mlp.w_in.weight");
       Scope s4(tmp);
-      float* s2_adj = tmp.alloc<float>(Ta * D);
+      const Rows s2_adj = maxima.fresh(tmp.alloc<float>(Ta * D), Ta);
       float* tok_a_adj = tmp.alloc<float>(Ta * D);
       // tokens_out = LN(s2), s2 = tok_a + mlp(tok_a)
-      norm_bwd(st, s2_adj, tokens_adj, b.s2, vec(tl + ".norm_mlp.weight"), true, T, D, T, tok_a_adj);
+      norm_bwd(st, s2_adj.p, tokens_adj.p, b.s2, vec(tl + ".norm_mlp.weight"), true, T, D, T, tok_a_adj, s2_adj.mx);
       {
         Scope s5(tmp);
-        float* h_adj = tmp.alloc<float>(Ta * w_in.rows);
+        const Rows h_adj = maxima.fresh(tmp.alloc<float>(Ta * w_in.rows), Ta);
         gm.linear_silu_bwd(h_adj, s2_adj, mat(tl + ".mlp.w_out.weight"), b.pre, T);
-        gm.linear_bwd(tok_a_adj, h_adj, w_in, T, true);
+        gm.linear_bwd({tok_a_adj}, h_adj, w_in, T, true);
       }
       // tok_a = LN(s1), s1 = tokens_in + attention(tokens_in)
-      float* s1_adj = alt;
-      norm_bwd(st, s1_adj, tok_a_adj, b.s1, vec(tl + ".norm_attention.weight"), true, T, D, T);
+      Rows s1_adj = maxima.fresh(alt, Ta);
+      norm_bwd(st, s1_adj.p, tok_a_adj, b.s1, vec(tl + ".norm_attention.weight"), true, T, D, T, nullptr, s1_adj.mx);
       {
         Scope s6(tmp);
         float* dmerged = tmp.alloc<float>(Ta * D);
-        float* qkv_adj = tmp.alloc<float>(Ta * 3 * D);
+        const Rows qkv_adj = maxima.fresh(tmp.alloc<float>(Ta * 3 * D), Ta);
         float* cfh = tmp.alloc<float>(Ta * H);
-        gm.linear_bwd(dmerged, s1_adj, mat(tl + ".attention.output_linear.weight"), T, false);
+        gm.linear_bwd({dmerged}, s1_adj, mat(tl + ".attention.output_linear.weight"), T, false);
         AttnArgs at;
         at.N = N, at.H = H, at.hd = hd, at.S = S, at.sc = sc, at.off = pk.off, at.cut = pk.cut;
       at.mode = attention_mode_for(mode);
         at.pairs = pk.pairs, at.T = T;
-        at.qkv = b.qkv, at.merged = b.merged, at.ml = b.ml, at.dmerged = dmerged, at.qkv_adj = qkv_adj, at.cfh = cfh;
+        at.qkv = b.qkv, at.merged = b.merged, at.ml = b.ml, at.dmerged = dmerged, at.qkv_adj = qkv_adj.p, at.cfh = cfh;
+        at.qkv_adj_max = qkv_adj.mx;
         attention_backward(st, at);
         cutoff_share(st, cf_adj, cfh, pk.cut, N, E, H);
+        s1_adj.mx = maxima.take(Ta);
         gm.linear_bwd(s1_adj, qkv_adj, mat(tl + ".attention.input_linear.weight"), T, true);
       }
-      alt = tokens_adj;
+      alt = tokens_adj.p;
       tokens_adj = s1_adj;
     }
     {  // tokens = [node_L ; et]: only et depends on the geometry
       Scope s7(tmp);
-      float* gz = tmp.alloc<float>(Ea * D);
-      gm.linear_silu_bwd(gz, tokens_adj + size_t(N) * D, mat(g + ".compress.2.weight"), sl.cpre, E);
-      compress_geometry_bwd(st, x4_adj, gz, mat(c0 + "@x4").w, E, D);
-      if (L > 0) gm.linear_bwd(ie_next, gz, mat(c0 + "@in"), E, true);
+      const Rows gz = maxima.fresh(tmp.alloc<float>(Ea * D), Ea);
+      gm.linear_silu_bwd(gz, tokens_adj.from(N, D), mat(g + ".compress.2.weight"), sl.cpre, E);
+      compress_geometry_bwd(st, x4_adj, gz.p, mat(c0 + "@x4").w, E, D);
+      if (L > 0) gm.linear_bwd({ie_next}, gz, mat(c0 + "@in"), E, true);
     }
     ie_adj = ie_next;
   }

@@ -12,19 +12,18 @@
 
 #include "checkpoint.h"
 #include "common.h"
+#include "gemm.h"
 #include "neighbors.h"
 #include "ops.h"
 
 namespace petb {
 
-// A weight on the device in both orientations: w [rows, cols] as stored, wt [cols, rows].
+// A weight on the device.
 struct Mat {
-  const float* w = nullptr;
-  const float* wt = nullptr;
+  const float* w = nullptr;  // [rows, cols]
   int rows = 0, cols = 0;
-  size_t lo_off = 0;  // w + lo_off and wt + lo_off: the low parts of the 3xTF32 split of w and wt
-  const uint16_t* w16 = nullptr;   // w and wt again as bf16 (round to nearest even), for the bf16 GEMM mode
-  const uint16_t* wt16 = nullptr;
+  // GEMM operands: w (and its transpose) packed for the native mode and for the mode the model was loaded for
+  PackedB nat, nat_t, fast, fast_t;
 };
 
 struct PassOut {
@@ -53,7 +52,7 @@ struct RunOptions {
 
 class Model {
  public:
-  explicit Model(const Checkpoint& ckpt);
+  Model(const Checkpoint& ckpt, int gemm_mode);
   ~Model();
   Model(const Model&) = delete;
   Model& operator=(const Model&) = delete;
@@ -81,6 +80,7 @@ class Model {
   size_t last_estimate() const { return last_estimate_; }
   // Bytes the pools hold for one evaluation with forces of N atoms and E kept edges under a tier.
   size_t memory_estimate(int tier, int N, int E) const;
+  size_t row_maxima_words(int N, int E) const;
   MemoryNeed memory_need(int tier, int N, int E, int n_live) const;
   int choose_tier(const RunOptions& opt, int N, int E) const;
   // Rows of a chunk of the edge MLP under Wide and Layers: an eighth of the edges, at least 64 Ki; PET_EDGE_CHUNK=rows
@@ -98,12 +98,13 @@ class Model {
   const Mat& mat(const std::string& name) const;
   const float* vec(const std::string& name) const;
   // `src` are doubles in DEVICE memory; the layouts the kernels read are made from them by kernels.
-  void put_mat(const std::string& name, const double* src, int ld, int rows, int cols, bool paired);
+  void put_mat(const std::string& name, const double* src, int ld, int rows, int cols, bool paired, bool operand);
   void put_vec(const std::string& name, const double* src, int len, bool paired);
   void fold_compress(const Checkpoint& ck, const std::string& c0, int layer);
 
   Hypers h_;
   double scale_ = 1.0;
+  int mode_ = 0;  // the GEMM mode the weights are packed for
   int last_tier_ = RECOMPUTE_NEVER;
   size_t last_estimate_ = 0;
   double* comp_ = nullptr;  // [n_species] composition energies

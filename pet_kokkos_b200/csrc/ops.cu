@@ -22,12 +22,32 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
+__device__ __forceinline__ float warp_max(float v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(kFull, v, o));
+  return v;
+}
+__device__ __forceinline__ float max4(const float4& v) { return max_abs4(v.x, v.y, v.z, v.w); }
+
+// Row r's largest magnitude raised to m, for kernels with a thread per run of four of a row's D4 runs: where a row is whole
+// warps, a warp's largest goes out once.
+__device__ __forceinline__ void raise_row(uint32_t* mx, int r, int D4, float m) {
+  if (!mx) return;
+  if (D4 % 32 == 0) {
+    m = warp_max(m);
+    if (threadIdx.x % 32) return;
+  }
+  atomicMax(mx + r, __float_as_uint(m));
+}
+
 __global__ void k_gather_rows(float* __restrict__ out, const float* __restrict__ table, const int* __restrict__ idx, int R,
-                              int D4) {
+                              int D4, uint32_t* __restrict__ mx) {
   const size_t t = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (t >= size_t(R) * D4) return;
   const int r = int(t / D4), q = int(t % D4);
-  reinterpret_cast<float4*>(out)[t] = reinterpret_cast<const float4*>(table)[size_t(idx[r]) * D4 + q];
+  const float4 v = reinterpret_cast<const float4*>(table)[size_t(idx[r]) * D4 + q];
+  reinterpret_cast<float4*>(out)[t] = v;
+  raise_row(mx, r, D4, max4(v));
 }
 
 __global__ void k_compress0(GemmArgs p) {
@@ -35,12 +55,14 @@ __global__ void k_compress0(GemmArgs p) {
   const int D4 = p.N / 4;
   if (t >= size_t(p.M) * D4) return;
   const float zero[4] = {0.f, 0.f, 0.f, 0.f};
-  epilogue_run4<EPI_COMPRESS>(p, int(t / D4), int(t % D4) * 4, zero);
+  const float m = epilogue_run4<EPI_COMPRESS>(p, int(t / D4), int(t % D4) * 4, zero);
+  raise_row(p.c_max, int(t / D4), D4, m);
 }
 
 // One warp per row. x = in (+ add, stored back); out = (x - mu) inv w + b.
 __global__ void __launch_bounds__(256) k_norm_fwd(float* __restrict__ out, float* __restrict__ in, const float* __restrict__ add,
-                                                  const float* __restrict__ w, const float* __restrict__ bias, int R, int D) {
+                                                  const float* __restrict__ w, const float* __restrict__ bias, int R, int D,
+                                                  uint32_t* __restrict__ mx) {
   const int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (r >= R) return;
   float* x = in + size_t(r) * D;
@@ -63,7 +85,14 @@ __global__ void __launch_bounds__(256) k_norm_fwd(float* __restrict__ out, float
   v = warp_sum(v);
   const float inv = 1.0f / sqrtf(v / D + (ln ? kLnEps : kRmsEps));
   float* o = out + size_t(r) * D;
-  for (int d = lane; d < D; d += 32) o[d] = (x[d] - mu) * inv * w[d] + (ln ? bias[d] : 0.f);
+  float big = 0.f;
+  for (int d = lane; d < D; d += 32) {
+    const float y = (x[d] - mu) * inv * w[d] + (ln ? bias[d] : 0.f);
+    o[d] = y, big = fmaxf(big, fabsf(y));
+  }
+  if (!mx) return;
+  big = warp_max(big);
+  if (lane == 0) mx[r] = __float_as_uint(big);
 }
 
 // Edge q's partner row: its reverse edge's, the row another rank sent for it, or none.
@@ -89,7 +118,8 @@ __global__ void k_gather_live(float* __restrict__ out, const float* __restrict__
 // once, 16 bytes at a time, for the statistics and for the output.
 template <int NV>
 __global__ void __launch_bounds__(256) k_norm_fwd_v(float* __restrict__ out, float* __restrict__ in, const float* __restrict__ add,
-                                                    const float* __restrict__ w, const float* __restrict__ bias, int R) {
+                                                    const float* __restrict__ w, const float* __restrict__ bias, int R,
+                                                    uint32_t* __restrict__ mx) {
   constexpr int D = 128 * NV;
   const int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (r >= R) return;
@@ -122,6 +152,7 @@ __global__ void __launch_bounds__(256) k_norm_fwd_v(float* __restrict__ out, flo
   q = warp_sum(q);
   const float inv = 1.0f / sqrtf(q / D + (ln ? kLnEps : kRmsEps));
   float* o = out + size_t(r) * D;
+  float big = 0.f;
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
     const float4 ww = ld4(w + 128 * i + 4 * lane);
@@ -132,13 +163,17 @@ __global__ void __launch_bounds__(256) k_norm_fwd_v(float* __restrict__ out, flo
       y.x += bb.x, y.y += bb.y, y.z += bb.z, y.w += bb.w;
     }
     st4(o + 128 * i + 4 * lane, y);
+    big = fmaxf(big, max4(y));
   }
+  if (!mx) return;
+  big = warp_max(big);
+  if (lane == 0) mx[r] = __float_as_uint(big);
 }
 
 __global__ void __launch_bounds__(256) k_concat_norm_fwd(float* __restrict__ out, const float* __restrict__ oe,
                                                          const int* __restrict__ rev, float* __restrict__ ie,
                                                          const float* __restrict__ w, const float* __restrict__ bias, int E,
-                                                         int D, RemoteRows rm) {
+                                                         int D, RemoteRows rm, uint32_t* __restrict__ mx) {
   const int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (k >= E) return;
   const int W = 2 * D;
@@ -159,10 +194,15 @@ __global__ void __launch_bounds__(256) k_concat_norm_fwd(float* __restrict__ out
   v = warp_sum(v);
   const float inv = 1.0f / sqrtf(v / W + kLnEps);
   float* o = out + size_t(k) * W;
+  float big = 0.f;
   for (int d = lane; d < D; d += 32) {
-    o[d] = (a[d] - mu) * inv * w[d] + bias[d];
-    o[D + d] = ((b ? b[d] : 0.f) - mu) * inv * w[D + d] + bias[D + d];
+    const float y0 = (a[d] - mu) * inv * w[d] + bias[d], y1 = ((b ? b[d] : 0.f) - mu) * inv * w[D + d] + bias[D + d];
+    o[d] = y0, o[D + d] = y1;
+    big = fmaxf(big, fmaxf(fabsf(y0), fabsf(y1)));
   }
+  if (!mx) return;
+  big = warp_max(big);
+  if (lane == 0) mx[k] = __float_as_uint(big);
 }
 
 struct RowStats {
@@ -171,7 +211,7 @@ struct RowStats {
 
 __global__ void __launch_bounds__(256) k_norm_bwd(float* __restrict__ in_adj, const float* __restrict__ out_adj,
                                                   const float* __restrict__ in, const float* __restrict__ w, bool ln, int R, int D,
-                                                  int acc_row0, float* __restrict__ also) {
+                                                  int acc_row0, float* __restrict__ also, uint32_t* __restrict__ mx) {
   const int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (r >= R) return;
   const float* x = in + size_t(r) * D;
@@ -192,18 +232,23 @@ __global__ void __launch_bounds__(256) k_norm_bwd(float* __restrict__ in_adj, co
   const float mg = ln ? sg / D : 0.f, mgx = sgx * inv / D;
   float* o = in_adj + size_t(r) * D;
   const bool acc = r >= acc_row0;
+  float big = 0.f;
   for (int d = lane; d < D; d += 32) {
     const float g = inv * (ga[d] * w[d] - mg - (x[d] - mu) * inv * mgx);
     const float v = acc ? o[d] + g : g;
     o[d] = v;
     if (also) also[size_t(r) * D + d] = v;
+    big = fmaxf(big, fabsf(v));
   }
+  if (!mx) return;
+  big = warp_max(big);
+  if (lane == 0) mx[r] = __float_as_uint(big);
 }
 
 template <int NV>
 __global__ void __launch_bounds__(256) k_norm_bwd_v(float* __restrict__ in_adj, const float* __restrict__ out_adj,
                                                     const float* __restrict__ in, const float* __restrict__ w, bool ln, int R,
-                                                    int acc_row0, float* __restrict__ also) {
+                                                    int acc_row0, float* __restrict__ also, uint32_t* __restrict__ mx) {
   constexpr int D = 128 * NV;
   const int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (r >= R) return;
@@ -234,6 +279,7 @@ __global__ void __launch_bounds__(256) k_norm_bwd_v(float* __restrict__ in_adj, 
   const float mg = ln ? sg / D : 0.f, mgx = sgx * inv / D;
   float* o = in_adj + size_t(r) * D;
   const bool acc = r >= acc_row0;
+  float big = 0.f;
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
     float4 g = make_float4(inv * (gw[i].x - mg - x[i].x * inv * mgx), inv * (gw[i].y - mg - x[i].y * inv * mgx),
@@ -244,7 +290,11 @@ __global__ void __launch_bounds__(256) k_norm_bwd_v(float* __restrict__ in_adj, 
     }
     st4(o + 128 * i + 4 * lane, g);
     if (also) st4(also + size_t(r) * D + 128 * i + 4 * lane, g);
+    big = fmaxf(big, max4(g));
   }
+  if (!mx) return;
+  big = warp_max(big);
+  if (lane == 0) mx[r] = __float_as_uint(big);
 }
 
 // The statistics of row q of the concat [oe(q) | partner(q) or 0] and of its adjoint.
@@ -270,7 +320,8 @@ __device__ __forceinline__ RowStats concat_stats(const float* oe, const float* b
 __global__ void __launch_bounds__(256) k_concat_norm_bwd(float* __restrict__ edge_adj, const float* __restrict__ out_adj,
                                                          const float* __restrict__ oe, const int* __restrict__ rev,
                                                          const float* __restrict__ ie_adj, const float* __restrict__ w, int E,
-                                                         int D, RemoteRows rm, const float* __restrict__ remote_adj) {
+                                                         int D, RemoteRows rm, const float* __restrict__ remote_adj,
+                                                         uint32_t* __restrict__ mx) {
   const int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (k >= E) return;
   const int W = 2 * D, r = rev[k];
@@ -283,6 +334,7 @@ __global__ void __launch_bounds__(256) k_concat_norm_bwd(float* __restrict__ edg
   }
   // An edge to another rank's atom: that rank computed the adjoint of the row it read from here.
   const float* far = (r < 0 && rm.of && remote_adj && rm.of[k] >= 0) ? remote_adj + size_t(rm.of[k]) * D : nullptr;
+  float big = 0.f;
   for (int d = lane; d < D; d += 32) {
     const float gk = sk.inv * (out_adj[size_t(k) * W + d] * w[d] - sk.mg - (oe[size_t(k) * D + d] - sk.mu) * sk.inv * sk.mgx);
     float back = 0.f;
@@ -292,8 +344,13 @@ __global__ void __launch_bounds__(256) k_concat_norm_bwd(float* __restrict__ edg
     } else if (far) {
       back = far[d];
     }
-    edge_adj[size_t(k) * D + d] = ie_adj[size_t(k) * D + d] + gk + back;
+    const float v = ie_adj[size_t(k) * D + d] + gk + back;
+    edge_adj[size_t(k) * D + d] = v;
+    big = fmaxf(big, fabsf(v));
   }
+  if (!mx) return;
+  big = warp_max(big);
+  if (lane == 0) mx[k] = __float_as_uint(big);
 }
 
 // The same, one warp per PAIR of partner rows (single-rank lists only). Row k's concat is [oe(k) | oe(r)] and row r's is
@@ -303,7 +360,7 @@ template <int NV>
 __global__ void __launch_bounds__(256) k_concat_norm_bwd_pair(float* __restrict__ edge_adj, const float* __restrict__ out_adj,
                                                               const float* __restrict__ oe, const int* __restrict__ rev,
                                                               const float* __restrict__ ie_adj, const float* __restrict__ w,
-                                                              int E) {
+                                                              int E, uint32_t* __restrict__ mx) {
   constexpr int D = 128 * NV, W = 2 * D;
   const int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (k >= E) return;
@@ -316,11 +373,18 @@ __global__ void __launch_bounds__(256) k_concat_norm_bwd_pair(float* __restrict_
     const RowStats sk = concat_stats(oe, oe + size_t(r) * D, out_adj, w, k, D, lane);
     const float* xr2 = partner_row(oe, rev, none, r, D);
     const RowStats sr = concat_stats(oe, xr2, out_adj, w, r, D, lane);
+    float big = 0.f;
     for (int d = lane; d < D; d += 32) {
       const float gk = sk.inv * (out_adj[size_t(k) * W + d] * w[d] - sk.mg - (oe[size_t(k) * D + d] - sk.mu) * sk.inv * sk.mgx);
       const float x = (xr2 ? xr2[d] : 0.f) - sr.mu;
       const float back = sr.inv * (out_adj[size_t(r) * W + D + d] * w[D + d] - sr.mg - x * sr.inv * sr.mgx);
-      edge_adj[size_t(k) * D + d] = ie_adj[size_t(k) * D + d] + gk + back;
+      const float v = ie_adj[size_t(k) * D + d] + gk + back;
+      edge_adj[size_t(k) * D + d] = v;
+      big = fmaxf(big, fabsf(v));
+    }
+    if (mx) {
+      big = warp_max(big);
+      if (lane == 0) mx[k] = __float_as_uint(big);
     }
     return;
   }
@@ -365,6 +429,7 @@ __global__ void __launch_bounds__(256) k_concat_norm_bwd_pair(float* __restrict_
   // input adjoint of a concat row's element with centred value x and weighted output adjoint g, for row k's / r's statistics
   auto in_k = [&](float g, float x) { return inv * (g - mgk - x * inv * mgxk); };
   auto in_r = [&](float g, float x) { return inv * (g - mgr - x * inv * mgxr); };
+  float big_k = 0.f, big_r = 0.f;
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
     const int c = 128 * i + 4 * lane;
@@ -376,8 +441,17 @@ __global__ void __launch_bounds__(256) k_concat_norm_bwd_pair(float* __restrict_
       t.x += in_r(h0[i].x, b[i].x) + in_k(g1[i].x, b[i].x), t.y += in_r(h0[i].y, b[i].y) + in_k(g1[i].y, b[i].y);
       t.z += in_r(h0[i].z, b[i].z) + in_k(g1[i].z, b[i].z), t.w += in_r(h0[i].w, b[i].w) + in_k(g1[i].w, b[i].w);
       st4(edge_adj + size_t(r) * D + c, t);
+      big_r = fmaxf(big_r, max4(t));
     }
     st4(edge_adj + size_t(k) * D + c, o);
+    big_k = fmaxf(big_k, max4(o));
+  }
+  if (!mx) return;
+  big_k = warp_max(big_k);
+  if (mutual) big_r = warp_max(big_r);
+  if (lane == 0) {
+    mx[k] = __float_as_uint(big_k);
+    if (mutual) mx[r] = __float_as_uint(big_r);
   }
 }
 
@@ -434,7 +508,8 @@ __global__ void k_readout_energy(float* __restrict__ net, double* __restrict__ p
 }
 
 __global__ void k_readout_seed_bwd(float* __restrict__ out, const float* __restrict__ w, const float* __restrict__ pre,
-                                   const float* __restrict__ cut, const int* __restrict__ center, int n_local, int R, int Dh4) {
+                                   const float* __restrict__ cut, const int* __restrict__ center, int n_local, int R, int Dh4,
+                                   uint32_t* __restrict__ mx) {
   const size_t t = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (t >= size_t(R) * Dh4) return;
   const int r = int(t / Dh4), q = int(t % Dh4);
@@ -442,8 +517,9 @@ __global__ void k_readout_seed_bwd(float* __restrict__ out, const float* __restr
   if (cut) seed = center[r] < n_local ? cut[r] : 0.f;
   else seed = r < n_local ? 1.f : 0.f;
   const float4 x = reinterpret_cast<const float4*>(pre)[t], ww = reinterpret_cast<const float4*>(w)[q];
-  reinterpret_cast<float4*>(out)[t] = make_float4(seed * ww.x * dsilu_f(x.x), seed * ww.y * dsilu_f(x.y),
-                                                  seed * ww.z * dsilu_f(x.z), seed * ww.w * dsilu_f(x.w));
+  const float4 v = make_float4(seed * ww.x * dsilu_f(x.x), seed * ww.y * dsilu_f(x.y), seed * ww.z * dsilu_f(x.z), seed * ww.w * dsilu_f(x.w));
+  reinterpret_cast<float4*>(out)[t] = v;
+  raise_row(mx, r, Dh4, max4(v));
 }
 
 __global__ void k_cutoff_share(float* __restrict__ cf_adj, const float* __restrict__ cfh, const float* __restrict__ cut, int N,
@@ -463,14 +539,16 @@ __global__ void k_add_inplace(float* __restrict__ a, const float* __restrict__ b
 }
 
 __global__ void k_message_average(float* __restrict__ ie, const float* __restrict__ oe, const int* __restrict__ rev, int E,
-                                  int D4, RemoteRows rm) {
+                                  int D4, RemoteRows rm, uint32_t* __restrict__ mx) {
   const size_t t = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (t >= size_t(E) * D4) return;
   const int k = int(t / D4), q = int(t % D4);
   float4 x = reinterpret_cast<float4*>(ie)[t];
   const float* pr = partner_row(oe, rev, rm, k, 4 * D4);
   const float4 y = pr ? ld4(pr + 4 * q) : make_float4(0, 0, 0, 0);
-  reinterpret_cast<float4*>(ie)[t] = make_float4(0.5f * (x.x + y.x), 0.5f * (x.y + y.y), 0.5f * (x.z + y.z), 0.5f * (x.w + y.w));
+  x = make_float4(0.5f * (x.x + y.x), 0.5f * (x.y + y.y), 0.5f * (x.z + y.z), 0.5f * (x.w + y.w));
+  reinterpret_cast<float4*>(ie)[t] = x;
+  raise_row(mx, k, D4, max4(x));
 }
 
 // The adjoint of message_average: ie_adj_out(k) = 0.5 ie_adj_in(k); oe_adj(k) += 0.5 ie_adj_in(rev k).
@@ -574,34 +652,34 @@ inline unsigned blocks_for(size_t n, int per) { return (unsigned) ((n + per - 1)
 
 }  // namespace
 
-void gather_rows(Stream& st, float* out, const float* table, const int* idx, int R, int D) {
+void gather_rows(Stream& st, float* out, const float* table, const int* idx, int R, int D, uint32_t* mx) {
   if (R == 0) return;
   const ProfScope ps(st, PC_GATHER, 0.0, 8.0 * double(R) * D);
-  k_gather_rows<<<blocks_for(size_t(R) * (D / 4), 256), 256, 0, st.s>>>(out, table, idx, R, D / 4);
+  k_gather_rows<<<blocks_for(size_t(R) * (D / 4), 256), 256, 0, st.s>>>(out, table, idx, R, D / 4, mx);
   PETB_LAUNCH_CHECK(st);
 }
 
 void compress0(Stream& st, float* out, float* pre, const float* b, const float* tab, const float* wx, const PackedEdges& pk,
-               int D) {
+               int D, uint32_t* mx) {
   if (pk.E == 0) return;
   const ProfScope ps(st, PC_ELEMENTWISE, 12.0 * double(pk.E) * D, 8.0 * double(pk.E) * D);
   GemmArgs p;
   p.M = pk.E, p.N = D, p.C = out, p.ldc = D, p.pre = pre, p.ldp = D, p.bias = b, p.tab = tab, p.wx = wx, p.sp = pk.species;
-  p.vec = pk.vec, p.dist = pk.dist, p.epi = EPI_COMPRESS;
+  p.vec = pk.vec, p.dist = pk.dist, p.c_max = mx, p.epi = EPI_COMPRESS;
   k_compress0<<<blocks_for(size_t(pk.E) * (D / 4), 256), 256, 0, st.s>>>(p);
   PETB_LAUNCH_CHECK(st);
 }
 
-void norm_fwd(Stream& st, float* out, float* in, const float* add, const float* w, const float* bias, int R, int D) {
+void norm_fwd(Stream& st, float* out, float* in, const float* add, const float* w, const float* bias, int R, int D, uint32_t* mx) {
   if (R == 0) return;
   const ProfScope ps(st, PC_NORM, 6.0 * double(R) * D, (add ? 16.0 : 8.0) * double(R) * D);
   const unsigned blocks = blocks_for(size_t(R) * 32, 256);
   switch (D) {  // whole rows in registers for the usual widths
-    case 128: k_norm_fwd_v<1><<<blocks, 256, 0, st.s>>>(out, in, add, w, bias, R); break;
-    case 256: k_norm_fwd_v<2><<<blocks, 256, 0, st.s>>>(out, in, add, w, bias, R); break;
-    case 512: k_norm_fwd_v<4><<<blocks, 256, 0, st.s>>>(out, in, add, w, bias, R); break;
-    case 1024: k_norm_fwd_v<8><<<blocks, 256, 0, st.s>>>(out, in, add, w, bias, R); break;
-    default: k_norm_fwd<<<blocks, 256, 0, st.s>>>(out, in, add, w, bias, R, D);
+    case 128: k_norm_fwd_v<1><<<blocks, 256, 0, st.s>>>(out, in, add, w, bias, R, mx); break;
+    case 256: k_norm_fwd_v<2><<<blocks, 256, 0, st.s>>>(out, in, add, w, bias, R, mx); break;
+    case 512: k_norm_fwd_v<4><<<blocks, 256, 0, st.s>>>(out, in, add, w, bias, R, mx); break;
+    case 1024: k_norm_fwd_v<8><<<blocks, 256, 0, st.s>>>(out, in, add, w, bias, R, mx); break;
+    default: k_norm_fwd<<<blocks, 256, 0, st.s>>>(out, in, add, w, bias, R, D, mx);
   }
   PETB_LAUNCH_CHECK(st);
 }
@@ -614,42 +692,42 @@ void gather_live(Stream& st, float* out, const float* src, int ld, int col0, con
 }
 
 void concat_norm_fwd(Stream& st, float* out, const float* oe, const int* rev, float* ie, const float* w, const float* bias,
-                     int E, int D, RemoteRows remote) {
+                     int E, int D, RemoteRows remote, uint32_t* mx) {
   if (E == 0) return;
   const ProfScope ps(st, PC_NORM, 12.0 * double(E) * D, 24.0 * double(E) * D);
-  k_concat_norm_fwd<<<blocks_for(size_t(E) * 32, 256), 256, 0, st.s>>>(out, oe, rev, ie, w, bias, E, D, remote);
+  k_concat_norm_fwd<<<blocks_for(size_t(E) * 32, 256), 256, 0, st.s>>>(out, oe, rev, ie, w, bias, E, D, remote, mx);
   PETB_LAUNCH_CHECK(st);
 }
 
 void norm_bwd(Stream& st, float* in_adj, const float* out_adj, const float* in, const float* w, bool layernorm, int R, int D,
-              int acc_row0, float* also) {
+              int acc_row0, float* also, uint32_t* mx) {
   if (R == 0) return;
   const ProfScope ps(st, PC_NORM, 10.0 * double(R) * D, (acc_row0 < R ? 16.0 : 12.0) * double(R) * D);
   const unsigned blocks = blocks_for(size_t(R) * 32, 256);
   switch (D) {
-    case 128: k_norm_bwd_v<1><<<blocks, 256, 0, st.s>>>(in_adj, out_adj, in, w, layernorm, R, acc_row0, also); break;
-    case 256: k_norm_bwd_v<2><<<blocks, 256, 0, st.s>>>(in_adj, out_adj, in, w, layernorm, R, acc_row0, also); break;
-    case 512: k_norm_bwd_v<4><<<blocks, 256, 0, st.s>>>(in_adj, out_adj, in, w, layernorm, R, acc_row0, also); break;
-    case 1024: k_norm_bwd_v<8><<<blocks, 256, 0, st.s>>>(in_adj, out_adj, in, w, layernorm, R, acc_row0, also); break;
-    default: k_norm_bwd<<<blocks, 256, 0, st.s>>>(in_adj, out_adj, in, w, layernorm, R, D, acc_row0, also);
+    case 128: k_norm_bwd_v<1><<<blocks, 256, 0, st.s>>>(in_adj, out_adj, in, w, layernorm, R, acc_row0, also, mx); break;
+    case 256: k_norm_bwd_v<2><<<blocks, 256, 0, st.s>>>(in_adj, out_adj, in, w, layernorm, R, acc_row0, also, mx); break;
+    case 512: k_norm_bwd_v<4><<<blocks, 256, 0, st.s>>>(in_adj, out_adj, in, w, layernorm, R, acc_row0, also, mx); break;
+    case 1024: k_norm_bwd_v<8><<<blocks, 256, 0, st.s>>>(in_adj, out_adj, in, w, layernorm, R, acc_row0, also, mx); break;
+    default: k_norm_bwd<<<blocks, 256, 0, st.s>>>(in_adj, out_adj, in, w, layernorm, R, D, acc_row0, also, mx);
   }
   PETB_LAUNCH_CHECK(st);
 }
 
 void concat_norm_bwd(Stream& st, float* edge_adj, const float* out_adj, const float* oe, const int* rev, const float* ie_adj,
-                     const float* w, int E, int D, RemoteRows remote, const float* remote_adj) {
+                     const float* w, int E, int D, RemoteRows remote, const float* remote_adj, uint32_t* mx) {
   if (E == 0) return;
   const ProfScope ps(st, PC_NORM, 20.0 * double(E) * D, 24.0 * double(E) * D);
   const auto grid = blocks_for(size_t(E) * 32, 256);
   const bool one_rank = !remote.of && !remote_adj;
   if (one_rank && D == 128)
-    k_concat_norm_bwd_pair<1><<<grid, 256, 0, st.s>>>(edge_adj, out_adj, oe, rev, ie_adj, w, E);
+    k_concat_norm_bwd_pair<1><<<grid, 256, 0, st.s>>>(edge_adj, out_adj, oe, rev, ie_adj, w, E, mx);
   else if (one_rank && D == 256)
-    k_concat_norm_bwd_pair<2><<<grid, 256, 0, st.s>>>(edge_adj, out_adj, oe, rev, ie_adj, w, E);
+    k_concat_norm_bwd_pair<2><<<grid, 256, 0, st.s>>>(edge_adj, out_adj, oe, rev, ie_adj, w, E, mx);
   else if (one_rank && D == 512)
-    k_concat_norm_bwd_pair<4><<<grid, 256, 0, st.s>>>(edge_adj, out_adj, oe, rev, ie_adj, w, E);
+    k_concat_norm_bwd_pair<4><<<grid, 256, 0, st.s>>>(edge_adj, out_adj, oe, rev, ie_adj, w, E, mx);
   else
-    k_concat_norm_bwd<<<grid, 256, 0, st.s>>>(edge_adj, out_adj, oe, rev, ie_adj, w, E, D, remote, remote_adj);
+    k_concat_norm_bwd<<<grid, 256, 0, st.s>>>(edge_adj, out_adj, oe, rev, ie_adj, w, E, D, remote, remote_adj, mx);
   PETB_LAUNCH_CHECK(st);
 }
 
@@ -679,10 +757,10 @@ void readout_energy(Stream& st, float* net, double* per_atom, const float* node_
 }
 
 void readout_seed_bwd(Stream& st, float* out, const float* w, const float* pre, const float* cut, const int* center,
-                      int n_local, int R, int Dh) {
+                      int n_local, int R, int Dh, uint32_t* mx) {
   if (R == 0) return;
   const ProfScope ps(st, PC_ELEMENTWISE, 8.0 * double(R) * Dh, 8.0 * double(R) * Dh);
-  k_readout_seed_bwd<<<blocks_for(size_t(R) * (Dh / 4), 256), 256, 0, st.s>>>(out, w, pre, cut, center, n_local, R, Dh / 4);
+  k_readout_seed_bwd<<<blocks_for(size_t(R) * (Dh / 4), 256), 256, 0, st.s>>>(out, w, pre, cut, center, n_local, R, Dh / 4, mx);
   PETB_LAUNCH_CHECK(st);
 }
 
@@ -700,10 +778,11 @@ void add_inplace(Stream& st, float* a, const float* b, size_t n) {
   PETB_LAUNCH_CHECK(st);
 }
 
-void message_average(Stream& st, float* ie, const float* oe, const int* rev, int E, int D, RemoteRows remote) {
+void message_average(Stream& st, float* ie, const float* oe, const int* rev, int E, int D, RemoteRows remote,
+                     uint32_t* mx) {
   if (E == 0) return;
   const ProfScope ps(st, PC_GATHER, 2.0 * double(E) * D, 12.0 * double(E) * D);
-  k_message_average<<<blocks_for(size_t(E) * (D / 4), 256), 256, 0, st.s>>>(ie, oe, rev, E, D / 4, remote);
+  k_message_average<<<blocks_for(size_t(E) * (D / 4), 256), 256, 0, st.s>>>(ie, oe, rev, E, D / 4, remote, mx);
   PETB_LAUNCH_CHECK(st);
 }
 

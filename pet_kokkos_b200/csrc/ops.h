@@ -1,7 +1,8 @@
 // The network's non-GEMM passes: lookups, norms (forward and backward, with the
 // gathers and residual sums that ride along), compress.0's folded terms, the
 // readout's ordered sums and the geometry end of the backward. Each names the
-// reference pass it stands for.
+// reference pass it stands for. `mx`, where a pass takes one and unless null, receives the bits of each output row's
+// largest magnitude, for the GEMM that reads the rows (zeroed by the caller).
 #pragma once
 
 #include "common.h"
@@ -10,14 +11,15 @@
 namespace petb {
 
 // out(r,:) = table(idx(r),:)   (gather, src/ops.cpp:109-114)
-void gather_rows(Stream& st, float* out, const float* table, const int* idx, int R, int D);
+void gather_rows(Stream& st, float* out, const float* table, const int* idx, int R, int D, uint32_t* mx = nullptr);
 
 // Layer 0's compress.0: pre = b + tab[species] + wx.(v,|v|); out = silu(pre)  (compress_fwd without a GEMM, src/ops.cpp:326-365)
 void compress0(Stream& st, float* out, float* pre, const float* b, const float* tab, const float* wx, const PackedEdges& pk,
-               int D);
+               int D, uint32_t* mx = nullptr);
 
 // out = norm(in [+ add, stored back into in]); RMSNorm when bias is null, else LayerNorm  (norm_rows, src/ops.hpp:381-401)
-void norm_fwd(Stream& st, float* out, float* in, const float* add, const float* w, const float* bias, int R, int D);
+void norm_fwd(Stream& st, float* out, float* in, const float* add, const float* w, const float* bias, int R, int D,
+              uint32_t* mx = nullptr);
 
 // Partner rows that live on another rank (an exchanged list): edge k's partner row is rows[of[k]] when its local
 // partner is missing and of[k] >= 0. All null without an exchange.
@@ -32,18 +34,18 @@ void gather_live(Stream& st, float* out, const float* src, int ld, int col0, con
 // The combination norm with its gather: row k of the input is [oe(k) | oe(rev k), the remote partner's row, or 0];
 // ie(k) += oe(k) on the way  (src/feedforward.cpp:182-193)
 void concat_norm_fwd(Stream& st, float* out, const float* oe, const int* rev, float* ie, const float* w, const float* bias,
-                     int E, int D, RemoteRows remote = {});
+                     int E, int D, RemoteRows remote = {}, uint32_t* mx = nullptr);
 
 // in_adj = g for rows < acc_row0, in_adj += g for the rest; g the norm's input adjoint
 // (norm_rows_bwd, src/ops.hpp:404-436). `also`, unless null, receives a copy of the result.
 void norm_bwd(Stream& st, float* in_adj, const float* out_adj, const float* in, const float* w, bool layernorm, int R, int D,
-              int acc_row0, float* also = nullptr);
+              int acc_row0, float* also = nullptr, uint32_t* mx = nullptr);
 
 // edge_adj(k) = ie_adj(k) + g(k)[:D] + g(rev k)[D:], g from out_adj [E,2D]  (concat_norm_bwd, src/ops.cpp:191-244)
 // With an exchange: `remote` holds the partner rows the forward read, `remote_adj` the partners' adjoints of this
 // rank's rows (what concat_norm_remote_bwd computed on the other side).
 void concat_norm_bwd(Stream& st, float* edge_adj, const float* out_adj, const float* oe, const int* rev, const float* ie_adj,
-                     const float* w, int E, int D, RemoteRows remote = {}, const float* remote_adj = nullptr);
+                     const float* w, int E, int D, RemoteRows remote = {}, const float* remote_adj = nullptr, uint32_t* mx = nullptr);
 // send(l, :) = the adjoint of the partner row that live edge l read: g(live_packed[l])[D:]  (src/feedforward.cpp:246-255)
 void concat_norm_remote_bwd(Stream& st, float* send, const float* out_adj, const float* oe, const float* w,
                             const int* live_packed, int n_live, int D, RemoteRows remote);
@@ -59,7 +61,7 @@ void readout_energy(Stream& st, float* net, double* per_atom, const float* node_
 // out(r,j) = seed(r) * w(j) * silu'(pre(r,j)); seed is 1 for rows < n_one when cut is null, else cut(r) for rows
 // whose centre is owned  (the seeds of readout_bwd fused with its first linear_silu_bwd, src/model.cpp:749-778)
 void readout_seed_bwd(Stream& st, float* out, const float* w, const float* pre, const float* cut, const int* center,
-                      int n_local, int R, int Dh);
+                      int n_local, int R, int Dh, uint32_t* mx = nullptr);
 
 // cf_adj(k) += (sum_h cfh(N+k,h)) / cut(k)  (attn_bwd_cf, src/attention.cpp:1829-1838; only edge slots carry a gradient)
 void cutoff_share(Stream& st, float* cf_adj, const float* cfh, const float* cut, int N, int E, int H);
@@ -67,7 +69,8 @@ void cutoff_share(Stream& st, float* cf_adj, const float* cfh, const float* cut,
 // a += b, elementwise
 void add_inplace(Stream& st, float* a, const float* b, size_t n);
 // input_edge(k) = 0.5 (input_edge(k) + oe(rev k) or 0)  (re_msg, src/residual.cpp:123-132)
-void message_average(Stream& st, float* ie, const float* oe, const int* rev, int E, int D, RemoteRows remote = {});
+void message_average(Stream& st, float* ie, const float* oe, const int* rev, int E, int D, RemoteRows remote = {},
+                     uint32_t* mx = nullptr);
 // With an exchange, `remote_adj` holds the partners' ie_adj_in rows (src/residual.cpp:189).
 void message_average_bwd(Stream& st, float* ie_adj_out, float* oe_adj, const float* ie_adj_in, const int* rev, int E, int D,
                          RemoteRows remote_adj = {});

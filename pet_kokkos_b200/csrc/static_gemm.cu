@@ -97,7 +97,7 @@ extern "C" int pet_gemm_host_static(int m, int n, int k, const float* A, const f
     // (no accumulation onto old values), so nothing needs clearing first.
     petb::GemmArgs a;
     a.A = dA, a.lda = k, a.B = dW, a.ldb = k, a.C = dC, a.ldc = n, a.M = m, a.N = n, a.K = k;
-    petb::gemm(st, unused, a, petb::GEMM_NATIVE);
+    petb::gemm(st, unused, a);  // no packed weight: the CUDA cores
     PETB_CUDA(cudaMemcpyAsync(C, dC, sizeof(float) * size_t(m) * n, cudaMemcpyDeviceToHost, st.s));
     PETB_CUDA(cudaStreamSynchronize(st.s));
   } catch (const petb::Error& err) {
