@@ -8,7 +8,16 @@
 
 namespace petb {
 
-__device__ __forceinline__ float sigmoid_f(float x) { return 1.0f / (1.0f + expf(-x)); }
+// 1 / (1 + exp(-x)), the reciprocal from the hardware's estimate (within 1 ulp) and one Newton-Raphson step, which leaves
+// the rounding of its last fma: 1.3 ulp at most with expf's own error, the quotient's 1.3. The quotient compiles into a
+// call that spends 140 clocks an element in a GEMM's epilogue, this into a dozen instructions that overlap. The argument
+// is bounded where the estimate of the reciprocal would no longer be a normal number (sigmoid(-87) = 1.6e-38).
+__device__ __forceinline__ float sigmoid_f(float x) {
+  const float d = 1.0f + expf(fminf(-x, 87.0f));
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+  return fmaf(r, fmaf(-d, r, 1.0f), r);
+}
 __device__ __forceinline__ float silu_f(float x) { return x * sigmoid_f(x); }
 // d silu / dx = s (1 + x (1 - s))
 __device__ __forceinline__ float dsilu_f(float x) {
