@@ -4,12 +4,12 @@
 // A persistent kernel, one CTA per SM, each walking 128 x BN tiles of C = A . B^T (A [M,K] fp32, B [N,K] a packed
 // weight) in an N-fastest order so that CTAs running side by side share their A rows in L2. K goes by steps of 32
 // columns (FMT_TF32X2: 16). Roles, by warp:
-//   warp 0      producer of A: one thread issues TMA loads of 128 x 32 fp32 slabs (128-byte rows, 128-byte swizzle) into a
+//   warp 0      producer of A: one lane issues TMA loads of 128 x 32 fp32 slabs (128-byte rows, 128-byte swizzle) into a
 //               ring of slots; warp 2 the same for B's tiles, which arrive as 16-bit parts;
-//   warps 12-15 converter: a thread takes one row's 128 bytes out of a landed slot, scales and splits it and writes the
+//   warps 12-15 converter: a lane takes one row's 128 bytes out of a landed slot, scales and splits it and writes the
 //               parts back into the same 128 bytes (64 bytes a part; FMT_F16X3's third part into a tile of its own): a slot costs no second copy of A. The fp32 activations are read from memory once;
-//   warp 1      issuer: one thread issues the products (M = 128, N = BN, K = 16 each) into one of TWO accumulators in
-//               tensor memory, small terms first, and frees the slots with tcgen05.commit;
+//   warp 1      issuer: one lane issues the products (M = 128, N = BN, K = 16 each) into one of TWO accumulators in
+//               tensor memory, small terms first, and frees the step's slots with one tcgen05.commit;
 //   warps 4-11  epilogue: tcgen05.ld the accumulator (a thread owns a row, a warp pair splits the columns), undo the
 //               row's and the weight's scale, and work through 32 x 32 chunks in shared memory: what the epilogue reads (a
 //               residual, a saved pre-activation) is brought there by TMA a chunk ahead, what it writes leaves by TMA. The
@@ -20,6 +20,12 @@
 // and over a network (two truncations per 32 columns were enough to move energies by 1e-6). The h.h sums have no such
 // bits, and the small products' truncations are 2^-8 of what they would be there. setmaxnreg moves the registers the sums
 // take from the producers' and converters' warp groups.
+// Large GEMMs in the formats of several parts run on pairs of CTAs (cta_group::2): 256 x 256 tiles, each CTA with 128 rows of
+// A and half of the weight's tile in its shared memory, its own converter and epilogue, one issuer for both. A CTA's
+// converter tells the issuer that a step's operands are complete by an arrival on its barrier across the cluster, without a
+// cluster-scope release: that one (or an acquire on the waiting side) costs 2500 clocks a step. The converter's own writes
+// are ordered by the proxy fence before the arrival, and nothing but the tensor core reads them.
+//
 // What bounds it: the SM's shared-memory data path (one 128-byte wavefront per clock for TMA traffic, the tensor core's
 // operand reads, the converter and the epilogue). Wavefronts per 8 columns of K of a 128 x 256 tile, K = 256: FMT_F16X2
 // operand reads 144, fills 96, converter 64, epilogue 64-128 = about 370-430 against 192 clocks of MMA; FMT_F16X3 288, 128,
@@ -91,26 +97,33 @@ __device__ __forceinline__ float tf32_low(float x) {
   return __uint_as_float(__float_as_uint(x - __uint_as_float(__float_as_uint(x) & 0xFFFFE000u)) + 0x1000u);
 }
 
-template <int BN, int FMT>
+template <int BN, int FMT, bool PAIR>
 struct Tile {
   static constexpr bool X3 = FMT == FMT_F16X3, X2 = FMT == FMT_F16X2, T2 = FMT == FMT_TF32X2, T1 = FMT == FMT_TF32;
   static constexpr bool kScaled = FMT == FMT_F16X3 || FMT == FMT_F16X2 || FMT == FMT_F16;
   static constexpr int BK = T2 ? 16 : 32;                                   // columns of K of a step
   static constexpr int kSlab = TBM * BK * 4;                                // A as it lands
   static constexpr int kA = kSlab + (X3 || T2 ? TBM * 64 : 0);              // the fp32 slab, then its parts; l behind it
-  static constexpr int kB = BN * (X3 ? 192 : X2 || T2 || T1 ? 128 : 64);          // [h | m] or [h | l] rows of 128 bytes (then l), or rows of 64
+  static constexpr int kRowsB = PAIR ? BN / 2 : BN;                         // of B's tile, in this CTA
+  static constexpr int kB = kRowsB * (X3 ? 192 : X2 || T2 || T1 ? 128 : 64);          // [h | m] or [h | l] rows of 128 bytes (then l), or rows of 64
   // An epilogue warp's two buffers of 32 rows x kWide columns; half as wide where the rings need the room.
   static constexpr int kWide = X3 ? 16 : 32;
   static constexpr int kBuf = 32 * kWide * 4;
   static constexpr int kEpi = kEpiWarps * 2 * kBuf;
   static constexpr int kBars = 640;
   // Slots: as many as shared memory has room for beside the epilogue's buffers, at most eight of each; of A, whose bytes come
-  // from HBM, no fewer than of B, whose bytes sit in L2.
+  // from HBM, no fewer than of B, whose bytes sit in L2; of A an even number, for the converter's groups.
   static constexpr int kRoom = 227 * 1024 - kEpi - 1024 - kBars;
-  static constexpr int kBoth = kRoom / (kA + kB);
-  static constexpr int NB = kBoth > 8 ? 8 : kBoth;
-  static constexpr int kMoreA = NB + (kRoom - NB * (kA + kB)) / kA;
-  static constexpr int NA = kMoreA > 8 ? 8 : kMoreA;
+  static constexpr int least(int a, int b) { return a < b ? a : b; }
+  static constexpr int slots_a(int nb) { return least(8, (kRoom - nb * kB) / kA); }
+  static constexpr int kBoth = least(8, kRoom / (kA + kB));
+  static constexpr bool kTrade = slots_a(kBoth) % 2 != 0 && slots_a(kBoth - 1) % 2 == 0;  // one of B's for one more of A's
+  static constexpr int NA = slots_a(kTrade ? kBoth - 1 : kBoth) / 2 * 2, NB = least(kTrade ? kBoth - 1 : kBoth, NA);
+  // The converter's warps work in groups on slots of their own: a slot takes a warp about a thousand clocks however few
+  // instructions its rows need (the wait, the loads, the fence), so two or four of them have to be under way at once. A
+  // slot always falls to the same group (NA a multiple of the groups): a group that met a slot's barrier only every other
+  // round could take the round before last for the one it waits for.
+  static constexpr int kGroups = NA % 4 == 0 && NA >= 8 ? 4 : 2;
   static constexpr int kRings = NA * kA + NB * kB;
   static constexpr int kTotal = kRings + kEpi + 1024 /*alignment slack*/ + kBars;
   static constexpr int kThreads = 512;
@@ -121,8 +134,8 @@ struct Tile {
   static constexpr int kAccs = X3 ? 2 : 1, kTurns = 512 / (kAccs * BN) >= 2 ? 2 : 1, kColumns = kTurns * kAccs * BN;
   static constexpr int kDrain = X3 ? 1024 / BK : 1 << 30;  // steps whose h.h products sum exactly
   static constexpr bool kMoveRegs = X3 && BN >= 128;
-  static_assert(NA >= 2 && NB >= 2, "two slots of each at least");
-  static_assert((3 * NA + 2 * NB + 4 + 2 * kEpiWarps) * 8 + 8 <= kBars, "the barriers");
+  static_assert(NA >= NB && NB >= 2 && NA % kGroups == 0, "the slots");
+  static_assert((3 * NA + 4 + 2 * kEpiWarps) * 8 + 8 <= kBars, "the barriers");
 };
 
 // ---- the epilogue ---------------------------------------------------------------------------
@@ -218,147 +231,167 @@ __device__ __forceinline__ void chunk_get(const uint8_t* tile, int r, float* x) 
   }
 }
 
-template <int EPI, int BN, int FMT>
-__global__ void __launch_bounds__(Tile<BN, FMT>::kThreads, 1)
+template <int EPI, int BN, int FMT, bool PAIR>
+__global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1)
     k_gemm_tc(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
               const __grid_constant__ CUtensorMap map_blo, const __grid_constant__ CUtensorMap map_in,
               const __grid_constant__ CUtensorMap map_c, const __grid_constant__ CUtensorMap map_pre,
               const __grid_constant__ GemmArgs p, const uint32_t* b_max, int* err) {
-  using L = Tile<BN, FMT>;
+  using L = Tile<BN, FMT, PAIR>;
   constexpr int NA = L::NA, NB = L::NB;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* ring_a = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* ring_b = ring_a + NA * L::kA;
   uint8_t* epi = ring_a + L::kRings;
-  uint64_t* full_a = reinterpret_cast<uint64_t*>(epi + L::kEpi);  // [NA] the fp32 slab has landed
-  uint64_t* conv_a = full_a + NA;   // [NA] it has been split
-  uint64_t* empty_a = conv_a + NA;  // [NA] its products are done
-  uint64_t* full_b = empty_a + NA;  // [NB]
-  uint64_t* empty_b = full_b + NB;  // [NB]
-  uint64_t* tfull = empty_b + NB;   // [2] accumulator complete
+  // Barriers of a step, in a ring as long as A's (B's is no longer, so a barrier's phase is over before B's next use of it).
+  // In a pair, `ready` and `tempty` are the leader's (rank 0), whose warp 1 issues the products of both; the commits of
+  // those arrive in both CTAs.
+  uint64_t* full_a = reinterpret_cast<uint64_t*>(epi + L::kEpi);  // [NA] the fp32 slab has landed (pair: and B's tile)
+  uint64_t* ready = full_a + NA;    // [NA] it has been split and B's tile has landed (FMT_TF32: both have landed)
+  uint64_t* done = ready + NA;      // [NA] the step's products are done
+  uint64_t* tfull = done + NA;      // [2] accumulator complete
   uint64_t* tempty = tfull + 2;     // [2] accumulator read back
   uint64_t* landed = tempty + 2;    // [kEpiWarps][2] an epilogue warp's chunk has landed
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(landed + 2 * kEpiWarps);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int tiles_n = (p.N + BN - 1) / BN, tiles_m = (p.M + TBM - 1) / TBM;
-  const int n_tiles = tiles_m * tiles_n;
+  // A pair walks tiles of 2 x 128 rows: its CTAs take 128 each, and half of B's rows each.
+  constexpr int CTAS = PAIR ? 2 : 1;
+  const int rank = PAIR ? int(cluster_ctarank()) : 0;
+  const int tiles_n = (p.N + BN - 1) / BN, tiles_m = (p.M + CTAS * TBM - 1) / (CTAS * TBM);
+  const int n_tiles = tiles_m * tiles_n, tile0 = blockIdx.x / CTAS, tile_step = gridDim.x / CTAS;
+  auto first_row = [&](int t) { return ((t / tiles_n) * CTAS + rank) * TBM; };
   constexpr int TBK = L::BK;
   const int nkb = (p.K + TBK - 1) / TBK;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < NA; ++s) mbar_init(full_a + s, 1), mbar_init(conv_a + s, 4), mbar_init(empty_a + s, 1);
-    for (int s = 0; s < NB; ++s) mbar_init(full_b + s, 1), mbar_init(empty_b + s, 1);
-    for (int b = 0; b < 2; ++b) mbar_init(tfull + b, 1), mbar_init(tempty + b, kEpiWarps);
+    for (int s = 0; s < NA; ++s) {
+      mbar_init(full_a + s, CTAS), mbar_init(ready + s, PAIR ? 2 * (4 / L::kGroups) : 1 + (L::T1 ? 1 : 4 / L::kGroups));
+      mbar_init(done + s, 1);
+    }
+    for (int b = 0; b < 2; ++b) mbar_init(tfull + b, 1), mbar_init(tempty + b, CTAS * kEpiWarps);
     for (int b = 0; b < 2 * kEpiWarps; ++b) mbar_init(landed + b, 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 1) {  // tensor memory: accumulators of BN fp32 columns x 128 lanes
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(L::kColumns) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
+  if (warp == 1) tmem_alloc<PAIR>(tmem_slot, L::kColumns);  // accumulators of BN fp32 columns x 128 lanes
   tcgen05_fence_before();
   __syncthreads();
+  if (PAIR) cluster_sync_all();  // the other CTA's barriers exist before anything signals them
   tcgen05_fence_after();
   const uint32_t tmem = *tmem_slot;
 
   if (warp < 4) {
-    // 40 + 208 + 208 + 56 registers a thread over the four warp groups are the 4 x 128 of the launch
-    if (L::kMoveRegs) asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
-    if (warp == 0 && lane == 0) {
-      int g = 0;  // steps issued so far, across tiles
-      bool ok = true;
-      for (int t = blockIdx.x; ok && t < n_tiles; t += gridDim.x) {
-        const int m0 = (t / tiles_n) * TBM;
-        for (int kb = 0; kb < nkb; ++kb, ++g) {
-          const int s = g % NA;
-          if (!(ok = mbar_wait(empty_a + s, ((g / NA) & 1) ^ 1, abort_flag))) break;
-          mbar_expect_tx(full_a + s, L::kSlab);
-          tma_load_2d(ring_a + s * L::kA, &map_a, full_a + s, kb * TBK, m0);
-        }
-      }
-    } else if (warp == 2 && lane == 0) {
-      int g = 0;
-      bool ok = true;
-      for (int t = blockIdx.x; ok && t < n_tiles; t += gridDim.x) {
-        const int n0 = (t % tiles_n) * BN;
-        for (int kb = 0; kb < nkb; ++kb, ++g) {
-          const int s = g % NB;
-          if (!(ok = mbar_wait(empty_b + s, ((g / NB) & 1) ^ 1, abort_flag))) break;
-          uint8_t* dst = ring_b + s * L::kB;
-          mbar_expect_tx(full_b + s, L::kB);
-          if (L::X3 || L::X2) {
-            tma_load_2d(dst, &map_b, full_b + s, kb * 64, n0);
-            if (L::X3) tma_load_2d(dst + BN * 128, &map_blo, full_b + s, kb * TBK, n0);
-          } else {
-            tma_load_2d(dst, &map_b, full_b + s, kb * TBK, n0);
-            if (L::T2) tma_load_2d(dst + BN * 64, &map_blo, full_b + s, kb * TBK, n0);
+    // 24 + 200 + 200 + 88 registers a thread over the four warp groups are the 4 x 128 of the launch
+    if (L::kMoveRegs) asm volatile("setmaxnreg.dec.sync.aligned.u32 24;");
+    // Each of the three roles is a whole warp's loop with one lane's instructions. `s` is the step's slot in its ring, `turn`
+    // the parity of the ring's round.
+    const bool one = elect_one();
+    bool ok = true;
+    if (warp == 0) {
+      int s = 0;
+      uint32_t turn = 0;
+      for (int t = tile0; ok && t < n_tiles; t += tile_step) {
+        const int m0 = first_row(t);
+        for (int kb = 0; kb < nkb; ++kb) {
+          if (!(ok = mbar_wait_warp(done + s, turn ^ 1, abort_flag))) break;
+          if (one) {
+            uint64_t* bar = L::T1 && !PAIR ? ready + s : full_a + s;
+            mbar_expect_tx(bar, L::kSlab);
+            tma_load_2d(ring_a + s * L::kA, &map_a, bar, kb * TBK, m0);
           }
+          if (++s == NA) s = 0, turn ^= 1;
         }
       }
-    } else if (warp == 1 && lane == 0) {
-      constexpr uint32_t idesc = L::T2 || L::T1 ? idesc_tf32(TBM, BN) : idesc_f16(TBM, BN, FMT == FMT_BF16);
-      int g = 0, i = 0;  // steps, accumulators handed over
-      bool ok = true;
-      for (int t = blockIdx.x; ok && t < n_tiles; t += gridDim.x) {
+    } else if (warp == 2) {
+      int s = 0, sb = 0, g = 0;  // the step's barrier, B's slot, steps so far
+      for (int t = tile0; ok && t < n_tiles; t += tile_step) {
+        const int n0 = (t % tiles_n) * BN + rank * L::kRowsB;
         for (int kb = 0; kb < nkb; ++kb, ++g) {
+          // the step that used this slot before, NB steps ago, has its barrier at (g - NB) % NA
+          if (g >= NB && !(ok = mbar_wait_warp(done + (g - NB) % NA, ((g - NB) / NA) & 1, abort_flag))) break;
+          if (one) {
+            uint8_t* dst = ring_b + sb * L::kB;
+            uint64_t* bar = PAIR ? full_a + s : ready + s;
+            mbar_expect_tx(bar, L::kB);
+            if (L::X3 || L::X2) {
+              tma_load_2d(dst, &map_b, bar, kb * 64, n0);
+              if (L::X3) tma_load_2d(dst + L::kRowsB * 128, &map_blo, bar, kb * TBK, n0);
+            } else {
+              tma_load_2d(dst, &map_b, bar, kb * TBK, n0);
+              if (L::T2) tma_load_2d(dst + L::kRowsB * 64, &map_blo, bar, kb * TBK, n0);
+            }
+          }
+          if (++s == NA) s = 0;
+          if (++sb == NB) sb = 0;
+        }
+      }
+    } else if (warp == 1 && rank == 0) {
+      constexpr uint32_t idesc = L::T2 || L::T1 ? idesc_tf32(CTAS * TBM, BN) : idesc_f16(CTAS * TBM, BN, FMT == FMT_BF16);
+      int s = 0, sb = 0, i = 0;  // the slots, accumulators handed over
+      uint32_t turn = 0;
+      for (int t = tile0; ok && t < n_tiles; t += tile_step) {
+        for (int kb = 0; kb < nkb; ++kb) {
           const bool first = kb % L::kDrain == 0, last = kb + 1 == nkb || (kb + 1) % L::kDrain == 0;
-          const int b = i % L::kTurns, sa = g % NA, sb = g % NB;
-          if (first && !(ok = mbar_wait(tempty + b, ((i / L::kTurns) & 1) ^ 1, abort_flag))) break;
-          if (!(ok = mbar_wait(full_b + sb, (g / NB) & 1, abort_flag))) break;
-          if (!(ok = mbar_wait(L::T1 ? full_a + sa : conv_a + sa, (g / NA) & 1, abort_flag))) break;
+          const int b = i % L::kTurns;
+          if (first && !(ok = mbar_wait_warp(tempty + b, ((i / L::kTurns) & 1) ^ 1, abort_flag))) break;
+          if (!(ok = mbar_wait_warp(ready + s, turn, abort_flag))) break;
           tcgen05_fence_after();
-          const uint32_t acc = tmem + uint32_t(b * L::kAccs * BN);
-          const uint32_t a0 = smem_u32(ring_a + sa * L::kA), b0 = smem_u32(ring_b + sb * L::kB);
-          const uint64_t ah = smem_desc<128>(a0), am = smem_desc<128>(a0 + 64);  // h and the part beside it
-          if (L::X3) {
-            const uint64_t al = smem_desc<64>(a0 + TBM * 128), bh = smem_desc<128>(b0), bm = smem_desc<128>(b0 + 64),
-                           bl = smem_desc<64>(b0 + BN * 128);
-            const uint32_t small = acc + BN;
+          if (one) {
+            const uint32_t acc = tmem + uint32_t(b * L::kAccs * BN);
+            const uint32_t a0 = smem_u32(ring_a + s * L::kA), b0 = smem_u32(ring_b + sb * L::kB);
+            const uint64_t ah = smem_desc<128>(a0), am = smem_desc<128>(a0 + 64);  // h and the part beside it
+            if (L::X3) {
+              const uint64_t al = smem_desc<64>(a0 + TBM * 128), bh = smem_desc<128>(b0), bm = smem_desc<128>(b0 + 64),
+                             bl = smem_desc<64>(b0 + L::kRowsB * 128);
+              const uint32_t small = acc + BN;
 #pragma unroll
-            for (int k = 0; k < 4; k += 2) {  // 16 columns are 32 bytes: 2 in the descriptors' 16-byte units
-              mma_f16(small, ah + k, bl + k, idesc, !first || k != 0);
-              mma_f16(small, al + k, bh + k, idesc, 1);
-              mma_f16(small, am + k, bm + k, idesc, 1);
-              mma_f16(small, ah + k, bm + k, idesc, 1);
-              mma_f16(small, am + k, bh + k, idesc, 1);
-              mma_f16(acc, ah + k, bh + k, idesc, !first || k != 0);
+              for (int k = 0; k < 4; k += 2) {  // 16 columns are 32 bytes: 2 in the descriptors' 16-byte units
+                mma_f16<PAIR>(small, ah + k, bl + k, idesc, !first || k != 0);
+                mma_f16<PAIR>(small, al + k, bh + k, idesc, 1);
+                mma_f16<PAIR>(small, am + k, bm + k, idesc, 1);
+                mma_f16<PAIR>(small, ah + k, bm + k, idesc, 1);
+                mma_f16<PAIR>(small, am + k, bh + k, idesc, 1);
+                mma_f16<PAIR>(acc, ah + k, bh + k, idesc, !first || k != 0);
+              }
+            } else if (L::X2) {
+              const uint64_t bh = smem_desc<128>(b0), bl = smem_desc<128>(b0 + 64);
+#pragma unroll
+              for (int k = 0; k < 4; k += 2) {
+                mma_f16<PAIR>(acc, ah + k, bl + k, idesc, kb != 0 || k != 0);
+                mma_f16<PAIR>(acc, am + k, bh + k, idesc, 1);
+                mma_f16<PAIR>(acc, ah + k, bh + k, idesc, 1);
+              }
+            } else if (L::T2) {
+              const uint64_t th = smem_desc<64>(a0), tl = smem_desc<64>(a0 + L::kSlab), bh = smem_desc<64>(b0), bl = smem_desc<64>(b0 + L::kRowsB * 64);
+#pragma unroll
+              for (int k = 0; k < 4; k += 2) {  // 8 columns are 32 bytes
+                mma_tf32<PAIR>(acc, th + k, bl + k, idesc, kb != 0 || k != 0);
+                mma_tf32<PAIR>(acc, tl + k, bh + k, idesc, 1);
+                mma_tf32<PAIR>(acc, th + k, bh + k, idesc, 1);
+              }
+            } else if (L::T1) {
+              const uint64_t bh = smem_desc<128>(b0);
+#pragma unroll
+              for (int k = 0; k < 8; k += 2) mma_tf32<PAIR>(acc, ah + k, bh + k, idesc, kb != 0 || k != 0);
+            } else {
+              const uint64_t bh = smem_desc<64>(b0);
+#pragma unroll
+              for (int k = 0; k < 4; k += 2) mma_f16<PAIR>(acc, ah + k, bh + k, idesc, kb != 0 || k != 0);
             }
-          } else if (L::X2) {
-            const uint64_t bh = smem_desc<128>(b0), bl = smem_desc<128>(b0 + 64);
-#pragma unroll
-            for (int k = 0; k < 4; k += 2) {
-              mma_f16(acc, ah + k, bl + k, idesc, kb != 0 || k != 0);
-              mma_f16(acc, am + k, bh + k, idesc, 1);
-              mma_f16(acc, ah + k, bh + k, idesc, 1);
-            }
-          } else if (L::T2) {
-            const uint64_t th = smem_desc<64>(a0), tl = smem_desc<64>(a0 + L::kSlab), bh = smem_desc<64>(b0), bl = smem_desc<64>(b0 + BN * 64);
-#pragma unroll
-            for (int k = 0; k < 4; k += 2) {  // 8 columns are 32 bytes
-              mma_tf32(acc, th + k, bl + k, idesc, kb != 0 || k != 0);
-              mma_tf32(acc, tl + k, bh + k, idesc, 1);
-              mma_tf32(acc, th + k, bh + k, idesc, 1);
-            }
-          } else if (L::T1) {
-            const uint64_t bh = smem_desc<128>(b0);
-#pragma unroll
-            for (int k = 0; k < 8; k += 2) mma_tf32(acc, ah + k, bh + k, idesc, kb != 0 || k != 0);
-          } else {
-            const uint64_t bh = smem_desc<64>(b0);
-#pragma unroll
-            for (int k = 0; k < 4; k += 2) mma_f16(acc, ah + k, bh + k, idesc, kb != 0 || k != 0);
+            mma_commit<PAIR>(done + s);
+            if (last) mma_commit<PAIR>(tfull + b);
           }
-          mma_commit(empty_a + sa);
-          mma_commit(empty_b + sb);
-          if (last) mma_commit(tfull + b), ++i;
+          __syncwarp();
+          i += last;
+          if (++s == NA) s = 0, turn ^= 1;
+          if (++sb == NB) sb = 0;
         }
       }
     }
   } else if (warp < kConvWarp0) {
-    if (L::kMoveRegs) asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");
+    if (L::kMoveRegs) asm volatile("setmaxnreg.inc.sync.aligned.u32 200;");
     const int ew = warp - kEpiWarp0;
     const int q = warp & 3;          // the quarter of the 128 lanes this warp may read
     const int half = ew >> 2;        // which half of the BN columns
@@ -372,17 +405,25 @@ __global__ void __launch_bounds__(Tile<BN, FMT>::kThreads, 1)
     auto chunks_of = [&](int t) { return max(0, min(BN / 2 / AC, (p.N - first_col(t) + AC - 1) / AC)); };
     auto ask = [&](int t, int c, int k) {  // lane 0: chunk c of tile t, the k-th this warp reads, into buffer k & 1
       mbar_expect_tx(bar + (k & 1), L::kBuf);
-      tma_load_2d(buf + (k & 1) * L::kBuf, &map_in, bar + (k & 1), (first_col(t) + c * AC) * (W / AC), (t / tiles_n) * TBM + q * 32);
+      tma_load_2d(buf + (k & 1) * L::kBuf, &map_in, bar + (k & 1), (first_col(t) + c * AC) * (W / AC), first_row(t) + q * 32);
+    };
+    auto release = [&](int b) {  // the accumulators of turn b have been read: the issuer may reuse them
+      tcgen05_fence_before();
+      __syncwarp();
+      if (lane == 0) {
+        if (PAIR) mbar_arrive_at(tempty + b, 0);
+        else mbar_arrive(tempty + b);
+      }
     };
     int i = 0, k = 0;  // accumulators and chunks so far
     bool ok = true;
     if (has_in && lane == 0) {
-      int t = blockIdx.x;
-      while (t < n_tiles && chunks_of(t) == 0) t += gridDim.x;
+      int t = tile0;
+      while (t < n_tiles && chunks_of(t) == 0) t += tile_step;
       if (t < n_tiles) ask(t, 0, 0);
     }
-    for (int t = blockIdx.x; ok && t < n_tiles; t += gridDim.x) {
-      const int r0 = (t / tiles_n) * TBM + q * 32, row = r0 + lane, n0 = first_col(t), nc = chunks_of(t);
+    for (int t = tile0; ok && t < n_tiles; t += tile_step) {
+      const int r0 = first_row(t) + q * 32, row = r0 + lane, n0 = first_col(t), nc = chunks_of(t);
       if (reads(EPI)) epilogue_prefetch<EPI>(p, row, n0, BN / 2);
       float unscale = 1.f, big = 0.f;
       RowTerms rt{};
@@ -402,7 +443,7 @@ __global__ void __launch_bounds__(Tile<BN, FMT>::kThreads, 1)
       if (L::X3) {
         for (int kb = 0; kb < nkb; kb += L::kDrain, ++i) {
           const int b = i % L::kTurns;
-          if (!(ok = __all_sync(0xffffffffu, mbar_wait(tfull + b, (i / L::kTurns) & 1, abort_flag)))) break;
+          if (!(ok = mbar_wait_warp(tfull + b, (i / L::kTurns) & 1, abort_flag))) break;
           tcgen05_fence_after();
           acc = accumulator(b);
 #pragma unroll
@@ -417,14 +458,12 @@ __global__ void __launch_bounds__(Tile<BN, FMT>::kThreads, 1)
               sum[(c + j) % L::kSums] = kb == 0 ? v : sum[(c + j) % L::kSums] + v;
             }
           }
-          tcgen05_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(tempty + b);
+          release(b);
         }
         if (!ok) break;
       } else {
         const int b = i % L::kTurns;
-        if (!(ok = __all_sync(0xffffffffu, mbar_wait(tfull + b, (i / L::kTurns) & 1, abort_flag)))) break;
+        if (!(ok = mbar_wait_warp(tfull + b, (i / L::kTurns) & 1, abort_flag))) break;
         tcgen05_fence_after();
         acc = accumulator(b);
       }
@@ -440,11 +479,7 @@ __global__ void __launch_bounds__(Tile<BN, FMT>::kThreads, 1)
           for (int j = 0; j + AC < L::kSums; ++j) sum[j] = sum[j + AC];
         } else {
           tmem_ld<AC == 32 ? 32 : 16>(acc + c * AC, v);
-          if (c + 1 == nc) {  // the accumulator has been read: the issuer may reuse it
-            tcgen05_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(tempty + i % L::kTurns);
-          }
+          if (c + 1 == nc) release(i % L::kTurns);
 #pragma unroll
           for (int j = 0; j < AC; ++j) v[j] = L::kScaled ? v[j] * b_unscale * unscale : v[j];
         }
@@ -455,13 +490,13 @@ __global__ void __launch_bounds__(Tile<BN, FMT>::kThreads, 1)
             if (c + 1 < nc) {
               ask(t, c + 1, k + 1);
             } else {
-              int u = t + gridDim.x;
-              while (u < n_tiles && chunks_of(u) == 0) u += gridDim.x;
+              int u = t + tile_step;
+              while (u < n_tiles && chunks_of(u) == 0) u += tile_step;
               if (u < n_tiles) ask(u, 0, k + 1);
             }
           }
           __syncwarp();
-          if (!(ok = __all_sync(0xffffffffu, mbar_wait(bar + (k & 1), (k >> 1) & 1, abort_flag)))) break;
+          if (!(ok = mbar_wait_warp(bar + (k & 1), (k >> 1) & 1, abort_flag))) break;
           chunk_get<W>(mine, lane, in);
         }
         epilogue_row<EPI, AC>(p, row, n0 + c * AC, rt, v, has_in, in, out, pre);
@@ -490,71 +525,75 @@ __global__ void __launch_bounds__(Tile<BN, FMT>::kThreads, 1)
       }
       if (!ok) break;
       if (!L::X3) {
-        if (nc == 0) {
-          tcgen05_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(tempty + i % L::kTurns);
-        }
+        if (nc == 0) release(i % L::kTurns);
         ++i;
       }
       if (p.c_max && row < p.M && nc > 0) atomicMax(p.c_max + row, __float_as_uint(big));
     }
     if (lane == 0) bulk_wait_all();
-  } else if (!L::T1) {
-    if (L::kMoveRegs) asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
-    // A thread owns a row: 16-byte chunk c of row r sits at chunk c ^ (r & 7) of its 128 bytes, so the eight lanes of a
-    // quarter warp touch eight different 16-byte columns on the reads and on the writes. The parts go back as chunks 0-3
+  } else if (!L::T1 || PAIR) {
+    if (L::kMoveRegs) asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
+    // A lane owns a row at a time: 16-byte chunk c of row r sits at chunk c ^ (r & 7) of its 128 bytes, so the eight lanes of
+    // a quarter warp touch eight different 16-byte columns on the reads and on the writes. The parts go back as chunks 0-3
     // (h) and 4-7 (m or l) of the same row; FMT_F16X3's l into rows of 64 bytes, chunk c at c ^ ((r >> 1) & 3).
-    const int r = threadIdx.x - kConvWarp0 * 32;
+    constexpr int WPG = 4 / L::kGroups;  // warps of a group
+    const int cw = warp - kConvWarp0, group = cw / WPG, first = cw % WPG;
     int g = 0;
     bool ok = true;
-    for (int t = blockIdx.x; ok && t < n_tiles; t += gridDim.x) {
-      float s = 1.f;
-      if (L::kScaled) {
-        const int row = (t / tiles_n) * TBM + r;
-        s = row < p.M ? scale_of(p.a_max[row]) : 1.f;
+    for (int t = tile0; ok && t < n_tiles; t += tile_step) {
+      const int m0 = first_row(t);
+      float scale[4 / WPG];
+#pragma unroll
+      for (int j = 0; j < 4 / WPG; ++j) {
+        const int row = m0 + (first + j * WPG) * 32 + lane;
+        scale[j] = L::kScaled && row < p.M ? scale_of(p.a_max[row]) : 1.f;
       }
       for (int kb = 0; kb < nkb; ++kb, ++g) {
+        if (g % L::kGroups != group) continue;
         const int sa = g % NA;
-        if (!(ok = __all_sync(0xffffffffu, mbar_wait(full_a + sa, (g / NA) & 1, abort_flag)))) break;
-        if (L::T2) {  // the slab is h; l goes beside it at the same place
-          uint8_t* slab = ring_a + sa * L::kA;
+        if (!(ok = mbar_wait_warp(full_a + sa, (g / NA) & 1, abort_flag))) break;
+        uint8_t* slab = ring_a + sa * L::kA;
+#pragma unroll
+        for (int j = 0; j < 4 / WPG; ++j) {
+          const int r = (first + j * WPG) * 32 + lane;
+          if (L::T1 || m0 + r - lane >= p.M) break;  // rows past the matrix: whatever their products are, nobody reads them
+          if (L::T2) {  // the slab is h; l goes beside it at the same place
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              const float4 x = *reinterpret_cast<const float4*>(slab + swizzled<64>(r, c));
+              *reinterpret_cast<float4*>(slab + L::kSlab + swizzled<64>(r, c)) =
+                  make_float4(tf32_low(x.x), tf32_low(x.y), tf32_low(x.z), tf32_low(x.w));
+            }
+            continue;
+          }
+          const float s = scale[j];
+          float4 x[8];
+#pragma unroll
+          for (int c = 0; c < 8; ++c) x[c] = *reinterpret_cast<const float4*>(slab + swizzled<128>(r, c));
 #pragma unroll
           for (int c = 0; c < 4; ++c) {
-            const float4 x = *reinterpret_cast<const float4*>(slab + swizzled<64>(r, c));
-            *reinterpret_cast<float4*>(slab + L::kSlab + swizzled<64>(r, c)) =
-                make_float4(tf32_low(x.x), tf32_low(x.y), tf32_low(x.z), tf32_low(x.w));
+            uint4 h, m, l;
+            const float4 a = x[2 * c], b = x[2 * c + 1];
+            split2<FMT>(a.x, a.y, s, h.x, m.x, l.x), split2<FMT>(a.z, a.w, s, h.y, m.y, l.y);
+            split2<FMT>(b.x, b.y, s, h.z, m.z, l.z), split2<FMT>(b.z, b.w, s, h.w, m.w, l.w);
+            *reinterpret_cast<uint4*>(slab + swizzled<128>(r, c)) = h;
+            if (L::X3 || L::X2) *reinterpret_cast<uint4*>(slab + swizzled<128>(r, 4 + c)) = m;
+            if (L::X3) *reinterpret_cast<uint4*>(slab + L::kSlab + swizzled<64>(r, c)) = l;
           }
-          fence_async_smem();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(conv_a + sa);
-          continue;
-        }
-        uint8_t* rowp = ring_a + sa * L::kA + r * 128;
-        float4 x[8];
-#pragma unroll
-        for (int c = 0; c < 8; ++c) x[c] = *reinterpret_cast<const float4*>(rowp + ((c ^ (r & 7)) << 4));
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          uint4 h, m, l;
-          const float4 a = x[2 * c], b = x[2 * c + 1];
-          split2<FMT>(a.x, a.y, s, h.x, m.x, l.x), split2<FMT>(a.z, a.w, s, h.y, m.y, l.y);
-          split2<FMT>(b.x, b.y, s, h.z, m.z, l.z), split2<FMT>(b.z, b.w, s, h.w, m.w, l.w);
-          *reinterpret_cast<uint4*>(rowp + ((c ^ (r & 7)) << 4)) = h;
-          if (L::X3 || L::X2) *reinterpret_cast<uint4*>(rowp + (((4 + c) ^ (r & 7)) << 4)) = m;
-          if (L::X3) *reinterpret_cast<uint4*>(ring_a + sa * L::kA + TBM * 128 + r * 64 + ((c ^ ((r >> 1) & 3)) << 4)) = l;
         }
         fence_async_smem();  // generic-proxy writes visible to the tensor core
         __syncwarp();
-        if (lane == 0) mbar_arrive(conv_a + sa);
+        if (lane == 0) {
+          if (PAIR) mbar_arrive_at(ready + sa, 0);
+          else mbar_arrive(ready + sa);
+        }
       }
     }
   }
   tcgen05_fence_before();
   __syncthreads();
-  if (warp == 1) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(L::kColumns) : "memory");
-  }
+  if (PAIR) cluster_sync_all();  // nobody leaves while the other CTA may still signal it or read its tiles
+  if (warp == 1) tmem_dealloc<PAIR>(tmem, L::kColumns);
   if (threadIdx.x == 0 && *abort_flag) atomicExch(err, 1);
 }
 
@@ -661,27 +700,41 @@ CUtensorMap map_2d(CUtensorMapDataType type, const void* base, int cols, int row
   return make_map(type, 2, base, dims, pitch, box, swizzle);
 }
 
-template <int EPI, int BN, int FMT>
+// As many pairs as the device holds at once (a pair needs two SMs of one GPC: fewer than half the SMs may fit), or the last
+// pairs of a persistent kernel would start when the first ones end.
+template <class K>
+int resident_pairs(K kernel, cudaLaunchConfig_t cfg) {
+  static PerDevice<int> table;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  return table.get(dev, [&](int& n) {
+    cfg.gridDim = dim3(unsigned(state().sms / 2 * 2));
+    if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n <= 0) n = state().sms / 2;
+    n = std::min(n, state().sms / 2);
+  });
+}
+
+template <int EPI, int BN, int FMT, bool PAIR>
 void launch_tc(Stream& st, const GemmArgs& a, const PackedB& w) {
-  using L = Tile<BN, FMT>;
+  using L = Tile<BN, FMT, PAIR>;
   static_assert(L::kTotal <= 227 * 1024, "the tile pipeline does not fit shared memory");
   static SmemOptIn opted;
-  auto kernel = k_gemm_tc<EPI, BN, FMT>;
+  auto kernel = k_gemm_tc<EPI, BN, FMT, PAIR>;
   opt_in_shared_memory(kernel, L::kTotal, opted);
   const CUtensorMap ma = map_2d(CU_TENSOR_MAP_DATA_TYPE_FLOAT32, a.A, a.K, a.M, size_t(a.lda) * 4, L::BK, TBM,
                                 L::T2 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B);
   const auto half = FMT == FMT_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
   CUtensorMap mb, ml;
   if (L::T1) {
-    ml = mb = map_2d(CU_TENSOR_MAP_DATA_TYPE_FLOAT32, w.main, w.Kp, a.N, size_t(w.Kp) * 4, L::BK, BN, CU_TENSOR_MAP_SWIZZLE_128B);
+    ml = mb = map_2d(CU_TENSOR_MAP_DATA_TYPE_FLOAT32, w.main, w.Kp, a.N, size_t(w.Kp) * 4, L::BK, L::kRowsB, CU_TENSOR_MAP_SWIZZLE_128B);
   } else if (L::T2) {
-    mb = map_2d(CU_TENSOR_MAP_DATA_TYPE_FLOAT32, w.main, w.Kp, a.N, size_t(w.Kp) * 4, L::BK, BN, CU_TENSOR_MAP_SWIZZLE_64B);
-    ml = map_2d(CU_TENSOR_MAP_DATA_TYPE_FLOAT32, w.low, w.Kp, a.N, size_t(w.Kp) * 4, L::BK, BN, CU_TENSOR_MAP_SWIZZLE_64B);
+    mb = map_2d(CU_TENSOR_MAP_DATA_TYPE_FLOAT32, w.main, w.Kp, a.N, size_t(w.Kp) * 4, L::BK, L::kRowsB, CU_TENSOR_MAP_SWIZZLE_64B);
+    ml = map_2d(CU_TENSOR_MAP_DATA_TYPE_FLOAT32, w.low, w.Kp, a.N, size_t(w.Kp) * 4, L::BK, L::kRowsB, CU_TENSOR_MAP_SWIZZLE_64B);
   } else if (L::X3 || L::X2) {
-    mb = map_2d(half, w.main, 2 * w.Kp, a.N, size_t(w.Kp) * 4, 64, BN, CU_TENSOR_MAP_SWIZZLE_128B);
-    ml = L::X3 ? map_2d(half, w.low, w.Kp, a.N, size_t(w.Kp) * 2, L::BK, BN, CU_TENSOR_MAP_SWIZZLE_64B) : mb;
+    mb = map_2d(half, w.main, 2 * w.Kp, a.N, size_t(w.Kp) * 4, 64, L::kRowsB, CU_TENSOR_MAP_SWIZZLE_128B);
+    ml = L::X3 ? map_2d(half, w.low, w.Kp, a.N, size_t(w.Kp) * 2, L::BK, L::kRowsB, CU_TENSOR_MAP_SWIZZLE_64B) : mb;
   } else {
-    ml = mb = map_2d(half, w.main, w.Kp, a.N, size_t(w.Kp) * 2, L::BK, BN, CU_TENSOR_MAP_SWIZZLE_64B);
+    ml = mb = map_2d(half, w.main, w.Kp, a.N, size_t(w.Kp) * 2, L::BK, L::kRowsB, CU_TENSOR_MAP_SWIZZLE_64B);
   }
   // the epilogue's chunks: 32 rows x kWide columns of what it reads and writes (C half as wide after a SwiGLU)
   constexpr int W = L::kWide;
@@ -695,9 +748,19 @@ void launch_tc(Stream& st, const GemmArgs& a, const PackedB& w) {
   if (EPI == EPI_PLAIN && a.res) mi = chunk(a.res, a.N, a.ldr, W);
   if (EPI == EPI_SILU_BWD || EPI == EPI_SWIGLU_BWD) mi = chunk(a.pre, c_cols, a.ldp, W);
   if (writes_two(EPI) && a.pre) mp = chunk(a.pre, a.N, a.ldp, W);
-  const long long tiles = (long long) cdiv(a.M, TBM) * cdiv(a.N, BN);
-  const int grid = int(tiles < state().sms ? tiles : state().sms);
-  kernel<<<grid, L::kThreads, L::kTotal, st.s>>>(ma, mb, ml, mi, mc, mp, a, w.amax, state().err);
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute attr{};
+  cfg.blockDim = dim3(L::kThreads), cfg.dynamicSmemBytes = L::kTotal, cfg.stream = st.s;
+  const long long tiles = (long long) cdiv(a.M, PAIR ? 2 * TBM : TBM) * cdiv(a.N, BN);
+  if (PAIR) {
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = 2, attr.val.clusterDim.y = 1, attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr, cfg.numAttrs = 1;
+    cfg.gridDim = dim3(unsigned(2 * std::min<long long>(tiles, resident_pairs(kernel, cfg))));
+  } else {
+    cfg.gridDim = dim3(unsigned(std::min<long long>(tiles, state().sms)));
+  }
+  PETB_CUDA(cudaLaunchKernelEx(&cfg, kernel, ma, mb, ml, mi, mc, mp, a, w.amax, state().err));
   PETB_LAUNCH_CHECK(st);
 }
 
@@ -722,9 +785,16 @@ void dispatch_width(Stream& st, const GemmArgs& a, const PackedB& w) {
     if (bn == 0 || rounds * wavefronts[i] < best) bn = widths[i], best = rounds * wavefronts[i];
   }
   if (bn == 0) bn = a.N <= 64 ? 64 : 128;  // ragged widths: a tile with a zero-filled edge
-  if (bn == 256) launch_tc<EPI, 256, FMT>(st, a, w);
-  else if (bn == 128) launch_tc<EPI, 128, FMT>(st, a, w);
-  else launch_tc<EPI, 64, FMT>(st, a, w);
+  // A pair of CTAs per 256-row tile halves what each reads and stages of the weight. It pays in the formats of two and three
+  // parts, whose weight tiles are the larger share (122138 rows: FMT_F16X3 w_in backward 258 us against 307, SwiGLU 353
+  // against 383; FMT_F16X2 215 against 274, plain 56 against 60), once there is a tile for every pair of SMs; the formats of
+  // one part are near HBM's rate without it, and the second CTA's signals make a step longer (SwiGLU 180 us against 164).
+  constexpr bool kPair = FMT == FMT_F16X3 || FMT == FMT_F16X2 || FMT == FMT_TF32X2;
+  if constexpr (kPair)
+    if (bn == 256 && cdiv(a.M, 2 * TBM) * (a.N / 256) >= sms / 2) return launch_tc<EPI, 256, FMT, true>(st, a, w);
+  if (bn == 256) launch_tc<EPI, 256, FMT, false>(st, a, w);
+  else if (bn == 128) launch_tc<EPI, 128, FMT, false>(st, a, w);
+  else launch_tc<EPI, 64, FMT, false>(st, a, w);
 }
 
 template <int EPI>

@@ -1,7 +1,7 @@
 """The tensor-core GEMM at the edges of its tiles, in every operand format, against the fp64 product.
 
 Rows: one, both sides of the 64 below which every mode runs in the native format, both sides of a 128-row tile, a ragged
-third tile. Columns: the least, both sides of a column tile's width of 64, 128 and 256, several tiles. Contraction: less than
+third tile, more tiles than SMs (several per block). Columns: the least, both sides of a column tile's width of 64, 128 and 256, several tiles. Contraction: less than
 a step of 32, a ragged last step, both sides of the 1024 after which the native format's exact sums are read out."""
 import numpy as np
 import pytest
@@ -9,7 +9,8 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 SHAPES = [(1, 4, 4), (1, 256, 32), (63, 60, 36), (64, 64, 64), (65, 68, 60), (127, 128, 128), (128, 132, 96), (129, 192, 100),
-          (257, 256, 1020), (257, 260, 1024), (130, 64, 1028), (300, 512, 2052), (5000, 256, 256), (2500, 768, 512)]
+          (257, 256, 1020), (257, 260, 1024), (130, 64, 1028), (300, 512, 2052), (5000, 256, 256), (2500, 768, 512),
+          (40001, 64, 160), (40001, 128, 96), (40001, 256, 288)]
 
 
 @pytest.fixture(scope="module")
@@ -53,3 +54,17 @@ def test_native_sums_are_not_biased(calc):
         C = calc.gemm(A, W, "native").astype(np.float64)
         assert abs((C * ref).sum() / (ref * ref).sum() - 1.0) < 1e-8
         assert np.sqrt(((C - ref) ** 2).mean()) < 1e-7 * np.sqrt((ref ** 2).mean())
+
+
+@pytest.mark.parametrize("mode", ["native", "3xtf32"])
+def test_a_pair_of_blocks_gives_the_bits_of_one(calc, mode):
+    """Large GEMMs run on pairs of blocks that share a 256-row tile; a row's bits stay those of the one-block kernel. A ragged
+    last tile whose second block has no rows, one that has a few, two column tiles, steps beyond a ring's length."""
+    rng = np.random.default_rng(11)
+    for m, n, k in [(38400 + 100, 256, 320), (38400 + 130, 256, 96), (20000, 512, 1056)]:
+        A = rng.normal(size=(m, k)).astype(np.float32)
+        W = rng.normal(size=(n, k)).astype(np.float32)
+        for _ in range(3):  # (operands handed from block to block: look at more than one run)
+            C = calc.gemm(A, W, mode)
+            for r0 in (0, 12800, m - 3000):
+                assert np.array_equal(C[r0:r0 + 3000], calc.gemm(A[r0:r0 + 3000], W, mode)), (m, n, k, r0)
