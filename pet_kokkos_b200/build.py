@@ -21,7 +21,7 @@ COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler",
           "--expt-relaxed-constexpr", "-Xcudafe", "--diag_suppress=177"]
 # neighbour kernels: every fp64 product and sum rounded on its own (bit-exact edge decisions)
 PER_FILE = {"neighbors.cu": ["-fmad=false"]}
-SOURCES = ["checkpoint.cpp", "neighbors.cu", "ops.cu", "adaptive.cu", "attention.cu", "attention_tile.cu", "attention_mma.cu", "gemm_simt.cu", "gemm_tc.cu", "model.cu", "static_gemm.cu", "nccl_exchange.cu",
+SOURCES = ["checkpoint.cpp", "neighbors.cu", "ops.cu", "adaptive.cu", "attention.cu", "attention_tile.cu", "attention_mma.cu", "attention_f16.cu", "gemm_simt.cu", "gemm_tc.cu", "model.cu", "static_gemm.cu", "nccl_exchange.cu",
            "engine.cu", "capi.cu"]
 
 

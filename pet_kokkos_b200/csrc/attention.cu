@@ -19,8 +19,9 @@ namespace petb {
 
 bool attention_forward_tiled(Stream& st, const AttnArgs& p);   // attention_tile.cu
 bool attention_backward_tiled(Stream& st, const AttnArgs& p);
+bool attention_forward_f16(Stream& st, const AttnArgs& p);  // attention_f16.cu
+bool attention_backward_f16(Stream& st, const AttnArgs& p);
 bool attention_forward_mma(Stream& st, const AttnArgs& p);  // attention_mma.cu
-bool attention_backward_mma(Stream& st, const AttnArgs& p);
 
 namespace {
 
@@ -251,6 +252,7 @@ void attention_forward(Stream& st, const AttnArgs& p) {
   // qkv read and the output written once.
   const double D = double(p.H) * p.hd;
   const ProfScope ps(st, PC_ATTN_FWD, 4.0 * p.pairs * D, 4.0 * p.T * (4.0 * D + 2.0 * p.H));
+  if (!(p.tf32 && p.mode != ATTN_NATIVE) && attention_forward_f16(st, p)) return;
   if (p.mode != ATTN_NATIVE && attention_forward_mma(st, p)) return;
   if (!attention_forward_tiled(st, p)) forward_streaming(st, p);
   // the CUDA-core kernels leave the rows' maxima to a pass of its own
@@ -261,7 +263,7 @@ void attention_backward(Stream& st, const AttnArgs& p) {
   if (p.N == 0) return;
   const double D = double(p.H) * p.hd;
   const ProfScope ps(st, PC_ATTN_BWD, 10.0 * p.pairs * D, 4.0 * p.T * (8.0 * D + 3.0 * p.H));
-  if (p.mode != ATTN_NATIVE && attention_backward_mma(st, p)) return;
+  if (attention_backward_f16(st, p)) return;
   if (!attention_backward_tiled(st, p)) backward_streaming(st, p);
   if (p.qkv_adj_max) row_max(st, p.qkv_adj_max, p.qkv_adj, int(3 * D), int(p.T), int(3 * D));
 }

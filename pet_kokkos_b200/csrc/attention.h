@@ -14,11 +14,16 @@ struct AttnArgs {
   // cores; ATTN_TF32X3, the split products on the tensor cores, as accurate but for the tensor core's truncating
   // accumulate; ATTN_TF32, one tf32 product per tile (a speed mode, about three decimal digits).
   int mode = 0;
+  bool tf32 = false;                // forward: the tensor-core modes on tf32 instructions (where energies depend on their bits)
   double pairs = 0.0;               // sum over atoms of tokens^2 (work accounting only)
   double T = 0.0;                   // token rows (work accounting only)
   const int* off = nullptr;         // [N+1] each atom's range of edge rows
   const float* cut = nullptr;       // [E] cutoff factor of each edge token
   const float* qkv = nullptr;       // [T,3D] columns Q | K | V
+  // [T] the bits of each row's largest |qkv| (and, in the backward, |dmerged|), which the kernels on fp16 parts scale by. Null:
+  // the pass goes to the others.
+  const uint32_t* qkv_max = nullptr;
+  const uint32_t* dmerged_max = nullptr;
   float* merged = nullptr;          // [T,D] attention output before the output projection
   uint32_t* merged_max = nullptr;   // [T] unless null, each row's largest |merged| is raised into it (zeroed by the caller)
   float* ml = nullptr;              // [T,H,2] each query's running max and 1/sum (null: not saved)

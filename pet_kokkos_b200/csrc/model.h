@@ -102,6 +102,8 @@ class Model {
   void put_vec(const std::string& name, const double* src, int len, bool paired);
   void fold_compress(const Checkpoint& ck, const std::string& c0, int layer);
 
+  bool wide() const { return h_.d_pet > 256; }  // the tensor-core modes' forward on tf32 instructions (put_mat)
+
   Hypers h_;
   double scale_ = 1.0;
   int mode_ = 0;  // the GEMM mode the weights are packed for
