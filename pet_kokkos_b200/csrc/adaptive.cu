@@ -60,6 +60,7 @@ __device__ inline double bump_dd(double d, double rc, double width) {
 __global__ void __launch_bounds__(256) k_solver(int N, const int* __restrict__ roff, const double* __restrict__ dist,
                                                 double rmax, double width, double target, double* __restrict__ acut,
                                                 double* __restrict__ root, double* __restrict__ slope) {
+  after_previous();
   const int a = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (a >= N) return;
   const int e0 = roff[a], e1 = roff[a + 1];
@@ -94,6 +95,7 @@ __global__ void __launch_bounds__(256) k_solver(int N, const int* __restrict__ r
 // One warp per atom, lanes striding the probes: each walks the atom's edges in order (a serial sweep's sums).
 __global__ void __launch_bounds__(256) k_grid_eff(int N, int P, const int* __restrict__ roff, const double* __restrict__ dist,
                                                   const double* __restrict__ probes, double width, double* __restrict__ eff) {
+  after_previous();
   const int a = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (a >= N) return;
   for (int p = lane; p < P; p += 32) {
@@ -117,6 +119,7 @@ __device__ inline double grid_stencil(const double* eff, int p, int P, double ta
 // One thread per atom: the softmax-weighted mean of the probes.
 __global__ void k_grid_cutoff(int N, int P, const double* __restrict__ eff_all, const double* __restrict__ probes, double target,
                               double* __restrict__ acut) {
+  after_previous();
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
   if (a >= N) return;
   const double* eff = eff_all + size_t(a) * P;
@@ -137,6 +140,7 @@ __global__ void k_grid_cutoff(int N, int P, const double* __restrict__ eff_all, 
 
 // adapted_adj(a) = sum over a's kept edges of half the edge's and half its partner's pair-cutoff adjoint.
 __global__ void k_adapted_adj(PackedEdges pk, const double* __restrict__ pc_adj, double* __restrict__ adapted_adj) {
+  after_previous();
   const int a = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (a >= pk.n_atoms) return;
   double s = 0.0;
@@ -154,6 +158,7 @@ __global__ void k_adapted_adj(PackedEdges pk, const double* __restrict__ pc_adj,
 __global__ void k_gmag_solver(int E, const int* __restrict__ center, const double* __restrict__ dist,
                               const double* __restrict__ root, const double* __restrict__ slope,
                               const double* __restrict__ adapted_adj, double width, double scale, double* __restrict__ gmag) {
+  after_previous();
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= E) return;
   const int c = center[e];
@@ -166,6 +171,7 @@ __global__ void k_gmag_solver(int E, const int* __restrict__ center, const doubl
 __global__ void k_grid_backward(int N, int P, const double* __restrict__ eff_all, const double* __restrict__ probes,
                                 double target, const double* __restrict__ adapted_adj, double* __restrict__ diff_adj_all,
                                 double* __restrict__ cq_all) {
+  after_previous();
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
   if (a >= N) return;
   const double* eff = eff_all + size_t(a) * P;
@@ -212,6 +218,7 @@ __global__ void k_grid_backward(int N, int P, const double* __restrict__ eff_all
 __global__ void k_gmag_grid(int E, int P, const int* __restrict__ center, const double* __restrict__ dist,
                             const double* __restrict__ probes, const double* __restrict__ diff_adj, double width, double scale,
                             double* __restrict__ gmag) {
+  after_previous();
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= E) return;
   const double d = dist[e];
@@ -230,6 +237,7 @@ __global__ void k_gmag_grid(int E, int P, const int* __restrict__ center, const 
 // a minus sign, so it adds. A warp per atom, a fixed combination order.
 __global__ void __launch_bounds__(256) k_raw_fold(int N, RawEdges re, const double* __restrict__ gmag, double* __restrict__ forces,
                                                   double* __restrict__ vir_atom) {
+  after_previous();
   const int a = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (a >= N) return;
   double s[12] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
@@ -259,17 +267,17 @@ AdaptiveCut adaptive_cutoffs(Stream& st, Arena& arena, const RawEdges& re, int n
   if (cs.adaptive == 2) {
     double* root = arena.alloc<double>(n_atoms);
     double* slope = arena.alloc<double>(n_atoms);
-    k_solver<<<cdiv(size_t(n_atoms) * 32, 256), 256, 0, st.s>>>(n_atoms, re.off, re.dist, cs.cutoff, cs.width_adaptive, cs.target,
+    launch(st, k_solver, cdiv(size_t(n_atoms) * 32, 256), 256, 0, n_atoms, re.off, re.dist, cs.cutoff, cs.width_adaptive, cs.target,
                                                                acut, root, slope);
     PETB_LAUNCH_CHECK(st);
     ad.root = root, ad.slope = slope;
   } else {
     if (cs.n_probes < 2) throw Error(1, "pet: the grid adaptive cutoff needs at least two probe radii");
     double* eff = arena.alloc<double>(size_t(n_atoms) * cs.n_probes);
-    k_grid_eff<<<cdiv(size_t(n_atoms) * 32, 256), 256, 0, st.s>>>(n_atoms, cs.n_probes, re.off, re.dist, cs.probes,
+    launch(st, k_grid_eff, cdiv(size_t(n_atoms) * 32, 256), 256, 0, n_atoms, cs.n_probes, re.off, re.dist, cs.probes,
                                                                  cs.width_adaptive, eff);
     PETB_LAUNCH_CHECK(st);
-    k_grid_cutoff<<<cdiv(n_atoms, 128), 128, 0, st.s>>>(n_atoms, cs.n_probes, eff, cs.probes, cs.target, acut);
+    launch(st, k_grid_cutoff, cdiv(n_atoms, 128), 128, 0, n_atoms, cs.n_probes, eff, cs.probes, cs.target, acut);
     PETB_LAUNCH_CHECK(st);
     ad.eff = eff;
   }
@@ -285,21 +293,21 @@ void adaptive_backward(Stream& st, Arena& arena, const PackedEdges& pk, const Cu
   const ProfScope ps(st, PC_FORCES, 60.0 * E, 120.0 * double(E));
   double* adapted_adj = arena.alloc<double>(N);
   double* gmag = arena.alloc<double>(E);
-  k_adapted_adj<<<cdiv(size_t(N) * 32, 256), 256, 0, st.s>>>(pk, pc_adj, adapted_adj);
+  launch(st, k_adapted_adj, cdiv(size_t(N) * 32, 256), 256, 0, pk, pc_adj, adapted_adj);
   PETB_LAUNCH_CHECK(st);
   if (cs.adaptive == 2) {
-    k_gmag_solver<<<cdiv(E, 256), 256, 0, st.s>>>(E, ad.raw.i, ad.raw.dist, ad.root, ad.slope, adapted_adj, cs.width_adaptive, scale,
+    launch(st, k_gmag_solver, cdiv(E, 256), 256, 0, E, ad.raw.i, ad.raw.dist, ad.root, ad.slope, adapted_adj, cs.width_adaptive, scale,
                                                  gmag);
     PETB_LAUNCH_CHECK(st);
   } else {
     double* diff_adj = arena.alloc<double>(size_t(N) * ad.P);
     double* cq = arena.alloc<double>(size_t(N) * ad.P);
-    k_grid_backward<<<cdiv(N, 128), 128, 0, st.s>>>(N, ad.P, ad.eff, ad.probes, cs.target, adapted_adj, diff_adj, cq);
+    launch(st, k_grid_backward, cdiv(N, 128), 128, 0, N, ad.P, ad.eff, ad.probes, cs.target, adapted_adj, diff_adj, cq);
     PETB_LAUNCH_CHECK(st);
-    k_gmag_grid<<<cdiv(E, 256), 256, 0, st.s>>>(E, ad.P, ad.raw.i, ad.raw.dist, ad.probes, diff_adj, cs.width_adaptive, scale, gmag);
+    launch(st, k_gmag_grid, cdiv(E, 256), 256, 0, E, ad.P, ad.raw.i, ad.raw.dist, ad.probes, diff_adj, cs.width_adaptive, scale, gmag);
     PETB_LAUNCH_CHECK(st);
   }
-  k_raw_fold<<<cdiv(size_t(N) * 32, 256), 256, 0, st.s>>>(N, ad.raw, gmag, forces, vir_atom);
+  launch(st, k_raw_fold, cdiv(size_t(N) * 32, 256), 256, 0, N, ad.raw, gmag, forces, vir_atom);
   PETB_LAUNCH_CHECK(st);
   *gmag_out = gmag;
 }

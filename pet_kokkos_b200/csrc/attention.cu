@@ -71,6 +71,7 @@ __device__ __forceinline__ void stage(float* dst, const float* src, size_t ld, i
 
 template <int HD>
 __global__ void __launch_bounds__(256) k_attn_fwd(AttnArgs p) {
+  after_previous();
   extern __shared__ __align__(16) float smem[];
   const int n = blockIdx.x / p.H, h = blockIdx.x % p.H, D = p.H * HD;
   const int e0 = p.off[n], cnt = p.off[n + 1] - e0 + 1;
@@ -119,6 +120,7 @@ __global__ void __launch_bounds__(256) k_attn_fwd(AttnArgs p) {
 
 template <int HD>
 __global__ void __launch_bounds__(256) k_attn_bwd(AttnArgs p) {
+  after_previous();
   extern __shared__ __align__(16) float smem[];
   const int n = blockIdx.x / p.H, h = blockIdx.x % p.H, D = p.H * HD;
   const int e0 = p.off[n], cnt = p.off[n + 1] - e0 + 1;
@@ -206,7 +208,7 @@ void launch(Stream& st, K kernel, const AttnArgs& p, size_t bytes, SmemOptIn& op
   opt_in_shared_memory(kernel, bytes, opted);
   int threads = (p.S + 31) / 32 * 32;
   if (threads > 256) threads = 256;
-  kernel<<<p.N * p.H, threads, bytes, st.s>>>(p);
+  launch(st, kernel, p.N * p.H, threads, bytes, p);
   PETB_LAUNCH_CHECK(st);
 }
 

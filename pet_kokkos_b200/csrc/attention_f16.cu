@@ -259,6 +259,7 @@ __host__ __device__ constexpr int resident(int rows) {
 
 template <int HD, int P, int MAXB>
 __global__ void __launch_bounds__(32 * MAXB, MAXB <= 5 ? resident<HD, P, 3>(16 * MAXB) : 1) k_attn_fwd_f16(AttnArgs p) {
+  after_previous();
   extern __shared__ __align__(16) uint8_t smem[];
   __shared__ uint32_t s_max;
   const int n = blockIdx.x / p.H, h = blockIdx.x % p.H, D = p.H * HD;
@@ -366,6 +367,7 @@ __global__ void __launch_bounds__(32 * MAXB, MAXB <= 5 ? resident<HD, P, 3>(16 *
 
 template <int HD, int P, int MAXT, int BLOCKS>
 __global__ void __launch_bounds__(MAXT, BLOCKS) k_attn_bwd_f16(AttnArgs p) {
+  after_previous();
   constexpr int KS = HD / 16;
   // The A operands of a block stay in registers over the whole loop where they are few enough; else each step's are loaded
   // where they are used.
@@ -524,7 +526,7 @@ __global__ void __launch_bounds__(MAXT, BLOCKS) k_attn_bwd_f16(AttnArgs p) {
 template <class K>
 void launch(Stream& st, K kernel, const AttnArgs& p, size_t bytes, int threads, SmemOptIn& opted) {
   opt_in_shared_memory(kernel, bytes, opted);
-  kernel<<<p.N * p.H, threads, bytes, st.s>>>(p);
+  launch(st, kernel, p.N * p.H, threads, bytes, p);
   PETB_LAUNCH_CHECK(st);
 }
 

@@ -112,6 +112,7 @@ __device__ __forceinline__ void load_a(Frag (*f)[4], const float* x, int r0, int
 
 template <int HD, int MAXKB, bool X3>
 __global__ void __launch_bounds__(32 * ((MAXKB + 1) / 2), MAXKB <= 10 ? 4 : 1) k_attn_fwd_mma(AttnArgs p) {
+  after_previous();
   constexpr int P = HD + 4, KS = HD / 8, R = 8 * MAXKB;  // R: staged token rows, the kernel's most (zero past the atom's)
   constexpr int G = MAXKB % 5 == 0 ? 5 : (MAXKB % 4 == 0 ? 4 : 2);  // key blocks whose score tiles advance together
   extern __shared__ __align__(16) float smem[];
@@ -235,7 +236,7 @@ size_t fwd_bytes(int maxkb, int HD) {
 template <class K>
 void launch(Stream& st, K kernel, const AttnArgs& p, size_t bytes, int threads, SmemOptIn& opted) {
   opt_in_shared_memory(kernel, bytes, opted);
-  kernel<<<p.N * p.H, threads, bytes, st.s>>>(p);
+  launch(st, kernel, p.N * p.H, threads, bytes, p);
   PETB_LAUNCH_CHECK(st);
 }
 

@@ -79,6 +79,7 @@ struct TileIter {
 
 template <int HD>
 __global__ void __launch_bounds__(192) k_attn_fwd_tile(AttnArgs p) {
+  after_previous();
   extern __shared__ __align__(16) float smem[];
   const Layout L = layout(p.S, HD);
   const int n = blockIdx.x / p.H, h = blockIdx.x % p.H, D = p.H * HD;
@@ -181,6 +182,7 @@ __global__ void __launch_bounds__(192) k_attn_fwd_tile(AttnArgs p) {
 
 template <int HD>
 __global__ void __launch_bounds__(192) k_attn_bwd_tile(AttnArgs p) {
+  after_previous();
   extern __shared__ __align__(16) float smem[];
   const Layout L = layout(p.S, HD);
   const int n = blockIdx.x / p.H, h = blockIdx.x % p.H, D = p.H * HD;
@@ -331,7 +333,7 @@ size_t bwd_bytes(int S, int HD) {
 template <class K>
 void launch(Stream& st, K kernel, const AttnArgs& p, size_t bytes, SmemOptIn& opted) {
   opt_in_shared_memory(kernel, bytes, opted);
-  kernel<<<p.N * p.H, 192, bytes, st.s>>>(p);
+  launch(st, kernel, p.N * p.H, 192, bytes, p);
   PETB_LAUNCH_CHECK(st);
 }
 

@@ -34,6 +34,7 @@ __device__ __forceinline__ void fma2(unsigned long long& d, unsigned long long a
 
 template <int EPI>
 __global__ void __launch_bounds__(256, 2) k_gemm_native(GemmArgs p) {
+  after_previous();
   __shared__ __align__(16) float As[2][BK][BM + PAD];
   __shared__ __align__(16) float Bs[2][BK][BN + PAD];
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
@@ -114,6 +115,7 @@ __global__ void __launch_bounds__(256, 2) k_gemm_native(GemmArgs p) {
 
 __global__ void k_gemv_rows(const float* __restrict__ A, int lda, const float* __restrict__ w, const float* __restrict__ bias,
                             float* __restrict__ out, int M, int K) {
+  after_previous();
   const int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (r >= M) return;
   float s = 0.0f;
@@ -126,7 +128,7 @@ __global__ void k_gemv_rows(const float* __restrict__ A, int lda, const float* _
 template <int EPI>
 void launch_native(Stream& st, const GemmArgs& a) {
   const long long tiles = (long long) cdiv(a.M, BM) * cdiv(a.N, BN);
-  k_gemm_native<EPI><<<(unsigned) tiles, 256, 0, st.s>>>(a);
+  launch(st, k_gemm_native<EPI>, (unsigned) tiles, 256, 0, a);
   PETB_LAUNCH_CHECK(st);
 }
 
@@ -161,7 +163,7 @@ void gemm(Stream& st, Arena& arena, const GemmArgs& a) {
 void gemv_rows(Stream& st, const float* A, int lda, const float* w, const float* bias, float* out, int M, int K) {
   if (M <= 0) return;
   const ProfScope ps(st, PC_GEMM, 2.0 * M * K, 4.0 * (double(M) * K + K + M));
-  k_gemv_rows<<<cdiv((long long) M * 32, 256), 256, 0, st.s>>>(A, lda, w, bias, out, M, K);
+  launch(st, k_gemv_rows, cdiv((long long) M * 32, 256), 256, 0, A, lda, w, bias, out, M, K);
   PETB_LAUNCH_CHECK(st);
 }
 

@@ -281,6 +281,7 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1)
   if (PAIR) cluster_sync_all();  // the other CTA's barriers exist before anything signals them
   tcgen05_fence_after();
   const uint32_t tmem = *tmem_slot;
+  after_previous();
 
   if (warp < 4) {
     // 24 + 200 + 200 + 88 registers a thread over the four warp groups are the 4 x 128 of the launch
@@ -335,9 +336,11 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1)
         for (int kb = 0; kb < nkb; ++kb) {
           const bool first = kb % L::kDrain == 0, last = kb + 1 == nkb || (kb + 1) % L::kDrain == 0;
           const int b = i % L::kTurns;
-          if (first && !(ok = mbar_wait_warp(tempty + b, ((i / L::kTurns) & 1) ^ 1, abort_flag))) break;
+          if (first) {
+            if (!(ok = mbar_wait_warp(tempty + b, ((i / L::kTurns) & 1) ^ 1, abort_flag))) break;
+            tcgen05_fence_after();
+          }
           if (!(ok = mbar_wait_warp(ready + s, turn, abort_flag))) break;
-          tcgen05_fence_after();
           if (one) {
             const uint32_t acc = tmem + uint32_t(b * L::kAccs * BN);
             const uint32_t a0 = smem_u32(ring_a + s * L::kA), b0 = smem_u32(ring_b + sb * L::kB);
@@ -632,6 +635,7 @@ __global__ void k_pack_weight(const float* __restrict__ W, size_t ld_r, size_t l
 }
 
 __global__ void __launch_bounds__(256) k_row_max(uint32_t* __restrict__ mx, const float* __restrict__ x, int ld, int R, int D4) {
+  after_previous();
   const int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (r >= R) return;
   float m = 0.f;
@@ -749,17 +753,19 @@ void launch_tc(Stream& st, const GemmArgs& a, const PackedB& w) {
   if (EPI == EPI_SILU_BWD || EPI == EPI_SWIGLU_BWD) mi = chunk(a.pre, c_cols, a.ldp, W);
   if (writes_two(EPI) && a.pre) mp = chunk(a.pre, a.N, a.ldp, W);
   cudaLaunchConfig_t cfg{};
-  cudaLaunchAttribute attr{};
-  cfg.blockDim = dim3(L::kThreads), cfg.dynamicSmemBytes = L::kTotal, cfg.stream = st.s;
+  cudaLaunchAttribute attr[2] = {};
+  cfg.blockDim = dim3(L::kThreads), cfg.dynamicSmemBytes = L::kTotal, cfg.stream = st.s, cfg.attrs = attr;
   const long long tiles = (long long) cdiv(a.M, PAIR ? 2 * TBM : TBM) * cdiv(a.N, BN);
   if (PAIR) {
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = 2, attr.val.clusterDim.y = 1, attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr, cfg.numAttrs = 1;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 1;
+    cfg.numAttrs = 1;
     cfg.gridDim = dim3(unsigned(2 * std::min<long long>(tiles, resident_pairs(kernel, cfg))));
   } else {
     cfg.gridDim = dim3(unsigned(std::min<long long>(tiles, state().sms)));
   }
+  attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // see launch()
+  attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
   PETB_CUDA(cudaLaunchKernelEx(&cfg, kernel, ma, mb, ml, mi, mc, mp, a, w.amax, state().err));
   PETB_LAUNCH_CHECK(st);
 }
@@ -829,7 +835,7 @@ PackedB pack_weight(cudaStream_t s, Format fmt, const float* W, size_t ld_r, siz
 
 void row_max(Stream& st, uint32_t* mx, const float* x, int ld, int R, int D) {
   if (R <= 0) return;
-  k_row_max<<<cdiv((long long) R * 32, 256), 256, 0, st.s>>>(mx, x, ld, R, D / 4);
+  launch(st, k_row_max, cdiv((long long) R * 32, 256), 256, 0, mx, x, ld, R, D / 4);
   PETB_LAUNCH_CHECK(st);
 }
 

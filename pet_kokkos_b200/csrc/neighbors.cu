@@ -96,6 +96,7 @@ __device__ inline int warp_inclusive(int v, int lane) {
 // Exclusive scan of a block's chunk into out, its total into sums[block].
 __global__ void __launch_bounds__(kScanThreads) k_scan_chunks(const int* __restrict__ in, int* __restrict__ out,
                                                               int* __restrict__ sums, int n) {
+  after_previous();
   __shared__ int warp_tot[kScanThreads / 32];
   const int base = blockIdx.x * kScanChunk + threadIdx.x * kScanItems;
   int v[kScanItems], t = 0;
@@ -125,6 +126,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_chunks(const int* __restr
 
 // One block: exclusive scan of the chunk totals in place, the grand total into *total.
 __global__ void __launch_bounds__(1024) k_scan_sums(int* __restrict__ sums, int nb, int* __restrict__ total) {
+  after_previous();
   __shared__ int warp_tot[32];
   __shared__ int carry_s;
   if (threadIdx.x == 0) carry_s = 0;
@@ -149,6 +151,7 @@ __global__ void __launch_bounds__(1024) k_scan_sums(int* __restrict__ sums, int 
 }
 
 __global__ void __launch_bounds__(kScanThreads) k_scan_add(int* __restrict__ out, const int* __restrict__ sums, int n) {
+  after_previous();
   const int add = sums[blockIdx.x];
   const int base = blockIdx.x * kScanChunk + threadIdx.x * kScanItems;
 #pragma unroll
@@ -165,12 +168,12 @@ void exclusive_scan(Stream& st, Arena& arena, const int* in, int* out, int n) {
   }
   const int nb = cdiv(n, kScanChunk);
   int* sums = arena.alloc<int>(nb);
-  k_scan_chunks<<<nb, kScanThreads, 0, st.s>>>(in, out, sums, n);
+  launch(st, k_scan_chunks, nb, kScanThreads, 0, in, out, sums, n);
   PETB_LAUNCH_CHECK(st);
-  k_scan_sums<<<1, 1024, 0, st.s>>>(sums, nb, out + n);
+  launch(st, k_scan_sums, 1, 1024, 0, sums, nb, out + n);
   PETB_LAUNCH_CHECK(st);
   if (nb > 1) {
-    k_scan_add<<<nb, kScanThreads, 0, st.s>>>(out, sums, n);
+    launch(st, k_scan_add, nb, kScanThreads, 0, out, sums, n);
     PETB_LAUNCH_CHECK(st);
   }
 }
@@ -180,6 +183,7 @@ void exclusive_scan(Stream& st, Arena& arena, const int* in, int* out, int n) {
 namespace {
 
 __global__ void k_wrap(Geom g, double* __restrict__ posw) {
+  after_previous();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= g.Ntot) return;
   const int b = g.sid[i], per = g.sper[b];
@@ -200,6 +204,7 @@ __global__ void k_wrap(Geom g, double* __restrict__ posw) {
 }
 
 __global__ void k_assign_bins(Geom g, const double* __restrict__ posw, int* __restrict__ abin, int* __restrict__ bcnt) {
+  after_previous();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= g.Ntot) return;
   const int b = g.sid[i];
@@ -224,6 +229,7 @@ __global__ void k_assign_bins(Geom g, const double* __restrict__ posw, int* __re
 // Atoms into their bins in arrival order; k_sort_bins then orders each bin by atom index.
 __global__ void k_fill_bins(int N, const int* __restrict__ abin, const int* __restrict__ bstart, int* __restrict__ fill,
                             int* __restrict__ unsorted) {
+  after_previous();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
   const int c = abin[i];
@@ -233,6 +239,7 @@ __global__ void k_fill_bins(int N, const int* __restrict__ abin, const int* __re
 // One warp per bin: each member goes to its rank among the bin's members.
 __global__ void k_sort_bins(int nbins, const int* __restrict__ bstart, const int* __restrict__ unsorted,
                             int* __restrict__ sorted) {
+  after_previous();
   const int bin = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (bin >= nbins) return;
   const int lo = bstart[bin], n = bstart[bin + 1] - lo;
@@ -264,6 +271,7 @@ struct Walk {
 
 template <bool FILL>
 __global__ void __launch_bounds__(128) k_walk(Walk w, int* __restrict__ ecnt, const int* __restrict__ eoff, RawEdges re) {
+  after_previous();
   const int gi = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (gi >= w.g.Ntot) return;
   const int b = w.g.sid[gi];
@@ -307,6 +315,7 @@ __global__ void __launch_bounds__(128) k_walk(Walk w, int* __restrict__ ecnt, co
 
 // Each edge's partner: the (j, i, -shift) entry in j's own range.
 __global__ void k_reverse(RawEdges re) {
+  after_previous();
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= re.E) return;
   const int i = re.i[e], j = re.j[e];
@@ -321,6 +330,7 @@ __global__ void k_reverse(RawEdges re) {
 }
 
 __global__ void k_edge_vectors(RawEdges re, const double* __restrict__ pos, const double* __restrict__ hc) {
+  after_previous();
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= re.E) return;
   const int i = re.i[e], j = re.j[e], a = re.shift[3 * e], b = re.shift[3 * e + 1], c = re.shift[3 * e + 2];
@@ -334,6 +344,7 @@ __global__ void k_edge_vectors(RawEdges re, const double* __restrict__ pos, cons
 
 // The same for a batch whose structures each have their own cell (the Verlet cache's pairs).
 __global__ void k_edge_vectors_batch(RawEdges re, Geom g) {
+  after_previous();
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= re.E) return;
   const int i = re.i[e], j = re.j[e], a = re.shift[3 * e], b = re.shift[3 * e + 1], c = re.shift[3 * e + 2];
@@ -363,6 +374,7 @@ __device__ inline void wrap_count(const Geom& g, int i, int n[3]) {
 // A searched pair's image in terms of the unwrapped positions: posw = pos - n.cell, so
 // posw_j + s.cell - posw_i = pos_j + (s - n_j + n_i).cell - pos_i (src/device_geometry.cpp:176-181).
 __global__ void k_unwrap_shifts(RawEdges re, Geom g, int* __restrict__ out) {
+  after_previous();
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= re.E) return;
   int ni[3], nj[3];
@@ -376,6 +388,7 @@ __global__ void k_unwrap_shifts(RawEdges re, Geom g, int* __restrict__ out) {
 // strained frame and D = H0^-1 H the strain since. worst = the largest such sum over the atoms.
 __global__ void k_verlet_check(Geom g, const double* __restrict__ pos0, const double* __restrict__ cinv0, double reach,
                                unsigned long long* __restrict__ worst) {
+  after_previous();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= g.Ntot) return;
   const int b = g.sid[i];
@@ -425,6 +438,7 @@ __device__ __forceinline__ double edge_cutoff(const double* acut, const int* nbr
 __global__ void k_keep_count(int NC, const int* __restrict__ roff, const double* __restrict__ dist, double rc,
                              int* __restrict__ kcnt, int* __restrict__ maxm, unsigned long long* __restrict__ pairs,
                              const double* __restrict__ acut, const int* __restrict__ nbr) {
+  after_previous();
   const int a = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (a >= NC) return;
   int c = 0;
@@ -440,6 +454,7 @@ __global__ void k_keep_count(int NC, const int* __restrict__ roff, const double*
 
 // One warp per centre atom: its kept edges to their packed rows, in raw order.
 __global__ void k_pack(int NC, RawEdges re, PackedEdges pk, CutoffSpec cs) {
+  after_previous();
   const int a = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (a >= NC) return;
   int row = pk.off[a];
@@ -472,6 +487,7 @@ __global__ void k_pack(int NC, RawEdges re, PackedEdges pk, CutoffSpec cs) {
 }
 
 __global__ void k_pack_reverse(PackedEdges pk, const int* __restrict__ raw_reverse) {
+  after_previous();
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= pk.E) return;
   if (p >= pk.off[pk.N]) {  // a capacity's dead row: no atom's, no partner
@@ -485,15 +501,18 @@ __global__ void k_pack_reverse(PackedEdges pk, const int* __restrict__ raw_rever
 // Fixed shapes: more kept edges than rows, or more of one atom's than the attention kernels were sized for.
 __global__ void k_check_capacity(const int* __restrict__ off, int NC, const int* __restrict__ maxm, int e_cap, int m_cap,
                                  int* __restrict__ overflow) {
+  after_previous();
   if (off[NC] > e_cap || *maxm > m_cap) *overflow = 1;
 }
 // A step that does not fit still has to stay inside its buffers until the host sees the flag and redoes it: no atom
 // keeps more than m_cap rows, and no row lies past e_cap.
 __global__ void k_clamp_counts(int* __restrict__ kcnt, int NC, int m_cap) {
+  after_previous();
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
   if (a < NC && kcnt[a] > m_cap) kcnt[a] = m_cap;
 }
 __global__ void k_clamp_offsets(int* __restrict__ off, int NC, int e_cap) {
+  after_previous();
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
   if (a <= NC && off[a] > e_cap) off[a] = e_cap;
 }
@@ -502,7 +521,7 @@ __global__ void k_clamp_offsets(int* __restrict__ off, int NC, int e_cap) {
 
 void wrap_positions(Stream& st, const Geom& g, double* posw) {
   if (g.Ntot == 0) return;
-  k_wrap<<<cdiv(g.Ntot, 256), 256, 0, st.s>>>(g, posw);
+  launch(st, k_wrap, cdiv(g.Ntot, 256), 256, 0, g, posw);
   PETB_LAUNCH_CHECK(st);
 }
 
@@ -524,16 +543,16 @@ RawEdges cell_list_search(Stream& st, Arena& arena, const Geom& g, const double*
   int* batom = arena.alloc<int>(N);
   int* ecnt = arena.alloc<int>(N);
   PETB_CUDA(cudaMemsetAsync(bcnt, 0, 2 * size_t(nbins) * sizeof(int), st.s));
-  k_assign_bins<<<cdiv(N, 256), 256, 0, st.s>>>(g, posw, abin, bcnt);
+  launch(st, k_assign_bins, cdiv(N, 256), 256, 0, g, posw, abin, bcnt);
   PETB_LAUNCH_CHECK(st);
   exclusive_scan(st, arena, bcnt, bstart, nbins);
-  k_fill_bins<<<cdiv(N, 256), 256, 0, st.s>>>(N, abin, bstart, fill, unsorted);
+  launch(st, k_fill_bins, cdiv(N, 256), 256, 0, N, abin, bstart, fill, unsorted);
   PETB_LAUNCH_CHECK(st);
-  k_sort_bins<<<cdiv(size_t(nbins) * 32, 128), 128, 0, st.s>>>(nbins, bstart, unsorted, batom);
+  launch(st, k_sort_bins, cdiv(size_t(nbins) * 32, 128), 128, 0, nbins, bstart, unsorted, batom);
   PETB_LAUNCH_CHECK(st);
 
   const Walk w{g, posw, abin, bstart, batom, cutoff * cutoff};
-  k_walk<false><<<cdiv(size_t(N) * 32, 128), 128, 0, st.s>>>(w, ecnt, nullptr, re);
+  launch(st, k_walk<false>, cdiv(size_t(N) * 32, 128), 128, 0, w, ecnt, nullptr, re);
   PETB_LAUNCH_CHECK(st);
   exclusive_scan(st, arena, ecnt, re.off, N);
   int E = 0;
@@ -549,7 +568,7 @@ RawEdges cell_list_search(Stream& st, Arena& arena, const Geom& g, const double*
   re.reverse = arena.alloc<int>(Ea);
   // The count and the fill are the same instantiated walk over the same inputs with
   // contraction off, so they agree on every candidate.
-  k_walk<true><<<cdiv(size_t(N) * 32, 128), 128, 0, st.s>>>(w, nullptr, re.off, re);
+  launch(st, k_walk<true>, cdiv(size_t(N) * 32, 128), 128, 0, w, nullptr, re.off, re);
   PETB_LAUNCH_CHECK(st);
   return re;
 }
@@ -557,33 +576,33 @@ RawEdges cell_list_search(Stream& st, Arena& arena, const Geom& g, const double*
 void find_reverse(Stream& st, const RawEdges& re, int) {
   if (re.E == 0) return;
   const ProfScope ps(st, PC_GEOMETRY, 0.0, 52.0 * re.E);
-  k_reverse<<<cdiv(re.E, 256), 256, 0, st.s>>>(re);
+  launch(st, k_reverse, cdiv(re.E, 256), 256, 0, re);
   PETB_LAUNCH_CHECK(st);
 }
 
 void edge_vectors(Stream& st, const RawEdges& re, const double* pos, const double* cell9) {
   if (re.E == 0) return;
-  k_edge_vectors<<<cdiv(re.E, 256), 256, 0, st.s>>>(re, pos, cell9);
+  launch(st, k_edge_vectors, cdiv(re.E, 256), 256, 0, re, pos, cell9);
   PETB_LAUNCH_CHECK(st);
 }
 
 void edge_vectors_batch(Stream& st, const RawEdges& re, const Geom& g) {
   if (re.E == 0) return;
   const ProfScope ps(st, PC_GEOMETRY, 0.0, 52.0 * re.E);
-  k_edge_vectors_batch<<<cdiv(re.E, 256), 256, 0, st.s>>>(re, g);
+  launch(st, k_edge_vectors_batch, cdiv(re.E, 256), 256, 0, re, g);
   PETB_LAUNCH_CHECK(st);
 }
 
 void unwrap_shifts(Stream& st, const RawEdges& re, const Geom& g, int* out) {
   if (re.E == 0) return;
-  k_unwrap_shifts<<<cdiv(re.E, 256), 256, 0, st.s>>>(re, g, out);
+  launch(st, k_unwrap_shifts, cdiv(re.E, 256), 256, 0, re, g, out);
   PETB_LAUNCH_CHECK(st);
 }
 
 void verlet_check(Stream& st, const Geom& g, const double* pos0, const double* cinv0, double reach, double* worst) {
   PETB_CUDA(cudaMemsetAsync(worst, 0, sizeof(double), st.s));
   if (g.Ntot == 0) return;
-  k_verlet_check<<<cdiv(g.Ntot, 256), 256, 0, st.s>>>(g, pos0, cinv0, reach, reinterpret_cast<unsigned long long*>(worst));
+  launch(st, k_verlet_check, cdiv(g.Ntot, 256), 256, 0, g, pos0, cinv0, reach, reinterpret_cast<unsigned long long*>(worst));
   PETB_LAUNCH_CHECK(st);
 }
 
@@ -601,7 +620,7 @@ PackedEdges pack_edges(Stream& st, Arena& arena, const RawEdges& re, int NC, con
   PETB_CUDA(cudaMemsetAsync(maxm, 0, sizeof(int), st.s));
   PETB_CUDA(cudaMemsetAsync(pairs, 0, 8, st.s));
   if (NC > 0) {
-    k_keep_count<<<cdiv(size_t(NC) * 32, 256), 256, 0, st.s>>>(NC, re.off, re.dist, cs.cutoff, kcnt, maxm, pairs, ad.acut, re.j);
+    launch(st, k_keep_count, cdiv(size_t(NC) * 32, 256), 256, 0, NC, re.off, re.dist, cs.cutoff, kcnt, maxm, pairs, ad.acut, re.j);
     PETB_LAUNCH_CHECK(st);
   }
   exclusive_scan(st, arena, kcnt, pk.off, NC);
@@ -624,11 +643,11 @@ PackedEdges pack_edges(Stream& st, Arena& arena, const RawEdges& re, int NC, con
   pk.raw_of = arena.alloc<int>(Ea);
   pk.packed_of_raw = arena.alloc<int>(Er);
   if (NC > 0 && re.E > 0) {
-    k_pack<<<cdiv(size_t(NC) * 32, 256), 256, 0, st.s>>>(NC, re, pk, cs);
+    launch(st, k_pack, cdiv(size_t(NC) * 32, 256), 256, 0, NC, re, pk, cs);
     PETB_LAUNCH_CHECK(st);
     // Edges whose centre is not a centre atom here (ghost rows of an exchanged list) keep no row.
     if (pk.E > 0) {
-      k_pack_reverse<<<cdiv(pk.E, 256), 256, 0, st.s>>>(pk, re.reverse);
+      launch(st, k_pack_reverse, cdiv(pk.E, 256), 256, 0, pk, re.reverse);
       PETB_LAUNCH_CHECK(st);
     }
   }
@@ -652,14 +671,14 @@ PackedEdges pack_edges_fixed(Stream& st, Arena& arena, const RawEdges& re, int N
   unsigned long long* pr = reinterpret_cast<unsigned long long*>(arena.alloc_bytes(8));
   PETB_CUDA(cudaMemsetAsync(maxm, 0, sizeof(int), st.s));
   PETB_CUDA(cudaMemsetAsync(pr, 0, 8, st.s));
-  k_keep_count<<<cdiv(size_t(NC) * 32, 256), 256, 0, st.s>>>(NC, re.off, re.dist, cs.cutoff, kcnt, maxm, pr, ad.acut, re.j);
+  launch(st, k_keep_count, cdiv(size_t(NC) * 32, 256), 256, 0, NC, re.off, re.dist, cs.cutoff, kcnt, maxm, pr, ad.acut, re.j);
   PETB_LAUNCH_CHECK(st);
-  k_clamp_counts<<<cdiv(NC, 256), 256, 0, st.s>>>(kcnt, NC, m_cap);  // maxm already holds the unclamped maximum
+  launch(st, k_clamp_counts, cdiv(NC, 256), 256, 0, kcnt, NC, m_cap);  // maxm already holds the unclamped maximum
   PETB_LAUNCH_CHECK(st);
   exclusive_scan(st, arena, kcnt, pk.off, NC);
-  k_check_capacity<<<1, 1, 0, st.s>>>(pk.off, NC, maxm, e_cap, m_cap, overflow);
+  launch(st, k_check_capacity, 1, 1, 0, pk.off, NC, maxm, e_cap, m_cap, overflow);
   PETB_LAUNCH_CHECK(st);
-  k_clamp_offsets<<<cdiv(NC + 1, 256), 256, 0, st.s>>>(pk.off, NC, e_cap);
+  launch(st, k_clamp_offsets, cdiv(NC + 1, 256), 256, 0, pk.off, NC, e_cap);
   PETB_LAUNCH_CHECK(st);
   const size_t Ea = e_cap > 0 ? e_cap : 1, Er = re.E > 0 ? re.E : 1;
   // one block for the row arrays, cleared in one go: dead rows read as zeros
@@ -680,11 +699,11 @@ PackedEdges pack_edges_fixed(Stream& st, Arena& arena, const RawEdges& re, int N
   }
   pk.packed_of_raw = arena.alloc<int>(Er);
   if (re.E > 0) {
-    k_pack<<<cdiv(size_t(NC) * 32, 256), 256, 0, st.s>>>(NC, re, pk, cs);
+    launch(st, k_pack, cdiv(size_t(NC) * 32, 256), 256, 0, NC, re, pk, cs);
     PETB_LAUNCH_CHECK(st);
   }
   if (e_cap > 0) {
-    k_pack_reverse<<<cdiv(e_cap, 256), 256, 0, st.s>>>(pk, re.reverse);
+    launch(st, k_pack_reverse, cdiv(e_cap, 256), 256, 0, pk, re.reverse);
     PETB_LAUNCH_CHECK(st);
   }
   return pk;

@@ -42,6 +42,7 @@ __device__ __forceinline__ void raise_row(uint32_t* mx, int r, int D4, float m) 
 
 __global__ void k_gather_rows(float* __restrict__ out, const float* __restrict__ table, const int* __restrict__ idx, int R,
                               int D4, uint32_t* __restrict__ mx) {
+  after_previous();
   const size_t t = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (t >= size_t(R) * D4) return;
   const int r = int(t / D4), q = int(t % D4);
@@ -51,6 +52,7 @@ __global__ void k_gather_rows(float* __restrict__ out, const float* __restrict__
 }
 
 __global__ void k_compress0(GemmArgs p) {
+  after_previous();
   const size_t t = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
   const int D4 = p.N / 4;
   if (t >= size_t(p.M) * D4) return;
@@ -63,6 +65,7 @@ __global__ void k_compress0(GemmArgs p) {
 __global__ void __launch_bounds__(256) k_norm_fwd(float* __restrict__ out, float* __restrict__ in, const float* __restrict__ add,
                                                   const float* __restrict__ w, const float* __restrict__ bias, int R, int D,
                                                   uint32_t* __restrict__ mx) {
+  after_previous();
   const int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (r >= R) return;
   float* x = in + size_t(r) * D;
@@ -108,6 +111,7 @@ __device__ __forceinline__ const float* partner_row(const float* oe, const int* 
 
 __global__ void k_gather_live(float* __restrict__ out, const float* __restrict__ src, int ld, int col0,
                               const int* __restrict__ live_packed, int n_live, int D4) {
+  after_previous();
   const size_t t = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (t >= size_t(n_live) * D4) return;
   const int l = int(t / D4), q = int(t % D4), k = live_packed[l];
@@ -120,6 +124,7 @@ template <int NV>
 __global__ void __launch_bounds__(256) k_norm_fwd_v(float* __restrict__ out, float* __restrict__ in, const float* __restrict__ add,
                                                     const float* __restrict__ w, const float* __restrict__ bias, int R,
                                                     uint32_t* __restrict__ mx) {
+  after_previous();
   constexpr int D = 128 * NV;
   const int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (r >= R) return;
@@ -174,6 +179,7 @@ __global__ void __launch_bounds__(256) k_concat_norm_fwd(float* __restrict__ out
                                                          const int* __restrict__ rev, float* __restrict__ ie,
                                                          const float* __restrict__ w, const float* __restrict__ bias, int E,
                                                          int D, RemoteRows rm, uint32_t* __restrict__ mx) {
+  after_previous();
   const int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (k >= E) return;
   const int W = 2 * D;
@@ -212,6 +218,7 @@ struct RowStats {
 __global__ void __launch_bounds__(256) k_norm_bwd(float* __restrict__ in_adj, const float* __restrict__ out_adj,
                                                   const float* __restrict__ in, const float* __restrict__ w, bool ln, int R, int D,
                                                   int acc_row0, float* __restrict__ also, uint32_t* __restrict__ mx) {
+  after_previous();
   const int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (r >= R) return;
   const float* x = in + size_t(r) * D;
@@ -249,6 +256,7 @@ template <int NV>
 __global__ void __launch_bounds__(256) k_norm_bwd_v(float* __restrict__ in_adj, const float* __restrict__ out_adj,
                                                     const float* __restrict__ in, const float* __restrict__ w, bool ln, int R,
                                                     int acc_row0, float* __restrict__ also, uint32_t* __restrict__ mx) {
+  after_previous();
   constexpr int D = 128 * NV;
   const int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (r >= R) return;
@@ -322,6 +330,7 @@ __global__ void __launch_bounds__(256) k_concat_norm_bwd(float* __restrict__ edg
                                                          const float* __restrict__ ie_adj, const float* __restrict__ w, int E,
                                                          int D, RemoteRows rm, const float* __restrict__ remote_adj,
                                                          uint32_t* __restrict__ mx) {
+  after_previous();
   const int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (k >= E) return;
   const int W = 2 * D, r = rev[k];
@@ -361,6 +370,7 @@ __global__ void __launch_bounds__(256) k_concat_norm_bwd_pair(float* __restrict_
                                                               const float* __restrict__ oe, const int* __restrict__ rev,
                                                               const float* __restrict__ ie_adj, const float* __restrict__ w,
                                                               int E, uint32_t* __restrict__ mx) {
+  after_previous();
   constexpr int D = 128 * NV, W = 2 * D;
   const int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (k >= E) return;
@@ -460,6 +470,7 @@ __global__ void __launch_bounds__(256) k_concat_norm_remote_bwd(float* __restric
                                                                 const float* __restrict__ oe, const float* __restrict__ w,
                                                                 const int* __restrict__ live_packed, int n_live, int D,
                                                                 RemoteRows rm) {
+  after_previous();
   const int l = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (l >= n_live) return;
   const int k = live_packed[l], W = 2 * D;
@@ -475,6 +486,7 @@ __global__ void __launch_bounds__(256) k_concat_norm_remote_bwd(float* __restric
 
 __global__ void __launch_bounds__(256) k_compress_geometry_bwd(float* __restrict__ x4_adj, const float* __restrict__ g,
                                                                const float* __restrict__ wx, int E, int D) {
+  after_previous();
   const int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (k >= E) return;
   float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
@@ -494,6 +506,7 @@ __global__ void __launch_bounds__(256) k_compress_geometry_bwd(float* __restrict
 __global__ void k_readout_energy(float* __restrict__ net, double* __restrict__ per_atom, const float* __restrict__ node_pred,
                                  const float* __restrict__ edge_pred, PackedEdges pk, const double* __restrict__ comp,
                                  double scale, bool acc, bool assemble) {
+  after_previous();
   const int n = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (n >= pk.N) return;
   double s = 0.0;
@@ -510,6 +523,7 @@ __global__ void k_readout_energy(float* __restrict__ net, double* __restrict__ p
 __global__ void k_readout_seed_bwd(float* __restrict__ out, const float* __restrict__ w, const float* __restrict__ pre,
                                    const float* __restrict__ cut, const int* __restrict__ center, int n_local, int R, int Dh4,
                                    uint32_t* __restrict__ mx) {
+  after_previous();
   const size_t t = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (t >= size_t(R) * Dh4) return;
   const int r = int(t / Dh4), q = int(t % Dh4);
@@ -524,6 +538,7 @@ __global__ void k_readout_seed_bwd(float* __restrict__ out, const float* __restr
 
 __global__ void k_cutoff_share(float* __restrict__ cf_adj, const float* __restrict__ cfh, const float* __restrict__ cut, int N,
                                int E, int H) {
+  after_previous();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= E) return;
   const float cf = cut[k];
@@ -534,12 +549,14 @@ __global__ void k_cutoff_share(float* __restrict__ cf_adj, const float* __restri
 }
 
 __global__ void k_add_inplace(float* __restrict__ a, const float* __restrict__ b, size_t n) {
+  after_previous();
   const size_t t = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (t < n) a[t] += b[t];
 }
 
 __global__ void k_message_average(float* __restrict__ ie, const float* __restrict__ oe, const int* __restrict__ rev, int E,
                                   int D4, RemoteRows rm, uint32_t* __restrict__ mx) {
+  after_previous();
   const size_t t = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (t >= size_t(E) * D4) return;
   const int k = int(t / D4), q = int(t % D4);
@@ -554,6 +571,7 @@ __global__ void k_message_average(float* __restrict__ ie, const float* __restric
 // The adjoint of message_average: ie_adj_out(k) = 0.5 ie_adj_in(k); oe_adj(k) += 0.5 ie_adj_in(rev k).
 __global__ void k_message_average_bwd(float* __restrict__ ie_out, float* __restrict__ oe_adj, const float* __restrict__ ie_in,
                                       const int* __restrict__ rev, int E, int D4, RemoteRows rm) {
+  after_previous();
   const size_t t = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (t >= size_t(E) * D4) return;
   const int k = int(t / D4), q = int(t % D4);
@@ -588,6 +606,7 @@ __device__ inline double cutoff_ddist(double d, double rc, double w, int kind) {
 __global__ void k_edge_grad(double* __restrict__ grad, PackedEdges pk, const float* __restrict__ x4_adj,
                             const float* __restrict__ cutoff_adj, const float* __restrict__ cf_adj, CutoffSpec cs,
                             double* __restrict__ pc_adj) {
+  after_previous();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= pk.E) return;
   if (pc_adj && k >= pk.off[pk.N]) {  // a capacity's dead row
@@ -608,6 +627,7 @@ __global__ void k_edge_grad(double* __restrict__ grad, PackedEdges pk, const flo
 // One warp per atom: F(i) = scale sum_k [g(k) - g(rev k)], W(i) = scale sum_k v (x) g, lanes striding
 // the atom's edges and combining in a fixed tree.
 __global__ void __launch_bounds__(256) k_fold_forces(ForceOut out, PackedEdges pk, double scale) {
+  after_previous();
   const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (i >= pk.n_atoms) return;
   double f[3] = {0, 0, 0}, w[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
@@ -630,6 +650,7 @@ __global__ void __launch_bounds__(256) k_fold_forces(ForceOut out, PackedEdges p
 
 // One warp per (structure, component): lane l sums every 32nd atom from the l-th, then a fixed tree.
 __global__ void k_struct_sum(double* __restrict__ out, const double* __restrict__ x, const int* __restrict__ soff, int B, int T) {
+  after_previous();
   const int u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (u >= B * T) return;
   const int b = u / T, t = u % T;
@@ -640,6 +661,7 @@ __global__ void k_struct_sum(double* __restrict__ out, const double* __restrict_
 }
 
 __global__ void k_voigt(double* __restrict__ w6, const double* __restrict__ w9, int B) {
+  after_previous();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= B) return;
   const double* w = w9 + 9 * b;
@@ -655,7 +677,7 @@ inline unsigned blocks_for(size_t n, int per) { return (unsigned) ((n + per - 1)
 void gather_rows(Stream& st, float* out, const float* table, const int* idx, int R, int D, uint32_t* mx) {
   if (R == 0) return;
   const ProfScope ps(st, PC_GATHER, 0.0, 8.0 * double(R) * D);
-  k_gather_rows<<<blocks_for(size_t(R) * (D / 4), 256), 256, 0, st.s>>>(out, table, idx, R, D / 4, mx);
+  launch(st, k_gather_rows, blocks_for(size_t(R) * (D / 4), 256), 256, 0, out, table, idx, R, D / 4, mx);
   PETB_LAUNCH_CHECK(st);
 }
 
@@ -666,7 +688,7 @@ void compress0(Stream& st, float* out, float* pre, const float* b, const float* 
   GemmArgs p;
   p.M = pk.E, p.N = D, p.C = out, p.ldc = D, p.pre = pre, p.ldp = D, p.bias = b, p.tab = tab, p.wx = wx, p.sp = pk.species;
   p.vec = pk.vec, p.dist = pk.dist, p.c_max = mx, p.epi = EPI_COMPRESS;
-  k_compress0<<<blocks_for(size_t(pk.E) * (D / 4), 256), 256, 0, st.s>>>(p);
+  launch(st, k_compress0, blocks_for(size_t(pk.E) * (D / 4), 256), 256, 0, p);
   PETB_LAUNCH_CHECK(st);
 }
 
@@ -675,11 +697,11 @@ void norm_fwd(Stream& st, float* out, float* in, const float* add, const float* 
   const ProfScope ps(st, PC_NORM, 6.0 * double(R) * D, (add ? 16.0 : 8.0) * double(R) * D);
   const unsigned blocks = blocks_for(size_t(R) * 32, 256);
   switch (D) {  // whole rows in registers for the usual widths
-    case 128: k_norm_fwd_v<1><<<blocks, 256, 0, st.s>>>(out, in, add, w, bias, R, mx); break;
-    case 256: k_norm_fwd_v<2><<<blocks, 256, 0, st.s>>>(out, in, add, w, bias, R, mx); break;
-    case 512: k_norm_fwd_v<4><<<blocks, 256, 0, st.s>>>(out, in, add, w, bias, R, mx); break;
-    case 1024: k_norm_fwd_v<8><<<blocks, 256, 0, st.s>>>(out, in, add, w, bias, R, mx); break;
-    default: k_norm_fwd<<<blocks, 256, 0, st.s>>>(out, in, add, w, bias, R, D, mx);
+    case 128: launch(st, k_norm_fwd_v<1>, blocks, 256, 0, out, in, add, w, bias, R, mx); break;
+    case 256: launch(st, k_norm_fwd_v<2>, blocks, 256, 0, out, in, add, w, bias, R, mx); break;
+    case 512: launch(st, k_norm_fwd_v<4>, blocks, 256, 0, out, in, add, w, bias, R, mx); break;
+    case 1024: launch(st, k_norm_fwd_v<8>, blocks, 256, 0, out, in, add, w, bias, R, mx); break;
+    default: launch(st, k_norm_fwd, blocks, 256, 0, out, in, add, w, bias, R, D, mx);
   }
   PETB_LAUNCH_CHECK(st);
 }
@@ -687,7 +709,7 @@ void norm_fwd(Stream& st, float* out, float* in, const float* add, const float* 
 void gather_live(Stream& st, float* out, const float* src, int ld, int col0, const int* live_packed, int n_live, int D) {
   if (n_live == 0) return;
   const ProfScope ps(st, PC_GATHER, 0.0, 8.0 * double(n_live) * D);
-  k_gather_live<<<blocks_for(size_t(n_live) * (D / 4), 256), 256, 0, st.s>>>(out, src, ld, col0, live_packed, n_live, D / 4);
+  launch(st, k_gather_live, blocks_for(size_t(n_live) * (D / 4), 256), 256, 0, out, src, ld, col0, live_packed, n_live, D / 4);
   PETB_LAUNCH_CHECK(st);
 }
 
@@ -695,7 +717,7 @@ void concat_norm_fwd(Stream& st, float* out, const float* oe, const int* rev, fl
                      int E, int D, RemoteRows remote, uint32_t* mx) {
   if (E == 0) return;
   const ProfScope ps(st, PC_NORM, 12.0 * double(E) * D, 24.0 * double(E) * D);
-  k_concat_norm_fwd<<<blocks_for(size_t(E) * 32, 256), 256, 0, st.s>>>(out, oe, rev, ie, w, bias, E, D, remote, mx);
+  launch(st, k_concat_norm_fwd, blocks_for(size_t(E) * 32, 256), 256, 0, out, oe, rev, ie, w, bias, E, D, remote, mx);
   PETB_LAUNCH_CHECK(st);
 }
 
@@ -705,11 +727,11 @@ void norm_bwd(Stream& st, float* in_adj, const float* out_adj, const float* in, 
   const ProfScope ps(st, PC_NORM, 10.0 * double(R) * D, (acc_row0 < R ? 16.0 : 12.0) * double(R) * D);
   const unsigned blocks = blocks_for(size_t(R) * 32, 256);
   switch (D) {
-    case 128: k_norm_bwd_v<1><<<blocks, 256, 0, st.s>>>(in_adj, out_adj, in, w, layernorm, R, acc_row0, also, mx); break;
-    case 256: k_norm_bwd_v<2><<<blocks, 256, 0, st.s>>>(in_adj, out_adj, in, w, layernorm, R, acc_row0, also, mx); break;
-    case 512: k_norm_bwd_v<4><<<blocks, 256, 0, st.s>>>(in_adj, out_adj, in, w, layernorm, R, acc_row0, also, mx); break;
-    case 1024: k_norm_bwd_v<8><<<blocks, 256, 0, st.s>>>(in_adj, out_adj, in, w, layernorm, R, acc_row0, also, mx); break;
-    default: k_norm_bwd<<<blocks, 256, 0, st.s>>>(in_adj, out_adj, in, w, layernorm, R, D, acc_row0, also, mx);
+    case 128: launch(st, k_norm_bwd_v<1>, blocks, 256, 0, in_adj, out_adj, in, w, layernorm, R, acc_row0, also, mx); break;
+    case 256: launch(st, k_norm_bwd_v<2>, blocks, 256, 0, in_adj, out_adj, in, w, layernorm, R, acc_row0, also, mx); break;
+    case 512: launch(st, k_norm_bwd_v<4>, blocks, 256, 0, in_adj, out_adj, in, w, layernorm, R, acc_row0, also, mx); break;
+    case 1024: launch(st, k_norm_bwd_v<8>, blocks, 256, 0, in_adj, out_adj, in, w, layernorm, R, acc_row0, also, mx); break;
+    default: launch(st, k_norm_bwd, blocks, 256, 0, in_adj, out_adj, in, w, layernorm, R, D, acc_row0, also, mx);
   }
   PETB_LAUNCH_CHECK(st);
 }
@@ -721,13 +743,13 @@ void concat_norm_bwd(Stream& st, float* edge_adj, const float* out_adj, const fl
   const auto grid = blocks_for(size_t(E) * 32, 256);
   const bool one_rank = !remote.of && !remote_adj;
   if (one_rank && D == 128)
-    k_concat_norm_bwd_pair<1><<<grid, 256, 0, st.s>>>(edge_adj, out_adj, oe, rev, ie_adj, w, E, mx);
+    launch(st, k_concat_norm_bwd_pair<1>, grid, 256, 0, edge_adj, out_adj, oe, rev, ie_adj, w, E, mx);
   else if (one_rank && D == 256)
-    k_concat_norm_bwd_pair<2><<<grid, 256, 0, st.s>>>(edge_adj, out_adj, oe, rev, ie_adj, w, E, mx);
+    launch(st, k_concat_norm_bwd_pair<2>, grid, 256, 0, edge_adj, out_adj, oe, rev, ie_adj, w, E, mx);
   else if (one_rank && D == 512)
-    k_concat_norm_bwd_pair<4><<<grid, 256, 0, st.s>>>(edge_adj, out_adj, oe, rev, ie_adj, w, E, mx);
+    launch(st, k_concat_norm_bwd_pair<4>, grid, 256, 0, edge_adj, out_adj, oe, rev, ie_adj, w, E, mx);
   else
-    k_concat_norm_bwd<<<grid, 256, 0, st.s>>>(edge_adj, out_adj, oe, rev, ie_adj, w, E, D, remote, remote_adj, mx);
+    launch(st, k_concat_norm_bwd, grid, 256, 0, edge_adj, out_adj, oe, rev, ie_adj, w, E, D, remote, remote_adj, mx);
   PETB_LAUNCH_CHECK(st);
 }
 
@@ -735,7 +757,7 @@ void concat_norm_remote_bwd(Stream& st, float* send, const float* out_adj, const
                             const int* live_packed, int n_live, int D, RemoteRows remote) {
   if (n_live == 0) return;
   const ProfScope ps(st, PC_NORM, 20.0 * double(n_live) * D, 16.0 * double(n_live) * D);
-  k_concat_norm_remote_bwd<<<blocks_for(size_t(n_live) * 32, 256), 256, 0, st.s>>>(send, out_adj, oe, w, live_packed, n_live, D,
+  launch(st, k_concat_norm_remote_bwd, blocks_for(size_t(n_live) * 32, 256), 256, 0, send, out_adj, oe, w, live_packed, n_live, D,
                                                                                   remote);
   PETB_LAUNCH_CHECK(st);
 }
@@ -743,7 +765,7 @@ void concat_norm_remote_bwd(Stream& st, float* send, const float* out_adj, const
 void compress_geometry_bwd(Stream& st, float* x4_adj, const float* g, const float* wx, int E, int D) {
   if (E == 0) return;
   const ProfScope ps(st, PC_ELEMENTWISE, 8.0 * double(E) * D, 4.0 * double(E) * D);
-  k_compress_geometry_bwd<<<blocks_for(size_t(E) * 32, 256), 256, 0, st.s>>>(x4_adj, g, wx, E, D);
+  launch(st, k_compress_geometry_bwd, blocks_for(size_t(E) * 32, 256), 256, 0, x4_adj, g, wx, E, D);
   PETB_LAUNCH_CHECK(st);
 }
 
@@ -751,7 +773,7 @@ void readout_energy(Stream& st, float* net, double* per_atom, const float* node_
                     const PackedEdges& pk, const double* composition, double scale, bool acc, bool assemble) {
   if (pk.N == 0) return;
   const ProfScope ps(st, PC_GATHER, 2.0 * pk.E, 8.0 * double(pk.E) + 16.0 * pk.N);
-  k_readout_energy<<<blocks_for(size_t(pk.N) * 32, 256), 256, 0, st.s>>>(net, per_atom, node_pred, edge_pred, pk, composition,
+  launch(st, k_readout_energy, blocks_for(size_t(pk.N) * 32, 256), 256, 0, net, per_atom, node_pred, edge_pred, pk, composition,
                                                                         scale, acc, assemble);
   PETB_LAUNCH_CHECK(st);
 }
@@ -760,21 +782,21 @@ void readout_seed_bwd(Stream& st, float* out, const float* w, const float* pre, 
                       int n_local, int R, int Dh, uint32_t* mx) {
   if (R == 0) return;
   const ProfScope ps(st, PC_ELEMENTWISE, 8.0 * double(R) * Dh, 8.0 * double(R) * Dh);
-  k_readout_seed_bwd<<<blocks_for(size_t(R) * (Dh / 4), 256), 256, 0, st.s>>>(out, w, pre, cut, center, n_local, R, Dh / 4, mx);
+  launch(st, k_readout_seed_bwd, blocks_for(size_t(R) * (Dh / 4), 256), 256, 0, out, w, pre, cut, center, n_local, R, Dh / 4, mx);
   PETB_LAUNCH_CHECK(st);
 }
 
 void cutoff_share(Stream& st, float* cf_adj, const float* cfh, const float* cut, int N, int E, int H) {
   if (E == 0) return;
   const ProfScope ps(st, PC_ELEMENTWISE, double(E) * H, 4.0 * double(E) * (H + 2));
-  k_cutoff_share<<<blocks_for(E, 256), 256, 0, st.s>>>(cf_adj, cfh, cut, N, E, H);
+  launch(st, k_cutoff_share, blocks_for(E, 256), 256, 0, cf_adj, cfh, cut, N, E, H);
   PETB_LAUNCH_CHECK(st);
 }
 
 void add_inplace(Stream& st, float* a, const float* b, size_t n) {
   if (n == 0) return;
   const ProfScope ps(st, PC_ELEMENTWISE, double(n), 12.0 * double(n));
-  k_add_inplace<<<blocks_for(n, 256), 256, 0, st.s>>>(a, b, n);
+  launch(st, k_add_inplace, blocks_for(n, 256), 256, 0, a, b, n);
   PETB_LAUNCH_CHECK(st);
 }
 
@@ -782,7 +804,7 @@ void message_average(Stream& st, float* ie, const float* oe, const int* rev, int
                      uint32_t* mx) {
   if (E == 0) return;
   const ProfScope ps(st, PC_GATHER, 2.0 * double(E) * D, 12.0 * double(E) * D);
-  k_message_average<<<blocks_for(size_t(E) * (D / 4), 256), 256, 0, st.s>>>(ie, oe, rev, E, D / 4, remote, mx);
+  launch(st, k_message_average, blocks_for(size_t(E) * (D / 4), 256), 256, 0, ie, oe, rev, E, D / 4, remote, mx);
   PETB_LAUNCH_CHECK(st);
 }
 
@@ -790,7 +812,7 @@ void message_average_bwd(Stream& st, float* ie_adj_out, float* oe_adj, const flo
                          RemoteRows remote_adj) {
   if (E == 0) return;
   const ProfScope ps(st, PC_GATHER, 2.0 * double(E) * D, 20.0 * double(E) * D);
-  k_message_average_bwd<<<blocks_for(size_t(E) * (D / 4), 256), 256, 0, st.s>>>(ie_adj_out, oe_adj, ie_adj_in, rev, E, D / 4,
+  launch(st, k_message_average_bwd, blocks_for(size_t(E) * (D / 4), 256), 256, 0, ie_adj_out, oe_adj, ie_adj_in, rev, E, D / 4,
                                                                               remote_adj);
   PETB_LAUNCH_CHECK(st);
 }
@@ -800,24 +822,24 @@ void forces_and_virial(Stream& st, Arena& arena, ForceOut& out, const PackedEdge
   const ProfScope ps(st, PC_FORCES, 40.0 * pk.E, 100.0 * double(pk.E) + 96.0 * pk.n_atoms);
   double* pc_adj = pk.adaptive.acut ? arena.alloc<double>(pk.E > 0 ? pk.E : 1) : nullptr;
   if (pk.E > 0) {
-    k_edge_grad<<<blocks_for(pk.E, 256), 256, 0, st.s>>>(out.edge_grad, pk, x4_adj, cutoff_adj, cf_adj, cs, pc_adj);
+    launch(st, k_edge_grad, blocks_for(pk.E, 256), 256, 0, out.edge_grad, pk, x4_adj, cutoff_adj, cf_adj, cs, pc_adj);
     PETB_LAUNCH_CHECK(st);
   }
   if (pk.n_atoms > 0) {
-    k_fold_forces<<<blocks_for(size_t(pk.n_atoms) * 32, 256), 256, 0, st.s>>>(out, pk, scale);
+    launch(st, k_fold_forces, blocks_for(size_t(pk.n_atoms) * 32, 256), 256, 0, out, pk, scale);
     PETB_LAUNCH_CHECK(st);
   }
   // the adaptive cutoff's share, folded over the raw list, before the per-structure sums
   if (pc_adj) adaptive_backward(st, arena, pk, cs, pc_adj, scale, out.forces, out.vir_atom, &out.adaptive_gmag);
-  k_struct_sum<<<blocks_for(size_t(pk.B) * 9 * 32, 256), 256, 0, st.s>>>(out.vir9, out.vir_atom, pk.soff, pk.B, 9);
+  launch(st, k_struct_sum, blocks_for(size_t(pk.B) * 9 * 32, 256), 256, 0, out.vir9, out.vir_atom, pk.soff, pk.B, 9);
   PETB_LAUNCH_CHECK(st);
-  k_voigt<<<blocks_for(pk.B, 128), 128, 0, st.s>>>(out.vir6, out.vir9, pk.B);
+  launch(st, k_voigt, blocks_for(pk.B, 128), 128, 0, out.vir6, out.vir9, pk.B);
   PETB_LAUNCH_CHECK(st);
 }
 
 void structure_energy(Stream& st, double* energy, const double* per_atom, const int* soff, int B) {
   const ProfScope ps(st, PC_FORCES, 0.0, 8.0 * B);
-  k_struct_sum<<<blocks_for(size_t(B) * 32, 256), 256, 0, st.s>>>(energy, per_atom, soff, B, 1);
+  launch(st, k_struct_sum, blocks_for(size_t(B) * 32, 256), 256, 0, energy, per_atom, soff, B, 1);
   PETB_LAUNCH_CHECK(st);
 }
 
