@@ -26,7 +26,16 @@
 // cluster-scope release: that one (or an acquire on the waiting side) costs 2500 clocks a step. The converter's own writes
 // are ordered by the proxy fence before the arrival, and nothing but the tensor core reads them.
 //
-// What bounds it: the SM's shared-memory data path (one 128-byte wavefront per clock for TMA traffic, the tensor core's
+// The other tiles (Tile::TA: not the pairs, not the tf32 formats, and with parts to spare in tensor memory) keep A's parts in
+// tensor memory instead: two groups of four converter warps (12-19) take a slab out of shared memory, which frees its slot at
+// once, and store the parts with tcgen05.st as the A operand of the products, 16 columns a part. That takes A's second trip
+// through shared memory and the proxy fence out of a step. Every role asks for its next step's barrier (mbar_test) before it
+// works on this step's: an answer takes 150 clocks, a third of a step of a narrow tile.
+// Where a GEMM has few tiles (the atoms' rows), a step's chain of barriers bounds it, not any unit's rate. 648 rows of a
+// recorded pass, FMT_F16X2: N 1024 K 4096 64.7 us -> 47.1, N 256 K 1024 18.3 -> 14.2, N 1024 K 256 7.7 -> 7.1; FMT_F16X3,
+// 21 rows, N 512 K 2048: 35.0 -> 27.4.
+//
+// What bounds the large ones: the SM's shared-memory data path (one 128-byte wavefront per clock for TMA traffic, the tensor core's
 // operand reads, the converter and the epilogue). Wavefronts per 8 columns of K of a 128 x 256 tile, K = 256: FMT_F16X2
 // operand reads 144, fills 96, converter 64, epilogue 64-128 = about 370-430 against 192 clocks of MMA; FMT_F16X3 288, 128,
 // 80, 64-128 = about 560-620 against 384. The 3xTF32 split it replaces (two tf32 parts, three products) took 610-640 for
@@ -102,8 +111,11 @@ struct Tile {
   static constexpr bool X3 = FMT == FMT_F16X3, X2 = FMT == FMT_F16X2, T2 = FMT == FMT_TF32X2, T1 = FMT == FMT_TF32;
   static constexpr bool kScaled = FMT == FMT_F16X3 || FMT == FMT_F16X2 || FMT == FMT_F16;
   static constexpr int BK = T2 ? 16 : 32;                                   // columns of K of a step
+  // A's parts in tensor memory, where the accumulators leave room for them.
+  static constexpr bool TA = !PAIR && !T1 && !T2 && (X2 || BN <= 128);
+  static constexpr int kParts = X3 ? 3 : X2 ? 2 : 1;
   static constexpr int kSlab = TBM * BK * 4;                                // A as it lands
-  static constexpr int kA = kSlab + (X3 || T2 ? TBM * 64 : 0);              // the fp32 slab, then its parts; l behind it
+  static constexpr int kA = kSlab + ((X3 && !TA) || T2 ? TBM * 64 : 0);     // the fp32 slab, then its parts; l behind it
   static constexpr int kRowsB = PAIR ? BN / 2 : BN;                         // of B's tile, in this CTA
   static constexpr int kB = kRowsB * (X3 ? 192 : X2 || T2 || T1 ? 128 : 64);          // [h | m] or [h | l] rows of 128 bytes (then l), or rows of 64
   // An epilogue warp's two buffers of 32 rows x kWide columns; half as wide where the rings need the room.
@@ -118,25 +130,38 @@ struct Tile {
   static constexpr int slots_a(int nb) { return least(8, (kRoom - nb * kB) / kA); }
   static constexpr int kBoth = least(8, kRoom / (kA + kB));
   static constexpr bool kTrade = slots_a(kBoth) % 2 != 0 && slots_a(kBoth - 1) % 2 == 0;  // one of B's for one more of A's
-  static constexpr int NA = slots_a(kTrade ? kBoth - 1 : kBoth) / 2 * 2, NB = least(kTrade ? kBoth - 1 : kBoth, NA);
+  // TA: A's slots are free as soon as they are read, four will do; B's no more than the steps of A's parts (NT).
+  static constexpr int kBesideFour = least(X3 ? 5 : 8, (kRoom - 4 * kA) / kB);
+  static constexpr int NB = TA ? kBesideFour : least(kTrade ? kBoth - 1 : kBoth, slots_a(kTrade ? kBoth - 1 : kBoth) / 2 * 2);
+  static constexpr int NA = slots_a(TA ? NB : kTrade ? kBoth - 1 : kBoth) / 2 * 2;
   // The converter's warps work in groups on slots of their own: a slot takes a warp about a thousand clocks however few
   // instructions its rows need (the wait, the loads, the fence), so two or four of them have to be under way at once. A
   // slot always falls to the same group (NA a multiple of the groups): a group that met a slot's barrier only every other
   // round could take the round before last for the one it waits for.
-  static constexpr int kGroups = NA % 4 == 0 && NA >= 8 ? 4 : 2;
+  // TA: a warp reaches only its quarter of tensor memory's lanes, so a group is four warps, and there are two of them.
+  static constexpr int kGroups = !TA && NA % 4 == 0 && NA >= 8 ? 4 : 2;
   static constexpr int kRings = NA * kA + NB * kB;
   static constexpr int kTotal = kRings + kEpi + 1024 /*alignment slack*/ + kBars;
-  static constexpr int kThreads = 512;
+  static constexpr int kThreads = TA ? 640 : 512;
   // registers of the tile's sums that an epilogue thread keeps over the steps (FMT_F16X3)
   static constexpr int kSums = X3 ? BN / 2 : 1;
   // accumulators in tensor memory: a tile takes one (two in FMT_F16X3), and while it is being read the next tile fills the
   // others, where there are others
-  static constexpr int kAccs = X3 ? 2 : 1, kTurns = 512 / (kAccs * BN) >= 2 ? 2 : 1, kColumns = kTurns * kAccs * BN;
+  static constexpr int kAccs = X3 ? 2 : 1, kTurns = (TA ? 384 : 512) / (kAccs * BN) >= 2 ? 2 : 1, kColumns = TA ? 512 : kTurns * kAccs * BN;
+  // TA: the steps of A's parts behind them, 16 columns a part; ND barriers for the steps' ends, no fewer than any ring's slots
+  static constexpr int kPartsAt = kTurns * kAccs * BN, NT = least(8, (512 - kPartsAt) / (16 * kParts)), ND = TA ? 8 : NA;
+  static constexpr int NS = TA ? NT : NA;  // `ready` barriers
   static constexpr int kDrain = X3 ? 1024 / BK : 1 << 30;  // steps whose h.h products sum exactly
-  static constexpr bool kMoveRegs = X3 && BN >= 128;
-  static_assert(NA >= NB && NB >= 2 && NA % kGroups == 0, "the slots");
-  static_assert((3 * NA + 4 + 2 * kEpiWarps) * 8 + 8 <= kBars, "the barriers");
+  // 24 + 2 x 200 + 88 registers a thread over the warp groups are the 4 x 128 of the launch, 40 + 2 x 136 + 2 x 80 within the 5 x 96
+  static constexpr bool kMoveRegs = TA || (X3 && BN >= 128);
+  static constexpr int kRegsProd = TA ? 40 : 24, kRegsEpi = TA ? 136 : 200, kRegsConv = TA ? 80 : 88;
+  static_assert((TA || NA >= NB) && NA >= 2 && NB >= 2 && NA % kGroups == 0, "the slots");
+  static_assert(!TA || (NT >= NB && NT <= ND), "the slots");
+  static_assert((2 * NA + NS + ND + 4 + 2 * kEpiWarps) * 8 + 8 <= kBars, "the barriers");
 };
+
+// Rows of A's TMA box: a matrix of few rows has only its own fetched (a box's rows past the matrix cost as much as others).
+__host__ __device__ constexpr int box_rows(int M) { return M >= TBM ? TBM : (M + 31) / 32 * 32; }
 
 // ---- the epilogue ---------------------------------------------------------------------------
 
@@ -247,9 +272,10 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1)
   // In a pair, `ready` and `tempty` are the leader's (rank 0), whose warp 1 issues the products of both; the commits of
   // those arrive in both CTAs.
   uint64_t* full_a = reinterpret_cast<uint64_t*>(epi + L::kEpi);  // [NA] the fp32 slab has landed (pair: and B's tile)
-  uint64_t* ready = full_a + NA;    // [NA] it has been split and B's tile has landed (FMT_TF32: both have landed)
-  uint64_t* done = ready + NA;      // [NA] the step's products are done
-  uint64_t* tfull = done + NA;      // [2] accumulator complete
+  uint64_t* ready = full_a + NA;    // [NS] it has been split and B's tile has landed (FMT_TF32: both have landed)
+  uint64_t* done = ready + L::NS;   // [ND] the step's products are done
+  uint64_t* empty_a = done + L::ND;                // TA: [NA] the slab has been read
+  uint64_t* tfull = empty_a + (L::TA ? NA : 0);    // [2] accumulator complete
   uint64_t* tempty = tfull + 2;     // [2] accumulator read back
   uint64_t* landed = tempty + 2;    // [kEpiWarps][2] an epilogue warp's chunk has landed
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(landed + 2 * kEpiWarps);
@@ -266,10 +292,12 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1)
   const int nkb = (p.K + TBK - 1) / TBK;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < NA; ++s) {
-      mbar_init(full_a + s, CTAS), mbar_init(ready + s, PAIR ? 2 * (4 / L::kGroups) : 1 + (L::T1 ? 1 : 4 / L::kGroups));
-      mbar_init(done + s, 1);
-    }
+    for (int s = 0; s < NA; ++s) mbar_init(full_a + s, CTAS);
+    if (L::TA)
+      for (int s = 0; s < NA; ++s) mbar_init(empty_a + s, 4);
+    for (int s = 0; s < L::NS; ++s)
+      mbar_init(ready + s, L::TA ? 1 + 4 : PAIR ? 2 * (4 / L::kGroups) : 1 + (L::T1 ? 1 : 4 / L::kGroups));
+    for (int s = 0; s < L::ND; ++s) mbar_init(done + s, 1);
     for (int b = 0; b < 2; ++b) mbar_init(tfull + b, 1), mbar_init(tempty + b, CTAS * kEpiWarps);
     for (int b = 0; b < 2 * kEpiWarps; ++b) mbar_init(landed + b, 1);
     *abort_flag = 0;
@@ -284,22 +312,24 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1)
   after_previous();
 
   if (warp < 4) {
-    // 24 + 200 + 200 + 88 registers a thread over the four warp groups are the 4 x 128 of the launch
-    if (L::kMoveRegs) asm volatile("setmaxnreg.dec.sync.aligned.u32 24;");
+    if (L::kMoveRegs) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(L::kRegsProd));
     // Each of the three roles is a whole warp's loop with one lane's instructions. `s` is the step's slot in its ring, `turn`
     // the parity of the ring's round.
     const bool one = elect_one();
     bool ok = true;
     if (warp == 0) {
+      uint64_t* freed = L::TA ? empty_a : done;
       int s = 0;
       uint32_t turn = 0;
+      bool peek = true;
       for (int t = tile0; ok && t < n_tiles; t += tile_step) {
         const int m0 = first_row(t);
         for (int kb = 0; kb < nkb; ++kb) {
-          if (!(ok = mbar_wait_warp(done + s, turn ^ 1, abort_flag))) break;
+          if (!(ok = mbar_wait_warp(freed + s, turn ^ 1, abort_flag, peek))) break;
+          peek = s + 1 < NA ? mbar_test(freed + s + 1, turn ^ 1) : mbar_test(freed, turn);
           if (one) {
             uint64_t* bar = L::T1 && !PAIR ? ready + s : full_a + s;
-            mbar_expect_tx(bar, L::kSlab);
+            mbar_expect_tx(bar, uint32_t(box_rows(p.M) * L::BK * 4));
             tma_load_2d(ring_a + s * L::kA, &map_a, bar, kb * TBK, m0);
           }
           if (++s == NA) s = 0, turn ^= 1;
@@ -307,11 +337,13 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1)
       }
     } else if (warp == 2) {
       int s = 0, sb = 0, g = 0;  // the step's barrier, B's slot, steps so far
+      bool peek = false;
       for (int t = tile0; ok && t < n_tiles; t += tile_step) {
         const int n0 = (t % tiles_n) * BN + rank * L::kRowsB;
         for (int kb = 0; kb < nkb; ++kb, ++g) {
-          // the step that used this slot before, NB steps ago, has its barrier at (g - NB) % NA
-          if (g >= NB && !(ok = mbar_wait_warp(done + (g - NB) % NA, ((g - NB) / NA) & 1, abort_flag))) break;
+          // the step that used this slot before, NB steps ago, has its barrier at (g - NB) % ND
+          if (g >= NB && !(ok = mbar_wait_warp(done + (g - NB) % L::ND, ((g - NB) / L::ND) & 1, abort_flag, peek))) break;
+          if (g + 1 >= NB) peek = mbar_test(done + (g + 1 - NB) % L::ND, ((g + 1 - NB) / L::ND) & 1);
           if (one) {
             uint8_t* dst = ring_b + sb * L::kB;
             uint64_t* bar = PAIR ? full_a + s : ready + s;
@@ -324,14 +356,15 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1)
               if (L::T2) tma_load_2d(dst + L::kRowsB * 64, &map_blo, bar, kb * TBK, n0);
             }
           }
-          if (++s == NA) s = 0;
+          if (++s == L::NS) s = 0;
           if (++sb == NB) sb = 0;
         }
       }
     } else if (warp == 1 && rank == 0) {
       constexpr uint32_t idesc = L::T2 || L::T1 ? idesc_tf32(CTAS * TBM, BN) : idesc_f16(CTAS * TBM, BN, FMT == FMT_BF16);
-      int s = 0, sb = 0, i = 0;  // the slots, accumulators handed over
+      int s = 0, sb = 0, sd = 0, i = 0;  // the slots, accumulators handed over
       uint32_t turn = 0;
+      bool peek = false;
       for (int t = tile0; ok && t < n_tiles; t += tile_step) {
         for (int kb = 0; kb < nkb; ++kb) {
           const bool first = kb % L::kDrain == 0, last = kb + 1 == nkb || (kb + 1) % L::kDrain == 0;
@@ -340,8 +373,38 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1)
             if (!(ok = mbar_wait_warp(tempty + b, ((i / L::kTurns) & 1) ^ 1, abort_flag))) break;
             tcgen05_fence_after();
           }
-          if (!(ok = mbar_wait_warp(ready + s, turn, abort_flag))) break;
-          if (one) {
+          if (!(ok = mbar_wait_warp(ready + s, turn, abort_flag, peek))) break;
+          peek = s + 1 < L::NS ? mbar_test(ready + s + 1, turn) : mbar_test(ready, turn ^ 1);
+          if (L::TA) tcgen05_fence_after();
+          if (L::TA && one) {
+            const uint32_t acc = tmem + uint32_t(b * L::kAccs * BN), b0 = smem_u32(ring_b + sb * L::kB);
+            const uint32_t th = tmem + uint32_t(L::kPartsAt + s * 16 * L::kParts);
+            constexpr int row = L::X3 || L::X2 ? 128 : 64;
+            const uint64_t bh = smem_desc<row>(b0), bm = smem_desc<row>(b0 + 64);
+#pragma unroll
+            for (int k = 0; k < 4; k += 2) {  // 16 columns: 8 of tensor memory, and as below
+              const uint32_t h = th + 4 * k, m = h + 16, l = h + 32;
+              if (L::X3) {
+                const uint64_t bl = smem_desc<64>(b0 + L::kRowsB * 128);
+                const uint32_t small = acc + BN;
+                mma_f16_ta(small, h, bl + k, idesc, !first || k != 0);
+                mma_f16_ta(small, l, bh + k, idesc, 1);
+                mma_f16_ta(small, m, bm + k, idesc, 1);
+                mma_f16_ta(small, h, bm + k, idesc, 1);
+                mma_f16_ta(small, m, bh + k, idesc, 1);
+                mma_f16_ta(acc, h, bh + k, idesc, !first || k != 0);
+              } else if (L::X2) {
+                mma_f16_ta(acc, h, bm + k, idesc, kb != 0 || k != 0);
+                mma_f16_ta(acc, m, bh + k, idesc, 1);
+                mma_f16_ta(acc, h, bh + k, idesc, 1);
+              } else {
+                mma_f16_ta(acc, h, bh + k, idesc, kb != 0 || k != 0);
+              }
+            }
+            mma_commit<false>(done + sd);
+            if (last) mma_commit<false>(tfull + b);
+          }
+          if (!L::TA && one) {
             const uint32_t acc = tmem + uint32_t(b * L::kAccs * BN);
             const uint32_t a0 = smem_u32(ring_a + s * L::kA), b0 = smem_u32(ring_b + sb * L::kB);
             const uint64_t ah = smem_desc<128>(a0), am = smem_desc<128>(a0 + 64);  // h and the part beside it
@@ -388,13 +451,14 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1)
           }
           __syncwarp();
           i += last;
-          if (++s == NA) s = 0, turn ^= 1;
+          if (++s == L::NS) s = 0, turn ^= 1;
           if (++sb == NB) sb = 0;
+          if (++sd == L::ND) sd = 0;
         }
       }
     }
   } else if (warp < kConvWarp0) {
-    if (L::kMoveRegs) asm volatile("setmaxnreg.inc.sync.aligned.u32 200;");
+    if (L::kMoveRegs) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(L::kRegsEpi));
     const int ew = warp - kEpiWarp0;
     const int q = warp & 3;          // the quarter of the 128 lanes this warp may read
     const int half = ew >> 2;        // which half of the BN columns
@@ -534,15 +598,58 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1)
       if (p.c_max && row < p.M && nc > 0) atomicMax(p.c_max + row, __float_as_uint(big));
     }
     if (lane == 0) bulk_wait_all();
+  } else if (L::TA) {
+    if (L::kMoveRegs) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(L::kRegsConv));
+    // A lane owns one of its warp's quarter of the rows; the groups take every other step.
+    const int quarter = warp & 3, group = (warp - kConvWarp0) >> 2;
+    int g = 0;
+    bool ok = true, peek = false;
+    for (int t = tile0; ok && t < n_tiles; t += tile_step) {
+      const int r = quarter * 32 + lane, row = first_row(t) + r;
+      const bool live = row - lane < p.M;  // rows past the matrix: whatever their products are, nobody reads them
+      const float s = L::kScaled && row < p.M ? scale_of(p.a_max[row]) : 1.f;
+      for (int kb = 0; kb < nkb; ++kb, ++g) {
+        if ((g & 1) != group) continue;
+        const int sa = g % NA, sp = g % L::NS, before = g - L::NS;
+        if (!(ok = mbar_wait_warp(full_a + sa, (g / NA) & 1, abort_flag, peek))) break;
+        const bool free_peek = before < 0 || mbar_test(done + before % L::ND, (before / L::ND) & 1);
+        peek = mbar_test(full_a + (g + 2) % NA, ((g + 2) / NA) & 1);
+        uint32_t part[3][16];
+        if (live) {
+          const uint8_t* slab = ring_a + sa * L::kA;
+          float4 x[8];
+#pragma unroll
+          for (int c = 0; c < 8; ++c) x[c] = *reinterpret_cast<const float4*>(slab + swizzled<128>(r, c));
+#pragma unroll
+          for (int c = 0; c < 8; ++c) {
+            split2<FMT>(x[c].x, x[c].y, s, part[0][2 * c], part[1][2 * c], part[2][2 * c]);
+            split2<FMT>(x[c].z, x[c].w, s, part[0][2 * c + 1], part[1][2 * c + 1], part[2][2 * c + 1]);
+          }
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(empty_a + sa);
+        if (!(ok = mbar_wait_warp(done + before % L::ND, (before / L::ND) & 1, abort_flag, free_peek))) break;
+        tcgen05_fence_after();
+        if (live) {
+          const uint32_t at = tmem + uint32_t(L::kPartsAt + sp * 16 * L::kParts) + (uint32_t(quarter * 32) << 16);
+#pragma unroll
+          for (int q = 0; q < L::kParts; ++q) tmem_st16_async(at + 16 * q, part[q]);
+          tmem_wait_st();
+        }
+        tcgen05_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(ready + sp);
+      }
+    }
   } else if (!L::T1 || PAIR) {
-    if (L::kMoveRegs) asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
+    if (L::kMoveRegs) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(L::kRegsConv));
     // A lane owns a row at a time: 16-byte chunk c of row r sits at chunk c ^ (r & 7) of its 128 bytes, so the eight lanes of
     // a quarter warp touch eight different 16-byte columns on the reads and on the writes. The parts go back as chunks 0-3
     // (h) and 4-7 (m or l) of the same row; FMT_F16X3's l into rows of 64 bytes, chunk c at c ^ ((r >> 1) & 3).
     constexpr int WPG = 4 / L::kGroups;  // warps of a group
     const int cw = warp - kConvWarp0, group = cw / WPG, first = cw % WPG;
     int g = 0;
-    bool ok = true;
+    bool ok = true, peek = false;
     for (int t = tile0; ok && t < n_tiles; t += tile_step) {
       const int m0 = first_row(t);
       float scale[4 / WPG];
@@ -554,7 +661,8 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1)
       for (int kb = 0; kb < nkb; ++kb, ++g) {
         if (g % L::kGroups != group) continue;
         const int sa = g % NA;
-        if (!(ok = mbar_wait_warp(full_a + sa, (g / NA) & 1, abort_flag))) break;
+        if (!(ok = mbar_wait_warp(full_a + sa, (g / NA) & 1, abort_flag, peek))) break;
+        peek = mbar_test(full_a + (g + L::kGroups) % NA, ((g + L::kGroups) / NA) & 1);
         uint8_t* slab = ring_a + sa * L::kA;
 #pragma unroll
         for (int j = 0; j < 4 / WPG; ++j) {
@@ -725,7 +833,7 @@ void launch_tc(Stream& st, const GemmArgs& a, const PackedB& w) {
   static SmemOptIn opted;
   auto kernel = k_gemm_tc<EPI, BN, FMT, PAIR>;
   opt_in_shared_memory(kernel, L::kTotal, opted);
-  const CUtensorMap ma = map_2d(CU_TENSOR_MAP_DATA_TYPE_FLOAT32, a.A, a.K, a.M, size_t(a.lda) * 4, L::BK, TBM,
+  const CUtensorMap ma = map_2d(CU_TENSOR_MAP_DATA_TYPE_FLOAT32, a.A, a.K, a.M, size_t(a.lda) * 4, L::BK, box_rows(a.M),
                                 L::T2 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B);
   const auto half = FMT == FMT_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
   CUtensorMap mb, ml;
