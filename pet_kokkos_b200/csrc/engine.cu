@@ -207,6 +207,7 @@ Engine::~Engine() {
   model.reset();
   if (pinned) cudaFreeHost(pinned);
   if (host_stage) cudaFreeHost(host_stage);
+  if (landing) cudaFreeHost(landing);
   if (ev0) cudaEventDestroy(ev0);
   if (ev1) cudaEventDestroy(ev1);
   if (st.legacy_fence) cudaEventDestroy(st.legacy_fence);
@@ -671,23 +672,46 @@ void Engine::fetch(pet_results* out) {
   PETB_CUDA(cudaSetDevice(device));
   if (!out) throw Error(2, "pet: no results struct given");
   const int B = last_B, N = last_N;
+  // Every result lands in one pinned block and goes on from there, with one wait for all of them: a copy straight into the
+  // caller's pageable memory is staged by the driver and waits on its own.
+  struct Piece {
+    void* to;
+    size_t bytes;
+  };
+  Piece pieces[5];
+  int n = 0;
+  size_t at = 0;
   if (have_out) {
     const PassOut& o = last_out;
-    if (out->energy) PETB_CUDA(cudaMemcpyAsync(out->energy, o.f.energy, sizeof(double) * B, cudaMemcpyDeviceToHost, st.s));
-    if (out->per_atom_energy)
-      PETB_CUDA(cudaMemcpyAsync(out->per_atom_energy, o.per_atom, sizeof(double) * N, cudaMemcpyDeviceToHost, st.s));
-    if (o.has_forces) {
-      if (out->forces) PETB_CUDA(cudaMemcpyAsync(out->forces, o.f.forces, sizeof(double) * 3 * N, cudaMemcpyDeviceToHost, st.s));
-      if (out->virial) PETB_CUDA(cudaMemcpyAsync(out->virial, o.f.vir6, sizeof(double) * 6 * B, cudaMemcpyDeviceToHost, st.s));
+    const size_t all = sizeof(double) * (7 * size_t(B) + 4 * size_t(N)) + sizeof(int) * size_t(N) + 64;
+    if (all > landing_bytes) {
+      if (landing) cudaFreeHost(landing);
+      landing = nullptr, landing_bytes = 0;
+      PETB_CUDA(cudaMallocHost(&landing, all + all / 2));
+      landing_bytes = all + all / 2;
     }
-    if (out->struct_id && last_pk.sid)
-      PETB_CUDA(cudaMemcpyAsync(out->struct_id, last_pk.sid, sizeof(int) * N, cudaMemcpyDeviceToHost, st.s));
+    auto bring = [&](void* to, const void* from, size_t bytes) {
+      if (!to || !from || !bytes) return;
+      PETB_CUDA(cudaMemcpyAsync(landing + at, from, bytes, cudaMemcpyDeviceToHost, st.s));
+      pieces[n++] = {to, bytes};
+      at += bytes;
+    };
+    bring(out->energy, o.f.energy, sizeof(double) * B);
+    bring(out->per_atom_energy, o.per_atom, sizeof(double) * N);
+    if (o.has_forces) {
+      bring(out->forces, o.f.forces, sizeof(double) * 3 * N);
+      bring(out->virial, o.f.vir6, sizeof(double) * 6 * B);
+    }
+    bring(out->struct_id, last_pk.sid, sizeof(int) * N);
   }
+  gemm_tensor_error_ask(st, pinned + kGaveUp);
   PETB_CUDA(cudaStreamSynchronize(st.s));
   float ms = 0.f;
   if (cudaEventElapsedTime(&ms, ev0, ev1) == cudaSuccess) last_ms = ms;
-  if (gemm_tensor_error(st))
+  if (gemm_tensor_error(st, pinned + kGaveUp))
     throw Error(5, "pet: a tensor-core GEMM gave up waiting on its pipeline; the results of this evaluation are invalid");
+  const char* from = landing;
+  for (int i = 0; i < n; from += pieces[i++].bytes) std::memcpy(pieces[i].to, from, pieces[i].bytes);
 }
 
 // How many neighbours an atom of this structure has, roughly: the density times the cutoff sphere for a periodic
@@ -1061,15 +1085,12 @@ static StepOut session_step(Engine& I, const double* positions, bool on_device, 
   return so;
 }
 
-// True when the latest fixed-shape step outgrew its capacities: they are dropped, and the caller redoes the step,
-// which then runs with the shapes read back and sizes new ones.
-static bool fixed_step_overflowed(Engine& I) {
-  Session& s = I.md;
+// Asks whether the latest fixed-shape step outgrew its capacities; false if it has none. The answer is in pinned[8] once the
+// stream has got there: an outgrown step's capacities are dropped and it is redone, with the shapes read back and new ones sized.
+static bool ask_overflow(Engine& I) {
+  const Session& s = I.md;
   if (!I.md_fixed || !s.caps_valid || s.has_exchange || !s.overflow) return false;
   PETB_CUDA(cudaMemcpyAsync(I.pinned + 8, s.overflow, sizeof(int), cudaMemcpyDeviceToHost, I.st.s));
-  PETB_CUDA(cudaStreamSynchronize(I.st.s));
-  if (I.pinned[8] == 0) return false;
-  s.caps_valid = false;
   return true;
 }
 
@@ -1077,14 +1098,24 @@ void Engine::compute_step(const double* positions, const double* cell, bool forc
   PETB_CUDA(cudaSetDevice(device));
   if (!positions && md.n_atoms > 0) throw Error(2, "pet: no positions given");
   StepOut so = session_step(*this, positions, false, cell, forces);
-  if (fixed_step_overflowed(*this)) so = session_step(*this, positions, false, cell, forces);
+  if (ask_overflow(*this)) {
+    if (out) fetch(out);
+    else PETB_CUDA(cudaStreamSynchronize(st.s));
+    if (pinned[8] != 0) {
+      md.caps_valid = false;
+      so = session_step(*this, positions, false, cell, forces);
+      if (out) fetch(out);
+    }
+  } else if (out) {
+    fetch(out);
+  }
+  if (!out) return;  // the results stay on the device (pet_device_results_of): a caller that reduces them there
   std::vector<double> g;
   if (forces && edge_gradients && out && out->edge_gradient && so.eg_raw) {
     g.resize(3 * size_t(md.E));
     PETB_CUDA(cudaMemcpyAsync(g.data(), so.eg_raw, 24 * size_t(md.E), cudaMemcpyDeviceToHost, st.s));
+    PETB_CUDA(cudaStreamSynchronize(st.s));
   }
-  if (!out) return;  // the results stay on the device (pet_device_results_of): a caller that reduces them there
-  fetch(out);
   if (forces && edge_gradients && out && out->edge_gradient) {
     // A half list's pair gets both directions: g(i -> j) - g(j -> i)  (src/calculator.cpp:689-699).
     std::fill(out->edge_gradient, out->edge_gradient + 3 * size_t(md.n_pairs), 0.0);
@@ -1115,9 +1146,10 @@ void Engine::compute_step_device(const pet_device_arrays* a, const double* cell,
     PETB_CUDA(cudaMemcpyAsync(h, last_out.f.energy, 8, cudaMemcpyDeviceToHost, st.s));
     if (forces) PETB_CUDA(cudaMemcpyAsync(h + 1, last_out.f.vir6, 48, cudaMemcpyDeviceToHost, st.s));
     if (skip) PETB_CUDA(cudaMemcpyAsync(pinned + 8, md.overflow, sizeof(int), cudaMemcpyDeviceToHost, st.s));
+    gemm_tensor_error_ask(st, pinned + kGaveUp);
     PETB_CUDA(cudaStreamSynchronize(st.s));
     // a tensor-core GEMM that gave up on a wait left garbage behind, and the adds above have put it into the caller's arrays
-    if (gemm_tensor_error(st))
+    if (gemm_tensor_error(st, pinned + kGaveUp))
       throw Error(5, "pet: a tensor-core GEMM gave up waiting on its pipeline; the arrays this step added into are invalid");
     if (skip && pinned[8] != 0) {  // outgrown: drop the capacities and run the step again, read back and resized
       md.caps_valid = false;
@@ -1280,8 +1312,16 @@ void Engine::compute_pairs(const pet_pair_list* v, const double* positions, cons
     PETB_CUDA(cudaStreamSynchronize(st.s));
   }
   session_step(*this, positions, true, cell, forces);
-  if (fixed_step_overflowed(*this)) session_step(*this, positions, true, cell, forces);
-  if (gemm_tensor_error(st))  // synchronizes the stream
+  if (ask_overflow(*this)) {
+    PETB_CUDA(cudaStreamSynchronize(st.s));
+    if (pinned[8] != 0) {
+      md.caps_valid = false;
+      session_step(*this, positions, true, cell, forces);
+    }
+  }
+  gemm_tensor_error_ask(st, pinned + kGaveUp);
+  PETB_CUDA(cudaStreamSynchronize(st.s));
+  if (gemm_tensor_error(st, pinned + kGaveUp))
     throw Error(5, "pet: a tensor-core GEMM gave up waiting on its pipeline; the results of this evaluation are invalid");
   if (out) {
     *out = pet_device_results{};
@@ -1326,8 +1366,9 @@ void Engine::gemm_host(int mode, bool w_transposed, int m, int n, int k, const f
   a.nat = pack(FMT_F16X3), a.fast = pack(format_of(mode));
   gemm(st, tmp_arena, a);
   PETB_CUDA(cudaMemcpyAsync(C, dC, 4 * size_t(m) * n, cudaMemcpyDeviceToHost, st.s));
+  gemm_tensor_error_ask(st, pinned + kGaveUp);
   PETB_CUDA(cudaStreamSynchronize(st.s));
-  if (gemm_tensor_error(st)) throw Error(5, "pet: a tensor-core GEMM gave up waiting on its pipeline");
+  if (gemm_tensor_error(st, pinned + kGaveUp)) throw Error(5, "pet: a tensor-core GEMM gave up waiting on its pipeline");
 }
 
 }  // namespace petb

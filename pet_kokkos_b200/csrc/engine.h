@@ -125,6 +125,9 @@ struct Engine {
   bool have_out = false;
   int last_B = 0, last_N = 0;
   int* pinned = nullptr;  // small pinned scratch for readbacks
+  static constexpr int kGaveUp = 9;  // the word of it that says whether a GEMM gave up on a wait
+  char* landing = nullptr;  // pinned: where results land before they go to the caller's arrays
+  size_t landing_bytes = 0;
   void* host_stage = nullptr;
   size_t host_stage_bytes = 0;
   std::map<std::string, std::pair<const float*, size_t>> taps;

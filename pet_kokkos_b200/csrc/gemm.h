@@ -112,9 +112,10 @@ void gemv_rows(Stream& st, const float* A, int lda, const float* w, const float*
 // mx[r] = bits of the largest |x(r, :)|.
 void row_max(Stream& st, uint32_t* mx, const float* x, int ld, int R, int D);
 
-// Non-zero if a tensor-core kernel launched on this stream gave up on a bounded wait since the
-// last call (synchronizes the stream; clears the flag).
-int gemm_tensor_error(Stream& st);
+// Whether a tensor-core kernel gave up on a bounded wait: the first puts a copy of the device's word into pinned memory on the
+// stream, the second, once the stream has got there, looks at it and clears the device's.
+void gemm_tensor_error_ask(Stream& st, int* host);
+bool gemm_tensor_error(Stream& st, const int* host);
 
 // True once the tensor-core path has been initialised on this device (driver entry point found).
 bool tensor_gemm_available();

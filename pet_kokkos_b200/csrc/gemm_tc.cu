@@ -762,13 +762,11 @@ using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, voi
                               const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                               CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
-// What the tensor-core path needs of one device: its SM count and an error word in its memory (with a pinned
-// mirror), plus the driver's tensor-map encoder (the same function for every device). One per device ordinal,
+// What the tensor-core path needs of one device: its SM count and an error word in its memory, plus the driver's tensor-map encoder (the same function for every device). One per device ordinal,
 // built on first use with that device current.
 struct TensorState {
   EncodeFn encode = nullptr;
   int* err = nullptr;       // device error word
-  int* err_host = nullptr;  // pinned mirror
   int sms = 0;
   bool ok = false;
 };
@@ -788,8 +786,6 @@ TensorState& state() {
     if (cudaMalloc(&s.err, sizeof(int)) != cudaSuccess) return;
     cudaMemset(s.err, 0, sizeof(int));
     cudaStreamSynchronize(cudaStreamLegacy);  // the callers' streams do not wait for the legacy one
-    if (cudaMallocHost(&s.err_host, sizeof(int)) != cudaSuccess) return;
-    *s.err_host = 0;
     s.encode = reinterpret_cast<EncodeFn>(fn);
     s.ok = true;
   });
@@ -976,15 +972,14 @@ void gemm_tensor(Stream& st, Arena& arena, const GemmArgs& given, const PackedB&
   arena.rewind(mark);
 }
 
-// Non-zero once a tensor-core kernel gave up on a wait; cleared by the read.
-int gemm_tensor_error(Stream& st) {
+void gemm_tensor_error_ask(Stream& st, int* host) {
   TensorState& s = state();
-  if (!s.ok) return 0;
-  cudaMemcpyAsync(s.err_host, s.err, sizeof(int), cudaMemcpyDeviceToHost, st.s);
-  cudaStreamSynchronize(st.s);
-  const int e = *s.err_host;
-  if (e) cudaMemsetAsync(s.err, 0, sizeof(int), st.s);
-  return e;
+  *host = 0;
+  if (s.ok) cudaMemcpyAsync(host, s.err, sizeof(int), cudaMemcpyDeviceToHost, st.s);
+}
+bool gemm_tensor_error(Stream& st, const int* host) {
+  if (*host) cudaMemsetAsync(state().err, 0, sizeof(int), st.s);
+  return *host != 0;
 }
 
 }  // namespace petb
