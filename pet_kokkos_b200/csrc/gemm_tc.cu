@@ -151,10 +151,13 @@ struct Tile {
   // TA: the steps of A's parts behind them, 16 columns a part; ND barriers for the steps' ends, no fewer than any ring's slots
   static constexpr int kPartsAt = kTurns * kAccs * BN, NT = least(8, (512 - kPartsAt) / (16 * kParts)), ND = TA ? 8 : NA;
   static constexpr int NS = TA ? NT : NA;  // `ready` barriers
-  static constexpr int kDrain = X3 ? 1024 / BK : 1 << 30;  // steps whose h.h products sum exactly
+  // Steps whose products go into one accumulator. FMT_F16X3's h.h products sum exactly over 1024 columns of K; up to 4096 a
+  // longer K goes in four pieces, one for each of four CTAs that share a tile (SPLIT).
+  static __device__ int drain(int K) { return !X3 ? 1 << 30 : K > 1024 && K <= 4096 ? (K + 127) / 128 : 1024 / BK; }
   // 24 + 2 x 200 + 88 registers a thread over the warp groups are the 4 x 128 of the launch, 40 + 2 x 136 + 2 x 80 within the 5 x 96
   static constexpr bool kMoveRegs = TA || (X3 && BN >= 128);
   static constexpr int kRegsProd = TA ? 40 : 24, kRegsEpi = TA ? 136 : 200, kRegsConv = TA ? 80 : 88;
+  static_assert(kRings >= TBM * BN * 4, "the shared sums of a split tile");
   static_assert((TA || NA >= NB) && NA >= 2 && NB >= 2 && NA % kGroups == 0, "the slots");
   static_assert(!TA || (NT >= NB && NT <= ND), "the slots");
   static_assert((2 * NA + NS + ND + 4 + 2 * kEpiWarps) * 8 + 8 <= kBars, "the barriers");
@@ -256,7 +259,7 @@ __device__ __forceinline__ void chunk_get(const uint8_t* tile, int r, float* x) 
   }
 }
 
-template <int EPI, int BN, int FMT, bool PAIR>
+template <int EPI, int BN, int FMT, bool PAIR, bool SPLIT>
 __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1)
     k_gemm_tc(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
               const __grid_constant__ CUtensorMap map_blo, const __grid_constant__ CUtensorMap map_in,
@@ -285,11 +288,14 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1)
   // A pair walks tiles of 2 x 128 rows: its CTAs take 128 each, and half of B's rows each.
   constexpr int CTAS = PAIR ? 2 : 1;
   const int rank = PAIR ? int(cluster_ctarank()) : 0;
+  // SPLIT: the CTAs of a cluster share a tile; each sums a run of K, then finishes a slice of the columns.
+  const int part = SPLIT ? int(cluster_ctarank()) : 0, parts = SPLIT ? int(cluster_size()) : 1, slice = BN / parts;
   const int tiles_n = (p.N + BN - 1) / BN, tiles_m = (p.M + CTAS * TBM - 1) / (CTAS * TBM);
-  const int n_tiles = tiles_m * tiles_n, tile0 = blockIdx.x / CTAS, tile_step = gridDim.x / CTAS;
+  const int n_tiles = tiles_m * tiles_n, tile0 = blockIdx.x / (CTAS * parts), tile_step = gridDim.x / (CTAS * parts);
   auto first_row = [&](int t) { return ((t / tiles_n) * CTAS + rank) * TBM; };
   constexpr int TBK = L::BK;
-  const int nkb = (p.K + TBK - 1) / TBK;
+  const int steps = (p.K + TBK - 1) / TBK / parts, kb0 = part * steps, kb1 = kb0 + steps;  // SPLIT: parts divides the steps of K
+  const int drain = L::drain(p.K);
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < NA; ++s) mbar_init(full_a + s, CTAS);
@@ -324,7 +330,7 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1)
       bool peek = true;
       for (int t = tile0; ok && t < n_tiles; t += tile_step) {
         const int m0 = first_row(t);
-        for (int kb = 0; kb < nkb; ++kb) {
+        for (int kb = kb0; kb < kb1; ++kb) {
           if (!(ok = mbar_wait_warp(freed + s, turn ^ 1, abort_flag, peek))) break;
           peek = s + 1 < NA ? mbar_test(freed + s + 1, turn ^ 1) : mbar_test(freed, turn);
           if (one) {
@@ -340,7 +346,7 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1)
       bool peek = false;
       for (int t = tile0; ok && t < n_tiles; t += tile_step) {
         const int n0 = (t % tiles_n) * BN + rank * L::kRowsB;
-        for (int kb = 0; kb < nkb; ++kb, ++g) {
+        for (int kb = kb0; kb < kb1; ++kb, ++g) {
           // the step that used this slot before, NB steps ago, has its barrier at (g - NB) % ND
           if (g >= NB && !(ok = mbar_wait_warp(done + (g - NB) % L::ND, ((g - NB) / L::ND) & 1, abort_flag, peek))) break;
           if (g + 1 >= NB) peek = mbar_test(done + (g + 1 - NB) % L::ND, ((g + 1 - NB) / L::ND) & 1);
@@ -362,12 +368,12 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1)
       }
     } else if (warp == 1 && rank == 0) {
       constexpr uint32_t idesc = L::T2 || L::T1 ? idesc_tf32(CTAS * TBM, BN) : idesc_f16(CTAS * TBM, BN, FMT == FMT_BF16);
-      int s = 0, sb = 0, sd = 0, i = 0;  // the slots, accumulators handed over
+      int s = 0, sb = 0, sd = 0, i = 0, run = 0;  // the slots, accumulators handed over, steps into this one
       uint32_t turn = 0;
       bool peek = false;
       for (int t = tile0; ok && t < n_tiles; t += tile_step) {
-        for (int kb = 0; kb < nkb; ++kb) {
-          const bool first = kb % L::kDrain == 0, last = kb + 1 == nkb || (kb + 1) % L::kDrain == 0;
+        for (int kb = kb0; kb < kb1; ++kb) {
+          const bool first = run == 0, last = kb + 1 == kb1 || run + 1 == drain;
           const int b = i % L::kTurns;
           if (first) {
             if (!(ok = mbar_wait_warp(tempty + b, ((i / L::kTurns) & 1) ^ 1, abort_flag))) break;
@@ -394,11 +400,11 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1)
                 mma_f16_ta(small, m, bh + k, idesc, 1);
                 mma_f16_ta(acc, h, bh + k, idesc, !first || k != 0);
               } else if (L::X2) {
-                mma_f16_ta(acc, h, bm + k, idesc, kb != 0 || k != 0);
+                mma_f16_ta(acc, h, bm + k, idesc, kb != kb0 || k != 0);
                 mma_f16_ta(acc, m, bh + k, idesc, 1);
                 mma_f16_ta(acc, h, bh + k, idesc, 1);
               } else {
-                mma_f16_ta(acc, h, bh + k, idesc, kb != 0 || k != 0);
+                mma_f16_ta(acc, h, bh + k, idesc, kb != kb0 || k != 0);
               }
             }
             mma_commit<false>(done + sd);
@@ -425,7 +431,7 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1)
               const uint64_t bh = smem_desc<128>(b0), bl = smem_desc<128>(b0 + 64);
 #pragma unroll
               for (int k = 0; k < 4; k += 2) {
-                mma_f16<PAIR>(acc, ah + k, bl + k, idesc, kb != 0 || k != 0);
+                mma_f16<PAIR>(acc, ah + k, bl + k, idesc, kb != kb0 || k != 0);
                 mma_f16<PAIR>(acc, am + k, bh + k, idesc, 1);
                 mma_f16<PAIR>(acc, ah + k, bh + k, idesc, 1);
               }
@@ -433,24 +439,24 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1)
               const uint64_t th = smem_desc<64>(a0), tl = smem_desc<64>(a0 + L::kSlab), bh = smem_desc<64>(b0), bl = smem_desc<64>(b0 + L::kRowsB * 64);
 #pragma unroll
               for (int k = 0; k < 4; k += 2) {  // 8 columns are 32 bytes
-                mma_tf32<PAIR>(acc, th + k, bl + k, idesc, kb != 0 || k != 0);
+                mma_tf32<PAIR>(acc, th + k, bl + k, idesc, kb != kb0 || k != 0);
                 mma_tf32<PAIR>(acc, tl + k, bh + k, idesc, 1);
                 mma_tf32<PAIR>(acc, th + k, bh + k, idesc, 1);
               }
             } else if (L::T1) {
               const uint64_t bh = smem_desc<128>(b0);
 #pragma unroll
-              for (int k = 0; k < 8; k += 2) mma_tf32<PAIR>(acc, ah + k, bh + k, idesc, kb != 0 || k != 0);
+              for (int k = 0; k < 8; k += 2) mma_tf32<PAIR>(acc, ah + k, bh + k, idesc, kb != kb0 || k != 0);
             } else {
               const uint64_t bh = smem_desc<64>(b0);
 #pragma unroll
-              for (int k = 0; k < 4; k += 2) mma_f16<PAIR>(acc, ah + k, bh + k, idesc, kb != 0 || k != 0);
+              for (int k = 0; k < 4; k += 2) mma_f16<PAIR>(acc, ah + k, bh + k, idesc, kb != kb0 || k != 0);
             }
             mma_commit<PAIR>(done + s);
             if (last) mma_commit<PAIR>(tfull + b);
           }
           __syncwarp();
-          i += last;
+          i += last, run = last ? 0 : run + 1;
           if (++s == L::NS) s = 0, turn ^= 1;
           if (++sb == NB) sb = 0;
           if (++sd == L::ND) sd = 0;
@@ -468,8 +474,11 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1)
     uint64_t* bar = landed + 2 * ew;
     const bool has_in = reads(EPI) && (EPI != EPI_PLAIN || p.res != nullptr);
     const float b_unscale = L::kScaled ? unscale_of(*b_max) : 1.f;
-    auto first_col = [&](int t) { return (t % tiles_n) * BN + half * (BN / 2); };
-    auto chunks_of = [&](int t) { return max(0, min(BN / 2 / AC, (p.N - first_col(t) + AC - 1) / AC)); };
+    // The chunks of a warp: its half of the columns; SPLIT: every other one of the CTA's slice.
+    auto first_col = [&](int t) { return (t % tiles_n) * BN + (SPLIT ? part * slice : half * (BN / 2)); };
+    auto chunks_of = [&](int t) { return max(0, min((SPLIT ? slice : BN / 2) / AC, (p.N - first_col(t) + AC - 1) / AC)); };
+    const int c0 = SPLIT ? half : 0;
+    constexpr int CS = SPLIT ? 2 : 1;
     auto ask = [&](int t, int c, int k) {  // lane 0: chunk c of tile t, the k-th this warp reads, into buffer k & 1
       mbar_expect_tx(bar + (k & 1), L::kBuf);
       tma_load_2d(buf + (k & 1) * L::kBuf, &map_in, bar + (k & 1), (first_col(t) + c * AC) * (W / AC), first_row(t) + q * 32);
@@ -486,8 +495,8 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1)
     bool ok = true;
     if (has_in && lane == 0) {
       int t = tile0;
-      while (t < n_tiles && chunks_of(t) == 0) t += tile_step;
-      if (t < n_tiles) ask(t, 0, 0);
+      while (t < n_tiles && chunks_of(t) <= c0) t += tile_step;
+      if (t < n_tiles) ask(t, c0, 0);
     }
     for (int t = tile0; ok && t < n_tiles; t += tile_step) {
       const int r0 = first_row(t) + q * 32, row = r0 + lane, n0 = first_col(t), nc = chunks_of(t);
@@ -507,8 +516,8 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1)
       float sum[L::kSums];
       uint32_t acc = 0;
       const auto accumulator = [&](int b) { return tmem + uint32_t(b * L::kAccs * BN + half * (BN / 2)) + (uint32_t(q * 32) << 16); };
-      if (L::X3) {
-        for (int kb = 0; kb < nkb; kb += L::kDrain, ++i) {
+      if (L::X3 && !SPLIT) {
+        for (int kb = kb0; kb < kb1; kb += drain, ++i) {
           const int b = i % L::kTurns;
           if (!(ok = mbar_wait_warp(tfull + b, (i / L::kTurns) & 1, abort_flag))) break;
           tcgen05_fence_after();
@@ -522,7 +531,7 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1)
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
               const float v = __uint_as_float(big16[j]) + __uint_as_float(small16[j]);
-              sum[(c + j) % L::kSums] = kb == 0 ? v : sum[(c + j) % L::kSums] + v;
+              sum[(c + j) % L::kSums] = kb == kb0 ? v : sum[(c + j) % L::kSums] + v;
             }
           }
           release(b);
@@ -530,23 +539,64 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1)
         if (!ok) break;
       } else {
         const int b = i % L::kTurns;
-        if (!(ok = mbar_wait_warp(tfull + b, (i / L::kTurns) & 1, abort_flag))) break;
+        ok = mbar_wait_warp(tfull + b, (i / L::kTurns) & 1, abort_flag);
+        if (!ok && !SPLIT) break;
         tcgen05_fence_after();
         acc = accumulator(b);
+      }
+      // SPLIT: where the rings were, each CTA gets its slice of every CTA's sums, four columns of 32 rows at a time. (One tile a
+      // CTA: nothing else is under way then, and the two barriers are met by every thread whatever happened.)
+      const auto piece = [&](int from, int run) {
+        return reinterpret_cast<float4*>(ring_a) + (size_t(from * 4 + q) * (slice / 4) + run) * 32 + lane;
+      };
+      if constexpr (SPLIT) {
+        cluster_sync_all();
+        if (ok) {
+#pragma unroll
+          for (int c = 0; c < BN / 2; c += 16) {
+            float x[16];
+            tmem_ld<16>(acc + c, x);
+            if (L::X3) {  // (one piece a CTA)
+              float small[16];
+              tmem_ld<16>(acc + BN + c, small);
+#pragma unroll
+              for (int j = 0; j < 16; ++j) x[j] += small[j];
+            }
+#pragma unroll
+            for (int j = 0; j < 16; j += 4) {
+              const int col = half * (BN / 2) + c + j;
+              store4_at(piece(part, col % slice / 4), col / slice, x[j], x[j + 1], x[j + 2], x[j + 3]);
+            }
+          }
+        }
+        cluster_sync_all();
+        if (!ok) break;
       }
       // One copy of the chunk's code; FMT_F16X3 moves its sums down after each chunk: unrolled, the compiler keeps every
       // chunk's addresses alive beside the sums and spills.
 #pragma unroll 1
-      for (int c = 0; c < nc; ++c) {
+      for (int c = c0; c < nc; c += CS) {
         float v[AC], in[W], out[W], pre[W];
-        if (L::X3) {
+        if constexpr (SPLIT) {
+#pragma unroll
+          for (int j = 0; j < AC; j += 4) {
+            float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int o = 0; o < parts; ++o) {  // in K's order
+              const float4 y = *piece(o, (c * AC + j) / 4);
+              x = o == 0 ? y : make_float4(x.x + y.x, x.y + y.y, x.z + y.z, x.w + y.w);
+            }
+            v[j] = x.x, v[j + 1] = x.y, v[j + 2] = x.z, v[j + 3] = x.w;
+          }
+#pragma unroll
+          for (int j = 0; j < AC; ++j) v[j] = L::kScaled ? v[j] * b_unscale * unscale : v[j];
+        } else if (L::X3) {
 #pragma unroll
           for (int j = 0; j < AC; ++j) v[j] = sum[j % L::kSums] * b_unscale * unscale;  // one after the other: their product may not be a normal number
 #pragma unroll
           for (int j = 0; j + AC < L::kSums; ++j) sum[j] = sum[j + AC];
         } else {
           tmem_ld<AC == 32 ? 32 : 16>(acc + c * AC, v);
-          if (c + 1 == nc) release(i % L::kTurns);
+          if (c + 1 == nc) release(i % L::kTurns);  // (not SPLIT)
 #pragma unroll
           for (int j = 0; j < AC; ++j) v[j] = L::kScaled ? v[j] * b_unscale * unscale : v[j];
         }
@@ -554,12 +604,12 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1)
         if (has_in) {
           if (lane == 0) {
             bulk_wait_read<0>();  // the chunk before this one has left the other buffer: the next one may come in
-            if (c + 1 < nc) {
-              ask(t, c + 1, k + 1);
+            if (c + CS < nc) {
+              ask(t, c + CS, k + 1);
             } else {
               int u = t + tile_step;
-              while (u < n_tiles && chunks_of(u) == 0) u += tile_step;
-              if (u < n_tiles) ask(u, 0, k + 1);
+              while (u < n_tiles && chunks_of(u) <= c0) u += tile_step;
+              if (u < n_tiles) ask(u, c0, k + 1);
             }
           }
           __syncwarp();
@@ -592,7 +642,7 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1)
       }
       if (!ok) break;
       if (!L::X3) {
-        if (nc == 0) release(i % L::kTurns);
+        if (!SPLIT && nc == 0) release(i % L::kTurns);
         ++i;
       }
       if (p.c_max && row < p.M && nc > 0) atomicMax(p.c_max + row, __float_as_uint(big));
@@ -608,7 +658,7 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1)
       const int r = quarter * 32 + lane, row = first_row(t) + r;
       const bool live = row - lane < p.M;  // rows past the matrix: whatever their products are, nobody reads them
       const float s = L::kScaled && row < p.M ? scale_of(p.a_max[row]) : 1.f;
-      for (int kb = 0; kb < nkb; ++kb, ++g) {
+      for (int kb = kb0; kb < kb1; ++kb, ++g) {
         if ((g & 1) != group) continue;
         const int sa = g % NA, sp = g % L::NS, before = g - L::NS;
         if (!(ok = mbar_wait_warp(full_a + sa, (g / NA) & 1, abort_flag, peek))) break;
@@ -658,7 +708,7 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1)
         const int row = m0 + (first + j * WPG) * 32 + lane;
         scale[j] = L::kScaled && row < p.M ? scale_of(p.a_max[row]) : 1.f;
       }
-      for (int kb = 0; kb < nkb; ++kb, ++g) {
+      for (int kb = kb0; kb < kb1; ++kb, ++g) {
         if (g % L::kGroups != group) continue;
         const int sa = g % NA;
         if (!(ok = mbar_wait_warp(full_a + sa, (g / NA) & 1, abort_flag, peek))) break;
@@ -700,6 +750,11 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1)
         }
       }
     }
+  }
+  if (SPLIT && (warp < kEpiWarp0 || warp >= kConvWarp0)) {
+    __syncwarp();
+    cluster_sync_all();
+    cluster_sync_all();
   }
   tcgen05_fence_before();
   __syncthreads();
@@ -822,12 +877,12 @@ int resident_pairs(K kernel, cudaLaunchConfig_t cfg) {
   });
 }
 
-template <int EPI, int BN, int FMT, bool PAIR>
-void launch_tc(Stream& st, const GemmArgs& a, const PackedB& w) {
+template <int EPI, int BN, int FMT, bool PAIR, bool SPLIT = false>
+void launch_tc(Stream& st, const GemmArgs& a, const PackedB& w, int parts = 1) {
   using L = Tile<BN, FMT, PAIR>;
   static_assert(L::kTotal <= 227 * 1024, "the tile pipeline does not fit shared memory");
   static SmemOptIn opted;
-  auto kernel = k_gemm_tc<EPI, BN, FMT, PAIR>;
+  auto kernel = k_gemm_tc<EPI, BN, FMT, PAIR, SPLIT>;
   opt_in_shared_memory(kernel, L::kTotal, opted);
   const CUtensorMap ma = map_2d(CU_TENSOR_MAP_DATA_TYPE_FLOAT32, a.A, a.K, a.M, size_t(a.lda) * 4, L::BK, box_rows(a.M),
                                 L::T2 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B);
@@ -860,7 +915,12 @@ void launch_tc(Stream& st, const GemmArgs& a, const PackedB& w) {
   cudaLaunchAttribute attr[2] = {};
   cfg.blockDim = dim3(L::kThreads), cfg.dynamicSmemBytes = L::kTotal, cfg.stream = st.s, cfg.attrs = attr;
   const long long tiles = (long long) cdiv(a.M, PAIR ? 2 * TBM : TBM) * cdiv(a.N, BN);
-  if (PAIR) {
+  if (SPLIT) {
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = parts, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 1;
+    cfg.numAttrs = 1;
+    cfg.gridDim = dim3(unsigned(tiles * parts));
+  } else if (PAIR) {
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 1;
     cfg.numAttrs = 1;
@@ -872,6 +932,42 @@ void launch_tc(Stream& st, const GemmArgs& a, const PackedB& w) {
   attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
   PETB_CUDA(cudaLaunchKernelEx(&cfg, kernel, ma, mb, ml, mi, mc, mp, a, w.amax, state().err));
   PETB_LAUNCH_CHECK(st);
+}
+
+// How many CTAs share a tile, and the tile's width, for a GEMM of few tiles and a long contraction (the atoms' rows); `parts`
+// is 1 if none should. A step of 32 columns takes about `clocks` however few tiles there are (see the head of this file), so
+// K is shared out as far as the SMs go; handing the sums over costs 4000 clocks and more with the tile's width. Clusters do
+// not fill every SM, those of eight hardly two thirds (96 fit, 112 took a second round).
+// FMT_F16X3, whose rows' bits must not depend on how many there are, adds its pieces in K's order either way, and so is
+// shared by as many CTAs as it has pieces, or not at all. From K = 1024 on: below that there is little to share, and GEMMs
+// over a few thousand tokens, whose row count moves, stay out of it.
+// Measured, recorded passes, whole -> shared: FMT_F16X2 648 x 1024 x 4096 47.5 us -> 28.2 (256 wide, 4 CTAs), 648 x 256 x 1024
+// 14.2 -> 10.7 (128, 4); FMT_F16X3 21 x 512 x 2048 28.0 -> 12.0 (64, 4), 648 x 1024 x 4096 65.6 -> 44.3 (256, 4).
+struct SplitPlan {
+  int bn = 0, parts = 1;
+};
+template <int FMT>
+SplitPlan plan_split(const GemmArgs& a, int bn_whole, int sms) {
+  constexpr bool X3 = FMT == FMT_F16X3, T2 = FMT == FMT_TF32X2, two = FMT == FMT_F16X2;
+  constexpr int clocks[3] = {X3 || T2 ? 1800 : two ? 850 : 640, X3 ? 1050 : T2 ? 1550 : two ? 700 : 530, X3 ? 850 : T2 ? 1500 : two ? 670 : 510};
+  const int widths[3] = {256, 128, 64}, steps = (a.K + 31) / 32, rows = cdiv(a.M, TBM);
+  SplitPlan best;
+  if (a.K < 1024 || a.K % 32 || a.N % 64) return best;
+  long long least = 0;
+  for (int i = 0; i < 3; ++i)
+    if (widths[i] == bn_whole) {
+      if (rows * cdiv(a.N, bn_whole) > sms) return best;
+      least = (long long) steps * clocks[i];
+    }
+  for (int i = 0; i < 3; ++i)
+    for (int parts = 2; parts <= 8; parts *= 2) {
+      if (a.N % widths[i] || widths[i] / parts < (X3 ? 16 : 32) || steps % parts || steps / parts < 4) continue;
+      if (X3 && parts != (a.K <= 1024 ? 1 : a.K <= 4096 ? 4 : cdiv(a.K, 1024))) continue;
+      if ((long long) rows * (a.N / widths[i]) * parts > (parts == 8 ? sms * 2 / 3 : sms * 7 / 8)) continue;
+      const long long cost = (long long) (steps / parts) * clocks[i] + 4000 + 55 * widths[i];
+      if (cost < least) best.bn = widths[i], best.parts = parts, least = cost;
+    }
+  return best;
 }
 
 template <int EPI, int FMT>
@@ -902,6 +998,14 @@ void dispatch_width(Stream& st, const GemmArgs& a, const PackedB& w) {
   constexpr bool kPair = FMT == FMT_F16X3 || FMT == FMT_F16X2 || FMT == FMT_TF32X2;
   if constexpr (kPair)
     if (bn == 256 && cdiv(a.M, 2 * TBM) * (a.N / 256) >= sms / 2) return launch_tc<EPI, 256, FMT, true>(st, a, w);
+  if constexpr (EPI == EPI_PLAIN) {
+    const SplitPlan sp = plan_split<FMT>(a, bn, sms);
+    if (sp.parts > 1) {
+      if (sp.bn == 256) return launch_tc<EPI, 256, FMT, false, true>(st, a, w, sp.parts);
+      if (sp.bn == 128) return launch_tc<EPI, 128, FMT, false, true>(st, a, w, sp.parts);
+      return launch_tc<EPI, 64, FMT, false, true>(st, a, w, sp.parts);
+    }
+  }
   if (bn == 256) launch_tc<EPI, 256, FMT, false>(st, a, w);
   else if (bn == 128) launch_tc<EPI, 128, FMT, false>(st, a, w);
   else launch_tc<EPI, 64, FMT, false>(st, a, w);

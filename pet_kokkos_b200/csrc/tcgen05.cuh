@@ -68,6 +68,18 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
   return r;
 }
+__device__ __forceinline__ uint32_t cluster_size() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+  return r;
+}
+// Four words to the place of `p` in CTA `rank`'s shared memory.
+__device__ __forceinline__ void store4_at(const void* p, uint32_t rank, float x, float y, float z, float w) {
+  asm volatile(
+      "{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %0, %1;\n\tst.shared::cluster.v4.f32 [a], {%2, %3, %4, %5};\n\t}" ::"r"(smem_u32(p)),
+      "r"(rank), "f"(x), "f"(y), "f"(z), "f"(w)
+      : "memory");
+}
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }

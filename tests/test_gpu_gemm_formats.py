@@ -68,3 +68,22 @@ def test_a_pair_of_blocks_gives_the_bits_of_one(calc, mode):
             C = calc.gemm(A, W, mode)
             for r0 in (0, 12800, m - 3000):
                 assert np.array_equal(C[r0:r0 + 3000], calc.gemm(A[r0:r0 + 3000], W, mode)), (m, n, k, r0)
+
+
+@pytest.mark.parametrize("mode", ["native", "3xtf32", "tf32", "bf16"])
+@pytest.mark.parametrize("shape", [(64, 64, 1024), (1, 128, 4096), (129, 256, 1024), (300, 192, 2048), (1000, 512, 2048),
+                                   (648, 1024, 4096), (640, 256, 1056), (40, 64, 8192), (70, 128, 1152)])
+def test_blocks_that_share_a_tile(calc, shape, mode):
+    """Few tiles and a long contraction: the blocks of a cluster sum a run of it each and finish a slice of the columns each.
+    Two, four and eight of them, tile widths of 64, 128 and 256, ragged rows, a length that cannot be shared out."""
+    m, n, k = shape
+    rng = np.random.default_rng(m + n + k)
+    A = rng.normal(size=(m, k)).astype(np.float32)
+    W = rng.normal(size=(n, k)).astype(np.float32)
+    C = calc.gemm(A, W, mode)
+    size = np.abs(A).astype(np.float64) @ np.abs(W).T.astype(np.float64)
+    band = {"native": 2.0 ** -22, "3xtf32": 2.0 ** -20 + k * 2.0 ** -25, "tf32": 2.0 ** -10, "bf16": 2.0 ** -7}[mode]
+    assert (np.abs(C - A.astype(np.float64) @ W.T.astype(np.float64)) <= band * size).all()
+    if mode == "native":  # among so many rows that nothing is shared, the same rows have the same bits
+        many = np.concatenate([A, rng.normal(size=(20000, k)).astype(np.float32)])
+        assert np.array_equal(C, calc.gemm(many, W, mode)[:m])
