@@ -244,6 +244,7 @@ void Engine::stage(const pet_system* systems, int B, bool keep_cache) {
   }
   if (Nll >= (1LL << 24)) throw Error(1, "pet: too many atoms for the edge key");
   const int N = int(Nll);
+  PETB_CUDA(cudaStreamSynchronize(st.s));  // the previous copy out of this block, an evaluation that still reads the staged one
   // One host block, one copy: doubles first, then ints.
   const size_t nd = size_t(N) * 3 + size_t(B) * 18, ni = size_t(N) * 2 + size_t(B) * 9 + 2;
   char* hb = static_cast<char*>(staging(nd * 8 + ni * 4));
@@ -280,7 +281,6 @@ void Engine::stage(const pet_system* systems, int B, bool keep_cache) {
   }
   h_soff[B] = gi;
   h_goff[B] = bins;
-  PETB_CUDA(cudaStreamSynchronize(st.s));  // the previous evaluation may still read the staged block
   geom_arena.reset();
   char* db = static_cast<char*>(geom_arena.alloc_bytes(nd * 8 + ni * 4));
   PETB_CUDA(cudaMemcpyAsync(db, hb, nd * 8 + ni * 4, cudaMemcpyHostToDevice, st.s));
@@ -301,8 +301,6 @@ void Engine::stage(const pet_system* systems, int B, bool keep_cache) {
   // Calculator::stage resets the neighbour cache (include/pet/calculator.hpp:210-212); an evaluation that stages
   // the same atoms again keeps it
   verlet.valid = verlet.valid && keep_cache && was_natoms == h_natoms && was_per == h_per && was_species == h_species;
-  // the copy must finish before the staging block is reused by another stage()
-  PETB_CUDA(cudaStreamSynchronize(st.s));
 }
 
 // A batch being stepped shrinks as its structures finish (a batched relaxation): the structures `keep` (indices into
@@ -502,6 +500,7 @@ void Engine::run_model(const PackedEdges& pk, bool forces) {
   }
   // An exchanged list calls back into the engine in the middle of the pass: it is never recorded.
   const bool eager_only = !graphs || want_taps || prof.on || pk.exchange != nullptr;
+  ++graph_clock;
   if (eager_only) {
     last_out = model->run(st, save_arena, tmp_arena, pk, forces, gemm_mode, want_taps ? &taps : nullptr, fixed);
     last_pk = pk, have_out = true;
@@ -527,16 +526,24 @@ void Engine::run_model(const PackedEdges& pk, bool forces) {
       PETB_CUDA(cudaGraphLaunch(g.exec, st.s));
       st.launches += g.launches;
       ++graph_replays;
-      g.stamp = ++graph_clock;
+      g.stamp = graph_clock;
       save_arena.rewind(g.save_after), tmp_arena.rewind(g.tmp_after);
       last_out = g.out, last_pk = pk, have_out = true;
       return;
     }
   bool seen = false;
   for (auto& k : graph_seen) seen = seen || k == key;
-  if (!seen) {  // first time: eagerly (the pools may still grow, which a capture cannot contain)
-    if (graph_seen.size() >= 32) graph_seen.erase(graph_seen.begin());
-    graph_seen.push_back(key);
+  // A full cache gives up the recording used least recently, if that is long ago. Otherwise the shapes in turn outnumber the
+  // cache, each would be recorded (which costs several passes' launches) only to be dropped before it is used, and the pass
+  // runs eagerly instead: 18 shapes in turn against a cache of eight made a step of the 24-structure relaxation 2.4 ms for 1.9.
+  size_t lru = 0;
+  for (size_t i = 1; i < graph_cache.size(); ++i)
+    if (graph_cache[i].stamp < graph_cache[lru].stamp) lru = i;
+  const bool full = graph_cache.size() >= kGraphs;
+  if (!seen || (full && graph_cache[lru].stamp + 4 * kGraphs > graph_clock)) {
+    // the first time always eagerly: the pools may still grow, which a capture cannot contain
+    if (graph_seen.size() >= 2 * kGraphs) graph_seen.erase(graph_seen.begin());
+    if (!seen) graph_seen.push_back(key);
     last_out = model->run(st, save_arena, tmp_arena, pk, forces, gemm_mode, nullptr, fixed);
     last_pk = pk, have_out = true;
     return;
@@ -566,11 +573,8 @@ void Engine::run_model(const PackedEdges& pk, bool forces) {
   cudaGraphDestroy(graph);
   if (ie != cudaSuccess) throw Error(5, std::string("cudaGraphInstantiate: ") + cudaGetErrorString(ie));
   PETB_CUDA(cudaGraphLaunch(g.exec, st.s));
-  g.stamp = ++graph_clock;
-  if (graph_cache.size() >= 8) {  // least recently used out
-    size_t lru = 0;
-    for (size_t i = 1; i < graph_cache.size(); ++i)
-      if (graph_cache[i].stamp < graph_cache[lru].stamp) lru = i;
+  g.stamp = graph_clock;
+  if (full) {
     cudaGraphExecDestroy(graph_cache[lru].exec);
     graph_cache.erase(graph_cache.begin() + lru);
   }
@@ -581,7 +585,8 @@ void Engine::run_model(const PackedEdges& pk, bool forces) {
 void Engine::compute_staged(bool forces) {
   PETB_CUDA(cudaSetDevice(device));
   have_out = false;
-  PETB_CUDA(cudaStreamSynchronize(st.s));
+  if (in_flight) PETB_CUDA(cudaStreamSynchronize(st.s));  // (not for the copy of what was just staged)
+  in_flight = true;
   nbr_arena.reset();
   save_arena.reset();
   tmp_arena.reset();
@@ -593,7 +598,7 @@ void Engine::compute_staged(bool forces) {
   } else {
     posw = nbr_arena.alloc<double>(3 * size_t(g.Ntot > 0 ? g.Ntot : 1));
     wrap_positions(st, g, posw);
-    re = cell_list_search(st, nbr_arena, g, posw, ckpt.hypers.cutoff);
+    re = cell_list_search(st, nbr_arena, g, posw, ckpt.hypers.cutoff, pinned);
     find_reverse(st, re, g.Ntot);
   }
   const CutoffSpec cs = model->cutoff_spec();
@@ -640,7 +645,7 @@ RawEdges Engine::cached_edges() {
     PETB_CUDA(cudaStreamSynchronize(st.s));  // gi leaves scope
     posw = nbr_arena.alloc<double>(3 * size_t(N > 0 ? N : 1));
     wrap_positions(st, gr, posw);
-    const RawEdges found = cell_list_search(st, nbr_arena, gr, posw, reach);
+    const RawEdges found = cell_list_search(st, nbr_arena, gr, posw, reach, pinned);
     find_reverse(st, found, N);
     cache_arena.reset();
     const size_t E = found.E, Ea = E > 0 ? E : 1, Na = N > 0 ? N : 1;
@@ -710,6 +715,7 @@ void Engine::fetch(pet_results* out) {
   if (cudaEventElapsedTime(&ms, ev0, ev1) == cudaSuccess) last_ms = ms;
   if (gemm_tensor_error(st, pinned + kGaveUp))
     throw Error(5, "pet: a tensor-core GEMM gave up waiting on its pipeline; the results of this evaluation are invalid");
+  in_flight = false;
   const char* from = landing;
   for (int i = 0; i < n; from += pieces[i++].bytes) std::memcpy(pieces[i].to, from, pieces[i].bytes);
 }
@@ -852,7 +858,7 @@ void Engine::neighbor_list(const pet_system* systems, int B, pet_raw_edges* out)
   const Geom& g = geom;
   posw = nbr_arena.alloc<double>(3 * size_t(g.Ntot > 0 ? g.Ntot : 1));
   wrap_positions(st, g, posw);
-  RawEdges re = cell_list_search(st, nbr_arena, g, posw, ckpt.hypers.cutoff);
+  RawEdges re = cell_list_search(st, nbr_arena, g, posw, ckpt.hypers.cutoff, pinned);
   find_reverse(st, re, g.Ntot);
   out->n_edges = re.E;
   if (re.E > out->capacity) throw Error(2, "pet: " + std::to_string(re.E) + " edges, above the given capacity");
@@ -1004,7 +1010,7 @@ static StepOut session_step(Engine& I, const double* positions, bool on_device, 
   if (!s.valid) throw Error(1, "pet: no neighbour list set");
   if (s.shifted && !cell) throw Error(1, "pet: an edge list with shifts needs the cell");
   PETB_CUDA(cudaStreamSynchronize(st.s));
-  I.have_out = false;
+  I.have_out = false, I.in_flight = true;
   I.nbr_arena.reset();
   I.save_arena.reset();
   I.tmp_arena.reset();

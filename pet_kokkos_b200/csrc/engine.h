@@ -123,6 +123,7 @@ struct Engine {
   PackedEdges last_pk;
   PassOut last_out;
   bool have_out = false;
+  bool in_flight = true;  // work that uses the pools may be on the stream
   int last_B = 0, last_N = 0;
   int* pinned = nullptr;  // small pinned scratch for readbacks
   static constexpr int kGaveUp = 9;  // the word of it that says whether a GEMM gave up on a wait
@@ -147,6 +148,7 @@ struct Engine {
     long long launches = 0;
     uint64_t stamp = 0;
   };
+  static constexpr size_t kGraphs = 32;  // recordings kept, a few hundred launches each
   std::vector<GraphEntry> graph_cache;
   std::vector<std::vector<uint64_t>> graph_seen;
   uint64_t graph_clock = 0;

@@ -525,7 +525,7 @@ void wrap_positions(Stream& st, const Geom& g, double* posw) {
   PETB_LAUNCH_CHECK(st);
 }
 
-RawEdges cell_list_search(Stream& st, Arena& arena, const Geom& g, const double* posw, double cutoff) {
+RawEdges cell_list_search(Stream& st, Arena& arena, const Geom& g, const double* posw, double cutoff, int* pinned) {
   const int N = g.Ntot, nbins = g.nbins > 0 ? g.nbins : 1;
   // 52 bytes per raw edge and 56 per atom: the reference's own count (tools/roofline.py:308-309).
   const ProfScope ps(st, PC_GEOMETRY, 0.0, 56.0 * N);
@@ -555,10 +555,9 @@ RawEdges cell_list_search(Stream& st, Arena& arena, const Geom& g, const double*
   launch(st, k_walk<false>, cdiv(size_t(N) * 32, 128), 128, 0, w, ecnt, nullptr, re);
   PETB_LAUNCH_CHECK(st);
   exclusive_scan(st, arena, ecnt, re.off, N);
-  int E = 0;
-  PETB_CUDA(cudaMemcpyAsync(&E, re.off + N, sizeof(int), cudaMemcpyDeviceToHost, st.s));
+  PETB_CUDA(cudaMemcpyAsync(pinned, re.off + N, sizeof(int), cudaMemcpyDeviceToHost, st.s));
   PETB_CUDA(cudaStreamSynchronize(st.s));
-  re.E = E;
+  const int E = re.E = *pinned;
   const size_t Ea = E > 0 ? E : 1;
   re.i = arena.alloc<int>(Ea);
   re.j = arena.alloc<int>(Ea);
@@ -606,27 +605,36 @@ void verlet_check(Stream& st, const Geom& g, const double* pos0, const double* c
   PETB_LAUNCH_CHECK(st);
 }
 
+namespace {
+// The offsets of NC atoms and, right behind off[NC], what is counted beside them: the most edges of an atom (an int) and the
+// sum of squares (eight bytes, aligned), so that one fill clears them and one copy brings all three.
+struct Counts {
+  int *off, *most;
+  unsigned long long* pairs;
+};
+Counts counts(Stream& st, Arena& arena, int NC) {
+  int* off = arena.alloc<int>(size_t(NC) + 8) + (NC & 1);
+  PETB_CUDA(cudaMemsetAsync(off + NC, 0, 16, st.s));
+  return {off, off + NC + 1, reinterpret_cast<unsigned long long*>(off + NC + 2)};
+}
+}  // namespace
+
 PackedEdges pack_edges(Stream& st, Arena& arena, const RawEdges& re, int NC, const int* atom_species,
                        const CutoffSpec& cs, int* pinned, const AdaptiveCut& ad) {
   PackedEdges pk;
   pk.N = NC;
   pk.adaptive = ad;
   pk.atom_species = atom_species;
-  pk.off = arena.alloc<int>(NC + 1);
   const ProfScope ps(st, PC_GEOMETRY, 0.0, 60.0 * double(re.E) + 8.0 * NC);
-  int* kcnt = arena.alloc<int>(NC + 4);
-  int* maxm = kcnt + NC;
-  unsigned long long* pairs = reinterpret_cast<unsigned long long*>(arena.alloc_bytes(8));
-  PETB_CUDA(cudaMemsetAsync(maxm, 0, sizeof(int), st.s));
-  PETB_CUDA(cudaMemsetAsync(pairs, 0, 8, st.s));
+  const Counts c = counts(st, arena, NC);
+  pk.off = c.off;
+  int* kcnt = arena.alloc<int>(NC + 1);
   if (NC > 0) {
-    launch(st, k_keep_count, cdiv(size_t(NC) * 32, 256), 256, 0, NC, re.off, re.dist, cs.cutoff, kcnt, maxm, pairs, ad.acut, re.j);
+    launch(st, k_keep_count, cdiv(size_t(NC) * 32, 256), 256, 0, NC, re.off, re.dist, cs.cutoff, kcnt, c.most, c.pairs, ad.acut, re.j);
     PETB_LAUNCH_CHECK(st);
   }
   exclusive_scan(st, arena, kcnt, pk.off, NC);
-  PETB_CUDA(cudaMemcpyAsync(pinned, pk.off + NC, sizeof(int), cudaMemcpyDeviceToHost, st.s));
-  PETB_CUDA(cudaMemcpyAsync(pinned + 1, maxm, sizeof(int), cudaMemcpyDeviceToHost, st.s));
-  PETB_CUDA(cudaMemcpyAsync(pinned + 2, pairs, 8, cudaMemcpyDeviceToHost, st.s));
+  PETB_CUDA(cudaMemcpyAsync(pinned, pk.off + NC, 16, cudaMemcpyDeviceToHost, st.s));
   PETB_CUDA(cudaStreamSynchronize(st.s));
   pk.E = pinned[0];
   pk.M = pinned[1] > 1 ? pinned[1] : 1;
@@ -664,19 +672,16 @@ PackedEdges pack_edges_fixed(Stream& st, Arena& arena, const RawEdges& re, int N
   pk.N = NC, pk.E = e_cap, pk.M = m_cap, pk.pairs = pairs;
   pk.adaptive = ad;
   pk.atom_species = atom_species;
-  pk.off = arena.alloc<int>(NC + 1);
   const ProfScope ps(st, PC_GEOMETRY, 0.0, 60.0 * double(re.E) + 8.0 * NC);
-  int* kcnt = arena.alloc<int>(NC + 4);
-  int* maxm = kcnt + NC;
-  unsigned long long* pr = reinterpret_cast<unsigned long long*>(arena.alloc_bytes(8));
-  PETB_CUDA(cudaMemsetAsync(maxm, 0, sizeof(int), st.s));
-  PETB_CUDA(cudaMemsetAsync(pr, 0, 8, st.s));
-  launch(st, k_keep_count, cdiv(size_t(NC) * 32, 256), 256, 0, NC, re.off, re.dist, cs.cutoff, kcnt, maxm, pr, ad.acut, re.j);
+  const Counts c = counts(st, arena, NC);
+  pk.off = c.off;
+  int* kcnt = arena.alloc<int>(NC + 1);
+  launch(st, k_keep_count, cdiv(size_t(NC) * 32, 256), 256, 0, NC, re.off, re.dist, cs.cutoff, kcnt, c.most, c.pairs, ad.acut, re.j);
   PETB_LAUNCH_CHECK(st);
-  launch(st, k_clamp_counts, cdiv(NC, 256), 256, 0, kcnt, NC, m_cap);  // maxm already holds the unclamped maximum
+  launch(st, k_clamp_counts, cdiv(NC, 256), 256, 0, kcnt, NC, m_cap);  // c.most already holds the unclamped maximum
   PETB_LAUNCH_CHECK(st);
   exclusive_scan(st, arena, kcnt, pk.off, NC);
-  launch(st, k_check_capacity, 1, 1, 0, pk.off, NC, maxm, e_cap, m_cap, overflow);
+  launch(st, k_check_capacity, 1, 1, 0, pk.off, NC, c.most, e_cap, m_cap, overflow);
   PETB_LAUNCH_CHECK(st);
   launch(st, k_clamp_offsets, cdiv(NC + 1, 256), 256, 0, pk.off, NC, e_cap);
   PETB_LAUNCH_CHECK(st);

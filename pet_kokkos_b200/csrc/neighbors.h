@@ -111,7 +111,7 @@ void verlet_check(Stream& st, const Geom& g, const double* pos0, const double* c
 // Wrapped positions for the search: posw [Ntot,3].
 void wrap_positions(Stream& st, const Geom& g, double* posw);
 // The cell-list search. Allocates from `arena`; reads back the edge count once.
-RawEdges cell_list_search(Stream& st, Arena& arena, const Geom& g, const double* posw, double cutoff);
+RawEdges cell_list_search(Stream& st, Arena& arena, const Geom& g, const double* posw, double cutoff, int* pinned_scratch);
 // Each raw edge's partner, by a search of the neighbour's own range.
 void find_reverse(Stream& st, const RawEdges& re, int N);
 // Edge vectors of an engine-supplied list from positions, shifts and the cell (the reference's md_vectors).
