@@ -599,8 +599,8 @@ def run_ours(args):
                        "tflops": v["flops"] / max(v["ms"], 1e-9) / 1e9, "gbs": v["bytes"] / max(v["ms"], 1e-9) / 1e6}
                    for k, v in prof.items()}
         # the other GEMM/attention modes on the same staged structures (N = 1 only), three steps each after two:
-        # native = fp32 on the CUDA cores (the default correctness mode); tf32 and bf16 = the speed modes (one
-        # tensor-core pass per product, single-pass tf32 attention), each with its measured distance from native
+        # native = fp32 accuracy (the default correctness mode); tf32 and bf16 = the speed modes (one
+        # tensor-core pass per product, in the attention too), each with its measured distance from native
         modes = None
         if world == 1 and not args.no_cpu:
             modes, results = {}, {args.gemm: r}

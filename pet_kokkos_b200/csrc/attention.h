@@ -10,9 +10,9 @@ enum AttnMode { ATTN_NATIVE = 0, ATTN_TF32X3 = 1, ATTN_TF32 = 2 };
 struct AttnArgs {
   int N = 0, H = 0, hd = 0, S = 0;  // atoms, heads, head_dim, most tokens of any atom (max neighbours + 1)
   float sc = 1.f;                   // 1 / (sqrt(head_dim) * temperature)
-  // How the products run (the reference's AttentionMode, include/pet/gemm.hpp): ATTN_NATIVE, fp32 on the CUDA
-  // cores; ATTN_TF32X3, the split products on the tensor cores, as accurate but for the tensor core's truncating
-  // accumulate; ATTN_TF32, one tf32 product per tile (a speed mode, about three decimal digits).
+  // How the products run (the reference's AttentionMode, include/pet/gemm.hpp): ATTN_NATIVE, operands in three fp16 parts (fp32
+  // accuracy); ATTN_TF32X3, in two, as accurate but for the tensor core's truncating accumulate; ATTN_TF32, in one of eleven
+  // bits (a speed mode, about three decimal digits). On the CUDA cores in fp32 where no tensor-core kernel takes the shape.
   int mode = 0;
   bool tf32 = false;                // forward: the tensor-core modes on tf32 instructions (where energies depend on their bits)
   double pairs = 0.0;               // sum over atoms of tokens^2 (work accounting only)

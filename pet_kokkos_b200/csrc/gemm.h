@@ -14,7 +14,8 @@
 //     into which, for each mode;
 //   * fp32 FMA on the CUDA cores (gemm_simt.cu): one accumulation chain per output in k order, for operands that have
 //     no packed weight (pet_gemm_host_static) or that TMA cannot address.
-// A row's bits depend on that row and the weight alone, in both: not on how many rows share its launch.
+// In the native format and on the CUDA cores a row's bits depend on that row and the weight alone, not on how many rows share
+// its launch. The other formats add a long K in another order where few rows leave SMs for it (plan_split, gemm_tc.cu).
 #pragma once
 
 #include "common.h"
