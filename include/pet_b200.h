@@ -334,6 +334,25 @@ int pet_debug_fetch(pet_calc* c, const char* name, float* out, size_t capacity, 
  * tests/test_gemm_modes.cpp:63-103). */
 int pet_gemm_host(pet_calc* c, int mode, int w_transposed, int m, int n, int k, const float* A, const float* W, float* C);
 
+/* The same with an epilogue and in one operand format, whatever the number of rows (testing aid: pet_gemm_host reaches the
+ * plain epilogue and the formats that a mode names). `format` and `epilogue` are the numbers of csrc/gemm.h's enums. */
+typedef struct pet_debug_gemm_args {
+  int format, epilogue, w_transposed, m, n, k;
+  const float *A, *W;
+  const float* bias;       /* [n], optional */
+  const float* res;        /* [m,n], optional: added to rows >= res_row0 */
+  int res_row0;
+  float* pre;              /* [m,n] written (optional), or read: SiLU' [m,n], SwiGLU' [m,2n] */
+  const float* tab;        /* compress: [n_tab,n] */
+  int n_tab;
+  const int* species;      /* [m] rows of tab */
+  const float* wx;         /* [n,4] */
+  const double *vec, *dist; /* [m,3], [m] */
+  float* C;                /* [m,n]; SwiGLU [m,n/2]; SwiGLU' [m,2n] */
+  float* row_max;          /* [m], optional: each row's largest |C| as the epilogue keeps it */
+} pet_debug_gemm_args;
+int pet_debug_gemm(pet_calc* c, const pet_debug_gemm_args* args);
+
 /* A ready-made pet_exchange over NCCL: what an MD engine's pair style does around pet::Exchange
  * (lammps/ML-PET/pair_pet.cpp:268-360 routing, :396-472 exchange_rows, :479-555 set_live / edges), inside the
  * library. Rows of edges to ghosts are packed by a kernel, cross with ncclSend / ncclRecv on the calculator's own

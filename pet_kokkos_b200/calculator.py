@@ -20,6 +20,9 @@ _LIB_PATH = Path(__file__).resolve().parent / "libpet_b200.so"
 _lib = None
 
 GEMM_MODES = {"native": 0, "tf32": 1, "bf16": 2, "3xtf32": 3}
+# operand formats and epilogues of the weight GEMM (csrc/gemm.h), for debug_gemm
+GEMM_FORMATS = {"f16x3": 0, "f16x2": 1, "f16": 2, "bf16": 3, "tf32x2": 4, "tf32": 5}
+GEMM_EPILOGUES = {"plain": 0, "silu": 1, "swiglu": 2, "silu_bwd": 3, "swiglu_bwd": 4, "compress": 5}
 RECOMPUTE_TIERS = {"auto": 0, "never": 1, "wide": 2, "layers": 3}
 
 
@@ -98,6 +101,14 @@ class PetProfileEntry(C.Structure):
                 ("bytes", C.c_double)]
 
 
+class PetDebugGemmArgs(C.Structure):
+    _fields_ = [(f, C.c_int) for f in ("format", "epilogue", "w_transposed", "m", "n", "k")] + \
+               [(f, C.POINTER(C.c_float)) for f in ("A", "W", "bias", "res")] + [("res_row0", C.c_int)] + \
+               [(f, C.POINTER(C.c_float)) for f in ("pre", "tab")] + \
+               [("n_tab", C.c_int), ("species", C.POINTER(C.c_int)), ("wx", C.POINTER(C.c_float)), ("vec", C.POINTER(C.c_double)),
+                ("dist", C.POINTER(C.c_double)), ("C", C.POINTER(C.c_float)), ("row_max", C.POINTER(C.c_float))]
+
+
 class PetRawEdges(C.Structure):
     _fields_ = [("capacity", C.c_int), ("n_edges", C.c_int), ("i", C.POINTER(C.c_int)), ("j", C.POINTER(C.c_int)),
                 ("shift", C.POINTER(C.c_int)), ("vec", C.POINTER(C.c_double)), ("dist", C.POINTER(C.c_double)),
@@ -159,6 +170,7 @@ SIGNATURES = {
     "pet_debug_fetch": (C.c_int, [C.c_void_p, C.c_char_p, _P(C.c_float), C.c_size_t, _P(C.c_size_t)]),
     "pet_gemm_host_static": (C.c_int, [C.c_int, C.c_int, C.c_int, _P(C.c_float), _P(C.c_float), _P(C.c_float), C.c_char_p,
                                        C.c_size_t]),
+    "pet_debug_gemm": (C.c_int, [C.c_void_p, _P(PetDebugGemmArgs)]),
     "pet_gemm_host": (C.c_int, [C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, _P(C.c_float), _P(C.c_float),
                                 _P(C.c_float)]),
 }
@@ -656,3 +668,34 @@ class Calculator:
         fp = lambda a: a.ctypes.data_as(C.POINTER(C.c_float))
         self._check(self._lib.pet_gemm_host(self._h, GEMM_MODES[mode], int(w_transposed), m, n, k, fp(A), fp(W), fp(Cm)))
         return Cm
+
+    def debug_gemm(self, A, W, fmt, epilogue="plain", w_transposed=True, bias=None, res=None, res_row0=0, pre=None, tab=None,
+                   species=None, wx=None, vec=None, dist=None, want_pre=True):
+        """One weight GEMM with an epilogue in one operand format: (C, pre as written or None, row maxima of C)."""
+        g, keep = PetDebugGemmArgs(), []
+
+        def ptr(x, dtype, pt):
+            if x is None:
+                return None
+            keep.append(np.ascontiguousarray(x, dtype=dtype))
+            return keep[-1].ctypes.data_as(pt)
+        f32 = lambda x: ptr(x, np.float32, C.POINTER(C.c_float))
+        m, k = np.shape(A)
+        n = np.shape(W)[0] if w_transposed else np.shape(W)[1]
+        g.format, g.epilogue = GEMM_FORMATS[fmt], GEMM_EPILOGUES[epilogue]
+        g.w_transposed, g.m, g.n, g.k, g.res_row0 = int(w_transposed), m, n, k, res_row0
+        g.A, g.W, g.bias, g.res, g.tab, g.wx = f32(A), f32(W), f32(bias), f32(res), f32(tab), f32(wx)
+        g.n_tab = 0 if tab is None else len(tab)
+        g.species = ptr(species, np.int32, C.POINTER(C.c_int))
+        g.vec, g.dist = ptr(vec, np.float64, C.POINTER(C.c_double)), ptr(dist, np.float64, C.POINTER(C.c_double))
+        out = np.zeros((m, {"swiglu": n // 2, "swiglu_bwd": 2 * n}.get(epilogue, n)), np.float32)
+        written = None
+        if pre is not None:
+            g.pre = f32(pre)
+        elif want_pre and epilogue in ("silu", "swiglu", "compress"):
+            written = np.zeros((m, n), np.float32)
+            g.pre = written.ctypes.data_as(C.POINTER(C.c_float))
+        row_max = np.zeros(m, np.float32)
+        g.C, g.row_max = out.ctypes.data_as(C.POINTER(C.c_float)), row_max.ctypes.data_as(C.POINTER(C.c_float))
+        self._check(self._lib.pet_debug_gemm(self._h, C.byref(g)))
+        return out, written, row_max

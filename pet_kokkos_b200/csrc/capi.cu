@@ -261,5 +261,11 @@ int pet_debug_fetch(pet_calc* c, const char* name, float* out, size_t capacity, 
 int pet_gemm_host(pet_calc* c, int mode, int w_transposed, int m, int n, int k, const float* A, const float* W, float* C) {
   return guarded(c, [&](Engine& e) { e.gemm_host(mode, w_transposed != 0, m, n, k, A, W, C); });
 }
+int pet_debug_gemm(pet_calc* c, const pet_debug_gemm_args* args) {
+  return guarded(c, [&](Engine& e) {
+    if (!args || args->format < 0 || args->format > petb::FMT_TF32) throw petb::Error(PET_ERR_INVALID, "pet: bad GEMM arguments");
+    e.gemm_on_host_arrays(*args, args->format, args->format);
+  });
+}
 
 }  // extern "C"

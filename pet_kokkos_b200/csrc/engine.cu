@@ -5,6 +5,7 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <type_traits>
 
 #include "gemm.h"
 
@@ -1353,25 +1354,57 @@ void Engine::debug_fetch(const char* name, float* out, size_t capacity, size_t* 
 }
 
 void Engine::gemm_host(int mode, bool w_transposed, int m, int n, int k, const float* A, const float* W, float* C) {
+  pet_debug_gemm_args g{};
+  g.w_transposed = w_transposed, g.m = m, g.n = n, g.k = k, g.A = A, g.W = W, g.C = C;
+  gemm_on_host_arrays(g, FMT_F16X3, format_of(mode));
+}
+
+void Engine::gemm_on_host_arrays(const pet_debug_gemm_args& g, int native_format, int fast_format) {
   PETB_CUDA(cudaSetDevice(device));
-  if (m <= 0 || n <= 0 || k <= 0 || !A || !W || !C) throw Error(2, "pet: bad GEMM arguments");
+  const size_t m = g.m, n = g.n, k = g.k;
+  const bool reads_pre = g.epilogue == EPI_SILU_BWD || g.epilogue == EPI_SWIGLU_BWD, compress = g.epilogue == EPI_COMPRESS;
+  if (g.m <= 0 || g.n <= 0 || g.k <= 0 || !g.A || !g.W || !g.C || (reads_pre && !g.pre) ||
+      (compress && (!g.tab || g.n_tab <= 0 || !g.species || !g.wx || !g.vec || !g.dist)))
+    throw Error(2, "pet: bad GEMM arguments");
+  if (compress)
+    for (size_t i = 0; i < m; ++i)
+      if (g.species[i] < 0 || g.species[i] >= g.n_tab) throw Error(2, "pet: bad GEMM arguments");
   PETB_CUDA(cudaStreamSynchronize(st.s));
   tmp_arena.reset();
-  float* dA = tmp_arena.alloc<float>(size_t(m) * k);
-  float* dW = tmp_arena.alloc<float>(size_t(n) * k);
-  float* dC = tmp_arena.alloc<float>(size_t(m) * n);
-  PETB_CUDA(cudaMemcpyAsync(dA, A, 4 * size_t(m) * k, cudaMemcpyHostToDevice, st.s));
-  PETB_CUDA(cudaMemcpyAsync(dW, W, 4 * size_t(n) * k, cudaMemcpyHostToDevice, st.s));
-  GemmArgs a;
-  a.A = dA, a.lda = k, a.C = dC, a.ldc = n, a.M = m, a.N = n, a.K = k;
-  // the weight packed from either orientation, as a loaded one is
-  auto pack = [&](Format fmt) {
-    uint16_t* out = tmp_arena.alloc<uint16_t>(packed_halves(fmt, n, k));
-    return pack_weight(st.s, fmt, dW, w_transposed ? k : 1, w_transposed ? 1 : n, n, k, out, tmp_arena.alloc<uint32_t>(1));
+  auto up = [&](const auto* from, size_t count) {
+    using T = std::remove_const_t<std::remove_pointer_t<decltype(from)>>;
+    if (!from) return static_cast<T*>(nullptr);
+    T* to = tmp_arena.alloc<T>(count);
+    PETB_CUDA(cudaMemcpyAsync(to, from, sizeof(T) * count, cudaMemcpyHostToDevice, st.s));
+    return to;
   };
-  a.nat = pack(FMT_F16X3), a.fast = pack(format_of(mode));
+  GemmArgs a;
+  a.M = g.m, a.N = g.n, a.K = g.k, a.epi = g.epilogue;
+  a.lda = a.K, a.ldc = g.epilogue == EPI_SWIGLU ? a.N / 2 : g.epilogue == EPI_SWIGLU_BWD ? 2 * a.N : a.N;
+  a.ldr = a.N, a.ldp = g.epilogue == EPI_SWIGLU_BWD ? 2 * a.N : a.N;
+  const size_t c_size = m * size_t(a.ldc), pre_size = m * size_t(a.ldp);
+  float* dC = tmp_arena.alloc<float>(c_size);
+  const float* dW = up(g.W, n * k);
+  a.A = up(g.A, m * k), a.C = dC, a.bias = up(g.bias, n), a.res = up(g.res, m * n), a.res_row0 = g.res_row0;
+  a.pre = reads_pre ? up(g.pre, pre_size) : g.pre ? tmp_arena.alloc<float>(pre_size) : nullptr;
+  if (compress) {
+    a.tab = up(g.tab, size_t(g.n_tab) * n), a.sp = up(g.species, m), a.wx = up(g.wx, 4 * n);
+    a.vec = up(g.vec, 3 * m), a.dist = up(g.dist, m);
+  }
+  if (g.row_max) {
+    a.c_max = tmp_arena.alloc<uint32_t>(m);
+    PETB_CUDA(cudaMemsetAsync(a.c_max, 0, 4 * m, st.s));
+  }
+  // the weight packed from either orientation, as a loaded one is
+  auto pack = [&](int fmt) {
+    uint16_t* out = tmp_arena.alloc<uint16_t>(packed_halves(fmt, a.N, a.K));
+    return pack_weight(st.s, Format(fmt), dW, g.w_transposed ? k : 1, g.w_transposed ? 1 : n, a.N, a.K, out, tmp_arena.alloc<uint32_t>(1));
+  };
+  a.nat = pack(native_format), a.fast = pack(fast_format);
   gemm(st, tmp_arena, a);
-  PETB_CUDA(cudaMemcpyAsync(C, dC, 4 * size_t(m) * n, cudaMemcpyDeviceToHost, st.s));
+  PETB_CUDA(cudaMemcpyAsync(g.C, dC, 4 * c_size, cudaMemcpyDeviceToHost, st.s));
+  if (g.pre && !reads_pre) PETB_CUDA(cudaMemcpyAsync(g.pre, a.pre, 4 * pre_size, cudaMemcpyDeviceToHost, st.s));
+  if (g.row_max) PETB_CUDA(cudaMemcpyAsync(g.row_max, a.c_max, 4 * m, cudaMemcpyDeviceToHost, st.s));
   gemm_tensor_error_ask(st, pinned + kGaveUp);
   PETB_CUDA(cudaStreamSynchronize(st.s));
   if (gemm_tensor_error(st, pinned + kGaveUp)) throw Error(5, "pet: a tensor-core GEMM gave up waiting on its pipeline");
