@@ -9,12 +9,15 @@
 namespace petb {
 
 // 1 / (1 + exp(-x)), the reciprocal from the hardware's estimate (within 1 ulp) and one Newton-Raphson step, which leaves
-// the rounding of its last fma: 1.3 ulp at most with expf's own error, the quotient's 1.3. The quotient compiles into a
-// call that spends 140 clocks an element in a GEMM's epilogue, this into a dozen instructions that overlap. The argument
-// is bounded where the estimate of the reciprocal would no longer be a normal number (sigmoid(-87) = 1.6e-38).
+// the rounding of its last fma. Relative error: expf's ulp (2^-23 at most), the sum's rounding and that one (2^-24 each), 2^-22
+// in all; the quotient's is the same. The quotient compiles into a call that spends 140 clocks an element in a GEMM's
+// epilogue, this into a dozen instructions that overlap. The argument is bounded so that exp stays finite; the bound passes a
+// NaN on (fminf would put 88 in its place). Below x = -87.3 the estimate is no longer a normal number and the result is 0,
+// where the quotient's last values are subnormal.
 __device__ __forceinline__ float sigmoid_f(float x) {
-  const float d = 1.0f + expf(fminf(-x, 87.0f));
-  float r;
+  float a, r;
+  asm("min.NaN.f32 %0, %1, %2;" : "=f"(a) : "f"(-x), "f"(88.0f));
+  const float d = 1.0f + expf(a);
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
   return fmaf(r, fmaf(-d, r, 1.0f), r);
 }

@@ -1,4 +1,4 @@
-"""Every epilogue of the tensor-core GEMM in every operand format that runs it, at ragged widths, against fp64.
+"""Every epilogue of the tensor-core GEMM in every operand format that runs it, at ragged widths, against fp64; the sigmoid and its limits.
 
 The widths are no multiple of a column tile (64, 128, 256) nor of a chunk of the epilogue (16 or 32 columns), the rows none of a
 row tile; one shape is large enough for pairs of blocks, one long enough for blocks that share a tile. The bands are the operand
@@ -84,3 +84,56 @@ def test_against_fp64(calc, fmt, epi, shape):
             other = calc.debug_gemm(A, W if transposed else W.T, fmt, epi, w_transposed=transposed, want_pre=False, **args)[0]
             assert np.array_equal(C, other)  # the same without the saved pre-activation
         assert np.array_equal(row_max, np.abs(C).max(axis=1))
+
+
+def gates(calc, x):
+    """sigmoid(x) as the SwiGLU epilogue computes it: values of one beside gates of x, both from the bias."""
+    n = 2 * len(x)
+    bias = np.ones(n, np.float32)
+    bias[1::2] = x
+    C, pre, _ = calc.debug_gemm(np.zeros((3, 4), np.float32), np.zeros((n, 4), np.float32), "f16x3", "swiglu", bias=bias)
+    assert np.array_equal(pre[0], bias, equal_nan=True) and np.array_equal(C[0], C[2], equal_nan=True)
+    return C[1]
+
+
+def test_the_sigmoid(calc):
+    """Within 2^-22 of itself (expf within one ulp, the sum, the last step of the reciprocal), with the quotient's limits; a result
+    that is no normal number may be zero."""
+    rng = np.random.default_rng(0)
+    x = np.concatenate([np.linspace(-87.3, 87.3, 20000), rng.normal(size=40000), 1e-3 * rng.normal(size=4000), [0.0] * 4]).astype(np.float32)
+    ref = sigmoid(x.astype(np.float64))
+    assert (np.abs(gates(calc, x) - ref) <= 2.0 ** -22 * ref).all()
+    low = np.linspace(-90.0, -87.3, 4000).astype(np.float32)
+    assert (np.abs(gates(calc, low) - sigmoid(low.astype(np.float64))) <= 2.0 ** -126).all()
+    far = np.array([-88.8, -1e3, -1e38, -np.inf, 1e3, 1e38, np.inf, 90.0], np.float32)
+    assert np.array_equal(gates(calc, far), np.array([0, 0, 0, 0, 1, 1, 1, 1], np.float32))
+
+
+@pytest.mark.parametrize("epi", ["silu", "swiglu", "silu_bwd", "swiglu_bwd", "compress"])
+def test_what_is_not_a_number_stays_so(calc, epi):
+    """A NaN in a gate or a pre-activation gives NaN in its own outputs and nowhere else."""
+    m, n, k = 70, 72, 36
+    rng = np.random.default_rng(1)
+    A, W = rng.normal(size=(m, k)), rng.normal(size=(n, k))
+    args, want = {}, np.zeros((m, {"swiglu": n // 2, "swiglu_bwd": 2 * n}.get(epi, n)), bool)
+    if epi.endswith("bwd"):
+        args["pre"] = rng.normal(size=(m, 2 * n if epi == "swiglu_bwd" else n))
+        args["pre"][7, 11] = np.nan
+        want[7, 10:12] = True  # the gate of a pair: both adjoints
+        if epi == "silu_bwd":
+            want[7, 10] = False
+    else:
+        args["bias"] = rng.normal(size=n)
+        args["bias"][11] = np.nan
+        want[:, 5 if epi == "swiglu" else 11] = True
+        if epi == "compress":
+            args.update(tab=rng.normal(size=(5, n)), species=rng.integers(0, 5, size=m), wx=rng.normal(size=(n, 4)), vec=rng.normal(size=(m, 3)),
+                        dist=np.ones(m))
+    assert np.array_equal(np.isnan(calc.debug_gemm(A, W, "f16x3", epi, **args)[0]), want)
+
+
+def test_large_negative_values_do_not_pass_the_gate(calc):
+    """silu(-1e38) is -0, not -1e38 times the smallest normal number."""
+    bias = np.array([-1e38, -3e38, -1e30, 0.0], np.float32)
+    C = calc.debug_gemm(np.zeros((2, 4), np.float32), np.zeros((4, 4), np.float32), "f16x3", "silu", bias=bias)[0]
+    assert (C == 0.0).all()
