@@ -34,7 +34,7 @@ enum Epilogue {
 enum GemmMode { GEMM_NATIVE = 0, GEMM_TF32 = 1, GEMM_BF16 = 2, GEMM_TF32X3 = 3 };
 
 // How an fp32 operand is handed to the 16-bit tensor cores. The fp16 formats scale it by a power of two first: s brings the
-// largest value of the row (of the matrix, for a weight) to [2^14, 2^15).
+// largest value of the row, of A and of B alike, to [2^14, 2^15).
 //   FMT_F16X3 (native)   s x = h + m + l: h is s x rounded to a multiple of 2^8, eight bits of the row's largest value; what
 //                        remains goes into two fp16 parts. Every value is represented to its last bit, or to 2^-23 of
 //                        itself where it is below 2^-6 of the row's largest. Six products; h.h on its own accumulator,
@@ -55,25 +55,28 @@ inline Format format_of(int mode) {
 constexpr bool scales_rows(int fmt) { return fmt == FMT_F16X3 || fmt == FMT_F16X2 || fmt == FMT_F16; }
 
 // A weight [rows, K] in one format, made once when it was loaded. K is padded with zeros to a multiple of 32.
-//   FMT_F16X3   main [rows][Kp/32][h 32 | m 32], low [rows][Kp] the l parts; `amax` the bits of the matrix's largest |x|
-//   FMT_F16X2   main [rows][Kp/32][h 32 | l 32]; `amax`
-//   FMT_F16     main [rows][Kp]; `amax`
+//   FMT_F16X3   main [rows][Kp/32][h 32 | m 32], low [rows][Kp] the l parts; `unscale` [rows] what undoes each row's scale, a power
+//               of two as bf16, with zeros up to a multiple of eight
+//   FMT_F16X2   main [rows][Kp/32][h 32 | l 32]; `unscale`
+//   FMT_F16     main [rows][Kp]; `unscale`
 //   FMT_BF16    main [rows][Kp]
 //   FMT_TF32X2  main [rows][Kp] and low [rows][Kp], fp32 words; FMT_TF32 main alone
 struct PackedB {
   Format fmt = FMT_F16X3;
   const uint16_t* main = nullptr;
   const uint16_t* low = nullptr;
-  const uint32_t* amax = nullptr;
+  const uint16_t* unscale = nullptr;
   int Kp = 0;
 };
 inline int packed_k(int K) { return (K + 31) / 32 * 32; }
+inline size_t unscale_halves(int rows) { return size_t(rows + 7) / 8 * 8; }
 // 16-bit values and bytes a packed weight takes (main and low together), rows padded apart to 16 bytes.
 inline size_t packed_halves(int fmt, int rows, int K) {
   return size_t(rows) * packed_k(K) * (fmt == FMT_F16X3 ? 3 : fmt == FMT_F16X2 || fmt == FMT_TF32 ? 2 : fmt == FMT_TF32X2 ? 4 : 1);
 }
-// Packs W [rows, K] (element (r, k) at W[r * ld_r + k * ld_k]) into `out`; `amax` is one device word, written here.
-PackedB pack_weight(cudaStream_t s, Format fmt, const float* W, size_t ld_r, size_t ld_k, int rows, int K, uint16_t* out, uint32_t* amax);
+// Packs W [rows, K] (element (r, k) at W[r * ld_r + k * ld_k]) into `out`, and writes `unscale` (unscale_halves(rows),
+// 16-byte aligned).
+PackedB pack_weight(cudaStream_t s, Format fmt, const float* W, size_t ld_r, size_t ld_k, int rows, int K, uint16_t* out, uint16_t* unscale);
 
 struct GemmArgs {
   const float* A = nullptr;  // [M,K]

@@ -11,7 +11,7 @@
 //   warp 1      issuer: one lane issues the products (M = 128, N = BN, K = 16 each) into one of TWO accumulators in
 //               tensor memory, small terms first, and frees the step's slots with one tcgen05.commit;
 //   warps 4-11  epilogue: tcgen05.ld the accumulator (a thread owns a row, a warp pair splits the columns), undo the
-//               row's and the weight's scale, and work through 32 x 32 chunks in shared memory: what the epilogue reads (a
+//               two rows' scales, and work through 32 x 32 chunks in shared memory: what the epilogue reads (a
 //               residual, a saved pre-activation) is brought there by TMA a chunk ahead, what it writes leaves by TMA. The
 //               accumulator is handed back as soon as it has been read.
 // FMT_F16X3 fills both accumulators for one tile (the exact h.h sum, and the small products); the epilogue warps add the two into
@@ -59,7 +59,7 @@ constexpr int TBM = 128;  // rows of a tile
 constexpr int kEpiWarp0 = 4, kEpiWarps = 8, kConvWarp0 = 12;
 
 // ---- the fp16 formats' scales --------------------------------------------------------------
-// The power of two that brings a row (or matrix) whose largest magnitude has these bits to [2^14, 2^15), and its inverse.
+// The power of two that brings a row whose largest magnitude has these bits to [2^14, 2^15), and its inverse.
 // Rows below 2^-112 are taken as that, which keeps both normal numbers.
 __device__ __forceinline__ uint32_t scale_exponent(uint32_t max_bits) { return max(max_bits >> 23, 15u); }
 __device__ __forceinline__ float scale_of(uint32_t max_bits) { return __uint_as_float((268u - scale_exponent(max_bits)) << 23); }
@@ -243,6 +243,15 @@ __device__ __forceinline__ void epilogue_row(const GemmArgs& p, int row, int col
   }
 }
 
+// (x, y) times (the floats with bits fx, fy), then both times s: two packed products. Taking a scale per column apart costs the
+// epilogue as many instructions as the packed form saves it.
+__device__ __forceinline__ void scale_pair(float& x, float& y, uint32_t fx, uint32_t fy, float s) {
+  asm("{ .reg .b64 v, f, t;\n\t"
+      "mov.b64 v, {%0, %1};\n\tmov.b64 f, {%2, %3};\n\tmov.b64 t, {%4, %4};\n\t"
+      "mul.rn.f32x2 v, v, f;\n\tmul.rn.f32x2 v, v, t;\n\tmov.b64 {%0, %1}, v; }"
+      : "+f"(x), "+f"(y) : "r"(fx), "r"(fy), "f"(s));
+}
+
 // A thread's row of a chunk to and from its tile in shared memory.
 template <int n>
 __device__ __forceinline__ void chunk_put(uint8_t* tile, int r, const float* x) {
@@ -264,7 +273,7 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1)
     k_gemm_tc(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
               const __grid_constant__ CUtensorMap map_blo, const __grid_constant__ CUtensorMap map_in,
               const __grid_constant__ CUtensorMap map_c, const __grid_constant__ CUtensorMap map_pre,
-              const __grid_constant__ GemmArgs p, const uint32_t* b_max, int* err) {
+              const __grid_constant__ GemmArgs p, const uint16_t* __restrict__ b_unscale, int* err) {
   using L = Tile<BN, FMT, PAIR>;
   constexpr int NA = L::NA, NB = L::NB;
   extern __shared__ uint8_t smem_raw[];
@@ -473,7 +482,6 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1)
     uint8_t* buf = epi + ew * 2 * L::kBuf;
     uint64_t* bar = landed + 2 * ew;
     const bool has_in = reads(EPI) && (EPI != EPI_PLAIN || p.res != nullptr);
-    const float b_unscale = L::kScaled ? unscale_of(*b_max) : 1.f;
     // The chunks of a warp: its half of the columns; SPLIT: every other one of the CTA's slice.
     auto first_col = [&](int t) { return (t % tiles_n) * BN + (SPLIT ? part * slice : half * (BN / 2)); };
     auto chunks_of = [&](int t) { return max(0, min((SPLIT ? slice : BN / 2) / AC, (p.N - first_col(t) + AC - 1) / AC)); };
@@ -501,6 +509,20 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1)
     for (int t = tile0; ok && t < n_tiles; t += tile_step) {
       const int r0 = first_row(t) + q * 32, row = r0 + lane, n0 = first_col(t), nc = chunks_of(t);
       if (reads(EPI)) epilogue_prefetch<EPI>(p, row, n0, BN / 2);
+      // The scales of a chunk's columns. FMT_F16X3, whose epilogue threads have registers to spare (and whose launches are the
+      // small structures'), asks for them a chunk ahead, the first ones while the accumulator is being filled: asked for where
+      // they are used they cost each launch of a 21-atom pass 0.7 us. The others, whose chunks are twice as wide, would spill.
+      // A scale per row against one for the matrix: GEMMs of diamond1728 3xTF32 7.57 -> 7.63 ms, of water1791 tf32 4.12 -> 4.19,
+      // of water648 native 3.86 -> 3.90.
+      constexpr bool kAhead = L::X3;
+      uint4 u[L::kScaled ? AC / 8 : 1];
+      const auto ask_scales = [&](int c) {
+        if (L::kScaled)
+#pragma unroll
+          for (int j = 0; j < AC / 8; ++j)
+            if (c < nc && n0 + c * AC + 8 * j < p.N) u[j] = __ldg(reinterpret_cast<const uint4*>(b_unscale + n0 + c * AC + 8 * j));
+      };
+      if (kAhead) ask_scales(c0);
       float unscale = 1.f, big = 0.f;
       RowTerms rt{};
       if (row < p.M) {
@@ -577,6 +599,7 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1)
 #pragma unroll 1
       for (int c = c0; c < nc; c += CS) {
         float v[AC], in[W], out[W], pre[W];
+        if (!kAhead) ask_scales(c);
         if constexpr (SPLIT) {
 #pragma unroll
           for (int j = 0; j < AC; j += 4) {
@@ -587,18 +610,24 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1)
             }
             v[j] = x.x, v[j + 1] = x.y, v[j + 2] = x.z, v[j + 3] = x.w;
           }
-#pragma unroll
-          for (int j = 0; j < AC; ++j) v[j] = L::kScaled ? v[j] * b_unscale * unscale : v[j];
         } else if (L::X3) {
 #pragma unroll
-          for (int j = 0; j < AC; ++j) v[j] = sum[j % L::kSums] * b_unscale * unscale;  // one after the other: their product may not be a normal number
+          for (int j = 0; j < AC; ++j) v[j] = sum[j % L::kSums];
 #pragma unroll
           for (int j = 0; j + AC < L::kSums; ++j) sum[j] = sum[j + AC];
         } else {
           tmem_ld<AC == 32 ? 32 : 16>(acc + c * AC, v);
           if (c + 1 == nc) release(i % L::kTurns);  // (not SPLIT)
+        }
+        if (L::kScaled) {
 #pragma unroll
-          for (int j = 0; j < AC; ++j) v[j] = L::kScaled ? v[j] * b_unscale * unscale : v[j];
+          for (int j = 0; j < AC; j += 8) {
+            const uint32_t two[4] = {u[j / 8].x, u[j / 8].y, u[j / 8].z, u[j / 8].w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i)  // one after the other: the two scales' product may not be a normal number
+              scale_pair(v[j + 2 * i], v[j + 2 * i + 1], two[i] << 16, two[i] & 0xFFFF0000u, unscale);
+          }
+          if (kAhead) ask_scales(c + CS);
         }
         uint8_t* mine = buf + (k & 1) * L::kBuf;
         if (has_in) {
@@ -765,24 +794,30 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1)
 
 // ---- packing, row maxima ----------------------------------------------------------------------
 
-__global__ void k_abs_max(const float* __restrict__ W, size_t ld_r, size_t ld_k, int rows, int K, uint32_t* amax) {
+// What undoes the scale of each row of a weight: a block per row (past the last one: zeros).
+__global__ void k_row_unscale(const float* __restrict__ W, size_t ld_r, size_t ld_k, int rows, int K, uint16_t* __restrict__ unscale) {
+  __shared__ uint32_t s_max;
+  const int r = blockIdx.x;
+  if (threadIdx.x == 0) s_max = 0;
+  __syncthreads();
   float m = 0.f;
-  for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < size_t(rows) * K; i += size_t(gridDim.x) * blockDim.x)
-    m = fmaxf(m, fabsf(W[(i / K) * ld_r + (i % K) * ld_k]));
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0) atomicMax(amax, __float_as_uint(m));
+  if (r < rows)
+    for (int k = threadIdx.x; k < K; k += blockDim.x) m = fmaxf(m, fabsf(W[r * ld_r + k * ld_k]));
+  const uint32_t most = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
+  if ((threadIdx.x & 31) == 0) atomicMax(&s_max, most);
+  __syncthreads();
+  if (threadIdx.x == 0) unscale[r] = r < rows ? __float_as_uint(unscale_of(s_max)) >> 16 : 0;
 }
 
 template <int FMT>
-__global__ void k_pack_weight(const float* __restrict__ W, size_t ld_r, size_t ld_k, int rows, int K, int Kp, const uint32_t* amax,
+__global__ void k_pack_weight(const float* __restrict__ W, size_t ld_r, size_t ld_k, int rows, int K, int Kp, const uint16_t* __restrict__ unscale,
                               uint16_t* __restrict__ main, uint16_t* __restrict__ low) {
   const size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= size_t(rows) * (Kp / 2)) return;
   const int r = int(i / (Kp / 2)), k = 2 * int(i % (Kp / 2));
   const float x = k < K ? W[r * ld_r + k * ld_k] : 0.f, y = k + 1 < K ? W[r * ld_r + (k + 1) * ld_k] : 0.f;
   uint32_t h, m, l;
-  split2<FMT>(x, y, scales_rows(FMT) ? scale_of(*amax) : 1.f, h, m, l);
+  split2<FMT>(x, y, scales_rows(FMT) ? 1.f / __uint_as_float(uint32_t(unscale[r]) << 16) : 1.f, h, m, l);  // (powers of two: exact)
   if (FMT == FMT_TF32X2 || FMT == FMT_TF32) {
     *reinterpret_cast<float2*>(reinterpret_cast<float*>(main) + size_t(r) * Kp + k) = make_float2(x, y);
     if (FMT == FMT_TF32X2) *reinterpret_cast<float2*>(reinterpret_cast<float*>(low) + size_t(r) * Kp + k) = make_float2(tf32_low(x), tf32_low(y));
@@ -930,7 +965,7 @@ void launch_tc(Stream& st, const GemmArgs& a, const PackedB& w, int parts = 1) {
   }
   attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // see launch()
   attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
-  PETB_CUDA(cudaLaunchKernelEx(&cfg, kernel, ma, mb, ml, mi, mc, mp, a, w.amax, state().err));
+  PETB_CUDA(cudaLaunchKernelEx(&cfg, kernel, ma, mb, ml, mi, mc, mp, a, w.unscale, state().err));
   PETB_LAUNCH_CHECK(st);
 }
 
@@ -1025,18 +1060,17 @@ void dispatch_format(Stream& st, const GemmArgs& a, const PackedB& w) {
 
 }  // namespace
 
-PackedB pack_weight(cudaStream_t s, Format fmt, const float* W, size_t ld_r, size_t ld_k, int rows, int K, uint16_t* out, uint32_t* amax) {
+PackedB pack_weight(cudaStream_t s, Format fmt, const float* W, size_t ld_r, size_t ld_k, int rows, int K, uint16_t* out, uint16_t* unscale) {
   PackedB w;
-  w.fmt = fmt, w.Kp = packed_k(K), w.main = out, w.amax = amax;
+  w.fmt = fmt, w.Kp = packed_k(K), w.main = out, w.unscale = unscale;
   uint16_t* low = fmt == FMT_F16X3 || fmt == FMT_TF32X2 ? out + 2 * size_t(rows) * w.Kp : nullptr;
   w.low = low;
   if (rows <= 0 || K <= 0) return w;
-  PETB_CUDA(cudaMemsetAsync(amax, 0, 4, s));
   const unsigned blocks = unsigned(cdiv((long long) rows * (w.Kp / 2), 256));
-  if (scales_rows(fmt)) k_abs_max<<<std::min(blocks, 592u), 256, 0, s>>>(W, ld_r, ld_k, rows, K, amax);
+  if (scales_rows(fmt)) k_row_unscale<<<unsigned(unscale_halves(rows)), 128, 0, s>>>(W, ld_r, ld_k, rows, K, unscale);
   auto kernel = fmt == FMT_F16X3 ? k_pack_weight<FMT_F16X3> : fmt == FMT_F16X2 ? k_pack_weight<FMT_F16X2> : fmt == FMT_F16 ? k_pack_weight<FMT_F16>
                 : fmt == FMT_BF16 ? k_pack_weight<FMT_BF16> : fmt == FMT_TF32X2 ? k_pack_weight<FMT_TF32X2> : k_pack_weight<FMT_TF32>;
-  kernel<<<blocks, 256, 0, s>>>(W, ld_r, ld_k, rows, K, w.Kp, amax, out, low);
+  kernel<<<blocks, 256, 0, s>>>(W, ld_r, ld_k, rows, K, w.Kp, unscale, out, low);
   PETB_CUDA(cudaGetLastError());
   return w;
 }

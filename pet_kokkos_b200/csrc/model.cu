@@ -150,10 +150,10 @@ void Model::put_mat(const std::string& name, const double* src, int ld, int rows
       const int r = transposed ? cols : rows, k = transposed ? rows : cols;
       uint16_t* out = nullptr;
       const size_t bytes = (packed_halves(f, r, k) * 2 + 15) & ~size_t(15);
-      PETB_CUDA(cudaMalloc(&out, bytes + 16));
+      PETB_CUDA(cudaMalloc(&out, bytes + 2 * unscale_halves(r)));
       owned_.push_back(out);
       return pack_weight(nullptr, f, dev, transposed ? 1 : cols, transposed ? cols : 1, r, k, out,
-                         reinterpret_cast<uint32_t*>(reinterpret_cast<char*>(out) + bytes));
+                         reinterpret_cast<uint16_t*>(reinterpret_cast<char*>(out) + bytes));
     };
     // At widths past 256 the forward of the 3xTF32 and tf32 modes keeps the tf32 instructions. The accumulator's
     // truncations pull every product sum toward zero by a factor that goes with their number, one per 8 columns of K and
