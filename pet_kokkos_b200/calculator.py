@@ -21,7 +21,7 @@ _lib = None
 
 GEMM_MODES = {"native": 0, "tf32": 1, "bf16": 2, "3xtf32": 3}
 # operand formats and epilogues of the weight GEMM (csrc/gemm.h), for debug_gemm
-GEMM_FORMATS = {"f16x3": 0, "f16x2": 1, "f16": 2, "bf16": 3, "tf32x2": 4, "tf32": 5}
+GEMM_FORMATS = {"f16x3": 0, "f16x2": 1, "f16": 2, "bf16": 3, "tf32x2": 4, "tf32": 5, "f16x3_full": 6}
 GEMM_EPILOGUES = {"plain": 0, "silu": 1, "swiglu": 2, "silu_bwd": 3, "swiglu_bwd": 4, "compress": 5}
 RECOMPUTE_TIERS = {"auto": 0, "never": 1, "wide": 2, "layers": 3}
 

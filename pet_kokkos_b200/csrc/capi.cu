@@ -263,7 +263,7 @@ int pet_gemm_host(pet_calc* c, int mode, int w_transposed, int m, int n, int k, 
 }
 int pet_debug_gemm(pet_calc* c, const pet_debug_gemm_args* args) {
   return guarded(c, [&](Engine& e) {
-    if (!args || args->format < 0 || args->format > petb::FMT_TF32) throw petb::Error(PET_ERR_INVALID, "pet: bad GEMM arguments");
+    if (!args || args->format < 0 || args->format > petb::FMT_F16X3_FULL) throw petb::Error(PET_ERR_INVALID, "pet: bad GEMM arguments");
     e.gemm_on_host_arrays(*args, args->format, args->format);
   });
 }

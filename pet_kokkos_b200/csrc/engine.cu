@@ -1398,7 +1398,10 @@ void Engine::gemm_on_host_arrays(const pet_debug_gemm_args& g, int native_format
   // the weight packed from either orientation, as a loaded one is
   auto pack = [&](int fmt) {
     uint16_t* out = tmp_arena.alloc<uint16_t>(packed_halves(fmt, a.N, a.K));
-    return pack_weight(st.s, Format(fmt), dW, g.w_transposed ? k : 1, g.w_transposed ? 1 : n, a.N, a.K, out, tmp_arena.alloc<uint16_t>(unscale_halves(a.N)));
+    PackedB w = pack_weight(st.s, Format(fmt), dW, g.w_transposed ? k : 1, g.w_transposed ? 1 : n, a.N, a.K, out, tmp_arena.alloc<uint16_t>(unscale_halves(a.N)));
+    PETB_CUDA(cudaStreamSynchronize(st.s));
+    full_if_spread(w, a.N);
+    return w;
   };
   a.nat = pack(native_format), a.fast = pack(fast_format);
   gemm(st, tmp_arena, a);

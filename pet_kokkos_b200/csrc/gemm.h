@@ -36,10 +36,19 @@ enum GemmMode { GEMM_NATIVE = 0, GEMM_TF32 = 1, GEMM_BF16 = 2, GEMM_TF32X3 = 3 }
 // How an fp32 operand is handed to the 16-bit tensor cores. The fp16 formats scale it by a power of two first: s brings the
 // largest value of the row, of A and of B alike, to [2^14, 2^15).
 //   FMT_F16X3 (native)   s x = h + m + l: h is s x rounded to a multiple of 2^8, eight bits of the row's largest value; what
-//                        remains goes into two fp16 parts. Every value is represented to its last bit, or to 2^-23 of
-//                        itself where it is below 2^-6 of the row's largest. Six products; h.h on its own accumulator,
-//                        where 1024 columns of K sum without any rounding; the rest (hm mh mm hl lh, 2^-8 of it and less;
-//                        what is left out is below 2^-27) on another. The two meet in one fp32 addition.
+//                        remains goes into two fp16 parts. Every value is represented to its last bit, or to 2^-23 of itself
+//                        down to 2^-17 of the row's largest; below that to 2^-40 of the largest. Six products; h.h on its own
+//                        accumulator, where 1024 columns of K sum without any rounding; the rest (hm mh mm hl lh, 2^-8 of it
+//                        and less) on another. The two meet in one fp32 addition. Left out are ml and lm: below 2^-27 of a
+//                        product of two values with a leading part, 2^-20 of one where one has none (it lies below 2^-8 of
+//                        its row's largest), 2^-12 where neither has.
+//   FMT_F16X3_FULL       the same parts, ml and lm among the products. A sum mostly of products without leading parts takes rows
+//                        of A and of the weight that are large in different columns (a gain and what undoes it): a weight with
+//                        rows or columns like that (k_row_unscale, k_column_spread) runs in this format. Columns that share
+//                        factors of 2^-8 .. 2^8 then give an error of 2^-20 of sum |a||w|, with six products 2^-14. What remains
+//                        is the second accumulator's truncation, where most of a sum goes over it: what 3xTF32 has. For every
+//                        weight it would cost a 1728-atom evaluation 11 % (and a fourth part, x to eleven bits as l's partner,
+//                        12 %); as a test in the issuer's loop a small structure's pass 1.5 to 4 %.
 //   FMT_F16X2 (3xTF32)   s x = h + l, two fp16 parts: 22 bits or more for every value down to 2^-18 of the row's largest, an
 //                        error of 2^-40 of the largest below that. Three products (hl lh hh), one accumulator.
 //   FMT_TF32X2 (3xTF32)  x = h + l, two tf32 parts: h is x as the tensor core reads it (its leading 11 bits, truncated), l the
@@ -48,15 +57,16 @@ enum GemmMode { GEMM_NATIVE = 0, GEMM_TF32 = 1, GEMM_BF16 = 2, GEMM_TF32X3 = 3 }
 //   FMT_F16 (tf32)       x's leading 11 bits, truncated: the value a tf32 tensor core reads of x, as one fp16.
 //   FMT_TF32 (tf32)      x as it is, read by a tf32 tensor core: the same operand value as FMT_F16's for twice the bytes.
 //   FMT_BF16 (bf16)      x rounded to bf16.
-enum Format { FMT_F16X3 = 0, FMT_F16X2 = 1, FMT_F16 = 2, FMT_BF16 = 3, FMT_TF32X2 = 4, FMT_TF32 = 5 };
+enum Format { FMT_F16X3 = 0, FMT_F16X2 = 1, FMT_F16 = 2, FMT_BF16 = 3, FMT_TF32X2 = 4, FMT_TF32 = 5, FMT_F16X3_FULL = 6 };
 inline Format format_of(int mode) {
   return mode == GEMM_TF32X3 ? FMT_F16X2 : mode == GEMM_TF32 ? FMT_F16 : mode == GEMM_BF16 ? FMT_BF16 : FMT_F16X3;
 }
-constexpr bool scales_rows(int fmt) { return fmt == FMT_F16X3 || fmt == FMT_F16X2 || fmt == FMT_F16; }
+constexpr bool three_parts(int fmt) { return fmt == FMT_F16X3 || fmt == FMT_F16X3_FULL; }
+constexpr bool scales_rows(int fmt) { return three_parts(fmt) || fmt == FMT_F16X2 || fmt == FMT_F16; }
 
 // A weight [rows, K] in one format, made once when it was loaded. K is padded with zeros to a multiple of 32.
 //   FMT_F16X3   main [rows][Kp/32][h 32 | m 32], low [rows][Kp] the l parts; `unscale` [rows] what undoes each row's scale, a power
-//               of two as bf16, with zeros up to a multiple of eight
+//               of two as bf16, with zeros up to a multiple of eight; behind them a word: whether the values are spread
 //   FMT_F16X2   main [rows][Kp/32][h 32 | l 32]; `unscale`
 //   FMT_F16     main [rows][Kp]; `unscale`
 //   FMT_BF16    main [rows][Kp]
@@ -69,14 +79,17 @@ struct PackedB {
   int Kp = 0;
 };
 inline int packed_k(int K) { return (K + 31) / 32 * 32; }
-inline size_t unscale_halves(int rows) { return size_t(rows + 7) / 8 * 8; }
+constexpr size_t unscale_halves(int rows) { return size_t(rows + 7) / 8 * 8 + 8; }
 // 16-bit values and bytes a packed weight takes (main and low together), rows padded apart to 16 bytes.
 inline size_t packed_halves(int fmt, int rows, int K) {
-  return size_t(rows) * packed_k(K) * (fmt == FMT_F16X3 ? 3 : fmt == FMT_F16X2 || fmt == FMT_TF32 ? 2 : fmt == FMT_TF32X2 ? 4 : 1);
+  return size_t(rows) * packed_k(K) * (three_parts(fmt) ? 3 : fmt == FMT_F16X2 || fmt == FMT_TF32 ? 2 : fmt == FMT_TF32X2 ? 4 : 1);
 }
 // Packs W [rows, K] (element (r, k) at W[r * ld_r + k * ld_k]) into `out`, and writes `unscale` (unscale_halves(rows),
 // 16-byte aligned).
 PackedB pack_weight(cudaStream_t s, Format fmt, const float* W, size_t ld_r, size_t ld_k, int rows, int K, uint16_t* out, uint16_t* unscale);
+// A weight in FMT_F16X3 whose values pack_weight found spread becomes one in FMT_F16X3_FULL. Copies a word from the device: the
+// packing has to have ended.
+void full_if_spread(PackedB& w, int rows);
 
 struct GemmArgs {
   const float* A = nullptr;  // [M,K]

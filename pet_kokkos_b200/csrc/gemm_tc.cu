@@ -78,7 +78,7 @@ __device__ __forceinline__ float2 unpack_f16(uint32_t u) { return __half22float2
 // Two neighbouring values into their parts. `s` is the row's scale (fp16 formats).
 template <int FMT>
 __device__ __forceinline__ void split2(float x, float y, float s, uint32_t& h, uint32_t& m, uint32_t& l) {
-  if (FMT == FMT_F16X3) {
+  if (three_parts(FMT)) {
     constexpr float kGrid = 3221225472.f;  // 1.5 2^31: adding it rounds to a multiple of 2^8
     x *= s, y *= s;
     const float xh = (x + kGrid) - kGrid, yh = (y + kGrid) - kGrid;
@@ -108,8 +108,8 @@ __device__ __forceinline__ float tf32_low(float x) {
 
 template <int BN, int FMT, bool PAIR>
 struct Tile {
-  static constexpr bool X3 = FMT == FMT_F16X3, X2 = FMT == FMT_F16X2, T2 = FMT == FMT_TF32X2, T1 = FMT == FMT_TF32;
-  static constexpr bool kScaled = FMT == FMT_F16X3 || FMT == FMT_F16X2 || FMT == FMT_F16;
+  static constexpr bool X3 = three_parts(FMT), kFull = FMT == FMT_F16X3_FULL, X2 = FMT == FMT_F16X2, T2 = FMT == FMT_TF32X2, T1 = FMT == FMT_TF32;
+  static constexpr bool kScaled = scales_rows(FMT);
   static constexpr int BK = T2 ? 16 : 32;                                   // columns of K of a step
   // A's parts in tensor memory, where the accumulators leave room for them.
   static constexpr bool TA = !PAIR && !T1 && !T2 && (X2 || BN <= 128);
@@ -402,7 +402,8 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1)
               if (L::X3) {
                 const uint64_t bl = smem_desc<64>(b0 + L::kRowsB * 128);
                 const uint32_t small = acc + BN;
-                mma_f16_ta(small, h, bl + k, idesc, !first || k != 0);
+                if (L::kFull) mma_f16_ta(small, m, bl + k, idesc, !first || k != 0), mma_f16_ta(small, l, bm + k, idesc, 1);
+                mma_f16_ta(small, h, bl + k, idesc, L::kFull || !first || k != 0);
                 mma_f16_ta(small, l, bh + k, idesc, 1);
                 mma_f16_ta(small, m, bm + k, idesc, 1);
                 mma_f16_ta(small, h, bm + k, idesc, 1);
@@ -429,7 +430,8 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1)
               const uint32_t small = acc + BN;
 #pragma unroll
               for (int k = 0; k < 4; k += 2) {  // 16 columns are 32 bytes: 2 in the descriptors' 16-byte units
-                mma_f16<PAIR>(small, ah + k, bl + k, idesc, !first || k != 0);
+                if (L::kFull) mma_f16<PAIR>(small, am + k, bl + k, idesc, !first || k != 0), mma_f16<PAIR>(small, al + k, bm + k, idesc, 1);
+                mma_f16<PAIR>(small, ah + k, bl + k, idesc, L::kFull || !first || k != 0);
                 mma_f16<PAIR>(small, al + k, bh + k, idesc, 1);
                 mma_f16<PAIR>(small, am + k, bm + k, idesc, 1);
                 mma_f16<PAIR>(small, ah + k, bm + k, idesc, 1);
@@ -794,11 +796,14 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1)
 
 // ---- packing, row maxima ----------------------------------------------------------------------
 
-// What undoes the scale of each row of a weight: a block per row (past the last one: zeros).
-__global__ void k_row_unscale(const float* __restrict__ W, size_t ld_r, size_t ld_k, int rows, int K, uint16_t* __restrict__ unscale) {
+// What undoes the scale of each row of a weight, a block per row (past the last one: zeros); and whether more than a quarter of a
+// row's values (and more than eight; zeros do not count) lie below 2^-7 of its largest. Of 256 normal values some 2 % do.
+__global__ void k_row_unscale(const float* __restrict__ W, size_t ld_r, size_t ld_k, int rows, int K, uint16_t* __restrict__ unscale,
+                              int* __restrict__ spread) {
   __shared__ uint32_t s_max;
+  __shared__ int s_low;
   const int r = blockIdx.x;
-  if (threadIdx.x == 0) s_max = 0;
+  if (threadIdx.x == 0) s_max = 0, s_low = 0;
   __syncthreads();
   float m = 0.f;
   if (r < rows)
@@ -807,6 +812,33 @@ __global__ void k_row_unscale(const float* __restrict__ W, size_t ld_r, size_t l
   if ((threadIdx.x & 31) == 0) atomicMax(&s_max, most);
   __syncthreads();
   if (threadIdx.x == 0) unscale[r] = r < rows ? __float_as_uint(unscale_of(s_max)) >> 16 : 0;
+  if (r >= rows) return;
+  const float low = __uint_as_float(s_max) * 0.0078125f;
+  int n = 0;
+  for (int k = threadIdx.x; k < K; k += blockDim.x) {
+    const float x = fabsf(W[r * ld_r + k * ld_k]);
+    n += x < low && x > 0.f;
+  }
+  n = __reduce_add_sync(0xffffffffu, n);
+  if ((threadIdx.x & 31) == 0) atomicAdd(&s_low, n);
+  __syncthreads();
+  if (threadIdx.x == 0 && s_low > 8 && 4 * s_low > K) *spread = 1;
+}
+
+// Whether a column's values all lie 2^-4 and more below their rows' scales. 32 columns a block, 32 rows at a time. (A column of
+// sixteen normal values does with a probability of 1e-9.)
+__global__ void k_column_spread(const float* __restrict__ W, size_t ld_r, size_t ld_k, int rows, int K, const uint16_t* __restrict__ unscale,
+                                int* __restrict__ spread) {
+  __shared__ float s_max[32][33];
+  const int k = blockIdx.x * 32 + threadIdx.x;
+  float m = 0.f;
+  if (k < K)
+    for (int r = threadIdx.y; r < rows; r += 32) m = fmaxf(m, fabsf(W[r * ld_r + k * ld_k]) / __uint_as_float(uint32_t(unscale[r]) << 16));
+  s_max[threadIdx.y][threadIdx.x] = m;
+  __syncthreads();
+  if (threadIdx.y != 0 || k >= K) return;
+  for (int r = 1; r < 32; ++r) m = fmaxf(m, s_max[r][threadIdx.x]);
+  if (m > 0.f && m < 2048.f) *spread = 1;
 }
 
 template <int FMT>
@@ -983,7 +1015,7 @@ struct SplitPlan {
 };
 template <int FMT>
 SplitPlan plan_split(const GemmArgs& a, int bn_whole, int sms) {
-  constexpr bool X3 = FMT == FMT_F16X3, T2 = FMT == FMT_TF32X2, two = FMT == FMT_F16X2;
+  constexpr bool X3 = three_parts(FMT), T2 = FMT == FMT_TF32X2, two = FMT == FMT_F16X2;
   constexpr int clocks[3] = {X3 || T2 ? 1800 : two ? 850 : 640, X3 ? 1050 : T2 ? 1550 : two ? 700 : 530, X3 ? 850 : T2 ? 1500 : two ? 670 : 510};
   const int widths[3] = {256, 128, 64}, steps = (a.K + 31) / 32, rows = cdiv(a.M, TBM);
   SplitPlan best;
@@ -1015,7 +1047,7 @@ void dispatch_width(Stream& st, const GemmArgs& a, const PackedB& w) {
   const long long mt = cdiv(a.M, TBM);
   const int sms = state().sms;
   const int widths[3] = {256, 128, 64};
-  constexpr bool twelve = FMT == FMT_F16X3 || FMT == FMT_TF32X2;  // twelve bytes of operand reads per value and tile side
+  constexpr bool twelve = three_parts(FMT) || FMT == FMT_TF32X2;  // twelve bytes of operand reads per value and tile side
   constexpr int wavefronts[3] = {twelve ? 608 : FMT == FMT_F16X2 ? 416 : 272, twelve ? 408 : FMT == FMT_F16X2 ? 280 : 184,
                                  twelve ? 308 : FMT == FMT_F16X2 ? 212 : 140};
   int bn = 0;
@@ -1030,7 +1062,7 @@ void dispatch_width(Stream& st, const GemmArgs& a, const PackedB& w) {
   // parts, whose weight tiles are the larger share (122138 rows: FMT_F16X3 w_in backward 258 us against 307, SwiGLU 353
   // against 383; FMT_F16X2 215 against 274, plain 56 against 60), once there is a tile for every pair of SMs; the formats of
   // one part are near HBM's rate without it, and the second CTA's signals make a step longer (SwiGLU 180 us against 164).
-  constexpr bool kPair = FMT == FMT_F16X3 || FMT == FMT_F16X2 || FMT == FMT_TF32X2;
+  constexpr bool kPair = three_parts(FMT) || FMT == FMT_F16X2 || FMT == FMT_TF32X2;
   if constexpr (kPair)
     if (bn == 256 && cdiv(a.M, 2 * TBM) * (a.N / 256) >= sms / 2) return launch_tc<EPI, 256, FMT, true>(st, a, w);
   if constexpr (EPI == EPI_PLAIN) {
@@ -1050,6 +1082,7 @@ template <int EPI>
 void dispatch_format(Stream& st, const GemmArgs& a, const PackedB& w) {
   switch (w.fmt) {
     case FMT_F16X3: return dispatch_width<EPI, FMT_F16X3>(st, a, w);
+    case FMT_F16X3_FULL: return dispatch_width<EPI, FMT_F16X3_FULL>(st, a, w);
     case FMT_F16X2: return dispatch_width<EPI, FMT_F16X2>(st, a, w);
     case FMT_F16: return dispatch_width<EPI, FMT_F16>(st, a, w);
     case FMT_BF16: return dispatch_width<EPI, FMT_BF16>(st, a, w);
@@ -1063,16 +1096,28 @@ void dispatch_format(Stream& st, const GemmArgs& a, const PackedB& w) {
 PackedB pack_weight(cudaStream_t s, Format fmt, const float* W, size_t ld_r, size_t ld_k, int rows, int K, uint16_t* out, uint16_t* unscale) {
   PackedB w;
   w.fmt = fmt, w.Kp = packed_k(K), w.main = out, w.unscale = unscale;
-  uint16_t* low = fmt == FMT_F16X3 || fmt == FMT_TF32X2 ? out + 2 * size_t(rows) * w.Kp : nullptr;
+  uint16_t* low = three_parts(fmt) || fmt == FMT_TF32X2 ? out + 2 * size_t(rows) * w.Kp : nullptr;
   w.low = low;
   if (rows <= 0 || K <= 0) return w;
   const unsigned blocks = unsigned(cdiv((long long) rows * (w.Kp / 2), 256));
-  if (scales_rows(fmt)) k_row_unscale<<<unsigned(unscale_halves(rows)), 128, 0, s>>>(W, ld_r, ld_k, rows, K, unscale);
-  auto kernel = fmt == FMT_F16X3 ? k_pack_weight<FMT_F16X3> : fmt == FMT_F16X2 ? k_pack_weight<FMT_F16X2> : fmt == FMT_F16 ? k_pack_weight<FMT_F16>
+  if (scales_rows(fmt)) {
+    int* spread = reinterpret_cast<int*>(unscale + unscale_halves(rows) - 8);
+    PETB_CUDA(cudaMemsetAsync(spread, 0, 16, s));
+    k_row_unscale<<<unsigned(unscale_halves(rows) - 8), 128, 0, s>>>(W, ld_r, ld_k, rows, K, unscale, spread);
+    if (fmt == FMT_F16X3 && rows >= 16) k_column_spread<<<cdiv(K, 32), dim3(32, 32), 0, s>>>(W, ld_r, ld_k, rows, K, unscale, spread);
+  }
+  auto kernel = three_parts(fmt) ? k_pack_weight<FMT_F16X3> : fmt == FMT_F16X2 ? k_pack_weight<FMT_F16X2> : fmt == FMT_F16 ? k_pack_weight<FMT_F16>
                 : fmt == FMT_BF16 ? k_pack_weight<FMT_BF16> : fmt == FMT_TF32X2 ? k_pack_weight<FMT_TF32X2> : k_pack_weight<FMT_TF32>;
   kernel<<<blocks, 256, 0, s>>>(W, ld_r, ld_k, rows, K, w.Kp, unscale, out, low);
   PETB_CUDA(cudaGetLastError());
   return w;
+}
+
+void full_if_spread(PackedB& w, int rows) {
+  if (w.fmt != FMT_F16X3 || rows <= 0) return;
+  int spread = 0;
+  PETB_CUDA(cudaMemcpy(&spread, w.unscale + unscale_halves(rows) - 8, sizeof(int), cudaMemcpyDeviceToHost));
+  if (spread) w.fmt = FMT_F16X3_FULL;
 }
 
 void row_max(Stream& st, uint32_t* mx, const float* x, int ld, int R, int D) {

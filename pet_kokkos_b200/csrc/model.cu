@@ -249,6 +249,13 @@ Model::Model(const Checkpoint& ck, int gemm_mode) : h_(ck.hypers), scale_(ck.ene
     PETB_CUDA(cudaMalloc(&probes_, (probes.size() ? probes.size() : 1) * sizeof(double)));
     PETB_CUDA(cudaMemcpy(probes_, probes.data(), probes.size() * sizeof(double), cudaMemcpyHostToDevice));
   }
+  PETB_CUDA(cudaDeviceSynchronize());
+  for (auto& [name, m] : mat_)
+    if (m.nat.main) {
+      full_if_spread(m.nat, m.rows), full_if_spread(m.nat_t, m.cols);
+      if (m.fast.fmt == FMT_F16X3) m.fast = m.nat;
+      if (m.fast_t.fmt == FMT_F16X3) m.fast_t = m.nat_t;
+    }
   // a blocking copy from pageable memory returns once staged: fence, since the evaluations run on a stream that
   // does not wait for the legacy one
   PETB_CUDA(cudaDeviceSynchronize());

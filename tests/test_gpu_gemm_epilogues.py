@@ -8,7 +8,7 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-FORMATS = ["f16x3", "f16x2", "f16", "bf16", "tf32x2", "tf32"]
+FORMATS = ["f16x3", "f16x3_full", "f16x2", "f16", "bf16", "tf32x2", "tf32"]
 FORWARD = ["plain", "silu", "swiglu", "compress"]
 BACKWARD = ["silu_bwd", "swiglu_bwd"]  # never packed in the tf32 formats
 CASES = [(f, e) for f in FORMATS for e in FORWARD + (BACKWARD if not f.startswith("tf32") else [])]
@@ -24,7 +24,7 @@ def calc(lib_path, models):
 
 
 def band_of(fmt, k):
-    return {"f16x3": 2.0 ** -22, "f16x2": 2.0 ** -20 + k * 2.0 ** -25, "tf32x2": 2.0 ** -20 + k * 2.0 ** -25, "f16": 2.0 ** -10,
+    return {"f16x3": 2.0 ** -22, "f16x3_full": 2.0 ** -22, "f16x2": 2.0 ** -20 + k * 2.0 ** -25, "tf32x2": 2.0 ** -20 + k * 2.0 ** -25, "f16": 2.0 ** -10,
             "tf32": 2.0 ** -10, "bf16": 2.0 ** -7}[fmt]
 
 
