@@ -20,10 +20,6 @@ struct AttnArgs {
   const int* off = nullptr;         // [N+1] each atom's range of edge rows
   const float* cut = nullptr;       // [E] cutoff factor of each edge token
   const float* qkv = nullptr;       // [T,3D] columns Q | K | V
-  // [T] the bits of each row's largest |qkv| (and, in the backward, |dmerged|), which the kernels on fp16 parts scale by. Null:
-  // the pass goes to the others.
-  const uint32_t* qkv_max = nullptr;
-  const uint32_t* dmerged_max = nullptr;
   float* merged = nullptr;          // [T,D] attention output before the output projection
   uint32_t* merged_max = nullptr;   // [T] unless null, each row's largest |merged| is raised into it (zeroed by the caller)
   float* ml = nullptr;              // [T,H,2] each query's running max and 1/sum (null: not saved)

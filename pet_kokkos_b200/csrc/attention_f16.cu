@@ -1,8 +1,8 @@
 // Attention on the tensor cores: warp-level mma.sync m16n8k16 on fp16 parts with fp32 accumulation. Same mathematics as
 // attention.cu; used when an atom's tokens fit shared memory.
 //
-// An operand is scaled by a power of two that brings the tile's largest value (from the maxima that the rows' writers
-// keep) to at most 2^15 and split into P parts:
+// An operand is scaled by a power of two that brings its largest value (of this atom and head, found while the tile is staged: Q, K,
+// V and dO each have their own, whatever the other heads hold) to [2^14, 2^15) and split into P parts:
 //   P = 3 (ATTN_NATIVE)  x = h + m + l, h a multiple of 2^8: eight bits of the largest value, so that the h.h products of up to
 //                        1024 terms sum exactly; six products, h.h on an accumulator of its own (gemm.h has the argument);
 //   P = 2 (ATTN_TF32X3)  x = h + l, 22 bits; three products;
@@ -207,12 +207,13 @@ __device__ __forceinline__ void make_a(uint32_t (*a)[4], const float (*x)[4]) {
     }
 }
 
-// The largest value a head's tile can hold, the largest of its rows' maxima (over all heads), raised into *slot.
-__device__ __forceinline__ void tile_max(const uint32_t* mx, int n, int N, int e0, int cnt, uint32_t* slot) {
-  uint32_t m = 0;
-  for (int r = threadIdx.x; r < cnt; r += blockDim.x) m = max(m, mx[r == 0 ? n : N + e0 + r - 1]);
-  m = __reduce_max_sync(0xffffffffu, m);
-  if ((threadIdx.x & 31) == 0) atomicMax(slot, m);
+// A thread's largest value of a tensor raised into the tile's.
+__device__ __forceinline__ void raise_tile(uint32_t* slot, float m) {
+  const uint32_t most = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
+  if ((threadIdx.x & 31) == 0) atomicMax(slot, most);
+}
+__device__ __forceinline__ float max_abs(float m, const float4& x) {
+  return fmaxf(fmaxf(m, fmaxf(fabsf(x.x), fabsf(x.y))), fmaxf(fabsf(x.z), fabsf(x.w)));
 }
 
 // A thread's 16 bytes of row r (a token row of the atom) of a tensor, in parts.
@@ -261,13 +262,14 @@ template <int HD, int P, int MAXB>
 __global__ void __launch_bounds__(32 * MAXB, MAXB <= 5 ? resident<HD, P, 3>(16 * MAXB) : 1) k_attn_fwd_f16(AttnArgs p) {
   after_previous();
   extern __shared__ __align__(16) uint8_t smem[];
-  __shared__ uint32_t s_max;
+  __shared__ uint32_t s_max[3];  // of Q, K, V
   const int n = blockIdx.x / p.H, h = blockIdx.x % p.H, D = p.H * HD;
   const int e0 = p.off[n], cnt = p.off[n + 1] - e0 + 1;
   const int S16 = round16(cnt), nb = S16 / 16, SM = round16(p.S);
   uint8_t *sq = smem, *sk = sq + SM * pitch<HD, P>(), *sv = sk + SM * pitch<HD, P>();
   float* slc = reinterpret_cast<float*>(sv + SM * pitch<HD, P>());
-  // Staging: a thread's loads of U rows' pieces are all under way before it looks for the tile's scale or splits any.
+  // Staging: a thread's loads of U rows' pieces are all under way before it looks at any. A head size of 64 takes two rounds of
+  // them, the second fetched again for the split.
   constexpr int Q = HD / 4, U = 4;
   float4 x0[U], x1[U], x2[U];
   auto fetch = [&](int t0) {
@@ -278,23 +280,32 @@ __global__ void __launch_bounds__(32 * MAXB, MAXB <= 5 ? resident<HD, P, 3>(16 *
       x0[u] = get(p.qkv, at, r < cnt), x1[u] = get(p.qkv, at + D, r < cnt), x2[u] = get(p.qkv, at + 2 * D, r < cnt);
     }
   };
-  fetch(threadIdx.x);
-  if (threadIdx.x == 0) s_max = 0;
+  if (threadIdx.x < 3) s_max[threadIdx.x] = 0;
   __syncthreads();
-  tile_max(p.qkv_max, n, p.N, e0, cnt, &s_max);
+  {
+    float mq = 0.f, mk = 0.f, mv = 0.f;
+    int t0 = threadIdx.x;
+    while (t0 + U * blockDim.x < S16 * Q) t0 += U * blockDim.x;  // the first round last: it stays in the registers
+    for (; t0 >= 0; t0 -= U * blockDim.x) {
+      fetch(t0);
+#pragma unroll
+      for (int u = 0; u < U; ++u) mq = max_abs(mq, x0[u]), mk = max_abs(mk, x1[u]), mv = max_abs(mv, x2[u]);
+    }
+    raise_tile(s_max, mq), raise_tile(s_max + 1, mk), raise_tile(s_max + 2, mv);
+  }
   for (int r = threadIdx.x; r < S16; r += blockDim.x) {
     const float cf = r == 0 ? 1.0f : (r < cnt ? p.cut[e0 + r - 1] : 0.f);
     slc[r] = cf > 0.f ? __logf(cf) * kLog2e : kOff;
   }
   __syncthreads();
-  const float s = scale_of(s_max), us = unscale_of(s_max);
+  const float scq = scale_of(s_max[0]), sck = scale_of(s_max[1]), scv = scale_of(s_max[2]);
   for (int t0 = threadIdx.x; t0 < S16 * Q; t0 += U * blockDim.x) {
     if (t0 != threadIdx.x) fetch(t0);
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int t = t0 + u * blockDim.x, r = t / Q, c = (t % Q) * 4;
       if (t >= S16 * Q) break;
-      put<HD, P>(sq, r, c, x0[u] * s), put<HD, P>(sk, r, c, x1[u] * s), put<HD, P>(sv, r, c, x2[u] * s);
+      put<HD, P>(sq, r, c, x0[u] * scq), put<HD, P>(sk, r, c, x1[u] * sck), put<HD, P>(sv, r, c, x2[u] * scv);
     }
   }
   __syncthreads();
@@ -302,7 +313,7 @@ __global__ void __launch_bounds__(32 * MAXB, MAXB <= 5 ? resident<HD, P, 3>(16 *
   const int r0 = 16 * warp;
   if (r0 >= cnt) return;
   const uint32_t aq = smem_u32(sq), ak = smem_u32(sk), av = smem_u32(sv);
-  const float f = us * us * p.sc * kLog2e;
+  const float us = unscale_of(s_max[2]), f = unscale_of(s_max[0]) * unscale_of(s_max[1]) * p.sc * kLog2e;
   uint32_t qa[HD / 16][P][4];
 #pragma unroll
   for (int ks = 0; ks < HD / 16; ++ks)
@@ -373,7 +384,7 @@ __global__ void __launch_bounds__(MAXT, BLOCKS) k_attn_bwd_f16(AttnArgs p) {
   // where they are used.
   constexpr bool KEEP = HD * P <= 32;
   extern __shared__ __align__(16) uint8_t smem[];
-  __shared__ uint32_t s_max, s_gmax, s_vnorm, s_gnorm;
+  __shared__ uint32_t s_max[4], s_vnorm, s_gnorm;  // of Q, K, V, dO
   const int n = blockIdx.x / p.H, h = blockIdx.x % p.H, D = p.H * HD;
   const int e0 = p.off[n], cnt = p.off[n + 1] - e0 + 1;
   const int S16 = round16(cnt), SM = round16(p.S);
@@ -394,11 +405,20 @@ __global__ void __launch_bounds__(MAXT, BLOCKS) k_attn_bwd_f16(AttnArgs p) {
       x3[u] = get(p.dmerged, ag, r < cnt), x4[u] = get(p.merged, ag, r < cnt);
     }
   };
-  fetch(threadIdx.x);
-  if (threadIdx.x == 0) s_max = s_gmax = s_vnorm = s_gnorm = 0;
+  if (threadIdx.x < 4) s_max[threadIdx.x] = 0;
+  if (threadIdx.x == 0) s_vnorm = s_gnorm = 0;
   __syncthreads();
-  tile_max(p.qkv_max, n, p.N, e0, cnt, &s_max);
-  tile_max(p.dmerged_max, n, p.N, e0, cnt, &s_gmax);
+  {
+    float mq = 0.f, mk = 0.f, mv = 0.f, mg = 0.f;
+    int t0 = threadIdx.x;
+    while (t0 + U * blockDim.x < S16 * Q) t0 += U * blockDim.x;  // the first round last: it stays in the registers
+    for (; t0 >= 0; t0 -= U * blockDim.x) {
+      fetch(t0);
+#pragma unroll
+      for (int u = 0; u < U; ++u) mq = max_abs(mq, x0[u]), mk = max_abs(mk, x1[u]), mv = max_abs(mv, x2[u]), mg = max_abs(mg, x3[u]);
+    }
+    raise_tile(s_max, mq), raise_tile(s_max + 1, mk), raise_tile(s_max + 2, mv), raise_tile(s_max + 3, mg);
+  }
   for (int r = threadIdx.x; r < S16; r += blockDim.x) {
     float lc = kOff, m = 1e30f, il = 0.f;
     if (r < cnt) {
@@ -412,22 +432,23 @@ __global__ void __launch_bounds__(MAXT, BLOCKS) k_attn_bwd_f16(AttnArgs p) {
     slc[r] = lc, sm[r] = m, sl[r] = il * 32768.f;
   }
   __syncthreads();
-  const float s = scale_of(s_max), us = unscale_of(s_max), sgs = scale_of(s_gmax), usg = unscale_of(s_gmax);
+  const float scq = scale_of(s_max[0]), sck = scale_of(s_max[1]), scv = scale_of(s_max[2]), scg = scale_of(s_max[3]);
+  const float usq = unscale_of(s_max[0]), usk = unscale_of(s_max[1]), usv = unscale_of(s_max[2]), usg = unscale_of(s_max[3]);
   for (int t0 = threadIdx.x; t0 < S16 * Q; t0 += U * blockDim.x) {
     if (t0 != threadIdx.x) fetch(t0);
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int t = t0 + u * blockDim.x, r = t / Q, c = (t % Q) * 4;
       if (t >= S16 * Q) break;  // whole warps: a row block of 16 is 16 Q threads
-      const float4 v = x2[u] * s, go = x3[u] * sgs;
-      put<HD, P>(sq, r, c, x0[u] * s), put<HD, P>(sk, r, c, x1[u] * s), put<HD, P>(sv, r, c, v), put<HD, P>(sg, r, c, go);
+      const float4 v = x2[u] * scv, go = x3[u] * scg;
+      put<HD, P>(sq, r, c, x0[u] * scq), put<HD, P>(sk, r, c, x1[u] * sck), put<HD, P>(sv, r, c, v), put<HD, P>(sg, r, c, go);
       float d = dot4(go, x4[u]), gg = dot4(go, go), vv = dot4(v, v);
 #pragma unroll
       for (int o = Q / 2; o > 0; o >>= 1) {
         d += __shfl_xor_sync(0xffffffffu, d, o), gg += __shfl_xor_sync(0xffffffffu, gg, o), vv += __shfl_xor_sync(0xffffffffu, vv, o);
       }
       if (c == 0) {
-        sd[r] = d * s, sn[r] = sqrtf(gg);  // in the units of the scaled products
+        sd[r] = d * scv, sn[r] = sqrtf(gg);  // in the units of the scaled products
         atomicMax(&s_vnorm, __float_as_uint(vv)), atomicMax(&s_gnorm, __float_as_uint(gg));
       }
     }
@@ -435,7 +456,7 @@ __global__ void __launch_bounds__(MAXT, BLOCKS) k_attn_bwd_f16(AttnArgs p) {
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5, g = lane >> 2, t = lane & 3;
   const uint32_t aq = smem_u32(sq), ak = smem_u32(sk), av = smem_u32(sv), ag = smem_u32(sg);
-  const float f = us * us * p.sc * kLog2e;  // a scaled score product to a score, base 2
+  const float f = usq * usk * p.sc * kLog2e;  // a scaled score product to a score, base 2
   const float vmax = sqrtf(__uint_as_float(s_vnorm)), gmax = sqrtf(__uint_as_float(s_gnorm));
   const int nb = S16 / 16;
   for (int task = warp; task < 2 * nb; task += nw) {
@@ -477,13 +498,13 @@ __global__ void __launch_bounds__(MAXT, BLOCKS) k_attn_bwd_f16(AttnArgs p) {
         make_a<P>(a, x);
         product_rows<HD, P>(dq, a, ak, b, lane);
       }
-      write_rows<HD>(p.qkv_adj, 3 * D, h * HD, g0, g1, i0 < cnt, i1 < cnt, dq, us * us * p.sc * unscale_of(b0) * usg, us * us * p.sc * unscale_of(b1) * usg,
+      write_rows<HD>(p.qkv_adj, 3 * D, h * HD, g0, g1, i0 < cnt, i1 < cnt, dq, usv * usk * p.sc * unscale_of(b0) * usg, usv * usk * p.sc * unscale_of(b1) * usg,
                         p.qkv_adj_max, t);
     } else {
       // transposed: rows are keys. S^T = K Q^T and dP^T = V dO^T per block of 16 queries
       const float lc0 = slc[i0], lc1 = slc[i1];
       const uint32_t bound = __float_as_uint(fmaxf(2.1f * gmax * vmax, 1e-9f));
-      const float ds = scale_of(bound) * (1.f / 32768.f), fds = us * unscale_of(bound) * usg;
+      const float ds = scale_of(bound) * (1.f / 32768.f), fds = usv * unscale_of(bound) * usg;
       float dk[HD / 8][4], dv[HD / 8][4];
       clear<HD>(dk), clear<HD>(dv);
       float cf0 = 0.f, cf1 = 0.f;
@@ -512,7 +533,7 @@ __global__ void __launch_bounds__(MAXT, BLOCKS) k_attn_bwd_f16(AttnArgs p) {
       }
       cf0 += __shfl_xor_sync(0xffffffffu, cf0, 1), cf0 += __shfl_xor_sync(0xffffffffu, cf0, 2);
       cf1 += __shfl_xor_sync(0xffffffffu, cf1, 1), cf1 += __shfl_xor_sync(0xffffffffu, cf1, 2);
-      write_rows<HD>(p.qkv_adj, 3 * D, D + h * HD, g0, g1, i0 < cnt, i1 < cnt, dk, fds * us * p.sc, fds * us * p.sc, p.qkv_adj_max, t);
+      write_rows<HD>(p.qkv_adj, 3 * D, D + h * HD, g0, g1, i0 < cnt, i1 < cnt, dk, fds * usq * p.sc, fds * usq * p.sc, p.qkv_adj_max, t);
       write_rows<HD>(p.qkv_adj, 3 * D, 2 * D + h * HD, g0, g1, i0 < cnt, i1 < cnt, dv, usg * (1.f / 32768.f), usg * (1.f / 32768.f),
                         p.qkv_adj_max, t);
       if (t == 0) {  // each key's dS summed over its queries: the cutoff factor's share from this head
@@ -580,11 +601,9 @@ bool bwd_p(Stream& st, const AttnArgs& p) {
 
 // True if these kernels took the pass; false leaves it to the others (an atom with too many tokens, another head size).
 bool attention_forward_f16(Stream& st, const AttnArgs& p) {
-  if (!p.qkv_max) return false;
   return p.mode == ATTN_NATIVE ? fwd_p<3>(st, p) : p.mode == ATTN_TF32X3 ? fwd_p<2>(st, p) : fwd_p<1>(st, p);
 }
 bool attention_backward_f16(Stream& st, const AttnArgs& p) {
-  if (!p.qkv_max || !p.dmerged_max) return false;
   return p.mode == ATTN_NATIVE ? bwd_p<3>(st, p) : p.mode == ATTN_TF32X3 ? bwd_p<2>(st, p) : bwd_p<1>(st, p);
 }
 

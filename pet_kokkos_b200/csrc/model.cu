@@ -286,7 +286,7 @@ int attention_mode_for(int gemm_mode) {
 }
 
 // Rows of an activation or adjoint, with the bits of each row's largest magnitude where the mode's operand format wants
-// them (gemm.h, attention.h); whatever writes the rows keeps them.
+// them (gemm.h); whatever writes the rows keeps them.
 struct Rows {
   float* p = nullptr;
   uint32_t* mx = nullptr;
@@ -298,26 +298,23 @@ struct Rows {
 // the block has no room left for (an edge MLP in very small chunks), whose GEMM then looks for the maxima itself.
 class RowMaxima {
  public:
-  RowMaxima(Stream& st, Arena& save, size_t words, bool gemms) : size_(words), gemms_(gemms) {
+  RowMaxima(Stream& st, Arena& save, size_t words) : size_(words) {
     if (!words) return;
     base_ = save.alloc<uint32_t>(words);
     PETB_CUDA(cudaMemsetAsync(base_, 0, words * sizeof(uint32_t), st.s));
   }
-  uint32_t* take(size_t rows) { return gemms_ ? part(rows) : nullptr; }
-  Rows fresh(float* p, size_t rows) { return {p, take(rows)}; }
-  Rows always(float* p, size_t rows) { return {p, part(rows)}; }  // what the attention reads, in every mode
-
- private:
-  uint32_t* part(size_t rows) {
+  uint32_t* take(size_t rows) {
     rows = (rows + 31) & ~size_t(31);
     if (used_ + rows > size_) return nullptr;
     uint32_t* p = base_ + used_;
     used_ += rows;
     return p;
   }
+  Rows fresh(float* p, size_t rows) { return {p, take(rows)}; }
+
+ private:
   uint32_t* base_ = nullptr;
   size_t size_ = 0, used_ = 0;
-  bool gemms_;
 };
 
 struct Gemms {
@@ -480,9 +477,8 @@ MemoryNeed Model::memory_need(int tier, int N, int E, int n_live) const {
 // Rows whose maxima a pass keeps (class RowMaxima): what each layer, block and readout writes for a GEMM to read.
 size_t Model::row_maxima_words(int N, int E) const {
   const size_t G = h_.num_gnn_layers, A = h_.num_attention_layers, T = size_t(N) + E + 64, n = size_t(N) + 64;
-  const size_t attention = G * 3 * A * T;
-  if (!scales_rows(format_of(mode_))) return attention;
-  return attention + G * ((11 * A + 8) * T + 6 * A * n) + 4 * T + 6 * n;
+  if (!scales_rows(format_of(mode_))) return 0;
+  return G * ((11 * A + 8) * T + 6 * A * n) + 4 * T + 6 * n;
 }
 
 size_t Model::memory_estimate(int tier, int N, int E) const {
@@ -511,7 +507,7 @@ PassOut Model::run_feedforward(Stream& st, Arena& save, Arena& tmp, const Packed
   last_tier_ = tier, last_estimate_ = memory_estimate(tier, N, E);
   const bool keep_wide = tier == RECOMPUTE_NEVER, relayer = grad && tier == RECOMPUTE_LAYERS;
   const int chunk = keep_wide ? 0 : edge_chunk_rows(E);
-  RowMaxima maxima(st, save, row_maxima_words(N, E) * (relayer ? 2 : 1), scales_rows(format_of(mode_)));  // a layer run again takes its own
+  RowMaxima maxima(st, save, row_maxima_words(N, E) * (relayer ? 2 : 1));  // a layer run again takes its own
 
   struct Block {
     float *tok, *ml, *node_res, *pre_c, *pre_e;
@@ -526,7 +522,7 @@ PassOut Model::run_feedforward(Stream& st, Arena& save, Arena& tmp, const Packed
     at.N = N, at.H = H, at.hd = hd, at.S = S, at.sc = sc, at.off = pk.off, at.cut = pk.cut;
     at.mode = attention_mode_for(mode), at.tf32 = wide();
     at.pairs = pk.pairs, at.T = T;
-    at.qkv = qkv.p, at.qkv_max = qkv.mx, at.merged = b.merged.p, at.ml = b.ml;
+    at.qkv = qkv.p, at.merged = b.merged.p, at.ml = b.ml;
     return at;
   };
   // qkv = W_in . norm(tokens) + b
@@ -578,7 +574,7 @@ PassOut Model::run_feedforward(Stream& st, Arena& save, Arena& tmp, const Packed
       b.eps = maxima.fresh(save.alloc<float>(Ta * D), Ta);  // rows < N: the attention output's atom rows; rows >= N: eps
       b.node_res = save.alloc<float>(Na * Dn);
       b.pre_c = save.alloc<float>(Na * w_cin.rows);
-      b.qkv = keep ? maxima.always(save.alloc<float>(Ta * 3 * D), Ta) : Rows{};
+      b.qkv = keep ? Rows{save.alloc<float>(Ta * 3 * D)} : Rows{};
       b.pre_e = keep ? save.alloc<float>(Ea * w_ein.rows) : nullptr;
       const Rows node_next = maxima.fresh(a + 1 == A ? node_out.p : save.alloc<float>(Na * Dn), Na);
       if (a + 1 == A) node_out = node_next;
@@ -587,7 +583,7 @@ PassOut Model::run_feedforward(Stream& st, Arena& save, Arena& tmp, const Packed
       gm.linear({b.tok}, node_cur, mat(tl + ".center_contraction.weight"), vec(tl + ".center_contraction.bias"), N);
       {
         Scope s1(tmp);
-        const Rows qkv = keep ? b.qkv : maxima.always(tmp.alloc<float>(Ta * 3 * D), Ta);
+        const Rows qkv = keep ? b.qkv : Rows{tmp.alloc<float>(Ta * 3 * D)};
         make_qkv(qkv, tl, b.tok);
         AttnArgs at = attention_args(b, qkv);
         at.merged_max = b.merged.mx;
@@ -789,19 +785,19 @@ PassOut Model::run_feedforward(Stream& st, Arena& save, Arena& tmp, const Packed
       }
       {  // attention: the output adjoint is [expansion's input adjoint ; eps adjoint] = tok_adj
         Scope s10(tmp);
-        const Rows dmerged = maxima.always(tmp.alloc<float>(Ta * D), Ta);
+        const Rows dmerged = Rows{tmp.alloc<float>(Ta * D)};
         const Rows qkv_adj = maxima.fresh(tmp.alloc<float>(Ta * 3 * D), Ta);
         float* cfh = tmp.alloc<float>(Ta * H);
         float* attn_in_adj = tmp.alloc<float>(Ta * D);
         Rows qkv = b.qkv;
         if (!qkv.p) {
-          qkv = maxima.always(tmp.alloc<float>(Ta * 3 * D), Ta);
+          qkv = Rows{tmp.alloc<float>(Ta * 3 * D)};
           make_qkv(qkv, tl, b.tok);
         }
         gm.linear_bwd(tok_adj, node_adj, mat(tl + ".center_expansion.weight"), N, false);
         gm.linear_bwd(dmerged, tok_adj, mat(tl + ".attention.output_linear.weight"), T, false);
         AttnArgs at = attention_args(b, qkv);
-        at.dmerged = dmerged.p, at.dmerged_max = dmerged.mx, at.qkv_adj = qkv_adj.p, at.qkv_adj_max = qkv_adj.mx, at.cfh = cfh;
+        at.dmerged = dmerged.p, at.qkv_adj = qkv_adj.p, at.qkv_adj_max = qkv_adj.mx, at.cfh = cfh;
         attention_backward(st, at);
         cutoff_share(st, cf_adj, cfh, pk.cut, N, E, H);
         gm.linear_bwd({attn_in_adj}, qkv_adj, mat(tl + ".attention.input_linear.weight"), T, false);
@@ -840,7 +836,7 @@ PassOut Model::run_residual(Stream& st, Arena& save, Arena& tmp, const PackedEdg
   const Gemms gm{st, tmp};
   const float sc = float(1.0 / (std::sqrt(double(hd)) * h_.attention_temperature));
   const size_t Ea = E > 0 ? E : 1, Ta = T > 0 ? T : 1, Na = N > 0 ? N : 1;
-  RowMaxima maxima(st, save, row_maxima_words(N, E), scales_rows(format_of(mode_)));
+  RowMaxima maxima(st, save, row_maxima_words(N, E));
 
   struct Block {
     Rows qkv;
@@ -881,7 +877,7 @@ PassOut Model::run_residual(Stream& st, Arena& save, Arena& tmp, const PackedEdg
       const std::string tl = g + ".trans.layers." + std::to_string(a);
       Block& b = sl.blk[a];
       const Mat& w_in = mat(tl + ".mlp.w_in.weight");
-      b.qkv = maxima.always(save.alloc<float>(Ta * 3 * D), Ta);
+      b.qkv = Rows{save.alloc<float>(Ta * 3 * D)};
       b.merged = save.alloc<float>(Ta * D);
       b.ml = save.alloc<float>(Ta * H * 2);
       b.s1 = save.alloc<float>(Ta * D);
@@ -893,7 +889,7 @@ PassOut Model::run_residual(Stream& st, Arena& save, Arena& tmp, const PackedEdg
       at.mode = attention_mode_for(mode), at.tf32 = wide();
       at.pairs = pk.pairs, at.T = T;
       const Rows merged = maxima.fresh(b.merged, Ta);
-      at.qkv = b.qkv.p, at.qkv_max = b.qkv.mx, at.merged = b.merged, at.ml = b.ml, at.merged_max = merged.mx;
+      at.qkv = b.qkv.p, at.merged = b.merged, at.ml = b.ml, at.merged_max = merged.mx;
       attention_forward(st, at);
       // s1 = attention(tokens) + tokens
       gm.linear({b.s1}, merged, mat(tl + ".attention.output_linear.weight"), vec(tl + ".attention.output_linear.bias"), T,
@@ -1010,7 +1006,7 @@ PassOut Model::run_residual(Stream& st, Arena& save, Arena& tmp, const PackedEdg
       norm_bwd(st, s1_adj.p, tok_a_adj, b.s1, vec(tl + ".norm_attention.weight"), true, T, D, T, nullptr, s1_adj.mx);
       {
         Scope s6(tmp);
-        const Rows dmerged = maxima.always(tmp.alloc<float>(Ta * D), Ta);
+        const Rows dmerged = Rows{tmp.alloc<float>(Ta * D)};
         const Rows qkv_adj = maxima.fresh(tmp.alloc<float>(Ta * 3 * D), Ta);
         float* cfh = tmp.alloc<float>(Ta * H);
         gm.linear_bwd(dmerged, s1_adj, mat(tl + ".attention.output_linear.weight"), T, false);
@@ -1018,7 +1014,7 @@ PassOut Model::run_residual(Stream& st, Arena& save, Arena& tmp, const PackedEdg
         at.N = N, at.H = H, at.hd = hd, at.S = S, at.sc = sc, at.off = pk.off, at.cut = pk.cut;
       at.mode = attention_mode_for(mode), at.tf32 = wide();
         at.pairs = pk.pairs, at.T = T;
-        at.qkv = b.qkv.p, at.qkv_max = b.qkv.mx, at.merged = b.merged, at.ml = b.ml, at.dmerged = dmerged.p, at.dmerged_max = dmerged.mx;
+        at.qkv = b.qkv.p, at.merged = b.merged, at.ml = b.ml, at.dmerged = dmerged.p;
         at.qkv_adj = qkv_adj.p, at.cfh = cfh;
         at.qkv_adj_max = qkv_adj.mx;
         attention_backward(st, at);
