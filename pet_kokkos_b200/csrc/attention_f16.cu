@@ -4,7 +4,12 @@
 // An operand is scaled by a power of two that brings its largest value (of this atom and head, found while the tile is staged: Q, K,
 // V and dO each have their own, whatever the other heads hold) to [2^14, 2^15) and split into P parts:
 //   P = 3 (ATTN_NATIVE)  x = h + m + l, h a multiple of 2^8: eight bits of the largest value, so that the h.h products of up to
-//                        1024 terms sum exactly; six products, h.h on an accumulator of its own (gemm.h has the argument);
+//                        1024 terms sum exactly; six products, h.h on an accumulator of its own (gemm.h has the argument): hh hm
+//                        mh mm tl lt with t = h + m to eleven bits, added up in registers. With h for t, as the GEMMs do on
+//                        weights that are not spread, ml and lm are left out; scores whose queries and keys are large in
+//                        different columns then put a force 1.7e-5 of the scale off for 2e-6. What an atom holds is not known
+//                        ahead, so the tile always takes t: attention of diamond1728 1.20 + 3.25 ms -> 1.32 + 3.44 (ml and lm as
+//                        products of their own: 1.38 + 3.85);
 //   P = 2 (ATTN_TF32X3)  x = h + l, 22 bits; three products;
 //   P = 1 (ATTN_TF32)    x rounded to 11 bits; one product.
 // Q, K, V (and dO) are split once, when a CTA stages its (atom, head): the parts of a row lie side by side in shared memory,
@@ -103,16 +108,32 @@ struct Acc {
   }
   __device__ __forceinline__ float get(int n, int i) const { return P == 3 ? big[n][i] + small[n][i] : big[n][i]; }
 };
-// The products of parts (i, j) in the order they are added, small terms first.
+// The products of parts (i, j) in the order they are added, small terms first. With three parts l's partner is h + m to eleven bits
+// (part 3, made in registers).
 template <int P>
 __device__ __forceinline__ constexpr int products() { return P == 3 ? 6 : P == 2 ? 3 : 1; }
 template <int P>
 __device__ __forceinline__ constexpr int part_a(int u) {
-  return P == 3 ? (u == 0 ? 0 : u == 1 ? 2 : u == 2 ? 1 : u == 3 ? 0 : u == 4 ? 1 : 0) : P == 2 ? (u == 0 ? 0 : u == 1 ? 1 : 0) : 0;
+  constexpr int three[6] = {3, 2, 1, 0, 1, 0}, two[3] = {0, 1, 0};
+  return P == 3 ? three[u] : P == 2 ? two[u] : 0;
 }
 template <int P>
 __device__ __forceinline__ constexpr int part_b(int u) {
-  return P == 3 ? (u == 0 ? 2 : u == 1 ? 0 : u == 2 ? 1 : u == 3 ? 1 : u == 4 ? 0 : 0) : P == 2 ? (u == 0 ? 1 : u == 1 ? 0 : 0) : 0;
+  constexpr int three[6] = {2, 3, 1, 1, 0, 0}, two[3] = {1, 0, 0};
+  return P == 3 ? three[u] : P == 2 ? two[u] : 0;
+}
+template <int P>
+__host__ __device__ constexpr int with_sum() { return P == 3 ? 4 : P; }
+// Part 3 of a fragment whose first two parts are x[0] and x[1].
+template <int P>
+__device__ __forceinline__ void add_sum(uint32_t (*x)[4]) {
+  if (P == 3) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const __half2 v = __hadd2(*reinterpret_cast<const __half2*>(&x[0][i]), *reinterpret_cast<const __half2*>(&x[1][i]));
+      x[3][i] = *reinterpret_cast<const uint32_t*>(&v);
+    }
+  }
 }
 
 // Rows r0 .. r0 + 15, columns 16 ks .. + 15 of a staged tensor as A operand, part j.
@@ -140,7 +161,8 @@ __device__ __forceinline__ void two_products(Acc<P, 2>& c1, Acc<P, 2>& c2, const
   if (BOTH) c2.zero();
 #pragma unroll
   for (int ks = 0; ks < HD / 16; ++ks) {
-    uint32_t b1[P][4], b2[P][4], t1[P][4], t2[P][4];
+    constexpr int R = with_sum<P>();
+    uint32_t b1[R][4], b2[R][4], t1[R][4], t2[R][4];
 #pragma unroll
     for (int j = 0; j < P; ++j) {
       load_bt<HD, P>(b1[j], y1, rb, ks, j, lane);
@@ -148,16 +170,24 @@ __device__ __forceinline__ void two_products(Acc<P, 2>& c1, Acc<P, 2>& c2, const
       if (!KEEP) {
         load_a<HD, P>(t1[j], xa1, ra, ks, j, lane);
         if (BOTH) load_a<HD, P>(t2[j], xa2, ra, ks, j, lane);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          t1[j][i] = a1[ks][j][i];
+          if (BOTH) t2[j][i] = a2[ks][j][i];
+        }
       }
     }
+    add_sum<P>(b1), add_sum<P>(t1);
+    if (BOTH) add_sum<P>(b2), add_sum<P>(t2);
 #pragma unroll
     for (int u = 0; u < products<P>(); ++u) {
       const int i = part_a<P>(u), j = part_b<P>(u);
       const bool lead = u + 1 == products<P>();
 #pragma unroll
       for (int n = 0; n < 2; ++n) {
-        mma(P == 3 && !lead ? c1.small[P == 3 ? n : 0] : c1.big[n], KEEP ? a1[ks][i] : t1[i], b1[j] + 2 * n);
-        if (BOTH) mma(P == 3 && !lead ? c2.small[P == 3 ? n : 0] : c2.big[n], KEEP ? a2[ks][i] : t2[i], b2[j] + 2 * n);
+        mma(P == 3 && !lead ? c1.small[P == 3 ? n : 0] : c1.big[n], t1[i], b1[j] + 2 * n);
+        if (BOTH) mma(P == 3 && !lead ? c2.small[P == 3 ? n : 0] : c2.big[n], t2[i], b2[j] + 2 * n);
       }
     }
   }
@@ -168,9 +198,10 @@ template <int HD, int P>
 __device__ __forceinline__ void product_rows(float (*c)[4], const uint32_t (*a)[4], uint32_t x, int r0, int lane) {
 #pragma unroll
   for (int d = 0; d < HD / 16; ++d) {
-    uint32_t b[P][4];
+    uint32_t b[with_sum<P>()][4];
 #pragma unroll
     for (int j = 0; j < P; ++j) load_b<HD, P>(b[j], x, r0, d, j, lane);
+    add_sum<P>(b);
     Acc<3, 2> tmp;
     if (P == 3) tmp.zero();
 #pragma unroll
@@ -205,6 +236,7 @@ __device__ __forceinline__ void make_a(uint32_t (*a)[4], const float (*x)[4]) {
 #pragma unroll
       for (int j = 0; j < P; ++j) a[j][2 * n + h] = part[j];
     }
+  add_sum<P>(a);
 }
 
 // A thread's largest value of a tensor raised into the tile's.
@@ -364,7 +396,7 @@ __global__ void __launch_bounds__(32 * MAXB, MAXB <= 5 ? resident<HD, P, 3>(16 *
     if (b < nb) {
 #pragma unroll
       for (int i = 0; i < 2; ++i) x[b][i][0] *= w0, x[b][i][1] *= w0, x[b][i][2] *= w1, x[b][i][3] *= w1;
-      uint32_t a[P][4];
+      uint32_t a[with_sum<P>()][4];
       make_a<P>(a, x[b]);
       product_rows<HD, P>(o, a, av, 16 * b, lane);
     }
@@ -494,7 +526,7 @@ __global__ void __launch_bounds__(MAXT, BLOCKS) k_attn_bwd_f16(AttnArgs p) {
           x[i][2] = exp2_fast(fmaf(c.get(i, 2), f, lc.x) - m1) * il1 * (w.get(i, 2) - d1);
           x[i][3] = exp2_fast(fmaf(c.get(i, 3), f, lc.y) - m1) * il1 * (w.get(i, 3) - d1);
         }
-        uint32_t a[P][4];
+        uint32_t a[with_sum<P>()][4];
         make_a<P>(a, x);
         product_rows<HD, P>(dq, a, ak, b, lane);
       }
@@ -525,7 +557,7 @@ __global__ void __launch_bounds__(MAXT, BLOCKS) k_attn_bwd_f16(AttnArgs p) {
           y[i][2] = x[i][2] * ((w.get(i, 2) - d.x) * ds), y[i][3] = x[i][3] * ((w.get(i, 3) - d.y) * ds);
           cf0 += y[i][0] + y[i][1], cf1 += y[i][2] + y[i][3];
         }
-        uint32_t a[P][4];
+        uint32_t a[with_sum<P>()][4];
         make_a<P>(a, y);
         product_rows<HD, P>(dk, a, aq, b, lane);
         make_a<P>(a, x);

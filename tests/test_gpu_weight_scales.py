@@ -1,6 +1,6 @@
 """A network whose weights are rescaled by powers of two that cancel exactly (a head's values against the output projection, a
-head's queries against its keys) is the same function. The evaluation has to stay within the bands of the plain network: no
-tensor may be held to the scale of another."""
+head's queries against its keys, a gate's values against the layer after it, a norm's gains against the layer after it) is the
+same function. The evaluation has to stay within the bands of the plain network: no tensor may be held to the scale of another."""
 import numpy as np
 import pytest
 import torch
@@ -25,9 +25,32 @@ def heads_apart(t, h, rng):
             t[p + ".output_linear.weight"][:, at] /= s
 
 
+def features_apart(t, h, rng):
+    """Columns of queries and keys, values of gates and gains of norms on scales of their own."""
+    D = h["d_pet"]
+    e = lambda n: np.float32(2.0) ** rng.integers(-6, 7, size=n).astype(np.float32)
+    for p in [n[:-len(".w_in.weight")] for n in t if n.endswith(".w_in.weight")]:
+        f = t[p + ".w_out.weight"].shape[1]
+        s = e(f)
+        t[p + ".w_in.weight"][:f] *= s[:, None]
+        t[p + ".w_in.bias"][:f] *= s
+        t[p + ".w_out.weight"] /= s
+    for p in [n[:-len(".attention.input_linear.weight")] for n in t if n.endswith(".attention.input_linear.weight")]:
+        s = e(D)
+        for name in (".attention.input_linear.weight", ".attention.input_linear.bias"):
+            t[p + name][:D] = (t[p + name][:D].T * s).T
+            t[p + name][D:2 * D] = (t[p + name][D:2 * D].T / s).T
+        g = e(D)
+        t[p + ".norm_attention.weight"] *= g
+        t[p + ".attention.input_linear.weight"] /= g
+        g = e(D)
+        t[p + ".norm_mlp.weight"] *= g
+        t[p + ".mlp.w_in.weight"] /= g
+
+
 @pytest.mark.parametrize("gemm", ["native", "3xtf32"])
 @pytest.mark.parametrize("heads", [1, 2, 4])  # head sizes 64, 32, 16
-@pytest.mark.parametrize("how", [heads_apart])
+@pytest.mark.parametrize("how", [heads_apart, features_apart])
 def test_same_function(lib_path, tmp_path, how, heads, gemm):
     from pet_kokkos_b200 import Calculator
     shape = dict(d_pet=64, num_heads=heads, d_feedforward=64, cutoff=4.5)
