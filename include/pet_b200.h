@@ -300,6 +300,9 @@ long long pet_batch_splits(const pet_calc* c);
  * device allocation of the scratch pools from now (0 = the next) reports out of memory once; k < 0 disarms. */
 long long pet_oom_recoveries(const pet_calc* c);
 void pet_debug_fail_alloc(long k);
+/* The test hook for a tensor-core kernel that gave up on a bounded wait: the calculator's device word is raised as such a
+ * kernel raises it. The next call that brings results to the host fails with PET_ERR_CUDA and lowers it. */
+int pet_debug_give_up(pet_calc* c);
 /* Times this calculator has asked the driver how much device memory is free (for the recompute tier and the batch
  * pieces it chooses by itself). The call goes into the kernel-mode driver and waits behind its other clients, so
  * the answer is kept for as long as the calculator's pools keep their size: a steady loop stops asking. */

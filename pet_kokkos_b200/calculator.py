@@ -163,6 +163,7 @@ SIGNATURES = {
     "pet_oom_recoveries": (C.c_longlong, [C.c_void_p]),
     "pet_driver_memory_queries": (C.c_longlong, [C.c_void_p]),
     "pet_debug_fail_alloc": (None, [C.c_long]),
+    "pet_debug_give_up": (C.c_int, [C.c_void_p]),
     "pet_neighbor_searches": (C.c_longlong, [C.c_void_p]),
     "pet_neighbor_reuses": (C.c_longlong, [C.c_void_p]),
     "pet_profile": (C.c_int, [C.c_void_p, C.c_int]),
@@ -646,6 +647,10 @@ class Calculator:
                 for i in range(n.value)}
 
     # ---- testing aids ----
+    def debug_give_up(self):
+        """Raises the word that a tensor-core kernel raises when it gives up on a wait."""
+        self._check(self._lib.pet_debug_give_up(self._h))
+
     def enable_taps(self):
         n = C.c_size_t()
         self._lib.pet_debug_fetch(self._h, b"", None, 0, C.byref(n))  # arms recording for the next evaluation

@@ -212,6 +212,12 @@ long long pet_graph_replays(const pet_calc* c) { return c && c->e ? c->e->graph_
 long long pet_oom_recoveries(const pet_calc* c) { return c && c->e ? c->e->oom_recoveries : 0; }
 long long pet_driver_memory_queries(const pet_calc* c) { return c && c->e ? c->e->mem_queries : 0; }
 void pet_debug_fail_alloc(long k) { petb::g_fail_alloc_in = k; }
+int pet_debug_give_up(pet_calc* c) {
+  return guarded(c, [&](Engine& e) {
+    PETB_CUDA(cudaSetDevice(e.device));
+    PETB_CUDA(cudaMemsetAsync(e.st.gave_up, 1, sizeof(int), e.st.s));
+  });
+}
 long long pet_batch_splits(const pet_calc* c) { return c && c->e ? c->e->batch_splits : 0; }
 long long pet_neighbor_searches(const pet_calc* c) { return c && c->e ? c->e->verlet.searches : 0; }
 long long pet_neighbor_reuses(const pet_calc* c) { return c && c->e ? c->e->verlet.reuses : 0; }

@@ -226,6 +226,7 @@ struct Stream {
   cudaStream_t s = nullptr;
   long long launches = 0;
   Profiler* prof = nullptr;
+  int* gave_up = nullptr;  // device word that a tensor-core kernel raises when it gives up on a bounded wait
   cudaEvent_t legacy_fence = nullptr;  // made at first use by order_after_legacy_stream, destroyed with the stream's owner
 };
 

@@ -195,6 +195,8 @@ Engine::Engine(const std::string& json, const std::string& weights, const pet_op
     }
   if (recompute > RECOMPUTE_LAYERS) throw Error(2, "pet: unknown recompute tier " + std::to_string(recompute));
   PETB_CUDA(cudaStreamCreateWithFlags(&st.s, cudaStreamNonBlocking));
+  PETB_CUDA(cudaMalloc(&st.gave_up, sizeof(int)));
+  PETB_CUDA(cudaMemsetAsync(st.gave_up, 0, sizeof(int), st.s));
   PETB_CUDA(cudaEventCreate(&ev0));
   PETB_CUDA(cudaEventCreate(&ev1));
   PETB_CUDA(cudaMallocHost(&pinned, 64 * sizeof(int)));
@@ -212,6 +214,7 @@ Engine::~Engine() {
   if (ev0) cudaEventDestroy(ev0);
   if (ev1) cudaEventDestroy(ev1);
   if (st.legacy_fence) cudaEventDestroy(st.legacy_fence);
+  cudaFree(st.gave_up);
   if (st.s) cudaStreamDestroy(st.s);
 }
 

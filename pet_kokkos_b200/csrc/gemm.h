@@ -129,8 +129,8 @@ void gemv_rows(Stream& st, const float* A, int lda, const float* w, const float*
 // mx[r] = bits of the largest |x(r, :)|.
 void row_max(Stream& st, uint32_t* mx, const float* x, int ld, int R, int D);
 
-// Whether a tensor-core kernel gave up on a bounded wait: the first puts a copy of the device's word into pinned memory on the
-// stream, the second, once the stream has got there, looks at it and clears the device's.
+// Whether a tensor-core kernel of this stream gave up on a bounded wait: the first puts a copy of the stream's word into pinned
+// memory, the second, once the stream has got there, looks at it and clears the word.
 void gemm_tensor_error_ask(Stream& st, int* host);
 bool gemm_tensor_error(Stream& st, const int* host);
 

@@ -12,7 +12,7 @@
 namespace petb {
 
 void gemm_tensor(Stream& st, Arena& arena, const GemmArgs& a, const PackedB& w);  // gemm_tc.cu
-bool gemm_tensor_usable(const GemmArgs& a, const PackedB& w);
+bool gemm_tensor_usable(const Stream& st, const GemmArgs& a, const PackedB& w);
 
 namespace {
 
@@ -147,7 +147,7 @@ void gemm(Stream& st, Arena& arena, const GemmArgs& a) {
   const ProfScope ps(st, PC_GEMM, 2.0 * a.M * a.N * a.K, bytes);
   // Fewer than half a tile of rows: the speed modes' products would not be felt there, so they run at full precision.
   const PackedB& w = a.M < 64 || a.N < 32 ? a.nat : a.fast;
-  if (gemm_tensor_usable(a, w)) return gemm_tensor(st, arena, a, w);
+  if (gemm_tensor_usable(st, a, w)) return gemm_tensor(st, arena, a, w);
   if (!a.B) throw Error(3, "gemm: this weight has no fp32 copy for the CUDA cores");
   switch (a.epi) {
     case EPI_PLAIN: return launch_native<EPI_PLAIN>(st, a);

@@ -884,11 +884,10 @@ using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, voi
                               const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                               CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
-// What the tensor-core path needs of one device: its SM count and an error word in its memory, plus the driver's tensor-map encoder (the same function for every device). One per device ordinal,
+// What the tensor-core path needs of one device: its SM count and the driver's tensor-map encoder (the same function for every device). One per device ordinal,
 // built on first use with that device current.
 struct TensorState {
   EncodeFn encode = nullptr;
-  int* err = nullptr;       // device error word
   int sms = 0;
   bool ok = false;
 };
@@ -905,9 +904,6 @@ TensorState& state() {
     cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev);
     cudaDeviceGetAttribute(&s.sms, cudaDevAttrMultiProcessorCount, dev);
     if (major != 10 || s.sms <= 0) return;
-    if (cudaMalloc(&s.err, sizeof(int)) != cudaSuccess) return;
-    cudaMemset(s.err, 0, sizeof(int));
-    cudaStreamSynchronize(cudaStreamLegacy);  // the callers' streams do not wait for the legacy one
     s.encode = reinterpret_cast<EncodeFn>(fn);
     s.ok = true;
   });
@@ -997,7 +993,7 @@ void launch_tc(Stream& st, const GemmArgs& a, const PackedB& w, int parts = 1) {
   }
   attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // see launch()
   attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
-  PETB_CUDA(cudaLaunchKernelEx(&cfg, kernel, ma, mb, ml, mi, mc, mp, a, w.unscale, state().err));
+  PETB_CUDA(cudaLaunchKernelEx(&cfg, kernel, ma, mb, ml, mi, mc, mp, a, w.unscale, st.gave_up));
   PETB_LAUNCH_CHECK(st);
 }
 
@@ -1129,10 +1125,10 @@ void row_max(Stream& st, uint32_t* mx, const float* x, int ld, int R, int D) {
 bool tensor_gemm_available() { return state().ok; }
 
 // Whether a tensor-core kernel takes this GEMM: a packed weight, and rows that TMA can address (16-byte aligned).
-bool gemm_tensor_usable(const GemmArgs& a, const PackedB& w) {
+bool gemm_tensor_usable(const Stream& st, const GemmArgs& a, const PackedB& w) {
   const uintptr_t at = reinterpret_cast<uintptr_t>(a.A) | reinterpret_cast<uintptr_t>(a.C) | reinterpret_cast<uintptr_t>(a.pre) |
                        reinterpret_cast<uintptr_t>(a.res);
-  return w.main && state().ok && !(at & 15) && a.lda % 4 == 0 && a.ldc % 4 == 0 && a.ldp % 4 == 0 && a.ldr % 4 == 0;
+  return w.main && st.gave_up && state().ok && !(at & 15) && a.lda % 4 == 0 && a.ldc % 4 == 0 && a.ldp % 4 == 0 && a.ldr % 4 == 0;
 }
 
 void gemm_tensor(Stream& st, Arena& arena, const GemmArgs& given, const PackedB& w) {
@@ -1156,12 +1152,11 @@ void gemm_tensor(Stream& st, Arena& arena, const GemmArgs& given, const PackedB&
 }
 
 void gemm_tensor_error_ask(Stream& st, int* host) {
-  TensorState& s = state();
   *host = 0;
-  if (s.ok) cudaMemcpyAsync(host, s.err, sizeof(int), cudaMemcpyDeviceToHost, st.s);
+  cudaMemcpyAsync(host, st.gave_up, sizeof(int), cudaMemcpyDeviceToHost, st.s);
 }
 bool gemm_tensor_error(Stream& st, const int* host) {
-  if (*host) cudaMemsetAsync(state().err, 0, sizeof(int), st.s);
+  if (*host) cudaMemsetAsync(st.gave_up, 0, sizeof(int), st.s);
   return *host != 0;
 }
 
