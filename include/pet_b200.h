@@ -387,7 +387,9 @@ int pet_nccl_exchange_reduce(pet_nccl_exchange* x, const double* forces, const d
                              void* stream, double* out_host);
 int pet_nccl_exchange_timing(pet_nccl_exchange* x, int enable, double* ms, int* calls);
 /* The latest evaluation's results where they lie on the device (forces [n_atoms,3], energy [B], virial [B,6]; null
- * before any evaluation or without forces) and the calculator's cudaStream_t: what pet_nccl_exchange_reduce reads. */
+ * before any evaluation or without forces) and the calculator's cudaStream_t: what pet_nccl_exchange_reduce reads.
+ * Nothing is waited for, so whether the evaluation ran to its end is not known yet: one of whose GEMMs gave up on a
+ * bounded wait has NaN in all of these once the stream has got there, and the next evaluation fails with PET_ERR_CUDA. */
 int pet_device_results_of(pet_calc* c, pet_device_results* out, void** stream);
 
 /* C[m,n] = A[m,k] . W^T, W [n,k], fp32 on the CUDA cores, on host arrays, WITHOUT allocating

@@ -591,6 +591,7 @@ void Engine::compute_staged(bool forces) {
   have_out = false;
   if (in_flight) PETB_CUDA(cudaStreamSynchronize(st.s));  // (not for the copy of what was just staged)
   in_flight = true;
+  check_left();
   nbr_arena.reset();
   save_arena.reset();
   tmp_arena.reset();
@@ -677,6 +678,40 @@ RawEdges Engine::cached_edges() {
   return c.ref;
 }
 
+// NaN in results on the device whose evaluation gave up on a wait: whoever reads them there never asks the host.
+static __global__ void k_void_results(const int* gave_up, double* energy, double* virial, int B, double* per_atom, double* forces, int N) {
+  if (*gave_up == 0) return;
+  const double nan = __longlong_as_double(0x7FF8000000000000ll);
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < max(N, B); i += gridDim.x * blockDim.x) {
+    if (i < B) energy[i] = nan;
+    if (i < N) per_atom[i] = nan;
+    for (int k = 0; virial && i < B && k < 6; ++k) virial[6 * i + k] = nan;
+    for (int k = 0; forces && i < N && k < 3; ++k) forces[3 * i + k] = nan;
+  }
+}
+
+void Engine::device_results(pet_device_results* out) {
+  PETB_CUDA(cudaSetDevice(device));
+  *out = pet_device_results{};
+  out->n_atoms = last_N;
+  if (!have_out) return;
+  const ForceOut& f = last_out.f;
+  const bool forces = last_out.has_forces;
+  k_void_results<<<32, 256, 0, st.s>>>(st.gave_up, f.energy, forces ? f.vir6 : nullptr, last_B, last_out.per_atom, forces ? f.forces : nullptr, last_N);
+  PETB_LAUNCH_CHECK(st);
+  gemm_tensor_error_ask(st, pinned + kGaveUpLeft);
+  left_asked = in_flight = true;
+  out->energy = f.energy, out->per_atom_energy = last_out.per_atom;
+  if (forces) out->forces = f.forces, out->virial = f.vir6;
+}
+
+void Engine::check_left() {
+  if (!left_asked) return;
+  left_asked = false;
+  if (gemm_tensor_error(st, pinned + kGaveUpLeft))
+    throw Error(5, "pet: a tensor-core GEMM gave up waiting on its pipeline in the evaluation before this one; the results it left on the device are invalid");
+}
+
 void Engine::fetch(pet_results* out) {
   PETB_CUDA(cudaSetDevice(device));
   if (!out) throw Error(2, "pet: no results struct given");
@@ -714,6 +749,7 @@ void Engine::fetch(pet_results* out) {
     bring(out->struct_id, last_pk.sid, sizeof(int) * N);
   }
   gemm_tensor_error_ask(st, pinned + kGaveUp);
+  left_asked = false;
   PETB_CUDA(cudaStreamSynchronize(st.s));
   float ms = 0.f;
   if (cudaEventElapsedTime(&ms, ev0, ev1) == cudaSuccess) last_ms = ms;
@@ -1015,6 +1051,7 @@ static StepOut session_step(Engine& I, const double* positions, bool on_device, 
   if (s.shifted && !cell) throw Error(1, "pet: an edge list with shifts needs the cell");
   PETB_CUDA(cudaStreamSynchronize(st.s));
   I.have_out = false, I.in_flight = true;
+  I.check_left();
   I.nbr_arena.reset();
   I.save_arena.reset();
   I.tmp_arena.reset();

@@ -76,6 +76,7 @@ struct Engine {
   void keep_staged(const int* keep, int n_keep);
   void compute_staged(bool forces);
   void fetch(pet_results* out);
+  void device_results(pet_device_results* out);
   void neighbor_list(const pet_system* systems, int B, pet_raw_edges* out);
   void set_neighbors(const pet_edge_list* list);
   void compute_step(const double* positions, const double* cell, bool forces, bool edge_gradients, pet_results* out);
@@ -128,6 +129,9 @@ struct Engine {
   int last_B = 0, last_N = 0;
   int* pinned = nullptr;  // small pinned scratch for readbacks
   static constexpr int kGaveUp = 9;  // the word of it that says whether a GEMM gave up on a wait
+  static constexpr int kGaveUpLeft = 10;  // the same of an evaluation whose results were handed out on the device
+  bool left_asked = false;                // that word is on its way
+  void check_left();                      // looks at it, the stream having been waited for
   char* landing = nullptr;  // pinned: where results land before they go to the caller's arrays
   size_t landing_bytes = 0;
   void* host_stage = nullptr;
