@@ -8,12 +8,12 @@
 // plus the residual add and compress.0's folded geometry/species terms
 // (src/ops.cpp:326-365).
 //
-// Two kernel families share the epilogue code:
+// Two kernel families:
 //   * tensor (gemm_tc.cu): tcgen05.mma kind::f16 with TMA-fed shared-memory tiles and the accumulator in tensor memory.
 //     Operands wider than 16 bits are split into 16-bit parts whose products are summed in fp32; the formats below say
 //     into which, for each mode;
-//   * fp32 FMA on the CUDA cores (gemm_simt.cu): one accumulation chain per output in k order, for operands that have
-//     no packed weight (pet_gemm_host_static) or that TMA cannot address.
+//   * fp32 FMA on the CUDA cores (gemm_simt.cu): one accumulation chain per output in k order, the plain product, for callers
+//     without a packed weight (pet_gemm_host_static).
 // In the native format and on the CUDA cores a row's bits depend on that row and the weight alone, not on how many rows share
 // its launch. The other formats add a long K in another order where few rows leave SMs for it (plan_split, gemm_tc.cu).
 #pragma once

@@ -32,7 +32,6 @@ __device__ __forceinline__ void fma2(unsigned long long& d, unsigned long long a
   asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
 }
 
-template <int EPI>
 __global__ void __launch_bounds__(256, 2) k_gemm_native(GemmArgs p) {
   after_previous();
   __shared__ __align__(16) float As[2][BK][BM + PAD];
@@ -108,7 +107,7 @@ __global__ void __launch_bounds__(256, 2) k_gemm_native(GemmArgs p) {
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       const int col = n0 + 64 * h + tx * 4;
-      if (col < p.N) epilogue_run4<EPI>(p, row, col, &acc[i][4 * h]);
+      if (col < p.N) st4(p.C + size_t(row) * p.ldc + col, ld4(&acc[i][4 * h]));
     }
   }
 }
@@ -123,13 +122,6 @@ __global__ void k_gemv_rows(const float* __restrict__ A, int lda, const float* _
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   if (lane == 0) out[r] = s + (bias ? bias[0] : 0.0f);
-}
-
-template <int EPI>
-void launch_native(Stream& st, const GemmArgs& a) {
-  const long long tiles = (long long) cdiv(a.M, BM) * cdiv(a.N, BN);
-  launch(st, k_gemm_native<EPI>, (unsigned) tiles, 256, 0, a);
-  PETB_LAUNCH_CHECK(st);
 }
 
 }  // namespace
@@ -149,15 +141,10 @@ void gemm(Stream& st, Arena& arena, const GemmArgs& a) {
   const PackedB& w = a.M < 64 || a.N < 32 ? a.nat : a.fast;
   if (gemm_tensor_usable(st, a, w)) return gemm_tensor(st, arena, a, w);
   if (!a.B) throw Error(3, "gemm: this weight has no fp32 copy for the CUDA cores");
-  switch (a.epi) {
-    case EPI_PLAIN: return launch_native<EPI_PLAIN>(st, a);
-    case EPI_SILU: return launch_native<EPI_SILU>(st, a);
-    case EPI_SWIGLU: return launch_native<EPI_SWIGLU>(st, a);
-    case EPI_SILU_BWD: return launch_native<EPI_SILU_BWD>(st, a);
-    case EPI_SWIGLU_BWD: return launch_native<EPI_SWIGLU_BWD>(st, a);
-    case EPI_COMPRESS: return launch_native<EPI_COMPRESS>(st, a);
-    default: throw Error(3, "gemm: unknown epilogue");
-  }
+  if (a.epi != EPI_PLAIN || a.bias || a.res || a.c_max) throw Error(3, "gemm: the CUDA cores give the plain product alone");
+  const long long tiles = (long long) cdiv(a.M, BM) * cdiv(a.N, BN);
+  launch(st, k_gemm_native, (unsigned) tiles, 256, 0, a);
+  PETB_LAUNCH_CHECK(st);
 }
 
 void gemv_rows(Stream& st, const float* A, int lda, const float* w, const float* bias, float* out, int M, int K) {

@@ -157,6 +157,7 @@ struct Tile {
   // 24 + 2 x 200 + 88 registers a thread over the warp groups are the 4 x 128 of the launch, 40 + 2 x 136 + 2 x 80 within the 5 x 96
   static constexpr bool kMoveRegs = TA || (X3 && BN >= 128);
   static constexpr int kRegsProd = TA ? 40 : 24, kRegsEpi = TA ? 136 : 200, kRegsConv = TA ? 80 : 88;
+  static_assert(!T1 || !PAIR, "FMT_TF32 has no converter to tell the other CTA's issuer that a slab has landed");
   static_assert(kRings >= TBM * BN * 4, "the shared sums of a split tile");
   static_assert((TA || NA >= NB) && NA >= 2 && NB >= 2 && NA % kGroups == 0, "the slots");
   static_assert(!TA || (NT >= NB && NT <= ND), "the slots");
@@ -343,7 +344,7 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1)
           if (!(ok = mbar_wait_warp(freed + s, turn ^ 1, abort_flag, peek))) break;
           peek = s + 1 < NA ? mbar_test(freed + s + 1, turn ^ 1) : mbar_test(freed, turn);
           if (one) {
-            uint64_t* bar = L::T1 && !PAIR ? ready + s : full_a + s;
+            uint64_t* bar = L::T1 ? ready + s : full_a + s;
             mbar_expect_tx(bar, uint32_t(box_rows(p.M) * L::BK * 4));
             tma_load_2d(ring_a + s * L::kA, &map_a, bar, kb * TBK, m0);
           }
@@ -722,7 +723,7 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1)
         if (lane == 0) mbar_arrive(ready + sp);
       }
     }
-  } else if (!L::T1 || PAIR) {
+  } else if (!L::T1) {
     if (L::kMoveRegs) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(L::kRegsConv));
     // A lane owns a row at a time: 16-byte chunk c of row r sits at chunk c ^ (r & 7) of its 128 bytes, so the eight lanes of
     // a quarter warp touch eight different 16-byte columns on the reads and on the writes. The parts go back as chunks 0-3
@@ -748,7 +749,7 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1)
 #pragma unroll
         for (int j = 0; j < 4 / WPG; ++j) {
           const int r = (first + j * WPG) * 32 + lane;
-          if (L::T1 || m0 + r - lane >= p.M) break;  // rows past the matrix: whatever their products are, nobody reads them
+          if (m0 + r - lane >= p.M) break;  // rows past the matrix: whatever their products are, nobody reads them
           if (L::T2) {  // the slab is h; l goes beside it at the same place
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
@@ -1082,9 +1083,14 @@ void dispatch_format(Stream& st, const GemmArgs& a, const PackedB& w) {
     case FMT_F16X2: return dispatch_width<EPI, FMT_F16X2>(st, a, w);
     case FMT_F16: return dispatch_width<EPI, FMT_F16>(st, a, w);
     case FMT_BF16: return dispatch_width<EPI, FMT_BF16>(st, a, w);
-    case FMT_TF32X2: return dispatch_width<EPI, FMT_TF32X2>(st, a, w);
-    default: return dispatch_width<EPI, FMT_TF32>(st, a, w);
+    default: break;
   }
+  // the tf32 formats: the forward of wide models (Model::put_mat)
+  if constexpr (EPI != EPI_SILU_BWD && EPI != EPI_SWIGLU_BWD) {
+    if (w.fmt == FMT_TF32X2) return dispatch_width<EPI, FMT_TF32X2>(st, a, w);
+    if (w.fmt == FMT_TF32) return dispatch_width<EPI, FMT_TF32>(st, a, w);
+  }
+  throw Error(3, "gemm: no kernel for this operand format and epilogue");
 }
 
 }  // namespace

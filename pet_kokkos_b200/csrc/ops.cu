@@ -56,9 +56,21 @@ __global__ void k_compress0(GemmArgs p) {
   const size_t t = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
   const int D4 = p.N / 4;
   if (t >= size_t(p.M) * D4) return;
-  const float zero[4] = {0.f, 0.f, 0.f, 0.f};
-  const float m = epilogue_run4<EPI_COMPRESS>(p, int(t / D4), int(t % D4) * 4, zero);
-  raise_row(p.c_max, int(t / D4), D4, m);
+  const size_t row = t / D4;
+  const int col = int(t % D4) * 4;
+  const float4 b = ld4(p.bias + col), tt = ld4(p.tab + size_t(p.sp[row]) * p.N + col);
+  const float e0 = (float) p.vec[3 * row], e1 = (float) p.vec[3 * row + 1], e2 = (float) p.vec[3 * row + 2], e3 = (float) p.dist[row];
+  float z[4] = {b.x, b.y, b.z, b.w};
+  const float from_table[4] = {tt.x, tt.y, tt.z, tt.w};
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float4 w = ld4(p.wx + size_t(col + j) * 4);
+    z[j] = z[j] + from_table[j] + w.x * e0 + w.y * e1 + w.z * e2 + w.w * e3;
+  }
+  st4(p.pre + row * p.ldp + col, make_float4(z[0], z[1], z[2], z[3]));
+  const float4 o = make_float4(silu_f(z[0]), silu_f(z[1]), silu_f(z[2]), silu_f(z[3]));
+  st4(p.C + row * p.ldc + col, o);
+  raise_row(p.c_max, int(row), D4, max_abs4(o.x, o.y, o.z, o.w));
 }
 
 // One warp per row. x = in (+ add, stored back); out = (x - mu) inv w + b.
@@ -648,7 +660,6 @@ __global__ void __launch_bounds__(256) k_fold_forces(ForceOut out, PackedEdges p
   }
 }
 
-// One warp per (structure, component): lane l sums every 32nd atom from the l-th, then a fixed tree.
 // out[b T + t] = the sum over structure b's atoms of x[a T + t]. A block per sum, whose warps' parts are added in order: a
 // warp alone takes 12 us for 1728 atoms, one trip to L2 after another.
 __global__ void __launch_bounds__(256) k_struct_sum(double* __restrict__ out, const double* __restrict__ x, const int* __restrict__ soff, int T) {

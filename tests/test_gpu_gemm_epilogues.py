@@ -137,3 +137,11 @@ def test_large_negative_values_do_not_pass_the_gate(calc):
     bias = np.array([-1e38, -3e38, -1e30, 0.0], np.float32)
     C = calc.debug_gemm(np.zeros((2, 4), np.float32), np.zeros((4, 4), np.float32), "f16x3", "silu", bias=bias)[0]
     assert (C == 0.0).all()
+
+
+def test_what_no_kernel_takes_is_refused(calc):
+    """The backward epilogues are never packed in the tf32 formats: asked for, they fail by name."""
+    for fmt in ("tf32", "tf32x2"):
+        for epi, wide in (("silu_bwd", 1), ("swiglu_bwd", 2)):
+            with pytest.raises(Exception, match="no kernel for this operand format"):
+                calc.debug_gemm(np.ones((70, 8)), np.ones((32, 8)), fmt, epi, pre=np.zeros((70, 32 * wide)))
