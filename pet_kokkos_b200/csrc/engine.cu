@@ -537,9 +537,10 @@ void Engine::run_model(const PackedEdges& pk, bool forces) {
     }
   bool seen = false;
   for (auto& k : graph_seen) seen = seen || k == key;
-  // A full cache gives up the recording used least recently, if that is long ago. Otherwise the shapes in turn outnumber the
-  // cache, each would be recorded (which costs several passes' launches) only to be dropped before it is used, and the pass
-  // runs eagerly instead: 18 shapes in turn against a cache of eight made a step of the 24-structure relaxation 2.4 ms for 1.9.
+  // A full cache gives up the recording used least recently, if that is long ago. Where the shapes in turn outnumber the cache,
+  // each would otherwise be recorded only to be dropped before it has paid (kGraphs); the pass runs eagerly instead, and the
+  // recordings there are go on serving. `graph_seen` tells up to 2 kGraphs shapes in turn from new ones, so a recording of such a
+  // turn is never older than that many passes: twice that long unused, it belongs to something the program has left.
   size_t lru = 0;
   for (size_t i = 1; i < graph_cache.size(); ++i)
     if (graph_cache[i].stamp < graph_cache[lru].stamp) lru = i;

@@ -153,7 +153,11 @@ struct Engine {
     long long launches = 0;
     uint64_t stamp = 0;
   };
-  static constexpr size_t kGraphs = 32;  // recordings kept, a few hundred launches each
+  // Recordings kept, 160 to 360 launches each. Making one takes 0.3 to 0.6 ms more than an eager pass, a replay takes 0.05 to
+  // 0.12 ms less (21 to 648 atoms): it pays from about six replays on. Each holds under 1 MB of device memory, so the bound is
+  // not memory's: a program that comes back to its shapes has tens of them (the structures of an ensemble, the pieces of a
+  // batch), and one whose shapes never repeat should not gather recordings that it will not use.
+  static constexpr size_t kGraphs = 32;
   std::vector<GraphEntry> graph_cache;
   std::vector<std::vector<uint64_t>> graph_seen;
   uint64_t graph_clock = 0;
