@@ -52,12 +52,12 @@ os.environ.setdefault("OMP_WAIT_POLICY", "passive")
 METRIC = "atom_evals_per_s"
 UNIT = "atom-evals/s"
 # DRAM traffic of one weight-GEMM launch per token row (atoms + kept edges), from one ncu capture:
-# dram__bytes_read.sum + dram__bytes_write.sum averaged over seven consecutive k_gemm_tc launches of the water648
-# workload, token-row and atom-row GEMMs as they come (50.2 MB at 25 320 rows; the capture is summarised under profiles/).
-# Captured with the kernel as of commit 002f4a5; the mainloop has been re-profiled since on one 122 138-row launch
-# (201 MB, 1646 B per row for a plain 256 x 256 GEMM: the same "A once, C once"), so the figure stands.
-# A GEMM reads A once and writes C once, so it grows with the rows.
-GEMM_DRAM_BYTES_PER_TOKEN_ROW = 50.2e6 / 25320
+# dram__bytes_read.sum + dram__bytes_write.sum averaged over the 86 k_gemm_tc launches of one evaluation of the water648
+# workload in the 3xTF32 mode, token-row and atom-row GEMMs as they come (47.6 MB at 25 320 rows;
+# profiles/gemm_launches_water648_s_3xtf32.md). A GEMM reads A once and writes C once, so it grows with the rows.
+GEMM_DRAM_BYTES_PER_TOKEN_ROW = 47.6e6 / 25320
+# products of 16-bit parts that one product of the mode takes on the tensor cores
+PRODUCTS_OF = {"native": 6, "3xtf32": 3, "tf32": 1, "bf16": 1}
 DTYPE_OF = {"native": "f32", "tf32": "tf32", "bf16": "bf16", "3xtf32": "f32 (3xTF32)"}
 MODEL_OF = {"diamond64": "xs", "water648": "s", "diamond1728": "s", "batch512x64": "s", "diamond13824": "l"}
 
@@ -581,15 +581,14 @@ def run_ours(args):
                         "peak": peaks["bf16_tflops_sustained"], "unit": "TFLOP/s", "frac": ach / peaks["bf16_tflops_sustained"],
                         "peak_source": f"{peaks['source']} cuBLAS bf16, sustained",
                         "traffic": GEMM_DRAM_BYTES_PER_TOKEN_ROW * (n_act + n_edges),
-                        "traffic_source": "ncu dram bytes per launch on water648 (capture of commit 002f4a5, summarised under profiles/), "
+                        "traffic_source": "ncu dram bytes per launch on water648 (profiles/gemm_launches_water648_s_3xtf32.md), "
                                           "scaled by token rows",
                         "launches": p["launches"], "avg_launch_ms": per_launch_ms}
-                # what the mode asks of the tensor cores: an fp32-accurate product is three tf32 MMAs, and tf32 runs at
-                # half the bf16 rate, so the algorithmic ceiling of this mode is a sixth of the bf16 peak
-                passes = {"3xtf32": 3, "tf32": 1, "bf16": 1}.get(args.gemm)
-                if passes:
-                    roof["mma_tflops"] = passes * ach
-                    roof["mode_ceiling_frac_of_peak"] = 0.5 / passes
+                # what the mode asks of the tensor cores: so many products of 16-bit parts for one of its own, at the bf16 rate
+                # (the forward of a model wider than 256 runs in the 3xTF32 and tf32 modes on tf32 instructions, at half of it)
+                passes = PRODUCTS_OF[args.gemm]
+                roof["mma_tflops"] = passes * ach
+                roof["mode_ceiling_frac_of_peak"] = 1.0 / passes
             else:
                 ach = p["bytes"] / (p["ms"] * 1e-3) / 1e9
                 roof = {"kernel": top, "bound": "hbm", "achieved": ach, "peak": peaks["hbm_gbs"], "unit": "GB/s",
