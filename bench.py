@@ -54,7 +54,7 @@ UNIT = "atom-evals/s"
 # DRAM traffic of one weight-GEMM launch per token row (atoms + kept edges), from one ncu capture:
 # dram__bytes_read.sum + dram__bytes_write.sum averaged over the 86 k_gemm_tc launches of one evaluation of the water648
 # workload in the 3xTF32 mode, token-row and atom-row GEMMs as they come (47.6 MB at 25 320 rows;
-# profiles/gemm_launches_water648_s_3xtf32.md). A GEMM reads A once and writes C once, so it grows with the rows.
+# summarised under profiles/). A GEMM reads A once and writes C once, so it grows with the rows.
 GEMM_DRAM_BYTES_PER_TOKEN_ROW = 47.6e6 / 25320
 # products of 16-bit parts that one product of the mode takes on the tensor cores
 PRODUCTS_OF = {"native": 6, "3xtf32": 3, "tf32": 1, "bf16": 1}
@@ -581,7 +581,7 @@ def run_ours(args):
                         "peak": peaks["bf16_tflops_sustained"], "unit": "TFLOP/s", "frac": ach / peaks["bf16_tflops_sustained"],
                         "peak_source": f"{peaks['source']} cuBLAS bf16, sustained",
                         "traffic": GEMM_DRAM_BYTES_PER_TOKEN_ROW * (n_act + n_edges),
-                        "traffic_source": "ncu dram bytes per launch on water648 (profiles/gemm_launches_water648_s_3xtf32.md), "
+                        "traffic_source": "ncu dram bytes per launch on water648 (summarised under profiles/), "
                                           "scaled by token rows",
                         "launches": p["launches"], "avg_launch_ms": per_launch_ms}
                 # what the mode asks of the tensor cores: so many products of 16-bit parts for one of its own, at the bf16 rate

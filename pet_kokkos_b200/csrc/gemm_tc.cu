@@ -7,7 +7,8 @@
 //   warp 0      producer of A: one lane issues TMA loads of 128 x 32 fp32 slabs (128-byte rows, 128-byte swizzle) into a
 //               ring of slots; warp 2 the same for B's tiles, which arrive as 16-bit parts;
 //   warps 12-15 converter: a lane takes one row's 128 bytes out of a landed slot, scales and splits it and writes the
-//               parts back into the same 128 bytes (64 bytes a part; FMT_F16X3's third part into a tile of its own): a slot costs no second copy of A. The fp32 activations are read from memory once;
+//               parts back into the same 128 bytes (64 bytes a part; FMT_F16X3's third part into a tile of its own): a slot costs
+//               no second copy of A. The fp32 activations are read from memory once;
 //   warp 1      issuer: one lane issues the products (M = 128, N = BN, K = 16 each) into one of TWO accumulators in
 //               tensor memory, small terms first, and frees the step's slots with one tcgen05.commit;
 //   warps 4-11  epilogue: tcgen05.ld the accumulator (a thread owns a row, a warp pair splits the columns), undo the
@@ -18,7 +19,8 @@
 // registers, rounding once, and hand them back before they start on the chunks. The tensor core truncates its fp32
 // accumulator at every instruction: on sums with more bits than it keeps that is a bias toward zero which adds up over K
 // and over a network (two truncations per 32 columns were enough to move energies by 1e-6). The h.h sums have no such
-// bits, and the small products' truncations are 2^-8 of what they would be there. setmaxnreg moves the registers the sums
+// bits, and the small products' truncations are 2^-8 of what they would be there (where most values have a leading part:
+// FMT_F16X3_FULL in gemm.h). setmaxnreg moves the registers the sums
 // take from the producers' and converters' warp groups.
 // Large GEMMs in the formats of several parts run on pairs of CTAs (cta_group::2): 256 x 256 tiles, each CTA with 128 rows of
 // A and half of the weight's tile in its shared memory, its own converter and epilogue, one issuer for both. A CTA's
@@ -35,11 +37,13 @@
 // recorded pass, FMT_F16X2: N 1024 K 4096 64.7 us -> 47.1, N 256 K 1024 18.3 -> 14.2, N 1024 K 256 7.7 -> 7.1; FMT_F16X3,
 // 21 rows, N 512 K 2048: 35.0 -> 27.4.
 //
-// What bounds the large ones: the SM's shared-memory data path (one 128-byte wavefront per clock for TMA traffic, the tensor core's
-// operand reads, the converter and the epilogue). Wavefronts per 8 columns of K of a 128 x 256 tile, K = 256: FMT_F16X2
-// operand reads 144, fills 96, converter 64, epilogue 64-128 = about 370-430 against 192 clocks of MMA; FMT_F16X3 288, 128,
-// 80, 64-128 = about 560-620 against 384. The 3xTF32 split it replaces (two tf32 parts, three products) took 610-640 for
-// the same tile, and fp32 FMAs 1024 clocks.
+// What bounds the large ones: no unit is at its rate. Counters of 122138 x 256 x 256 in three, two and one parts: tensor pipe
+// active 69, 53 and 21 % of the active cycles, SM memory throughput 60, 45 and 18 %, DRAM 29, 43 and 50 %, issue slots 50, 39 and
+// 42 %; in a fifth of the elapsed cycles no SM is active. The most work falls on the shared-memory data path (one 128-byte
+// wavefront per clock for TMA traffic, the tensor core's operand reads, the converter and the epilogue). Wavefronts per 8
+// columns of K of a 128 x 256 tile, K = 256, by count: FMT_F16X2 operand reads 144, fills 96, converter 64, epilogue 64-128 =
+// about 370-430 against 192 clocks of MMA; FMT_F16X3 288, 128, 80, 64-128 = about 560-620 against 384. A step's chain of
+// barriers, and an epilogue that has the one accumulator of 256 columns to itself, leave each of them idle in between.
 // No TMA load here uses cluster multicast. Every wait is bounded: a wait that runs out sets an error word the host checks,
 // every role then leaves its loop, and the CTA still reaches its tensor-memory release.
 #include <cuda_bf16.h>

@@ -73,8 +73,8 @@ def test_pairs_of_blocks_give_the_bits_of_one_block(calc, fmt):
 @pytest.mark.parametrize("mode", ["3xtf32", "tf32", "bf16"])
 def test_token_row_gemm_of_the_benchmark(calc, mode):
     """The most frequent GEMM of the 1728-atom benchmark at its full size (atoms + kept edges = 122 138 rows, d_pet 256
-    in and out), in every tensor-core mode, against the fp64 product. profiles/k_gemm_tc_122k_256_256.md is an ncu capture
-    of this test."""
+    in and out), in every tensor-core mode, against the fp64 product (an ncu capture of it is
+    summarised under profiles/)."""
     m, n, k = 122138, 256, 256
     rng = np.random.default_rng(0)
     A = rng.normal(size=(m, k)).astype(np.float32)
