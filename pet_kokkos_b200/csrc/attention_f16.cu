@@ -300,8 +300,8 @@ __global__ void __launch_bounds__(32 * MAXB, MAXB <= 5 ? resident<HD, P, 3>(16 *
   const int S16 = round16(cnt), nb = S16 / 16, SM = round16(p.S);
   uint8_t *sq = smem, *sk = sq + SM * pitch<HD, P>(), *sv = sk + SM * pitch<HD, P>();
   float* slc = reinterpret_cast<float*>(sv + SM * pitch<HD, P>());
-  // Staging: a thread's loads of U rows' pieces are all under way before it looks at any. A head size of 64 takes two rounds of
-  // them, the second fetched again for the split.
+  // Staging: a thread's loads of U rows' pieces are under way while it sees to the cutoffs; then it looks for the tile's largest
+  // values, also among the pieces it takes later (a head size of 64: read here, and again for the split).
   constexpr int Q = HD / 4, U = 4;
   float4 x0[U], x1[U], x2[U];
   auto fetch = [&](int t0) {
@@ -312,22 +312,23 @@ __global__ void __launch_bounds__(32 * MAXB, MAXB <= 5 ? resident<HD, P, 3>(16 *
       x0[u] = get(p.qkv, at, r < cnt), x1[u] = get(p.qkv, at + D, r < cnt), x2[u] = get(p.qkv, at + 2 * D, r < cnt);
     }
   };
+  fetch(threadIdx.x);
   if (threadIdx.x < 3) s_max[threadIdx.x] = 0;
-  __syncthreads();
-  {
-    float mq = 0.f, mk = 0.f, mv = 0.f;
-    int t0 = threadIdx.x;
-    while (t0 + U * blockDim.x < S16 * Q) t0 += U * blockDim.x;  // the first round last: it stays in the registers
-    for (; t0 >= 0; t0 -= U * blockDim.x) {
-      fetch(t0);
-#pragma unroll
-      for (int u = 0; u < U; ++u) mq = max_abs(mq, x0[u]), mk = max_abs(mk, x1[u]), mv = max_abs(mv, x2[u]);
-    }
-    raise_tile(s_max, mq), raise_tile(s_max + 1, mk), raise_tile(s_max + 2, mv);
-  }
   for (int r = threadIdx.x; r < S16; r += blockDim.x) {
     const float cf = r == 0 ? 1.0f : (r < cnt ? p.cut[e0 + r - 1] : 0.f);
     slc[r] = cf > 0.f ? __logf(cf) * kLog2e : kOff;
+  }
+  __syncthreads();
+  {
+    float mq = 0.f, mk = 0.f, mv = 0.f;
+    for (int t = threadIdx.x + U * blockDim.x; t < cnt * Q; t += blockDim.x) {
+      const int r = t / Q;
+      const size_t at = (r == 0 ? size_t(n) : size_t(p.N) + e0 + r - 1) * 3 * D + h * HD + (t % Q) * 4;
+      mq = max_abs(mq, get(p.qkv, at, true)), mk = max_abs(mk, get(p.qkv, at + D, true)), mv = max_abs(mv, get(p.qkv, at + 2 * D, true));
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) mq = max_abs(mq, x0[u]), mk = max_abs(mk, x1[u]), mv = max_abs(mv, x2[u]);
+    raise_tile(s_max, mq), raise_tile(s_max + 1, mk), raise_tile(s_max + 2, mv);
   }
   __syncthreads();
   const float scq = scale_of(s_max[0]), sck = scale_of(s_max[1]), scv = scale_of(s_max[2]);
@@ -437,20 +438,9 @@ __global__ void __launch_bounds__(MAXT, BLOCKS) k_attn_bwd_f16(AttnArgs p) {
       x3[u] = get(p.dmerged, ag, r < cnt), x4[u] = get(p.merged, ag, r < cnt);
     }
   };
+  fetch(threadIdx.x);
   if (threadIdx.x < 4) s_max[threadIdx.x] = 0;
   if (threadIdx.x == 0) s_vnorm = s_gnorm = 0;
-  __syncthreads();
-  {
-    float mq = 0.f, mk = 0.f, mv = 0.f, mg = 0.f;
-    int t0 = threadIdx.x;
-    while (t0 + U * blockDim.x < S16 * Q) t0 += U * blockDim.x;  // the first round last: it stays in the registers
-    for (; t0 >= 0; t0 -= U * blockDim.x) {
-      fetch(t0);
-#pragma unroll
-      for (int u = 0; u < U; ++u) mq = max_abs(mq, x0[u]), mk = max_abs(mk, x1[u]), mv = max_abs(mv, x2[u]), mg = max_abs(mg, x3[u]);
-    }
-    raise_tile(s_max, mq), raise_tile(s_max + 1, mk), raise_tile(s_max + 2, mv), raise_tile(s_max + 3, mg);
-  }
   for (int r = threadIdx.x; r < S16; r += blockDim.x) {
     float lc = kOff, m = 1e30f, il = 0.f;
     if (r < cnt) {
@@ -462,6 +452,19 @@ __global__ void __launch_bounds__(MAXT, BLOCKS) k_attn_bwd_f16(AttnArgs p) {
       if (il > 0.f) m = ml.x * kLog2e;  // a dead query's weights are exp(-1e30) = 0
     }
     slc[r] = lc, sm[r] = m, sl[r] = il * 32768.f;
+  }
+  __syncthreads();
+  {
+    float mq = 0.f, mk = 0.f, mv = 0.f, mg = 0.f;
+    for (int t = threadIdx.x + U * blockDim.x; t < cnt * Q; t += blockDim.x) {
+      const int r = t / Q;
+      const size_t row = r == 0 ? size_t(n) : size_t(p.N) + e0 + r - 1, at = row * 3 * D + h * HD + (t % Q) * 4;
+      mq = max_abs(mq, get(p.qkv, at, true)), mk = max_abs(mk, get(p.qkv, at + D, true)), mv = max_abs(mv, get(p.qkv, at + 2 * D, true));
+      mg = max_abs(mg, get(p.dmerged, row * D + h * HD + (t % Q) * 4, true));
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) mq = max_abs(mq, x0[u]), mk = max_abs(mk, x1[u]), mv = max_abs(mv, x2[u]), mg = max_abs(mg, x3[u]);
+    raise_tile(s_max, mq), raise_tile(s_max + 1, mk), raise_tile(s_max + 2, mv), raise_tile(s_max + 3, mg);
   }
   __syncthreads();
   const float scq = scale_of(s_max[0]), sck = scale_of(s_max[1]), scv = scale_of(s_max[2]), scg = scale_of(s_max[3]);
