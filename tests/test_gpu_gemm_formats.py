@@ -1,4 +1,4 @@
-"""The tensor-core GEMM at the edges of its tiles, in every operand format, against the fp64 product.
+"""The tensor-core GEMM at the edges of its tiles, in every mode, against the fp64 product.
 
 Rows: one, both sides of the 64 below which every mode runs in the native format, both sides of a 128-row tile, a ragged
 third tile, more tiles than SMs (several per block). Columns: the least, both sides of a column tile's width of 64, 128 and 256, several tiles. Contraction: less than
