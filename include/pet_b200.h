@@ -355,6 +355,9 @@ typedef struct pet_debug_gemm_args {
   float* row_max;          /* [m], optional: each row's largest |C| as the epilogue keeps it */
 } pet_debug_gemm_args;
 int pet_debug_gemm(pet_calc* c, const pet_debug_gemm_args* args);
+/* Two of one format, args[0] and args[1], handed over together as the atoms' and the edges' GEMM of a step are: one launch
+ * where that is the faster way (testing aid). */
+int pet_debug_gemm_two(pet_calc* c, const pet_debug_gemm_args* args);
 
 /* A ready-made pet_exchange over NCCL: what an MD engine's pair style does around pet::Exchange
  * (lammps/ML-PET/pair_pet.cpp:268-360 routing, :396-472 exchange_rows, :479-555 set_live / edges), inside the

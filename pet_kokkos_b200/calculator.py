@@ -172,6 +172,7 @@ SIGNATURES = {
     "pet_gemm_host_static": (C.c_int, [C.c_int, C.c_int, C.c_int, _P(C.c_float), _P(C.c_float), _P(C.c_float), C.c_char_p,
                                        C.c_size_t]),
     "pet_debug_gemm": (C.c_int, [C.c_void_p, _P(PetDebugGemmArgs)]),
+    "pet_debug_gemm_two": (C.c_int, [C.c_void_p, _P(PetDebugGemmArgs)]),
     "pet_gemm_host": (C.c_int, [C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, _P(C.c_float), _P(C.c_float),
                                 _P(C.c_float)]),
 }
@@ -677,6 +678,19 @@ class Calculator:
     def debug_gemm(self, A, W, fmt, epilogue="plain", w_transposed=True, bias=None, res=None, res_row0=0, pre=None, tab=None,
                    species=None, wx=None, vec=None, dist=None, want_pre=True):
         """One weight GEMM with an epilogue in one operand format: (C, pre as written or None, row maxima of C)."""
+        g, keep, results = self._debug_gemm_args(A, W, fmt, epilogue, w_transposed, bias, res, res_row0, pre, tab, species, wx, vec, dist,
+                                                 want_pre)
+        self._check(self._lib.pet_debug_gemm(self._h, C.byref(g)))
+        return results
+
+    def debug_gemm_two(self, first, second):
+        """Two of them handed over together, each a dict of debug_gemm's arguments."""
+        given = [self._debug_gemm_args(**first), self._debug_gemm_args(**second)]
+        self._check(self._lib.pet_debug_gemm_two(self._h, (PetDebugGemmArgs * 2)(given[0][0], given[1][0])))
+        return given[0][2], given[1][2]
+
+    def _debug_gemm_args(self, A, W, fmt, epilogue="plain", w_transposed=True, bias=None, res=None, res_row0=0, pre=None, tab=None,
+                         species=None, wx=None, vec=None, dist=None, want_pre=True):
         g, keep = PetDebugGemmArgs(), []
 
         def ptr(x, dtype, pt):
@@ -702,5 +716,4 @@ class Calculator:
             g.pre = written.ctypes.data_as(C.POINTER(C.c_float))
         row_max = np.zeros(m, np.float32)
         g.C, g.row_max = out.ctypes.data_as(C.POINTER(C.c_float)), row_max.ctypes.data_as(C.POINTER(C.c_float))
-        self._check(self._lib.pet_debug_gemm(self._h, C.byref(g)))
-        return out, written, row_max
+        return g, keep, (out, written, row_max)

@@ -265,7 +265,14 @@ int pet_gemm_host(pet_calc* c, int mode, int w_transposed, int m, int n, int k, 
 int pet_debug_gemm(pet_calc* c, const pet_debug_gemm_args* args) {
   return guarded(c, [&](Engine& e) {
     if (!args || args->format < 0 || args->format > petb::FMT_F16X3_FULL) throw petb::Error(PET_ERR_INVALID, "pet: bad GEMM arguments");
-    e.gemm_on_host_arrays(*args, args->format, args->format);
+    e.gemm_on_host_arrays(args, 1, args->format, args->format);
+  });
+}
+int pet_debug_gemm_two(pet_calc* c, const pet_debug_gemm_args* args) {
+  return guarded(c, [&](Engine& e) {
+    if (!args || args->format < 0 || args->format > petb::FMT_F16X3_FULL || args[1].format != args->format)
+      throw petb::Error(PET_ERR_INVALID, "pet: bad GEMM arguments");
+    e.gemm_on_host_arrays(args, 2, args->format, args->format);
   });
 }
 

@@ -1397,11 +1397,31 @@ void Engine::debug_fetch(const char* name, float* out, size_t capacity, size_t* 
 void Engine::gemm_host(int mode, bool w_transposed, int m, int n, int k, const float* A, const float* W, float* C) {
   pet_debug_gemm_args g{};
   g.w_transposed = w_transposed, g.m = m, g.n = n, g.k = k, g.A = A, g.W = W, g.C = C;
-  gemm_on_host_arrays(g, FMT_F16X3, format_of(mode));
+  gemm_on_host_arrays(&g, 1, FMT_F16X3, format_of(mode));
 }
 
-void Engine::gemm_on_host_arrays(const pet_debug_gemm_args& g, int native_format, int fast_format) {
+// One GEMM, or two as gemm_two runs them.
+void Engine::gemm_on_host_arrays(const pet_debug_gemm_args* g, int count, int native_format, int fast_format) {
   PETB_CUDA(cudaSetDevice(device));
+  PETB_CUDA(cudaStreamSynchronize(st.s));
+  tmp_arena.reset();
+  GemmArgs a[2];
+  for (int i = 0; i < count; ++i) a[i] = gemm_from_host_arrays(g[i], native_format, fast_format);
+  if (count == 1) gemm(st, tmp_arena, a[0]);
+  else gemm_two(st, tmp_arena, a[0], a[1]);
+  for (int i = 0; i < count; ++i) {
+    const size_t m = a[i].M;
+    const bool reads_pre = g[i].epilogue == EPI_SILU_BWD || g[i].epilogue == EPI_SWIGLU_BWD;
+    PETB_CUDA(cudaMemcpyAsync(g[i].C, a[i].C, 4 * m * a[i].ldc, cudaMemcpyDeviceToHost, st.s));
+    if (g[i].pre && !reads_pre) PETB_CUDA(cudaMemcpyAsync(g[i].pre, a[i].pre, 4 * m * a[i].ldp, cudaMemcpyDeviceToHost, st.s));
+    if (g[i].row_max) PETB_CUDA(cudaMemcpyAsync(g[i].row_max, a[i].c_max, 4 * m, cudaMemcpyDeviceToHost, st.s));
+  }
+  gemm_tensor_error_ask(st, pinned + kGaveUp);
+  PETB_CUDA(cudaStreamSynchronize(st.s));
+  if (gemm_tensor_error(st, pinned + kGaveUp)) throw Error(5, "pet: a tensor-core GEMM gave up waiting on its pipeline");
+}
+
+GemmArgs Engine::gemm_from_host_arrays(const pet_debug_gemm_args& g, int native_format, int fast_format) {
   const size_t m = g.m, n = g.n, k = g.k;
   const bool reads_pre = g.epilogue == EPI_SILU_BWD || g.epilogue == EPI_SWIGLU_BWD, compress = g.epilogue == EPI_COMPRESS;
   if (g.m <= 0 || g.n <= 0 || g.k <= 0 || !g.A || !g.W || !g.C || (reads_pre && !g.pre) ||
@@ -1410,8 +1430,6 @@ void Engine::gemm_on_host_arrays(const pet_debug_gemm_args& g, int native_format
   if (compress)
     for (size_t i = 0; i < m; ++i)
       if (g.species[i] < 0 || g.species[i] >= g.n_tab) throw Error(2, "pet: bad GEMM arguments");
-  PETB_CUDA(cudaStreamSynchronize(st.s));
-  tmp_arena.reset();
   auto up = [&](const auto* from, size_t count) {
     using T = std::remove_const_t<std::remove_pointer_t<decltype(from)>>;
     if (!from) return static_cast<T*>(nullptr);
@@ -1423,8 +1441,8 @@ void Engine::gemm_on_host_arrays(const pet_debug_gemm_args& g, int native_format
   a.M = g.m, a.N = g.n, a.K = g.k, a.epi = g.epilogue;
   a.lda = a.K, a.ldc = g.epilogue == EPI_SWIGLU ? a.N / 2 : g.epilogue == EPI_SWIGLU_BWD ? 2 * a.N : a.N;
   a.ldr = a.N, a.ldp = g.epilogue == EPI_SWIGLU_BWD ? 2 * a.N : a.N;
-  const size_t c_size = m * size_t(a.ldc), pre_size = m * size_t(a.ldp);
-  float* dC = tmp_arena.alloc<float>(c_size);
+  const size_t pre_size = m * size_t(a.ldp);
+  float* dC = tmp_arena.alloc<float>(m * size_t(a.ldc));
   const float* dW = up(g.W, n * k);
   a.A = up(g.A, m * k), a.C = dC, a.bias = up(g.bias, n), a.res = up(g.res, m * n), a.res_row0 = g.res_row0;
   a.pre = reads_pre ? up(g.pre, pre_size) : g.pre ? tmp_arena.alloc<float>(pre_size) : nullptr;
@@ -1445,13 +1463,7 @@ void Engine::gemm_on_host_arrays(const pet_debug_gemm_args& g, int native_format
     return w;
   };
   a.nat = pack(native_format), a.fast = pack(fast_format);
-  gemm(st, tmp_arena, a);
-  PETB_CUDA(cudaMemcpyAsync(g.C, dC, 4 * c_size, cudaMemcpyDeviceToHost, st.s));
-  if (g.pre && !reads_pre) PETB_CUDA(cudaMemcpyAsync(g.pre, a.pre, 4 * pre_size, cudaMemcpyDeviceToHost, st.s));
-  if (g.row_max) PETB_CUDA(cudaMemcpyAsync(g.row_max, a.c_max, 4 * m, cudaMemcpyDeviceToHost, st.s));
-  gemm_tensor_error_ask(st, pinned + kGaveUp);
-  PETB_CUDA(cudaStreamSynchronize(st.s));
-  if (gemm_tensor_error(st, pinned + kGaveUp)) throw Error(5, "pet: a tensor-core GEMM gave up waiting on its pipeline");
+  return a;
 }
 
 }  // namespace petb

@@ -86,7 +86,8 @@ struct Engine {
                      pet_device_results* out);
   void debug_fetch(const char* name, float* out, size_t capacity, size_t* n);
   void gemm_host(int mode, bool w_transposed, int m, int n, int k, const float* A, const float* W, float* C);
-  void gemm_on_host_arrays(const pet_debug_gemm_args& g, int native_format, int fast_format);
+  void gemm_on_host_arrays(const pet_debug_gemm_args* g, int count, int native_format, int fast_format);
+  GemmArgs gemm_from_host_arrays(const pet_debug_gemm_args& g, int native_format, int fast_format);
 
   int species_index(int Z) const;
 

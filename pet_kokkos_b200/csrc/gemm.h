@@ -9,13 +9,13 @@
 // (src/ops.cpp:326-365).
 //
 // Two kernel families:
-//   * tensor (gemm_tc.cu): tcgen05.mma kind::f16 with TMA-fed shared-memory tiles and the accumulator in tensor memory.
+//   * tensor (gemm_tc.cuh): tcgen05.mma kind::f16 with TMA-fed shared-memory tiles and the accumulator in tensor memory.
 //     Operands wider than 16 bits are split into 16-bit parts whose products are summed in fp32; the formats below say
 //     into which, for each mode;
 //   * fp32 FMA on the CUDA cores (gemm_simt.cu): one accumulation chain per output in k order, the plain product, for callers
 //     without a packed weight (pet_gemm_host_static).
 // In the native format and on the CUDA cores a row's bits depend on that row and the weight alone, not on how many rows share
-// its launch. The other formats add a long K in another order where few rows leave SMs for it (plan_split, gemm_tc.cu).
+// its launch. The other formats add a long K in another order where few rows leave SMs for it (plan_split, gemm_tc.cuh).
 #pragma once
 
 #include "common.h"
@@ -122,6 +122,9 @@ struct GemmArgs {
 
 // Runs the GEMM in the format of `fast`, or of `nat` where it has fewer than 64 rows.
 void gemm(Stream& st, Arena& arena, const GemmArgs& a);
+// Two that do not depend on each other and share no output, as one launch where that is the faster way (plan_two, gemm_tc.cuh);
+// `a` the one of fewer rows and longer contraction.
+void gemm_two(Stream& st, Arena& arena, const GemmArgs& a, const GemmArgs& b);
 
 // out[M] = A[M,K] . w[K] + b (a one-column linear layer), one warp per row.
 void gemv_rows(Stream& st, const float* A, int lda, const float* w, const float* bias, float* out, int M, int K);

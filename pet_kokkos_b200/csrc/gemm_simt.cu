@@ -8,10 +8,11 @@
 // weight has no packed form (pet_gemm_host_static): with the weight's parts at hand
 // the tensor cores are four times faster and no less exact.
 #include "epilogue.cuh"
+#include "gemm_tc.h"
 
 namespace petb {
 
-void gemm_tensor(Stream& st, Arena& arena, const GemmArgs& a, const PackedB& w);  // gemm_tc.cu
+void gemm_tensor(Stream& st, Arena& arena, const GemmTask* q, int n);  // gemm_tc.cu
 bool gemm_tensor_usable(const Stream& st, const GemmArgs& a, const PackedB& w);
 
 namespace {
@@ -126,25 +127,51 @@ __global__ void k_gemv_rows(const float* __restrict__ A, int lda, const float* _
 
 }  // namespace
 
-void gemm(Stream& st, Arena& arena, const GemmArgs& a) {
-  if (a.M <= 0 || a.N <= 0) return;
+namespace {
+
+void check(const GemmArgs& a) {
   if (a.N % 4 || a.K % 4 || a.lda % 4 || (a.B && a.ldb % 4) || a.ldc % 2)
     throw Error(2, "gemm: widths must be multiples of 4 (N=" + std::to_string(a.N) + ", K=" + std::to_string(a.K) + ")");
-  // Algorithmic work: 2MNK flops; A, B, C once each, plus what the epilogue reads and writes.
+}
+// Algorithmic work: 2MNK flops; A, B, C once each, plus what the epilogue reads and writes.
+double flops_of(const GemmArgs& a) { return 2.0 * a.M * a.N * a.K; }
+double bytes_of(const GemmArgs& a) {
   double bytes = 4.0 * (double(a.M) * a.K + double(a.N) * a.K + double(a.M) * a.N);
   if (a.res) bytes += 4.0 * a.M * a.N;
   if (a.pre) bytes += 4.0 * a.M * a.N * (a.epi == EPI_SWIGLU_BWD ? 2.0 : 1.0);
   if (a.epi == EPI_SWIGLU) bytes -= 2.0 * a.M * a.N;      // h is half as wide as the product
   if (a.epi == EPI_SWIGLU_BWD) bytes += 4.0 * a.M * a.N;  // pre_adj is twice as wide
-  const ProfScope ps(st, PC_GEMM, 2.0 * a.M * a.N * a.K, bytes);
-  // Fewer than half a tile of rows: the speed modes' products would not be felt there, so they run at full precision.
-  const PackedB& w = a.M < 64 || a.N < 32 ? a.nat : a.fast;
-  if (gemm_tensor_usable(st, a, w)) return gemm_tensor(st, arena, a, w);
+  return bytes;
+}
+// Fewer than half a tile of rows: the speed modes' products would not be felt there, so they run at full precision.
+const PackedB& weight_of(const GemmArgs& a) { return a.M < 64 || a.N < 32 ? a.nat : a.fast; }
+
+}  // namespace
+
+void gemm(Stream& st, Arena& arena, const GemmArgs& a) {
+  if (a.M <= 0 || a.N <= 0) return;
+  check(a);
+  const ProfScope ps(st, PC_GEMM, flops_of(a), bytes_of(a));
+  const GemmTask q{a, weight_of(a)};
+  if (gemm_tensor_usable(st, a, q.w)) return gemm_tensor(st, arena, &q, 1);
   if (!a.B) throw Error(3, "gemm: this weight has no fp32 copy for the CUDA cores");
   if (a.epi != EPI_PLAIN || a.bias || a.res || a.c_max) throw Error(3, "gemm: the CUDA cores give the plain product alone");
   const long long tiles = (long long) cdiv(a.M, BM) * cdiv(a.N, BN);
   launch(st, k_gemm_native, (unsigned) tiles, 256, 0, a);
   PETB_LAUNCH_CHECK(st);
+}
+
+void gemm_two(Stream& st, Arena& arena, const GemmArgs& a, const GemmArgs& b) {
+  const bool one_launch = a.M > 0 && b.M > 0 && a.N > 0 && b.N > 0 && a.epi == b.epi && weight_of(a).fmt == weight_of(b).fmt &&
+                          gemm_tensor_usable(st, a, weight_of(a)) && gemm_tensor_usable(st, b, weight_of(b));
+  if (!one_launch) {
+    gemm(st, arena, a);
+    return gemm(st, arena, b);
+  }
+  check(a), check(b);
+  const ProfScope ps(st, PC_GEMM, flops_of(a) + flops_of(b), bytes_of(a) + bytes_of(b));
+  const GemmTask q[2] = {{a, weight_of(a)}, {b, weight_of(b)}};
+  gemm_tensor(st, arena, q, 2);
 }
 
 void gemv_rows(Stream& st, const float* A, int lda, const float* w, const float* bias, float* out, int M, int K) {

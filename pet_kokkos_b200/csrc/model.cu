@@ -330,41 +330,57 @@ struct Gemms {
     return a;
   }
   // out[M, W.rows] = in[M, W.cols] . W^T + bias (+ res for rows >= res_row0)
-  void linear(const Rows& out, const Rows& in, const Mat& W, const float* bias, int M, const float* res = nullptr,
-              int res_row0 = 0) const {
+  static GemmArgs linear_args(const Rows& out, const Rows& in, const Mat& W, const float* bias, int M, const float* res = nullptr,
+                              int res_row0 = 0) {
     GemmArgs a = args(out, in, W, false, M);
     a.bias = bias, a.res = res, a.res_row0 = res_row0;
-    gemm(st, tmp, a);
+    return a;
   }
   // out = silu(pre), pre = in . W^T + bias, kept when `pre` is given
-  void linear_silu(const Rows& out, float* pre, const Rows& in, const Mat& W, const float* bias, int M) const {
+  static GemmArgs silu_args(const Rows& out, float* pre, const Rows& in, const Mat& W, const float* bias, int M) {
     GemmArgs a = args(out, in, W, false, M);
     a.bias = bias, a.pre = pre, a.epi = EPI_SILU;
-    gemm(st, tmp, a);
+    return a;
   }
   // pre[M, 2F] = in . W^T + bias (interleaved v, g); h[M, F] = v * sigmoid(g)
-  void swiglu_in(const Rows& h, float* pre, const Rows& in, const Mat& W, const float* bias, int M) const {
+  static GemmArgs swiglu_args(const Rows& h, float* pre, const Rows& in, const Mat& W, const float* bias, int M) {
     GemmArgs a = args(h, in, W, false, M);
     a.ldc = W.rows / 2, a.bias = bias, a.pre = pre, a.epi = EPI_SWIGLU;
-    gemm(st, tmp, a);
+    return a;
   }
   // in_adj[M, W.cols] (+)= out_adj[M, W.rows] . W
-  void linear_bwd(const Rows& in_adj, const Rows& out_adj, const Mat& W, int M, bool acc) const {
+  static GemmArgs linear_bwd_args(const Rows& in_adj, const Rows& out_adj, const Mat& W, int M, bool acc) {
     GemmArgs a = args(in_adj, out_adj, W, true, M);
     a.res = acc ? in_adj.p : nullptr;
-    gemm(st, tmp, a);
+    return a;
   }
   // grad[M, W.cols] = (out_adj . W) * silu'(pre)
-  void linear_silu_bwd(const Rows& grad, const Rows& out_adj, const Mat& W, const float* pre, int M) const {
+  static GemmArgs silu_bwd_args(const Rows& grad, const Rows& out_adj, const Mat& W, const float* pre, int M) {
     GemmArgs a = args(grad, out_adj, W, true, M);
     a.pre = const_cast<float*>(pre), a.epi = EPI_SILU_BWD;
-    gemm(st, tmp, a);
+    return a;
   }
   // pre_adj[M, 2F] from h_adj = out_adj . W_out and the saved pre
-  void swiglu_out_bwd(const Rows& pre_adj, const Rows& out_adj, const Mat& w_out, const float* pre, int M) const {
+  static GemmArgs swiglu_bwd_args(const Rows& pre_adj, const Rows& out_adj, const Mat& w_out, const float* pre, int M) {
     GemmArgs a = args(pre_adj, out_adj, w_out, true, M);
     a.ldc = a.ldp = 2 * w_out.cols, a.pre = const_cast<float*>(pre), a.epi = EPI_SWIGLU_BWD;
-    gemm(st, tmp, a);
+    return a;
+  }
+  void one(const GemmArgs& a) const { gemm(st, tmp, a); }
+  // The atoms' GEMM and the edges' of one step.
+  void two(const GemmArgs& atoms, const GemmArgs& edges) const { gemm_two(st, tmp, atoms, edges); }
+  void linear(const Rows& out, const Rows& in, const Mat& W, const float* bias, int M, const float* res = nullptr, int res_row0 = 0) const {
+    one(linear_args(out, in, W, bias, M, res, res_row0));
+  }
+  void linear_silu(const Rows& out, float* pre, const Rows& in, const Mat& W, const float* bias, int M) const {
+    one(silu_args(out, pre, in, W, bias, M));
+  }
+  void swiglu_in(const Rows& h, float* pre, const Rows& in, const Mat& W, const float* bias, int M) const {
+    one(swiglu_args(h, pre, in, W, bias, M));
+  }
+  void linear_bwd(const Rows& in_adj, const Rows& out_adj, const Mat& W, int M, bool acc) const { one(linear_bwd_args(in_adj, out_adj, W, M, acc)); }
+  void linear_silu_bwd(const Rows& grad, const Rows& out_adj, const Mat& W, const float* pre, int M) const {
+    one(silu_bwd_args(grad, out_adj, W, pre, M));
   }
   // act = silu(pre), pre = in . W_in^T + b + tab[species] + wx . (v, |v|): compress.0 past the first layer
   void compress(const Rows& act, float* pre, const Rows& in, const Mat& W, const float* b, const Mat& tab, const Mat& x4,
@@ -464,7 +480,7 @@ MemoryNeed Model::memory_need(int tier, int N, int E, int n_live) const {
   // tmp: the fullest scope
   const double attention_bwd = T * (5 * D + H) + (keep ? 0.0 : T * 4 * D);
   const double attention_fwd = T * D + (keep ? 0.0 : T * 3 * D);
-  const double edge_mlp = c * (2 * F + D) + (keep ? c * F : c * (2 * F + D));
+  const double edge_mlp = c * (2 * F + D) + (keep ? c * F : c * (2 * F + D)) + n * 5 * Dn;  // (beside the atoms')
   const double combination = e * 4 * D + 2 * live * D;
   const double heads = 2 * n * Dh + 2 * e * Dh;
   double tmp = std::max(std::max(attention_bwd, attention_fwd), std::max(std::max(edge_mlp, combination), heads));
@@ -536,7 +552,7 @@ PassOut Model::run_feedforward(Stream& st, Arena& save, Arena& tmp, const Packed
   auto edge_mlp_in = [&](const Rows& he, float* pre, const float* eps_rows, const std::string& tl, int nr) {
     const Rows edge_norm = maxima.fresh(tmp.alloc<float>(size_t(nr) * D), nr);
     norm_fwd(st, edge_norm.p, const_cast<float*>(eps_rows), nullptr, vec(tl + ".norm_mlp.weight"), nullptr, nr, D, edge_norm.mx);
-    gm.swiglu_in(he, pre, edge_norm, mat(tl + ".mlp.w_in.weight"), vec(tl + ".mlp.w_in.bias"), nr);
+    return Gemms::swiglu_args(he, pre, edge_norm, mat(tl + ".mlp.w_in.weight"), vec(tl + ".mlp.w_in.bias"), nr);
   };
 
   // One message-passing layer forward: node_in [N,Dn] -> node_out, input_edge [E,D] updated in place, saves in `sl`
@@ -551,6 +567,10 @@ PassOut Model::run_feedforward(Stream& st, Arena& save, Arena& tmp, const Packed
     std::vector<float*> tokbuf(A + 1);
     for (int a = 0; a <= A; ++a) tokbuf[a] = save.alloc<float>(Ta * D);
     sl.cpre = save.alloc<float>(Ea * D);
+    const auto contraction = [&](int a, const Rows& node) {  // block a's atom tokens
+      const std::string tl = g + ".trans.layers." + std::to_string(a);
+      return Gemms::linear_args({tokbuf[a]}, node, mat(tl + ".center_contraction.weight"), vec(tl + ".center_contraction.bias"), N);
+    };
     {
       Scope s0(tmp);
       const Rows cact = maxima.fresh(tmp.alloc<float>(Ea * D), Ea);
@@ -559,7 +579,8 @@ PassOut Model::run_feedforward(Stream& st, Arena& save, Arena& tmp, const Packed
       } else {
         gm.compress(cact, sl.cpre, input_edge, mat(c0 + "@in"), vec(c0 + "@b"), mat(c0 + "@tab"), mat(c0 + "@x4"), pk);
       }
-      gm.linear({tokbuf[0] + size_t(N) * D}, cact, mat(g + ".compress.2.weight"), vec(g + ".compress.2.bias"), E);
+      gm.two(contraction(0, node_in), Gemms::linear_args({tokbuf[0] + size_t(N) * D}, cact, mat(g + ".compress.2.weight"),
+                                                         vec(g + ".compress.2.bias"), E));
     }
     tap(taps, "et" + ls, tokbuf[0] + size_t(N) * D, size_t(E) * D);
 
@@ -580,7 +601,7 @@ PassOut Model::run_feedforward(Stream& st, Arena& save, Arena& tmp, const Packed
       if (a + 1 == A) node_out = node_next;
       float* edge_next = tokbuf[a + 1] + size_t(N) * D;
 
-      gm.linear({b.tok}, node_cur, mat(tl + ".center_contraction.weight"), vec(tl + ".center_contraction.bias"), N);
+      if (a > 0) gm.one(contraction(a, node_cur));
       {
         Scope s1(tmp);
         const Rows qkv = keep ? b.qkv : Rows{tmp.alloc<float>(Ta * 3 * D)};
@@ -595,24 +616,33 @@ PassOut Model::run_feedforward(Stream& st, Arena& save, Arena& tmp, const Packed
                 b.tok, N);
       // node_res = node_cur + expansion(atom rows of attn_out)
       gm.linear({b.node_res}, b.eps, mat(tl + ".center_expansion.weight"), vec(tl + ".center_expansion.bias"), N, node_cur.p, 0);
-      {
-        Scope s2(tmp);
-        const Rows node_norm = maxima.fresh(tmp.alloc<float>(Na * Dn), Na);
-        const Rows hc = maxima.fresh(tmp.alloc<float>(Na * (w_cin.rows / 2)), Na);
-        norm_fwd(st, node_norm.p, b.node_res, nullptr, vec(tl + ".norm_center_features.weight"), nullptr, N, Dn, node_norm.mx);
-        gm.swiglu_in(hc, b.pre_c, node_norm, w_cin, vec(tl + ".center_mlp.w_in.bias"), N);
-        gm.linear(node_next, hc, mat(tl + ".center_mlp.w_out.weight"), vec(tl + ".center_mlp.w_out.bias"), N, b.node_res, 0);
-      }
+      // the atoms' MLP, and the edges' a chunk at a time: the first chunk's GEMMs share their launches with the atoms'
+      Scope s2(tmp);
+      const Rows node_norm = maxima.fresh(tmp.alloc<float>(Na * Dn), Na);
+      const Rows hc = maxima.fresh(tmp.alloc<float>(Na * (w_cin.rows / 2)), Na);
+      norm_fwd(st, node_norm.p, b.node_res, nullptr, vec(tl + ".norm_center_features.weight"), nullptr, N, Dn, node_norm.mx);
+      const GemmArgs node_in_args = Gemms::swiglu_args(hc, b.pre_c, node_norm, w_cin, vec(tl + ".center_mlp.w_in.bias"), N);
+      const GemmArgs node_out_args =
+          Gemms::linear_args(node_next, hc, mat(tl + ".center_mlp.w_out.weight"), vec(tl + ".center_mlp.w_out.bias"), N, b.node_res, 0);
       const int rows = keep || chunk <= 0 ? (E > 0 ? E : 1) : chunk;
-      for (int r0 = 0; r0 < E; r0 += rows) {
+      int r0 = 0;
+      do {
         const int nr = std::min(rows, E - r0);
         Scope s3(tmp);
         float* eps_rows = b.eps.p + (size_t(N) + r0) * D;
         const Rows he = maxima.fresh(tmp.alloc<float>(size_t(nr) * (w_ein.rows / 2)), nr);
         float* pre = keep ? b.pre_e + size_t(r0) * w_ein.rows : tmp.alloc<float>(size_t(nr) * w_ein.rows);
-        edge_mlp_in(he, pre, eps_rows, tl, nr);
-        gm.linear({edge_next + size_t(r0) * D}, he, mat(tl + ".mlp.w_out.weight"), vec(tl + ".mlp.w_out.bias"), nr, eps_rows, 0);
-      }
+        const GemmArgs edge_in_args = edge_mlp_in(he, pre, eps_rows, tl, nr);
+        const GemmArgs edge_out_args = Gemms::linear_args({edge_next + size_t(r0) * D}, he, mat(tl + ".mlp.w_out.weight"),
+                                                          vec(tl + ".mlp.w_out.bias"), nr, eps_rows, 0);
+        if (r0 == 0) {
+          gm.two(node_in_args, edge_in_args);
+          gm.two(node_out_args, edge_out_args);
+        } else {
+          gm.one(edge_in_args), gm.one(edge_out_args);
+        }
+        r0 += rows;
+      } while (r0 < E);
       node_cur = node_next;
       tap(taps, "node" + tag, node_cur.p, size_t(N) * Dn);
       tap(taps, "edge" + tag, edge_next, size_t(E) * D);
@@ -680,12 +710,12 @@ PassOut Model::run_feedforward(Stream& st, Arena& save, Arena& tmp, const Packed
     const Rows nh0 = maxima.fresh(tmp.alloc<float>(Na * Dh), Na), eh0 = maxima.fresh(tmp.alloc<float>(Ea * Dh), Ea);
     float* nh1 = tmp.alloc<float>(Na * Dh);
     float* eh1 = tmp.alloc<float>(Ea * Dh);
-    gm.linear_silu(nh0, nh0_pre, node, mat("node_heads.energy.0.0.weight"), vec("node_heads.energy.0.0.bias"), N);
-    gm.linear_silu({nh1}, nh1_pre, nh0, mat("node_heads.energy.0.2.weight"), vec("node_heads.energy.0.2.bias"), N);
+    gm.two(Gemms::silu_args(nh0, nh0_pre, node, mat("node_heads.energy.0.0.weight"), vec("node_heads.energy.0.0.bias"), N),
+           Gemms::silu_args(eh0, eh0_pre, input_edge, mat("edge_heads.energy.0.0.weight"), vec("edge_heads.energy.0.0.bias"), E));
+    gm.two(Gemms::silu_args({nh1}, nh1_pre, nh0, mat("node_heads.energy.0.2.weight"), vec("node_heads.energy.0.2.bias"), N),
+           Gemms::silu_args({eh1}, eh1_pre, eh0, mat("edge_heads.energy.0.2.weight"), vec("edge_heads.energy.0.2.bias"), E));
     gemv_rows(st, nh1, Dh, mat("node_last_layers.energy.0.energy___0.weight").w, vec("node_last_layers.energy.0.energy___0.bias"),
               node_pred, N, Dh);
-    gm.linear_silu(eh0, eh0_pre, input_edge, mat("edge_heads.energy.0.0.weight"), vec("edge_heads.energy.0.0.bias"), E);
-    gm.linear_silu({eh1}, eh1_pre, eh0, mat("edge_heads.energy.0.2.weight"), vec("edge_heads.energy.0.2.bias"), E);
     gemv_rows(st, eh1, Dh, mat("edge_last_layers.energy.0.energy___0.weight").w, vec("edge_last_layers.energy.0.energy___0.bias"),
               edge_pred, E, Dh);
   }
@@ -708,12 +738,12 @@ PassOut Model::run_feedforward(Stream& st, Arena& save, Arena& tmp, const Packed
     const Rows eh1_adj = maxima.fresh(tmp.alloc<float>(Ea * Dh), Ea), eh0_adj = maxima.fresh(tmp.alloc<float>(Ea * Dh), Ea);
     readout_seed_bwd(st, nh1_adj.p, mat("node_last_layers.energy.0.energy___0.weight").w, nh1_pre, nullptr, nullptr, pk.n_local, N, Dh,
                      nh1_adj.mx);
-    gm.linear_silu_bwd(nh0_adj, nh1_adj, mat("node_heads.energy.0.2.weight"), nh0_pre, N);
-    gm.linear_bwd(node_adj, nh0_adj, mat("node_heads.energy.0.0.weight"), N, false);
     readout_seed_bwd(st, eh1_adj.p, mat("edge_last_layers.energy.0.energy___0.weight").w, eh1_pre, pk.cut, pk.center, pk.n_local, E, Dh,
                      eh1_adj.mx);
-    gm.linear_silu_bwd(eh0_adj, eh1_adj, mat("edge_heads.energy.0.2.weight"), eh0_pre, E);
-    gm.linear_bwd(ie_adj, eh0_adj, mat("edge_heads.energy.0.0.weight"), E, false);
+    gm.two(Gemms::silu_bwd_args(nh0_adj, nh1_adj, mat("node_heads.energy.0.2.weight"), nh0_pre, N),
+           Gemms::silu_bwd_args(eh0_adj, eh1_adj, mat("edge_heads.energy.0.2.weight"), eh0_pre, E));
+    gm.two(Gemms::linear_bwd_args(node_adj, nh0_adj, mat("node_heads.energy.0.0.weight"), N, false),
+           Gemms::linear_bwd_args(ie_adj, eh0_adj, mat("edge_heads.energy.0.0.weight"), E, false));
   }
   // The adjoint of a layer's tokens is one buffer written again and again: each writer of its edge rows or of all of it
   // takes fresh maxima.
@@ -757,29 +787,37 @@ PassOut Model::run_feedforward(Stream& st, Arena& save, Arena& tmp, const Packed
       tok_adj.mx = maxima.take(Ta);
       const Rows eps_adj = tok_adj.from(N, D);   // the same rows once the MLP's backward has added to them
       const int rows = b.pre_e || chunk <= 0 ? (E > 0 ? E : 1) : chunk;
-      for (int r0 = 0; r0 < E; r0 += rows) {
-        const int nr = std::min(rows, E - r0);
-        Scope s8(tmp);
-        const float* eps_rows = b.eps.p + (size_t(N) + r0) * D;
-        const Rows adj_rows = edge_adj.from(r0, D);
-        const float* pre = b.pre_e ? b.pre_e + size_t(r0) * w_ein.rows : nullptr;
-        if (!pre) {  // the pre-activation was not kept: these rows' again
-          float* again_pre = tmp.alloc<float>(size_t(nr) * w_ein.rows);
-          edge_mlp_in({}, again_pre, eps_rows, tl, nr);
-          pre = again_pre;
-        }
-        const Rows pre_adj = maxima.fresh(tmp.alloc<float>(size_t(nr) * w_ein.rows), nr);
-        float* enorm_adj = tmp.alloc<float>(size_t(nr) * D);
-        gm.swiglu_out_bwd(pre_adj, adj_rows, mat(tl + ".mlp.w_out.weight"), pre, nr);
-        gm.linear_bwd({enorm_adj}, pre_adj, w_ein, nr, false);
-        norm_bwd(st, adj_rows.p, enorm_adj, eps_rows, vec(tl + ".norm_mlp.weight"), false, nr, D, 0, nullptr, eps_adj.from(r0, D).mx);
-      }
       {
         Scope s9(tmp);
         const Rows prec_adj = maxima.fresh(tmp.alloc<float>(Na * w_cin.rows), Na);
         float* cnorm_adj = tmp.alloc<float>(Na * Dn);
-        gm.swiglu_out_bwd(prec_adj, node_adj, mat(tl + ".center_mlp.w_out.weight"), b.pre_c, N);
-        gm.linear_bwd({cnorm_adj}, prec_adj, w_cin, N, false);
+        const GemmArgs node_out_args = Gemms::swiglu_bwd_args(prec_adj, node_adj, mat(tl + ".center_mlp.w_out.weight"), b.pre_c, N);
+        const GemmArgs node_in_args = Gemms::linear_bwd_args({cnorm_adj}, prec_adj, w_cin, N, false);
+        int r0 = 0;
+        do {
+          const int nr = std::min(rows, E - r0);
+          Scope s8(tmp);
+          const float* eps_rows = b.eps.p + (size_t(N) + r0) * D;
+          const Rows adj_rows = edge_adj.from(r0, D);
+          const float* pre = b.pre_e ? b.pre_e + size_t(r0) * w_ein.rows : nullptr;
+          if (!pre) {  // the pre-activation was not kept: these rows' again
+            float* again_pre = tmp.alloc<float>(size_t(nr) * w_ein.rows);
+            gm.one(edge_mlp_in({}, again_pre, eps_rows, tl, nr));
+            pre = again_pre;
+          }
+          const Rows pre_adj = maxima.fresh(tmp.alloc<float>(size_t(nr) * w_ein.rows), nr);
+          float* enorm_adj = tmp.alloc<float>(size_t(nr) * D);
+          const GemmArgs edge_out_args = Gemms::swiglu_bwd_args(pre_adj, adj_rows, mat(tl + ".mlp.w_out.weight"), pre, nr);
+          const GemmArgs edge_in_args = Gemms::linear_bwd_args({enorm_adj}, pre_adj, w_ein, nr, false);
+          if (r0 == 0) {
+            gm.two(node_out_args, edge_out_args);
+            gm.two(node_in_args, edge_in_args);
+          } else {
+            gm.one(edge_out_args), gm.one(edge_in_args);
+          }
+          norm_bwd(st, adj_rows.p, enorm_adj, eps_rows, vec(tl + ".norm_mlp.weight"), false, nr, D, 0, nullptr, eps_adj.from(r0, D).mx);
+          r0 += rows;
+        } while (r0 < E);
         node_adj.mx = maxima.take(Na);
         norm_bwd(st, node_adj.p, cnorm_adj, b.node_res, vec(tl + ".norm_center_features.weight"), false, N, Dn, 0, nullptr, node_adj.mx);
       }
@@ -915,11 +953,11 @@ PassOut Model::run_residual(Stream& st, Arena& save, Arena& tmp, const PackedEdg
       float* eh1 = tmp.alloc<float>(Ea * Dh);
       const std::string nh = "node_heads.energy." + ls, eh = "edge_heads.energy." + ls;
       const std::string nl = "node_last_layers.energy." + ls + ".energy___0", el = "edge_last_layers.energy." + ls + ".energy___0";
-      gm.linear_silu(nh0, sl.nh0_pre, tokens, mat(nh + ".0.weight"), vec(nh + ".0.bias"), N);
-      gm.linear_silu({nh1}, sl.nh1_pre, nh0, mat(nh + ".2.weight"), vec(nh + ".2.bias"), N);
+      gm.two(Gemms::silu_args(nh0, sl.nh0_pre, tokens, mat(nh + ".0.weight"), vec(nh + ".0.bias"), N),
+             Gemms::silu_args(eh0, sl.eh0_pre, tokens.from(N, D), mat(eh + ".0.weight"), vec(eh + ".0.bias"), E));
+      gm.two(Gemms::silu_args({nh1}, sl.nh1_pre, nh0, mat(nh + ".2.weight"), vec(nh + ".2.bias"), N),
+             Gemms::silu_args({eh1}, sl.eh1_pre, eh0, mat(eh + ".2.weight"), vec(eh + ".2.bias"), E));
       gemv_rows(st, nh1, Dh, mat(nl + ".weight").w, vec(nl + ".bias"), node_pred, N, Dh);
-      gm.linear_silu(eh0, sl.eh0_pre, tokens.from(N, D), mat(eh + ".0.weight"), vec(eh + ".0.bias"), E);
-      gm.linear_silu({eh1}, sl.eh1_pre, eh0, mat(eh + ".2.weight"), vec(eh + ".2.bias"), E);
       gemv_rows(st, eh1, Dh, mat(el + ".weight").w, vec(el + ".bias"), sl.edge_pred, E, Dh);
       readout_energy(st, net, per_atom, node_pred, sl.edge_pred, pk, comp_, scale_, L > 0, L + 1 == G);
       tap(taps, "node_pred" + ls, node_pred, N);
@@ -966,11 +1004,11 @@ PassOut Model::run_residual(Stream& st, Arena& save, Arena& tmp, const PackedEdg
       const std::string nh = "node_heads.energy." + ls, eh = "edge_heads.energy." + ls;
       const std::string nl = "node_last_layers.energy." + ls + ".energy___0", el = "edge_last_layers.energy." + ls + ".energy___0";
       readout_seed_bwd(st, nh1_adj.p, mat(nl + ".weight").w, sl.nh1_pre, nullptr, nullptr, pk.n_local, N, Dh, nh1_adj.mx);
-      gm.linear_silu_bwd(nh0_adj, nh1_adj, mat(nh + ".2.weight"), sl.nh0_pre, N);
-      gm.linear_bwd(tokens_adj, nh0_adj, mat(nh + ".0.weight"), N, false);
       readout_seed_bwd(st, eh1_adj.p, mat(el + ".weight").w, sl.eh1_pre, pk.cut, pk.center, pk.n_local, E, Dh, eh1_adj.mx);
-      gm.linear_silu_bwd(eh0_adj, eh1_adj, mat(eh + ".2.weight"), sl.eh0_pre, E);
-      gm.linear_bwd(tokens_adj.from(N, D), eh0_adj, mat(eh + ".0.weight"), E, false);
+      gm.two(Gemms::silu_bwd_args(nh0_adj, nh1_adj, mat(nh + ".2.weight"), sl.nh0_pre, N),
+             Gemms::silu_bwd_args(eh0_adj, eh1_adj, mat(eh + ".2.weight"), sl.eh0_pre, E));
+      gm.two(Gemms::linear_bwd_args(tokens_adj, nh0_adj, mat(nh + ".0.weight"), N, false),
+             Gemms::linear_bwd_args(tokens_adj.from(N, D), eh0_adj, mat(eh + ".0.weight"), E, false));
     }
     float* ie_next = ie_adj == ie_a ? ie_b : ie_a;
     if (L + 1 < G) {

@@ -83,7 +83,7 @@ __device__ __forceinline__ void store4_at(const void* p, uint32_t rank, float x,
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-// Arrives on the barrier at the same place in CTA `rank` of the cluster (the default, CTA-scope release: see gemm_tc.cu).
+// Arrives on the barrier at the same place in CTA `rank` of the cluster (the default, CTA-scope release: see gemm_tc.cuh).
 __device__ __forceinline__ void mbar_arrive_at(uint64_t* bar, uint32_t rank) {
   asm volatile(
       "{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %0, %1;\n\tmbarrier.arrive.shared::cluster.b64 _, [a];\n\t}" ::"r"(smem_u32(bar)),
