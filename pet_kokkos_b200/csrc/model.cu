@@ -66,6 +66,17 @@ __global__ void k_fold_species(const double* W, int K, const double* T, int ns, 
   tab[i] = acc;
 }
 
+// W = A . B and b = A . x + y, what two linear layers without anything between them come to. In fp64.
+__global__ void k_fold_layers(const double* A, const double* B, const double* x, const double* y, int rows, int inner, int cols, double* W, double* b) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= rows * (cols + 1)) return;
+  const int r = i / (cols + 1), c = i % (cols + 1);
+  double acc = c < cols ? 0.0 : y[r];
+  for (int j = 0; j < inner; ++j) acc += A[size_t(r) * inner + j] * (c < cols ? B[size_t(j) * cols + c] : x[j]);
+  if (c < cols) W[size_t(r) * cols + c] = acc;
+  else b[r] = acc;
+}
+
 // A tensor's doubles on the device for the duration of the load.
 struct Staged {
   double* p = nullptr;
@@ -83,7 +94,7 @@ struct Staged {
 };
 
 // What the network reads from a checkpoint, as (tensor name, how it is prepared).
-enum class Prep { Table, Matrix, Vector, PairedMatrix, PairedVector, CompressFold };  // Table: read row by row, never a GEMM operand
+enum class Prep { Table, Matrix, Vector, PairedMatrix, PairedVector, CompressFold, ExpansionFold };  // Table: read row by row, never a GEMM operand
 struct PlanItem {
   std::string name;
   Prep prep;
@@ -112,7 +123,8 @@ std::vector<PlanItem> weight_plan(const Hypers& h) {
       dense(block + ".mlp.w_in", paired);
       norm(block + ".norm_attention"), norm(block + ".norm_mlp");
       if (!h.expanded_node()) continue;
-      for (const char* part : {".center_contraction", ".center_expansion", ".center_mlp.w_out"}) dense(block + part);
+      for (const char* part : {".center_contraction", ".center_mlp.w_out"}) dense(block + part);
+      plan.push_back({block, Prep::ExpansionFold});
       dense(block + ".center_mlp.w_in", paired);
       norm(block + ".norm_center_features");
     }
@@ -212,6 +224,20 @@ void Model::fold_compress(const Checkpoint& ck, const std::string& c0, int L) {
   PETB_CUDA(cudaDeviceSynchronize());  // the staged tensors are freed on return
 }
 
+// A block's expansion of the atoms' rows of the attention's output, with the output layer before it: nothing else reads those rows.
+// "@expand" [d_node, d_pet], "@expand_b". Two GEMMs on the atoms' chain become one, beside the edges' output layer.
+void Model::fold_expansion(const Checkpoint& ck, const std::string& block) {
+  const Staged A(ck.at(block + ".center_expansion.weight")), y(ck.at(block + ".center_expansion.bias"));
+  const Staged B(ck.at(block + ".attention.output_linear.weight")), x(ck.at(block + ".attention.output_linear.bias"));
+  if (A.cols != B.rows) throw Error(1, "model: '" + block + ".center_expansion' does not have the shape of an expansion");
+  const Staged W(size_t(A.rows) * B.cols), b(size_t(A.rows));
+  k_fold_layers<<<cdiv((long long) A.rows * (B.cols + 1), 128), 128>>>(A.p, B.p, x.p, y.p, A.rows, A.cols, B.cols, W.p, b.p);
+  PETB_CUDA(cudaGetLastError());
+  put_mat(block + "@expand", W.p, B.cols, A.rows, B.cols, false, true);
+  put_vec(block + "@expand_b", b.p, A.rows, false);
+  PETB_CUDA(cudaDeviceSynchronize());  // the staged tensors are freed on return
+}
+
 Model::Model(const Checkpoint& ck, int gemm_mode) : h_(ck.hypers), scale_(ck.energy_scale), mode_(gemm_mode) {
   const bool ff = h_.feedforward, ln = h_.layernorm, expanded = h_.expanded_node(), swiglu = h_.swiglu;
 
@@ -228,6 +254,10 @@ Model::Model(const Checkpoint& ck, int gemm_mode) : h_(ck.hypers), scale_(ck.ene
   for (const PlanItem& it : weight_plan(h_)) {
     if (it.prep == Prep::CompressFold) {
       fold_compress(ck, it.name, it.layer);
+      continue;
+    }
+    if (it.prep == Prep::ExpansionFold) {
+      fold_expansion(ck, it.name);
       continue;
     }
     const Tensor& t = ck.at(it.name);
@@ -471,7 +501,7 @@ MemoryNeed Model::memory_need(int tier, int N, int E, int n_live) const {
   const double c = keep ? e : std::min(e, double(edge_chunk_rows(E)));
   // save: what lives for the whole pass
   double save = (G + 1) * n * Dn + e * D + G * live * D + (relayer ? G * e * D : 0.0);
-  const double block = T * (2 * D + 2 * H) + n * (Dn + 4 * Dn + Dn) + (keep ? T * 3 * D + e * 2 * F : 0.0);
+  const double block = T * (D + 2 * H) + e * D + n * (Dn + 4 * Dn + Dn) + (keep ? T * 3 * D + e * 2 * F : 0.0);
   const double layer = (A + 1) * T * D + e * 3 * D + A * block + (relayer ? n * Dn : 0.0);
   save += (relayer ? 1.0 : G) * layer;
   save += 2 * n * Dh + 2 * e * Dh + 2 * n + e + 2 * n;              // readout
@@ -526,8 +556,8 @@ PassOut Model::run_feedforward(Stream& st, Arena& save, Arena& tmp, const Packed
   RowMaxima maxima(st, save, row_maxima_words(N, E) * (relayer ? 2 : 1));  // a layer run again takes its own
 
   struct Block {
-    float *tok, *ml, *node_res, *pre_c, *pre_e;
-    Rows qkv, merged, eps;
+    float *tok, *ml, *eps, *node_res, *pre_c, *pre_e;
+    Rows qkv, merged;
   };
   struct Layer {
     float *cpre, *cph_pre, *out_edge;
@@ -592,7 +622,7 @@ PassOut Model::run_feedforward(Stream& st, Arena& save, Arena& tmp, const Packed
       b.tok = tokbuf[a];
       b.merged = maxima.fresh(save.alloc<float>(Ta * D), Ta);
       b.ml = save.alloc<float>(Ta * H * 2);
-      b.eps = maxima.fresh(save.alloc<float>(Ta * D), Ta);  // rows < N: the attention output's atom rows; rows >= N: eps
+      b.eps = save.alloc<float>(Ea * D);
       b.node_res = save.alloc<float>(Na * Dn);
       b.pre_c = save.alloc<float>(Na * w_cin.rows);
       b.qkv = keep ? Rows{save.alloc<float>(Ta * 3 * D)} : Rows{};
@@ -611,11 +641,10 @@ PassOut Model::run_feedforward(Stream& st, Arena& save, Arena& tmp, const Packed
         attention_forward(st, at);
       }
       tap(taps, "merged" + tag, b.merged.p, size_t(T) * D);
-      // attn_out = merged W_out^T + b; its edge rows take the residual: eps = attn_out + edge_cur.
-      gm.linear(b.eps, b.merged, mat(tl + ".attention.output_linear.weight"), vec(tl + ".attention.output_linear.bias"), T,
-                b.tok, N);
-      // node_res = node_cur + expansion(atom rows of attn_out)
-      gm.linear({b.node_res}, b.eps, mat(tl + ".center_expansion.weight"), vec(tl + ".center_expansion.bias"), N, node_cur.p, 0);
+      // eps = output layer(merged) + edge_cur on the edges' rows, node_res = expansion(output layer(merged)) + node_cur on the atoms'
+      gm.two(Gemms::linear_args({b.node_res}, b.merged, mat(tl + "@expand"), vec(tl + "@expand_b"), N, node_cur.p, 0),
+             Gemms::linear_args({b.eps}, b.merged.from(N, D), mat(tl + ".attention.output_linear.weight"),
+                                vec(tl + ".attention.output_linear.bias"), E, b.tok + size_t(N) * D, 0));
       // the atoms' MLP, and the edges' a chunk at a time: the first chunk's GEMMs share their launches with the atoms'
       Scope s2(tmp);
       const Rows node_norm = maxima.fresh(tmp.alloc<float>(Na * Dn), Na);
@@ -629,7 +658,7 @@ PassOut Model::run_feedforward(Stream& st, Arena& save, Arena& tmp, const Packed
       do {
         const int nr = std::min(rows, E - r0);
         Scope s3(tmp);
-        float* eps_rows = b.eps.p + (size_t(N) + r0) * D;
+        float* eps_rows = b.eps + size_t(r0) * D;
         const Rows he = maxima.fresh(tmp.alloc<float>(size_t(nr) * (w_ein.rows / 2)), nr);
         float* pre = keep ? b.pre_e + size_t(r0) * w_ein.rows : tmp.alloc<float>(size_t(nr) * w_ein.rows);
         const GemmArgs edge_in_args = edge_mlp_in(he, pre, eps_rows, tl, nr);
@@ -797,7 +826,7 @@ PassOut Model::run_feedforward(Stream& st, Arena& save, Arena& tmp, const Packed
         do {
           const int nr = std::min(rows, E - r0);
           Scope s8(tmp);
-          const float* eps_rows = b.eps.p + (size_t(N) + r0) * D;
+          const float* eps_rows = b.eps + size_t(r0) * D;
           const Rows adj_rows = edge_adj.from(r0, D);
           const float* pre = b.pre_e ? b.pre_e + size_t(r0) * w_ein.rows : nullptr;
           if (!pre) {  // the pre-activation was not kept: these rows' again
@@ -821,7 +850,7 @@ PassOut Model::run_feedforward(Stream& st, Arena& save, Arena& tmp, const Packed
         node_adj.mx = maxima.take(Na);
         norm_bwd(st, node_adj.p, cnorm_adj, b.node_res, vec(tl + ".norm_center_features.weight"), false, N, Dn, 0, nullptr, node_adj.mx);
       }
-      {  // attention: the output adjoint is [expansion's input adjoint ; eps adjoint] = tok_adj
+      {  // attention
         Scope s10(tmp);
         const Rows dmerged = Rows{tmp.alloc<float>(Ta * D)};
         const Rows qkv_adj = maxima.fresh(tmp.alloc<float>(Ta * 3 * D), Ta);
@@ -832,8 +861,8 @@ PassOut Model::run_feedforward(Stream& st, Arena& save, Arena& tmp, const Packed
           qkv = Rows{tmp.alloc<float>(Ta * 3 * D)};
           make_qkv(qkv, tl, b.tok);
         }
-        gm.linear_bwd(tok_adj, node_adj, mat(tl + ".center_expansion.weight"), N, false);
-        gm.linear_bwd(dmerged, tok_adj, mat(tl + ".attention.output_linear.weight"), T, false);
+        gm.two(Gemms::linear_bwd_args(dmerged, node_adj, mat(tl + "@expand"), N, false),
+               Gemms::linear_bwd_args(dmerged.from(N, D), eps_adj, mat(tl + ".attention.output_linear.weight"), E, false));
         AttnArgs at = attention_args(b, qkv);
         at.dmerged = dmerged.p, at.qkv_adj = qkv_adj.p, at.qkv_adj_max = qkv_adj.mx, at.cfh = cfh;
         attention_backward(st, at);

@@ -101,6 +101,7 @@ class Model {
   void put_mat(const std::string& name, const double* src, int ld, int rows, int cols, bool paired, bool operand);
   void put_vec(const std::string& name, const double* src, int len, bool paired);
   void fold_compress(const Checkpoint& ck, const std::string& c0, int layer);
+  void fold_expansion(const Checkpoint& ck, const std::string& block);
 
   bool wide() const { return h_.d_pet > 256; }  // the tensor-core modes' forward on tf32 instructions (put_mat)
 
