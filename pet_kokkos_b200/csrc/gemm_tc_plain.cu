@@ -1,4 +1,4 @@
-// The tensor-core GEMM with EPI_PLAIN.
+// The tensor-core GEMM with EPI_PLAIN, but for the formats of three parts.
 #include "gemm_tc.cuh"
 
 namespace petb {
