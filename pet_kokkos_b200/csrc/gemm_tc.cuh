@@ -133,7 +133,8 @@ struct Tile {
   static constexpr int kBars = 640;
   // Slots: as many as shared memory has room for beside the epilogue's buffers, at most eight of each; of A, whose bytes come
   // from HBM, no fewer than of B, whose bytes sit in L2; of A an even number, for the converter's groups.
-  static constexpr int kRoom = 227 * 1024 - kEpi - 1024 - kBars;
+  static constexpr int kRows = 2 * TBM * 4;  // a tile's rows' sums of squares, by group of the converter
+  static constexpr int kRoom = 227 * 1024 - kEpi - 1024 - kBars - kRows;
   static constexpr int least(int a, int b) { return a < b ? a : b; }
   static constexpr int slots_a(int nb) { return least(8, (kRoom - nb * kB) / kA); }
   static constexpr int kBoth = least(8, kRoom / (kA + kB));
@@ -149,7 +150,7 @@ struct Tile {
   // TA: a warp reaches only its quarter of tensor memory's lanes, so a group is four warps, and there are two of them.
   static constexpr int kGroups = !TA && NA % 4 == 0 && NA >= 8 ? 4 : 2;
   static constexpr int kRings = NA * kA + NB * kB;
-  static constexpr int kTotal = kRings + kEpi + 1024 /*alignment slack*/ + kBars;
+  static constexpr int kTotal = kRings + kEpi + 1024 /*alignment slack*/ + kBars + kRows;
   static constexpr int kThreads = TA ? 640 : 512;
   // registers of the tile's sums that an epilogue thread keeps over the steps (FMT_F16X3)
   static constexpr int kSums = X3 ? BN / 2 : 1;
@@ -169,7 +170,7 @@ struct Tile {
   static_assert(kRings >= TBM * BN * 4, "the shared sums of a split tile");
   static_assert((TA || NA >= NB) && NA >= 2 && NB >= 2 && NA % kGroups == 0, "the slots");
   static_assert(!TA || (NT >= NB && NT <= ND), "the slots");
-  static_assert((2 * NA + NS + ND + 4 + 2 * kEpiWarps) * 8 + 8 <= kBars, "the barriers");
+  static_assert((2 * NA + NS + ND + 6 + 2 * kEpiWarps) * 8 + 8 <= kBars, "the barriers");
 };
 
 // Rows of A's TMA box: a matrix of few rows has only its own fetched (a box's rows past the matrix cost as much as others).
@@ -328,7 +329,10 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1) k_gemm_tc(co
   uint64_t* tfull = empty_a + (L::TA ? NA : 0);    // [2] accumulator complete
   uint64_t* tempty = tfull + 2;     // [2] accumulator read back
   uint64_t* landed = tempty + 2;    // [kEpiWarps][2] an epilogue warp's chunk has landed
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(landed + 2 * kEpiWarps);
+  uint64_t* squares_there = landed + 2 * kEpiWarps;  // RMSNorm: a tile's rows' sums of squares are there,
+  uint64_t* squares_read = squares_there + 1;        // and have been read
+  float* squares = reinterpret_cast<float*>(epi + L::kEpi + L::kBars);  // [2][TBM]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(squares_read + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -365,9 +369,18 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1) k_gemm_tc(co
     return have;
   };
   constexpr int TBK = L::BK;
+  // RMSNorm before the product (GemmArgs::rms). The converter, which sees every value of a row, adds up its squares; the epilogue
+  // scales. 122138 rows, FMT_F16X2, norm and attention's input layer 169 us -> 143; the edges' SwiGLU 254 -> 260 with the atoms' tiles in
+  // it; and a launch of 4 us less on a small structure's chain. (Sums of squares left in memory by the GEMM before cost it 10-18 us
+  // and this one, which has to wait for them, 35-45.)
+  constexpr bool kNorms = (EPI == EPI_PLAIN || EPI == EPI_SWIGLU) && !SPLIT && (L::X3 || L::X2 || L::T2);
+  static_assert(!kNorms || L::kGroups == 2, "two sums a row");
   // SPLIT: parts divides the steps of K
   const auto steps = [&](const GemmArgs& p) { return (p.K + TBK - 1) / TBK / parts; };
 
+  // The maps on their way while the kernel before this one still runs: the first load through one waits for it.
+  if (warp == 3)
+    for (int i = lane; i < 6 * SIDES; i += 32) prefetch_map(&g.side[i / 6].map_a + i % 6);
   if (threadIdx.x == 0) {
     for (int s = 0; s < NA; ++s) mbar_init(full_a + s, CTAS);
     if (L::TA)
@@ -377,6 +390,7 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1) k_gemm_tc(co
     for (int s = 0; s < L::ND; ++s) mbar_init(done + s, 1);
     for (int b = 0; b < 2; ++b) mbar_init(tfull + b, 1), mbar_init(tempty + b, CTAS * kEpiWarps);
     for (int b = 0; b < 2 * kEpiWarps; ++b) mbar_init(landed + b, 1);
+    mbar_init(squares_there, L::TA ? 8 : 4), mbar_init(squares_read, kEpiWarps);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -387,6 +401,21 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1) k_gemm_tc(co
   tcgen05_fence_after();
   const uint32_t tmem = *tmem_slot;
   after_previous();
+
+  // A converter lane's squares of a row's 32 columns, added to what it has of the row; and the sums of a tile's rows handed over
+  // to the epilogue, by a warp for `n` rows a lane, `step` apart.
+  const auto add_squares = [](float* sq, const float4& v) {
+    asm("{ .reg .b64 s, a, b;\n\tmov.b64 s, {%0, %1};\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\t"
+        "fma.rn.f32x2 s, a, a, s;\n\tfma.rn.f32x2 s, b, b, s;\n\tmov.b64 {%0, %1}, s; }"
+        : "+f"(sq[0]), "+f"(sq[1]) : "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w));
+  };
+  const auto hand_over = [&](int norms, int group, int r, int step, const float (*sq)[2], int n) {
+    if (norms > 0 && !mbar_wait_warp(squares_read, (norms - 1) & 1, abort_flag)) return false;
+    for (int j = 0; j < n; ++j) squares[group * TBM + r + j * step] = sq[j][0] + sq[j][1];
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) mbar_arrive(squares_there);
+    return true;
+  };
 
   if (warp < 4) {
     if (L::kMoveRegs) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(L::kRegsProd));
@@ -575,7 +604,15 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1) k_gemm_tc(co
         else mbar_arrive(tempty + b);
       }
     };
-    int i = 0, k = 0;  // accumulators and chunks so far
+    int i = 0, k = 0, norms = 0;  // accumulators, chunks and tiles after a norm so far
+    const auto row_max = [&](int tile) {  // of this thread's row of a tile
+      At y;
+      if (!L::kScaled || !at(tile, y)) return 0u;
+      const GemmArgs& p = g.side[y.side].p;
+      return __ldg(p.a_max + min(y.row + q * 32 + lane, p.M - 1));
+    };
+    // asked for a tile ahead (FMT_F16X3, which has no register to spare, waits longer for its sums than for this)
+    uint32_t next_max = L::X3 ? 0 : row_max(0);
     bool ok = true;
     if (has_in && lane == 0) ask_first(0, 0);
     const auto finish = [&](const Side& sd, int tile, const At& x) {
@@ -596,10 +633,9 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1) k_gemm_tc(co
             if (c < nc && n0 + c * AC + 8 * j < p.N) u[j] = __ldg(reinterpret_cast<const uint4*>(sd.b_unscale + n0 + c * AC + 8 * j));
       };
       if (kAhead) ask_scales(c0);
-      float unscale = 1.f, big = 0.f;
+      float big = 0.f;
       RowTerms rt{};
       if (row < p.M) {
-        if (L::kScaled) unscale = unscale_of(p.a_max[row]);
         if (EPI == EPI_COMPRESS) {
           rt.tab = p.tab + size_t(p.sp[row]) * p.N;
           rt.e0 = (float) p.vec[3 * size_t(row)], rt.e1 = (float) p.vec[3 * size_t(row) + 1], rt.e2 = (float) p.vec[3 * size_t(row) + 2];
@@ -607,6 +643,13 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1) k_gemm_tc(co
         }
       } else if (EPI == EPI_COMPRESS) {
         rt.tab = p.tab;
+      }
+      float unscale = 1.f;
+      if (L::X3) {
+        if (row < p.M) unscale = unscale_of(p.a_max[row]);
+      } else {
+        if (L::kScaled) unscale = unscale_of(next_max);
+        next_max = row_max(tile + 1);
       }
       float sum[L::kSums];
       uint32_t acc = 0;
@@ -672,6 +715,14 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1) k_gemm_tc(co
         cluster_sync_all();
         if (!ok) return;
       }
+      if (kNorms && p.rms) {
+        if (!(ok = mbar_wait_warp(squares_there, norms & 1, abort_flag))) return;
+        // (a row's largest value over its root mean square lies in [1, sqrt K]: the product with its scale is a normal number)
+        unscale *= 1.0f / sqrtf((squares[q * 32 + lane] + squares[TBM + q * 32 + lane]) / p.K + kRmsEps);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(squares_read);
+        ++norms;
+      }
       // One copy of the chunk's code; FMT_F16X3 moves its sums down after each chunk: unrolled, the compiler keeps every
       // chunk's addresses alive beside the sums and spills.
 #pragma unroll 1
@@ -706,6 +757,9 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1) k_gemm_tc(co
               scale_pair(v[j + 2 * i], v[j + 2 * i + 1], two[i] << 16, two[i] & 0xFFFF0000u, unscale);
           }
           if (kAhead) ask_scales(c + CS);
+        } else if (kNorms && p.rms) {
+#pragma unroll
+          for (int j = 0; j < AC; ++j) v[j] *= unscale;
         }
         uint8_t* mine = buf + (k & 1) * L::kBuf;
         if (has_in) {
@@ -757,14 +811,24 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1) k_gemm_tc(co
     if (L::kMoveRegs) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(L::kRegsConv));
     // A lane owns one of its warp's quarter of the rows; the groups take every other step.
     const int quarter = warp & 3, group = (warp - kConvWarp0) >> 2;
-    int gone = 0;
+    int gone = 0, norms = 0;
     bool ok = true, peek = false;
+    const int r = quarter * 32 + lane;
+    const auto row_max = [&](int k) {
+      At y;
+      if (!L::kScaled || !at(k, y)) return 0u;
+      const GemmArgs& p = g.side[y.side].p;
+      return y.row + r < p.M ? __ldg(p.a_max + y.row + r) : 0u;
+    };
+    uint32_t next = row_max(0);  // asked for a tile ahead: HBM is a sixth of a tile's time away
     At x;
     for (int k = 0; ok && at(k, x); ++k) {
       const GemmArgs& p = g.side[x.side].p;
-      const int r = quarter * 32 + lane, row = x.row + r, kb0 = part * steps(p), kb1 = kb0 + steps(p);
+      const int row = x.row + r, kb0 = part * steps(p), kb1 = kb0 + steps(p);
       const bool live = row - lane < p.M;  // rows past the matrix: whatever their products are, nobody reads them
-      const float s = L::kScaled && row < p.M ? scale_of(p.a_max[row]) : 1.f;
+      const float s = L::kScaled ? scale_of(next) : 1.f;
+      next = row_max(k + 1);
+      float sq[1][2] = {{0.f, 0.f}};
       for (int kb = kb0; kb < kb1; ++kb, ++gone) {
         if ((gone & 1) != group) continue;
         const int sa = gone % NA, sp = gone % L::NS, before = gone - L::NS;
@@ -779,6 +843,7 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1) k_gemm_tc(co
           for (int c = 0; c < 8; ++c) v[c] = *reinterpret_cast<const float4*>(slab + swizzled<128>(r, c));
 #pragma unroll
           for (int c = 0; c < 8; ++c) {
+            if (kNorms && p.rms) add_squares(sq[0], v[c]);
             split2<FMT>(v[c].x, v[c].y, s, part[0][2 * c], part[1][2 * c], part[2][2 * c]);
             split2<FMT>(v[c].z, v[c].w, s, part[0][2 * c + 1], part[1][2 * c + 1], part[2][2 * c + 1]);
           }
@@ -797,6 +862,7 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1) k_gemm_tc(co
         __syncwarp();
         if (lane == 0) mbar_arrive(ready + sp);
       }
+      if (ok && kNorms && p.rms) ok = hand_over(norms++, group, r, 0, sq, 1);
     }
   } else if (!L::T1) {
     if (L::kMoveRegs) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(L::kRegsConv));
@@ -805,18 +871,28 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1) k_gemm_tc(co
     // (h) and 4-7 (m or l) of the same row; FMT_F16X3's l into rows of 64 bytes, chunk c at c ^ ((r >> 1) & 3).
     constexpr int WPG = 4 / L::kGroups;  // warps of a group
     const int cw = warp - kConvWarp0, group = cw / WPG, first = cw % WPG;
-    int gone = 0;
+    int gone = 0, norms = 0;
     bool ok = true, peek = false;
+    uint32_t next[4 / WPG];  // the rows' maxima, asked for a tile ahead
+    const auto row_max = [&](int k) {
+      At y;
+      const bool have = L::kScaled && at(k, y);
+#pragma unroll
+      for (int j = 0; j < 4 / WPG; ++j) {
+        const int row = have ? y.row + (first + j * WPG) * 32 + lane : 0;
+        next[j] = have && row < g.side[y.side].p.M ? __ldg(g.side[y.side].p.a_max + row) : 0;
+      }
+    };
+    row_max(0);
     At x;
     for (int k = 0; ok && at(k, x); ++k) {
       const GemmArgs& p = g.side[x.side].p;
       const int m0 = x.row, kb0 = part * steps(p), kb1 = kb0 + steps(p);
       float scale[4 / WPG];
 #pragma unroll
-      for (int j = 0; j < 4 / WPG; ++j) {
-        const int row = m0 + (first + j * WPG) * 32 + lane;
-        scale[j] = L::kScaled && row < p.M ? scale_of(p.a_max[row]) : 1.f;
-      }
+      for (int j = 0; j < 4 / WPG; ++j) scale[j] = L::kScaled ? scale_of(next[j]) : 1.f;
+      row_max(k + 1);
+      float sq[4 / WPG][2] = {};
       for (int kb = kb0; kb < kb1; ++kb, ++gone) {
         if (gone % L::kGroups != group) continue;
         const int sa = gone % NA;
@@ -831,6 +907,7 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1) k_gemm_tc(co
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
               const float4 v = *reinterpret_cast<const float4*>(slab + swizzled<64>(r, c));
+              if (kNorms && p.rms) add_squares(sq[j], v);
               *reinterpret_cast<float4*>(slab + L::kSlab + swizzled<64>(r, c)) =
                   make_float4(tf32_low(v.x), tf32_low(v.y), tf32_low(v.z), tf32_low(v.w));
             }
@@ -844,6 +921,7 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1) k_gemm_tc(co
           for (int c = 0; c < 4; ++c) {
             uint4 h, m, l;
             const float4 a = v[2 * c], b = v[2 * c + 1];
+            if (kNorms && p.rms) add_squares(sq[j], a), add_squares(sq[j], b);
             split2<FMT>(a.x, a.y, s, h.x, m.x, l.x), split2<FMT>(a.z, a.w, s, h.y, m.y, l.y);
             split2<FMT>(b.x, b.y, s, h.z, m.z, l.z), split2<FMT>(b.z, b.w, s, h.w, m.w, l.w);
             *reinterpret_cast<uint4*>(slab + swizzled<128>(r, c)) = h;
@@ -858,6 +936,7 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1) k_gemm_tc(co
           else mbar_arrive(ready + sa);
         }
       }
+      if (ok && kNorms && p.rms) ok = hand_over(norms++, group, first * 32 + lane, 32 * WPG, sq, 4 / WPG);
     }
   }
   if (SPLIT && (warp < kEpiWarp0 || warp >= kConvWarp0)) {
@@ -1019,7 +1098,7 @@ Plan plan_split(const GemmArgs& a, int bn_whole, int sms) {
   constexpr bool X3 = three_parts(FMT);
   const int steps = (a.K + 31) / 32, rows = cdiv(a.M, TBM);
   Plan best;
-  if (a.K < 1024 || a.K % 32 || a.N % 64) return best;
+  if (a.K < 1024 || a.K % 32 || a.N % 64 || a.rms) return best;
   if (rows * cdiv(a.N, bn_whole) > sms) return best;
   best.clocks = (long long) steps * step_clocks<FMT>(width_index(bn_whole));
   for (int i = 0; i < 3; ++i)
@@ -1109,7 +1188,7 @@ Plan plan_two(const GemmArgs& a, const GemmArgs& b, int sms) {
       if (X3 && (EPI == EPI_SWIGLU || EPI == EPI_SWIGLU_BWD)) most += most / 4;
       if (most < best.clocks) best.bn = bn, best.pair = pair, best.parts = 1, best.rounds = rounds, best.clocks = most;
     }
-    if (EPI != EPI_PLAIN || bn != 64 || a.K < 1024 || a.K % 32 || (X3 && b.K > 1024)) continue;
+    if (EPI != EPI_PLAIN || bn != 64 || a.K < 1024 || a.K % 32 || a.rms || b.rms || (X3 && b.K > 1024)) continue;
     for (int parts = 2; parts <= 8; parts *= 2) {  // side 0's tiles shared as plan_split would (few rows: narrow tiles)
       if (bn / parts < (X3 ? 16 : 32) || sa % parts || sa / parts < 4) continue;
       if (X3 && parts != (a.K <= 1024 ? 1 : a.K <= 4096 ? 4 : cdiv(a.K, 1024))) continue;
@@ -1160,6 +1239,9 @@ extern template void run_format<EPI_PLAIN, FMT_F16X3_FULL>(Stream&, const GemmTa
 
 template <int EPI>
 void run_tensor(Stream& st, const GemmTask* q, int n) {
+  for (int i = 0; i < n; ++i)
+    if (q[i].a.rms && ((EPI != EPI_PLAIN && EPI != EPI_SWIGLU) || (!three_parts(q[i].w.fmt) && q[i].w.fmt != FMT_F16X2 && q[i].w.fmt != FMT_TF32X2)))
+      throw Error(3, "gemm: no kernel for this operand format and epilogue after a norm");
   switch (q[0].w.fmt) {
     case FMT_F16X3: return run_format<EPI, FMT_F16X3>(st, q, n);
     case FMT_F16X3_FULL: return run_format<EPI, FMT_F16X3_FULL>(st, q, n);

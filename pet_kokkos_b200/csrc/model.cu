@@ -28,11 +28,13 @@ namespace {
 __device__ __forceinline__ int stored_row(int a, int rows, int paired) { return paired ? (a & 1) * (rows / 2) + (a >> 1) : a; }
 
 // src [rows, ld] doubles (the first `cols` columns of each row) -> [rows, cols] floats.
-__global__ void k_weight_rows(const double* src, int ld, int rows, int cols, int paired, float* out) {
+// Times gain[column], unless null.
+__global__ void k_weight_rows(const double* src, int ld, int rows, int cols, int paired, const double* gain, float* out) {
   const size_t n = size_t(rows) * cols, i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int a = int(i / cols), b = int(i % cols);
-  out[i] = float(src[size_t(stored_row(a, rows, paired)) * ld + b]);
+  const double x = src[size_t(stored_row(a, rows, paired)) * ld + b];
+  out[i] = float(gain ? x * gain[b] : x);
 }
 __global__ void k_weight_vector(const double* src, int len, int paired, float* out) {
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
@@ -99,18 +101,24 @@ struct PlanItem {
   std::string name;
   Prep prep;
   int layer = 0;
+  std::string gain;  // an RMSNorm's weight that the matrix takes with it: the norm before it is then the row's 1 / rms alone
 };
 
-std::vector<PlanItem> weight_plan(const Hypers& h) {
+std::vector<PlanItem> weight_plan(const Hypers& h, bool gains) {
   std::vector<PlanItem> plan;
   const bool ff = h.feedforward, paired = h.swiglu;
-  auto dense = [&](const std::string& stem, bool pair_rows = false) {
-    plan.push_back({stem + ".weight", pair_rows ? Prep::PairedMatrix : Prep::Matrix});
+  auto dense = [&](const std::string& stem, bool pair_rows = false, const std::string& gain = "") {
+    plan.push_back({stem + ".weight", pair_rows ? Prep::PairedMatrix : Prep::Matrix, 0, gain});
     plan.push_back({stem + ".bias", pair_rows ? Prep::PairedVector : Prep::Vector});
   };
   auto norm = [&](const std::string& stem) {
     plan.push_back({stem + ".weight", Prep::Vector});
     if (h.layernorm) plan.push_back({stem + ".bias", Prep::Vector});
+  };
+  // a layer and the norm before it
+  auto normed = [&](const std::string& stem, bool pair_rows, const std::string& before) {
+    dense(stem, pair_rows, gains ? before + ".weight" : "");
+    if (!gains) norm(before);
   };
   plan.push_back({"edge_embedder.weight", Prep::Table});
   for (int L = 0; L < h.num_gnn_layers; ++L) {
@@ -119,14 +127,13 @@ std::vector<PlanItem> weight_plan(const Hypers& h) {
     dense(layer + ".compress.2");
     for (int a = 0; a < h.num_attention_layers; ++a) {
       const std::string block = layer + ".trans.layers." + std::to_string(a);
-      for (const char* part : {".attention.input_linear", ".attention.output_linear", ".mlp.w_out"}) dense(block + part);
-      dense(block + ".mlp.w_in", paired);
-      norm(block + ".norm_attention"), norm(block + ".norm_mlp");
+      for (const char* part : {".attention.output_linear", ".mlp.w_out"}) dense(block + part);
+      normed(block + ".attention.input_linear", false, block + ".norm_attention");
+      normed(block + ".mlp.w_in", paired, block + ".norm_mlp");
       if (!h.expanded_node()) continue;
       for (const char* part : {".center_contraction", ".center_mlp.w_out"}) dense(block + part);
       plan.push_back({block, Prep::ExpansionFold});
-      dense(block + ".center_mlp.w_in", paired);
-      norm(block + ".norm_center_features");
+      normed(block + ".center_mlp.w_in", paired, block + ".norm_center_features");
     }
     if (ff) {
       const std::string n = "combination_norms." + std::to_string(L), m = "combination_mlps." + std::to_string(L);
@@ -148,12 +155,12 @@ std::vector<PlanItem> weight_plan(const Hypers& h) {
 
 }  // namespace
 
-void Model::put_mat(const std::string& name, const double* src, int ld, int rows, int cols, bool paired, bool operand) {
+void Model::put_mat(const std::string& name, const double* src, int ld, int rows, int cols, bool paired, bool operand, const double* gain) {
   const size_t n = size_t(rows) * cols;
   float* dev = nullptr;
   PETB_CUDA(cudaMalloc(&dev, (n + 4) * sizeof(float)));
   owned_.push_back(dev);
-  if (n) k_weight_rows<<<cdiv((long long) n, 256), 256>>>(src, ld, rows, cols, paired ? 1 : 0, dev);
+  if (n) k_weight_rows<<<cdiv((long long) n, 256), 256>>>(src, ld, rows, cols, paired ? 1 : 0, gain, dev);
   PETB_CUDA(cudaGetLastError());
   Mat m;
   m.w = dev, m.rows = rows, m.cols = cols;
@@ -251,7 +258,7 @@ Model::Model(const Checkpoint& ck, int gemm_mode) : h_(ck.hypers), scale_(ck.ene
   if (h_.d_pet % 4 || h_.d_node % 4 || h_.d_head % 4 || h_.d_feedforward % 4)
     throw Error(1, "model: layer widths must be multiples of 4");
 
-  for (const PlanItem& it : weight_plan(h_)) {
+  for (const PlanItem& it : weight_plan(h_, folds_norms())) {
     if (it.prep == Prep::CompressFold) {
       fold_compress(ck, it.name, it.layer);
       continue;
@@ -265,7 +272,12 @@ Model::Model(const Checkpoint& ck, int gemm_mode) : h_(ck.hypers), scale_(ck.ene
     const bool paired = it.prep == Prep::PairedMatrix || it.prep == Prep::PairedVector;
     if (matrix && t.shape.size() != 2) throw Error(1, "model: expected a 2-D tensor '" + it.name + "'");
     const Staged dev(t);
-    if (matrix) put_mat(it.name, dev.p, dev.cols, dev.rows, dev.cols, paired, it.prep != Prep::Table);
+    if (!it.gain.empty()) {
+      const Staged gain(ck.at(it.gain));
+      if (gain.rows * gain.cols != dev.cols) throw Error(1, "model: '" + it.gain + "' does not have the width of the layer after it");
+      put_mat(it.name, dev.p, dev.cols, dev.rows, dev.cols, paired, true, gain.p);
+      PETB_CUDA(cudaDeviceSynchronize());
+    } else if (matrix) put_mat(it.name, dev.p, dev.cols, dev.rows, dev.cols, paired, it.prep != Prep::Table);
     else put_vec(it.name, dev.p, int(t.numel()), paired);
     PETB_CUDA(cudaDeviceSynchronize());
   }
@@ -509,8 +521,9 @@ MemoryNeed Model::memory_need(int tier, int N, int E, int n_live) const {
   save += double(row_maxima_words(N, E)) * (relayer ? 2 : 1);       // (a layer run again takes its own)
   // tmp: the fullest scope
   const double attention_bwd = T * (5 * D + H) + (keep ? 0.0 : T * 4 * D);
-  const double attention_fwd = T * D + (keep ? 0.0 : T * 3 * D);
-  const double edge_mlp = c * (2 * F + D) + (keep ? c * F : c * (2 * F + D)) + n * 5 * Dn;  // (beside the atoms')
+  const double norms = folds_norms() ? 0.0 : 1.0;  // the norms' rows
+  const double attention_fwd = norms * T * D + (keep ? 0.0 : T * 3 * D);
+  const double edge_mlp = c * (2 * F + D) + (keep ? c * F : c * (2 * F + norms * D)) + n * 5 * Dn;  // (beside the atoms')
   const double combination = e * 4 * D + 2 * live * D;
   const double heads = 2 * n * Dh + 2 * e * Dh;
   double tmp = std::max(std::max(attention_bwd, attention_fwd), std::max(std::max(edge_mlp, combination), heads));
@@ -524,7 +537,7 @@ MemoryNeed Model::memory_need(int tier, int N, int E, int n_live) const {
 size_t Model::row_maxima_words(int N, int E) const {
   const size_t G = h_.num_gnn_layers, A = h_.num_attention_layers, T = size_t(N) + E + 64, n = size_t(N) + 64;
   if (!scales_rows(format_of(mode_))) return 0;
-  return G * ((11 * A + 8) * T + 6 * A * n) + 4 * T + 6 * n;
+  return G * ((13 * A + 8) * T + 8 * A * n) + 4 * T + 6 * n;
 }
 
 size_t Model::memory_estimate(int tier, int N, int E) const {
@@ -556,7 +569,8 @@ PassOut Model::run_feedforward(Stream& st, Arena& save, Arena& tmp, const Packed
   RowMaxima maxima(st, save, row_maxima_words(N, E) * (relayer ? 2 : 1));  // a layer run again takes its own
 
   struct Block {
-    float *tok, *ml, *eps, *node_res, *pre_c, *pre_e;
+    Rows tok, eps, node_res;  // what the block's three norms read
+    float *ml, *pre_c, *pre_e;
     Rows qkv, merged;
   };
   struct Layer {
@@ -571,18 +585,30 @@ PassOut Model::run_feedforward(Stream& st, Arena& save, Arena& tmp, const Packed
     at.qkv = qkv.p, at.merged = b.merged.p, at.ml = b.ml;
     return at;
   };
+  // The RMSNorms of a block: folded into the GEMM that reads them, or by themselves in the modes of one part (folds_norms). norm_of
+  // is the input of that GEMM, normed what makes of it the GEMM of the norm.
+  const bool fold = folds_norms();
+  const auto norm_of = [&](const Rows& x, const std::string& name, int R, int width) {
+    if (fold) return x;
+    const Rows y = maxima.fresh(tmp.alloc<float>(size_t(R > 0 ? R : 1) * width), R);
+    norm_fwd(st, y.p, x.p, nullptr, vec(name + ".weight"), nullptr, R, width, y.mx);
+    return y;
+  };
+  const auto gain_of = [&](const std::string& name) { return fold ? nullptr : vec(name + ".weight"); };
+  const auto normed = [&](GemmArgs a) {
+    a.rms = fold;
+    return a;
+  };
   // qkv = W_in . norm(tokens) + b
-  auto make_qkv = [&](const Rows& qkv, const std::string& tl, float* tok) {
+  auto make_qkv = [&](const Rows& qkv, const std::string& tl, const Block& b) {
     Scope s(tmp);
-    const Rows attn_in = maxima.fresh(tmp.alloc<float>(Ta * D), Ta);
-    norm_fwd(st, attn_in.p, tok, nullptr, vec(tl + ".norm_attention.weight"), nullptr, T, D, attn_in.mx);
-    gm.linear(qkv, attn_in, mat(tl + ".attention.input_linear.weight"), vec(tl + ".attention.input_linear.bias"), T);
+    const Rows in = norm_of(b.tok, tl + ".norm_attention", T, D);
+    gm.one(normed(Gemms::linear_args(qkv, in, mat(tl + ".attention.input_linear.weight"), vec(tl + ".attention.input_linear.bias"), T)));
   };
   // The edge MLP's first half on rows [r0, r0 + nr): pre = W_in . norm(eps) + b and, with `he`, v * sigmoid(g).
-  auto edge_mlp_in = [&](const Rows& he, float* pre, const float* eps_rows, const std::string& tl, int nr) {
-    const Rows edge_norm = maxima.fresh(tmp.alloc<float>(size_t(nr) * D), nr);
-    norm_fwd(st, edge_norm.p, const_cast<float*>(eps_rows), nullptr, vec(tl + ".norm_mlp.weight"), nullptr, nr, D, edge_norm.mx);
-    return Gemms::swiglu_args(he, pre, edge_norm, mat(tl + ".mlp.w_in.weight"), vec(tl + ".mlp.w_in.bias"), nr);
+  auto edge_mlp_in = [&](const Rows& he, float* pre, const Block& b, int r0, const std::string& tl, int nr) {
+    const Rows in = norm_of(b.eps.from(r0, D), tl + ".norm_mlp", nr, D);
+    return normed(Gemms::swiglu_args(he, pre, in, mat(tl + ".mlp.w_in.weight"), vec(tl + ".mlp.w_in.bias"), nr));
   };
 
   // One message-passing layer forward: node_in [N,Dn] -> node_out, input_edge [E,D] updated in place, saves in `sl`
@@ -594,12 +620,12 @@ PassOut Model::run_feedforward(Stream& st, Arena& save, Arena& tmp, const Packed
     sl.blk.resize(A);
     // Token buffers: block a's tokens are [input_node ; edge_cur]; its edge output is written
     // straight into the edge rows of block a+1's, the last one's being the layer's out_edge.
-    std::vector<float*> tokbuf(A + 1);
-    for (int a = 0; a <= A; ++a) tokbuf[a] = save.alloc<float>(Ta * D);
+    std::vector<Rows> tokbuf(A + 1);
+    for (int a = 0; a <= A; ++a) tokbuf[a] = {save.alloc<float>(Ta * D), fold && a < A ? maxima.take(Ta) : nullptr};
     sl.cpre = save.alloc<float>(Ea * D);
     const auto contraction = [&](int a, const Rows& node) {  // block a's atom tokens
       const std::string tl = g + ".trans.layers." + std::to_string(a);
-      return Gemms::linear_args({tokbuf[a]}, node, mat(tl + ".center_contraction.weight"), vec(tl + ".center_contraction.bias"), N);
+      return Gemms::linear_args(tokbuf[a], node, mat(tl + ".center_contraction.weight"), vec(tl + ".center_contraction.bias"), N);
     };
     {
       Scope s0(tmp);
@@ -609,10 +635,10 @@ PassOut Model::run_feedforward(Stream& st, Arena& save, Arena& tmp, const Packed
       } else {
         gm.compress(cact, sl.cpre, input_edge, mat(c0 + "@in"), vec(c0 + "@b"), mat(c0 + "@tab"), mat(c0 + "@x4"), pk);
       }
-      gm.two(contraction(0, node_in), Gemms::linear_args({tokbuf[0] + size_t(N) * D}, cact, mat(g + ".compress.2.weight"),
-                                                         vec(g + ".compress.2.bias"), E));
+      gm.two(contraction(0, node_in),
+             Gemms::linear_args(tokbuf[0].from(N, D), cact, mat(g + ".compress.2.weight"), vec(g + ".compress.2.bias"), E));
     }
-    tap(taps, "et" + ls, tokbuf[0] + size_t(N) * D, size_t(E) * D);
+    tap(taps, "et" + ls, tokbuf[0].p + size_t(N) * D, size_t(E) * D);
 
     Rows node_cur = node_in;
     for (int a = 0; a < A; ++a) {
@@ -622,48 +648,45 @@ PassOut Model::run_feedforward(Stream& st, Arena& save, Arena& tmp, const Packed
       b.tok = tokbuf[a];
       b.merged = maxima.fresh(save.alloc<float>(Ta * D), Ta);
       b.ml = save.alloc<float>(Ta * H * 2);
-      b.eps = save.alloc<float>(Ea * D);
-      b.node_res = save.alloc<float>(Na * Dn);
+      b.eps = {save.alloc<float>(Ea * D), fold ? maxima.take(Ea) : nullptr};
+      b.node_res = {save.alloc<float>(Na * Dn), fold ? maxima.take(Na) : nullptr};
       b.pre_c = save.alloc<float>(Na * w_cin.rows);
       b.qkv = keep ? Rows{save.alloc<float>(Ta * 3 * D)} : Rows{};
       b.pre_e = keep ? save.alloc<float>(Ea * w_ein.rows) : nullptr;
       const Rows node_next = maxima.fresh(a + 1 == A ? node_out.p : save.alloc<float>(Na * Dn), Na);
       if (a + 1 == A) node_out = node_next;
-      float* edge_next = tokbuf[a + 1] + size_t(N) * D;
-
       if (a > 0) gm.one(contraction(a, node_cur));
       {
         Scope s1(tmp);
         const Rows qkv = keep ? b.qkv : Rows{tmp.alloc<float>(Ta * 3 * D)};
-        make_qkv(qkv, tl, b.tok);
+        make_qkv(qkv, tl, b);
         AttnArgs at = attention_args(b, qkv);
         at.merged_max = b.merged.mx;
         attention_forward(st, at);
       }
       tap(taps, "merged" + tag, b.merged.p, size_t(T) * D);
       // eps = output layer(merged) + edge_cur on the edges' rows, node_res = expansion(output layer(merged)) + node_cur on the atoms'
-      gm.two(Gemms::linear_args({b.node_res}, b.merged, mat(tl + "@expand"), vec(tl + "@expand_b"), N, node_cur.p, 0),
-             Gemms::linear_args({b.eps}, b.merged.from(N, D), mat(tl + ".attention.output_linear.weight"),
-                                vec(tl + ".attention.output_linear.bias"), E, b.tok + size_t(N) * D, 0));
+      gm.two(Gemms::linear_args(b.node_res, b.merged, mat(tl + "@expand"), vec(tl + "@expand_b"), N, node_cur.p, 0),
+             Gemms::linear_args(b.eps, b.merged.from(N, D), mat(tl + ".attention.output_linear.weight"),
+                                vec(tl + ".attention.output_linear.bias"), E, b.tok.p + size_t(N) * D, 0));
       // the atoms' MLP, and the edges' a chunk at a time: the first chunk's GEMMs share their launches with the atoms'
       Scope s2(tmp);
-      const Rows node_norm = maxima.fresh(tmp.alloc<float>(Na * Dn), Na);
       const Rows hc = maxima.fresh(tmp.alloc<float>(Na * (w_cin.rows / 2)), Na);
-      norm_fwd(st, node_norm.p, b.node_res, nullptr, vec(tl + ".norm_center_features.weight"), nullptr, N, Dn, node_norm.mx);
-      const GemmArgs node_in_args = Gemms::swiglu_args(hc, b.pre_c, node_norm, w_cin, vec(tl + ".center_mlp.w_in.bias"), N);
+      const Rows node_in_rows = norm_of(b.node_res, tl + ".norm_center_features", N, Dn);
+      const GemmArgs node_in_args =
+          normed(Gemms::swiglu_args(hc, b.pre_c, node_in_rows, w_cin, vec(tl + ".center_mlp.w_in.bias"), N));
       const GemmArgs node_out_args =
-          Gemms::linear_args(node_next, hc, mat(tl + ".center_mlp.w_out.weight"), vec(tl + ".center_mlp.w_out.bias"), N, b.node_res, 0);
+          Gemms::linear_args(node_next, hc, mat(tl + ".center_mlp.w_out.weight"), vec(tl + ".center_mlp.w_out.bias"), N, b.node_res.p, 0);
       const int rows = keep || chunk <= 0 ? (E > 0 ? E : 1) : chunk;
       int r0 = 0;
       do {
         const int nr = std::min(rows, E - r0);
         Scope s3(tmp);
-        float* eps_rows = b.eps + size_t(r0) * D;
         const Rows he = maxima.fresh(tmp.alloc<float>(size_t(nr) * (w_ein.rows / 2)), nr);
         float* pre = keep ? b.pre_e + size_t(r0) * w_ein.rows : tmp.alloc<float>(size_t(nr) * w_ein.rows);
-        const GemmArgs edge_in_args = edge_mlp_in(he, pre, eps_rows, tl, nr);
-        const GemmArgs edge_out_args = Gemms::linear_args({edge_next + size_t(r0) * D}, he, mat(tl + ".mlp.w_out.weight"),
-                                                          vec(tl + ".mlp.w_out.bias"), nr, eps_rows, 0);
+        const GemmArgs edge_in_args = edge_mlp_in(he, pre, b, r0, tl, nr);
+        const GemmArgs edge_out_args = Gemms::linear_args(tokbuf[a + 1].from(size_t(N) + r0, D), he, mat(tl + ".mlp.w_out.weight"),
+                                                          vec(tl + ".mlp.w_out.bias"), nr, b.eps.p + size_t(r0) * D, 0);
         if (r0 == 0) {
           gm.two(node_in_args, edge_in_args);
           gm.two(node_out_args, edge_out_args);
@@ -674,9 +697,9 @@ PassOut Model::run_feedforward(Stream& st, Arena& save, Arena& tmp, const Packed
       } while (r0 < E);
       node_cur = node_next;
       tap(taps, "node" + tag, node_cur.p, size_t(N) * Dn);
-      tap(taps, "edge" + tag, edge_next, size_t(E) * D);
+      tap(taps, "edge" + tag, tokbuf[a + 1].p + size_t(N) * D, size_t(E) * D);
     }
-    sl.out_edge = tokbuf[A] + size_t(N) * D;
+    sl.out_edge = tokbuf[A].p + size_t(N) * D;
     sl.cph_pre = save.alloc<float>(Ea * 2 * D);
     {
       Scope s4(tmp);
@@ -826,12 +849,12 @@ PassOut Model::run_feedforward(Stream& st, Arena& save, Arena& tmp, const Packed
         do {
           const int nr = std::min(rows, E - r0);
           Scope s8(tmp);
-          const float* eps_rows = b.eps + size_t(r0) * D;
+          const float* eps_rows = b.eps.p + size_t(r0) * D;
           const Rows adj_rows = edge_adj.from(r0, D);
           const float* pre = b.pre_e ? b.pre_e + size_t(r0) * w_ein.rows : nullptr;
           if (!pre) {  // the pre-activation was not kept: these rows' again
             float* again_pre = tmp.alloc<float>(size_t(nr) * w_ein.rows);
-            gm.one(edge_mlp_in({}, again_pre, eps_rows, tl, nr));
+            gm.one(edge_mlp_in({}, again_pre, b, r0, tl, nr));
             pre = again_pre;
           }
           const Rows pre_adj = maxima.fresh(tmp.alloc<float>(size_t(nr) * w_ein.rows), nr);
@@ -841,14 +864,16 @@ PassOut Model::run_feedforward(Stream& st, Arena& save, Arena& tmp, const Packed
           if (r0 == 0) {
             gm.two(node_out_args, edge_out_args);
             gm.two(node_in_args, edge_in_args);
+            node_adj.mx = maxima.take(Na);
+            norm_bwd_two(st, node_adj.p, cnorm_adj, b.node_res.p, gain_of(tl + ".norm_center_features"), N, Dn, node_adj.mx, adj_rows.p,
+                         enorm_adj, eps_rows, gain_of(tl + ".norm_mlp"), nr, D, eps_adj.mx);
           } else {
             gm.one(edge_out_args), gm.one(edge_in_args);
+            norm_bwd_two(st, nullptr, nullptr, nullptr, nullptr, 0, Dn, nullptr, adj_rows.p, enorm_adj, eps_rows, gain_of(tl + ".norm_mlp"), nr, D,
+                         eps_adj.from(r0, D).mx);
           }
-          norm_bwd(st, adj_rows.p, enorm_adj, eps_rows, vec(tl + ".norm_mlp.weight"), false, nr, D, 0, nullptr, eps_adj.from(r0, D).mx);
           r0 += rows;
         } while (r0 < E);
-        node_adj.mx = maxima.take(Na);
-        norm_bwd(st, node_adj.p, cnorm_adj, b.node_res, vec(tl + ".norm_center_features.weight"), false, N, Dn, 0, nullptr, node_adj.mx);
       }
       {  // attention
         Scope s10(tmp);
@@ -859,7 +884,7 @@ PassOut Model::run_feedforward(Stream& st, Arena& save, Arena& tmp, const Packed
         Rows qkv = b.qkv;
         if (!qkv.p) {
           qkv = Rows{tmp.alloc<float>(Ta * 3 * D)};
-          make_qkv(qkv, tl, b.tok);
+          make_qkv(qkv, tl, b);
         }
         gm.two(Gemms::linear_bwd_args(dmerged, node_adj, mat(tl + "@expand"), N, false),
                Gemms::linear_bwd_args(dmerged.from(N, D), eps_adj, mat(tl + ".attention.output_linear.weight"), E, false));
@@ -871,7 +896,7 @@ PassOut Model::run_feedforward(Stream& st, Arena& save, Arena& tmp, const Packed
         // through the norm, back to where the tokens came from: atom rows to the contraction's
         // output adjoint (written), edge rows onto the edge residual (accumulated)
         tok_adj.mx = maxima.take(Ta);
-        norm_bwd(st, tok_adj.p, attn_in_adj, b.tok, vec(tl + ".norm_attention.weight"), false, T, D, N, nullptr, tok_adj.mx);
+        norm_bwd(st, tok_adj.p, attn_in_adj, b.tok.p, gain_of(tl + ".norm_attention"), false, T, D, N, nullptr, tok_adj.mx);
       }
       node_adj.mx = maxima.take(Na);
       gm.linear_bwd(node_adj, tok_adj, mat(tl + ".center_contraction.weight"), N, true);

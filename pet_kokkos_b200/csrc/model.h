@@ -98,11 +98,16 @@ class Model {
   const Mat& mat(const std::string& name) const;
   const float* vec(const std::string& name) const;
   // `src` are doubles in DEVICE memory; the layouts the kernels read are made from them by kernels.
-  void put_mat(const std::string& name, const double* src, int ld, int rows, int cols, bool paired, bool operand);
+  void put_mat(const std::string& name, const double* src, int ld, int rows, int cols, bool paired, bool operand,
+               const double* gain = nullptr);
   void put_vec(const std::string& name, const double* src, int len, bool paired);
   void fold_compress(const Checkpoint& ck, const std::string& c0, int layer);
   void fold_expansion(const Checkpoint& ck, const std::string& block);
 
+  // The feedforward featurizer's RMSNorms go into the GEMMs that read them (gain in the weight, 1 / rms in the epilogue), but for the
+  // modes of one part: there what a weight loses to its operand's 8 or 11 bits is most of a mode's error, and W times a gain loses
+  // something else than W (pet-mad-s shape, two sets of random weights: forces off by 0.094 -> 0.117 and 0.044 -> 0.035 meV/A).
+  bool folds_norms() const { return h_.feedforward && (mode_ == GEMM_NATIVE || mode_ == GEMM_TF32X3); }
   bool wide() const { return h_.d_pet > 256; }  // the tensor-core modes' forward on tf32 instructions (put_mat)
 
   Hypers h_;

@@ -7,7 +7,6 @@ namespace petb {
 
 namespace {
 
-constexpr float kRmsEps = 1.1920928955078125e-07f;  // the reference's kRmsNormEps (src/ops.hpp:195)
 constexpr float kLnEps = 1e-5f;                     // kLayerNormEps (:196)
 constexpr unsigned kFull = 0xffffffffu;
 
@@ -243,7 +242,7 @@ __global__ void __launch_bounds__(256) k_norm_bwd(float* __restrict__ in_adj, co
   }
   float sq = 0.f, sg = 0.f, sgx = 0.f;
   for (int d = lane; d < D; d += 32) {
-    const float c = x[d] - mu, gw = ga[d] * w[d];
+    const float c = x[d] - mu, gw = w ? ga[d] * w[d] : ga[d];
     sq += c * c, sg += gw, sgx += gw * c;
   }
   sq = warp_sum(sq), sg = warp_sum(sg), sgx = warp_sum(sgx);
@@ -253,7 +252,7 @@ __global__ void __launch_bounds__(256) k_norm_bwd(float* __restrict__ in_adj, co
   const bool acc = r >= acc_row0;
   float big = 0.f;
   for (int d = lane; d < D; d += 32) {
-    const float g = inv * (ga[d] * w[d] - mg - (x[d] - mu) * inv * mgx);
+    const float g = inv * ((w ? ga[d] * w[d] : ga[d]) - mg - (x[d] - mu) * inv * mgx);
     const float v = acc ? o[d] + g : g;
     o[d] = v;
     if (also) also[size_t(r) * D + d] = v;
@@ -276,8 +275,11 @@ __global__ void __launch_bounds__(256) k_norm_bwd_v(float* __restrict__ in_adj, 
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
     x[i] = ld4(in + size_t(r) * D + 128 * i + 4 * lane);
-    const float4 g = ld4(out_adj + size_t(r) * D + 128 * i + 4 * lane), ww = ld4(w + 128 * i + 4 * lane);
-    gw[i] = make_float4(g.x * ww.x, g.y * ww.y, g.z * ww.z, g.w * ww.w);
+    gw[i] = ld4(out_adj + size_t(r) * D + 128 * i + 4 * lane);
+    if (w) {
+      const float4 ww = ld4(w + 128 * i + 4 * lane);
+      gw[i].x *= ww.x, gw[i].y *= ww.y, gw[i].z *= ww.z, gw[i].w *= ww.w;
+    }
   }
   float mu = 0.f;
   if (ln) {
@@ -315,6 +317,95 @@ __global__ void __launch_bounds__(256) k_norm_bwd_v(float* __restrict__ in_adj, 
   if (!mx) return;
   big = warp_max(big);
   if (lane == 0) mx[r] = __float_as_uint(big);
+}
+
+// RMSNorm's backward (`w` null for a gain of one) onto the atoms' rows, a block a row, and the edges', a warp a row, in one
+// launch: the few atoms' rows by themselves take 5-10 us, as a warp's rows of 1024 columns and more registers they would take the
+// edges' loads their warps.
+struct NormBwdRows {
+  float* in_adj;         // += the adjoint
+  const float* out_adj;
+  const float* in;
+  const float* w;
+  uint32_t* mx;
+  int R, D;
+};
+__device__ __forceinline__ float4 with_gain(float4 g, const float* w, int c) {
+  if (!w) return g;
+  const float4 x = ld4(w + c);
+  return make_float4(g.x * x.x, g.y * x.y, g.z * x.z, g.w * x.w);
+}
+template <int NV>
+__global__ void __launch_bounds__(256) k_norm_bwd_two(NormBwdRows n, NormBwdRows e) {
+  after_previous();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (int(blockIdx.x) < n.R) {
+    __shared__ float s_sq[8], s_gx[8], s_big[8];
+    const size_t at = size_t(blockIdx.x) * n.D;
+    float4 x[2], g[2];
+    float sq = 0.f, sgx = 0.f;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int c = 1024 * i + 4 * threadIdx.x;
+      x[i] = c < n.D ? ld4(n.in + at + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+      g[i] = c < n.D ? with_gain(ld4(n.out_adj + at + c), n.w, c) : make_float4(0.f, 0.f, 0.f, 0.f);
+      sq += (x[i].x * x[i].x + x[i].y * x[i].y) + (x[i].z * x[i].z + x[i].w * x[i].w);
+      sgx += (g[i].x * x[i].x + g[i].y * x[i].y) + (g[i].z * x[i].z + g[i].w * x[i].w);
+    }
+    sq = warp_sum(sq), sgx = warp_sum(sgx);
+    if (lane == 0) s_sq[warp] = sq, s_gx[warp] = sgx;
+    __syncthreads();
+    sq = sgx = 0.f;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) sq += s_sq[w], sgx += s_gx[w];
+    const float inv = 1.0f / sqrtf(sq / n.D + kRmsEps), mgx = sgx * inv / n.D;
+    float big = 0.f;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int c = 1024 * i + 4 * threadIdx.x;
+      if (c >= n.D) continue;
+      float4 o = ld4(n.in_adj + at + c);
+      o.x += inv * (g[i].x - x[i].x * inv * mgx), o.y += inv * (g[i].y - x[i].y * inv * mgx);
+      o.z += inv * (g[i].z - x[i].z * inv * mgx), o.w += inv * (g[i].w - x[i].w * inv * mgx);
+      st4(n.in_adj + at + c, o);
+      big = fmaxf(big, max4(o));
+    }
+    if (!n.mx) return;
+    big = warp_max(big);
+    if (lane == 0) s_big[warp] = big;
+    __syncthreads();
+    if (threadIdx.x) return;
+    for (int w = 1; w < 8; ++w) big = fmaxf(big, s_big[w]);
+    n.mx[blockIdx.x] = __float_as_uint(big);
+    return;
+  }
+  constexpr int D = 128 * NV;
+  const int r = (blockIdx.x - n.R) * 8 + warp;
+  if (r >= e.R) return;
+  float4 x[NV], g[NV];
+  float sq = 0.f, sgx = 0.f;
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const int c = 128 * i + 4 * lane;
+    x[i] = ld4(e.in + size_t(r) * D + c), g[i] = with_gain(ld4(e.out_adj + size_t(r) * D + c), e.w, c);
+    sq += (x[i].x * x[i].x + x[i].y * x[i].y) + (x[i].z * x[i].z + x[i].w * x[i].w);
+    sgx += (g[i].x * x[i].x + g[i].y * x[i].y) + (g[i].z * x[i].z + g[i].w * x[i].w);
+  }
+  sq = warp_sum(sq), sgx = warp_sum(sgx);
+  const float inv = 1.0f / sqrtf(sq / D + kRmsEps), mgx = sgx * inv / D;
+  float* o = e.in_adj + size_t(r) * D;
+  float big = 0.f;
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    float4 old = ld4(o + 128 * i + 4 * lane);
+    old.x += inv * (g[i].x - x[i].x * inv * mgx), old.y += inv * (g[i].y - x[i].y * inv * mgx);
+    old.z += inv * (g[i].z - x[i].z * inv * mgx), old.w += inv * (g[i].w - x[i].w * inv * mgx);
+    st4(o + 128 * i + 4 * lane, old);
+    big = fmaxf(big, max4(old));
+  }
+  if (!e.mx) return;
+  big = warp_max(big);
+  if (lane == 0) e.mx[r] = __float_as_uint(big);
 }
 
 // The statistics of row q of the concat [oe(q) | partner(q) or 0] and of its adjoint.
@@ -750,6 +841,21 @@ void norm_bwd(Stream& st, float* in_adj, const float* out_adj, const float* in, 
     case 1024: launch(st, k_norm_bwd_v<8>, blocks, 256, 0, in_adj, out_adj, in, w, layernorm, R, acc_row0, also, mx); break;
     default: launch(st, k_norm_bwd, blocks, 256, 0, in_adj, out_adj, in, w, layernorm, R, D, acc_row0, also, mx);
   }
+  PETB_LAUNCH_CHECK(st);
+}
+
+void norm_bwd_two(Stream& st, float* n_adj, const float* n_out_adj, const float* n_in, const float* n_w, int N, int Dn, uint32_t* n_mx,
+                  float* e_adj, const float* e_out_adj, const float* e_in, const float* e_w, int E, int D, uint32_t* e_mx) {
+  if (N == 0 && E == 0) return;
+  if (Dn > 2048 || (D != 128 && D != 256 && D != 512)) {
+    norm_bwd(st, e_adj, e_out_adj, e_in, e_w, false, E, D, 0, nullptr, e_mx);
+    return norm_bwd(st, n_adj, n_out_adj, n_in, n_w, false, N, Dn, 0, nullptr, n_mx);
+  }
+  const double values = double(N) * Dn + double(E) * D;
+  const ProfScope ps(st, PC_NORM, 10.0 * values, 16.0 * values);
+  const NormBwdRows n{n_adj, n_out_adj, n_in, n_w, n_mx, N, Dn}, e{e_adj, e_out_adj, e_in, e_w, e_mx, E, D};
+  const auto kernel = D == 128 ? k_norm_bwd_two<1> : D == 256 ? k_norm_bwd_two<2> : k_norm_bwd_two<4>;
+  launch(st, kernel, size_t(N) + blocks_for(E, 8), 256, 0, n, e);
   PETB_LAUNCH_CHECK(st);
 }
 

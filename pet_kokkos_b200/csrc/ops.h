@@ -37,9 +37,13 @@ void concat_norm_fwd(Stream& st, float* out, const float* oe, const int* rev, fl
                      int E, int D, RemoteRows remote = {}, uint32_t* mx = nullptr);
 
 // in_adj = g for rows < acc_row0, in_adj += g for the rest; g the norm's input adjoint
-// (norm_rows_bwd, src/ops.hpp:404-436). `also`, unless null, receives a copy of the result.
+// (norm_rows_bwd, src/ops.hpp:404-436); w null for a gain of one. `also`, unless null, receives a copy of the result.
 void norm_bwd(Stream& st, float* in_adj, const float* out_adj, const float* in, const float* w, bool layernorm, int R, int D,
               int acc_row0, float* also = nullptr, uint32_t* mx = nullptr);
+
+// RMSNorm's backward added to the atoms' rows [N, Dn] and the edges' [E, D] in one launch.
+void norm_bwd_two(Stream& st, float* n_adj, const float* n_out_adj, const float* n_in, const float* n_w, int N, int Dn, uint32_t* n_mx,
+                  float* e_adj, const float* e_out_adj, const float* e_in, const float* e_w, int E, int D, uint32_t* e_mx);
 
 // edge_adj(k) = ie_adj(k) + g(k)[:D] + g(rev k)[D:], g from out_adj [E,2D]  (concat_norm_bwd, src/ops.cpp:191-244)
 // With an exchange: `remote` holds the partner rows the forward read, `remote_adj` the partners' adjoints of this
