@@ -353,6 +353,7 @@ typedef struct pet_debug_gemm_args {
   const double *vec, *dist; /* [m,3], [m] */
   float* C;                /* [m,n]; SwiGLU [m,n/2]; SwiGLU' [m,2n] */
   float* row_max;          /* [m], optional: each row's largest |C| as the epilogue keeps it */
+  int rms;                 /* A's rows over their root mean squares first (an RMSNorm without a gain) */
 } pet_debug_gemm_args;
 int pet_debug_gemm(pet_calc* c, const pet_debug_gemm_args* args);
 /* Two of one format, args[0] and args[1], handed over together as the atoms' and the edges' GEMM of a step are: one launch

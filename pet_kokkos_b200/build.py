@@ -21,8 +21,6 @@ COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler",
           "--expt-relaxed-constexpr", "-Xcudafe", "--diag_suppress=177"]
 # neighbour kernels: every fp64 product and sum rounded on its own (bit-exact edge decisions)
 PER_FILE = {"neighbors.cu": ["-fmad=false"]}
-# many instances of one kernel to a file
-APART = ["--split-compile=8"]
 # (the longest to compile first)
 SOURCES = ["gemm_tc_plain_x3.cu", "gemm_tc_plain.cu", "gemm_tc_silu.cu", "gemm_tc_swiglu.cu", "gemm_tc_swiglu_bwd.cu", "gemm_tc_silu_bwd.cu",
            "attention_f16.cu", "gemm_tc_compress.cu", "checkpoint.cpp", "neighbors.cu", "ops.cu", "adaptive.cu", "attention.cu",
@@ -48,7 +46,7 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     for src in SOURCES:
         s, o = CSRC / src, OBJ / (src + ".o")
         if force or _stale(o, [s] + headers):
-            cmd = [nvcc(), *ARCH, *COMMON, *PER_FILE.get(src, []), *(APART if src.startswith("gemm_tc_") else []), "-c", str(s), "-o", str(o)]
+            cmd = [nvcc(), *ARCH, *COMMON, *PER_FILE.get(src, []), "-c", str(s), "-o", str(o)]
             if verbose:
                 cmd.insert(1, "-Xptxas=-v")
             jobs.append(cmd)

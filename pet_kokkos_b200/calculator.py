@@ -106,7 +106,7 @@ class PetDebugGemmArgs(C.Structure):
                [(f, C.POINTER(C.c_float)) for f in ("A", "W", "bias", "res")] + [("res_row0", C.c_int)] + \
                [(f, C.POINTER(C.c_float)) for f in ("pre", "tab")] + \
                [("n_tab", C.c_int), ("species", C.POINTER(C.c_int)), ("wx", C.POINTER(C.c_float)), ("vec", C.POINTER(C.c_double)),
-                ("dist", C.POINTER(C.c_double)), ("C", C.POINTER(C.c_float)), ("row_max", C.POINTER(C.c_float))]
+                ("dist", C.POINTER(C.c_double)), ("C", C.POINTER(C.c_float)), ("row_max", C.POINTER(C.c_float)), ("rms", C.c_int)]
 
 
 class PetRawEdges(C.Structure):
@@ -676,10 +676,10 @@ class Calculator:
         return Cm
 
     def debug_gemm(self, A, W, fmt, epilogue="plain", w_transposed=True, bias=None, res=None, res_row0=0, pre=None, tab=None,
-                   species=None, wx=None, vec=None, dist=None, want_pre=True):
+                   species=None, wx=None, vec=None, dist=None, want_pre=True, rms=False):
         """One weight GEMM with an epilogue in one operand format: (C, pre as written or None, row maxima of C)."""
         g, keep, results = self._debug_gemm_args(A, W, fmt, epilogue, w_transposed, bias, res, res_row0, pre, tab, species, wx, vec, dist,
-                                                 want_pre)
+                                                 want_pre, rms)
         self._check(self._lib.pet_debug_gemm(self._h, C.byref(g)))
         return results
 
@@ -690,7 +690,7 @@ class Calculator:
         return given[0][2], given[1][2]
 
     def _debug_gemm_args(self, A, W, fmt, epilogue="plain", w_transposed=True, bias=None, res=None, res_row0=0, pre=None, tab=None,
-                         species=None, wx=None, vec=None, dist=None, want_pre=True):
+                         species=None, wx=None, vec=None, dist=None, want_pre=True, rms=False):
         g, keep = PetDebugGemmArgs(), []
 
         def ptr(x, dtype, pt):
@@ -702,7 +702,7 @@ class Calculator:
         m, k = np.shape(A)
         n = np.shape(W)[0] if w_transposed else np.shape(W)[1]
         g.format, g.epilogue = GEMM_FORMATS[fmt], GEMM_EPILOGUES[epilogue]
-        g.w_transposed, g.m, g.n, g.k, g.res_row0 = int(w_transposed), m, n, k, res_row0
+        g.w_transposed, g.m, g.n, g.k, g.res_row0, g.rms = int(w_transposed), m, n, k, res_row0, int(rms)
         g.A, g.W, g.bias, g.res, g.tab, g.wx = f32(A), f32(W), f32(bias), f32(res), f32(tab), f32(wx)
         g.n_tab = 0 if tab is None else len(tab)
         g.species = ptr(species, np.int32, C.POINTER(C.c_int))

@@ -1438,7 +1438,7 @@ GemmArgs Engine::gemm_from_host_arrays(const pet_debug_gemm_args& g, int native_
     return to;
   };
   GemmArgs a;
-  a.M = g.m, a.N = g.n, a.K = g.k, a.epi = g.epilogue;
+  a.M = g.m, a.N = g.n, a.K = g.k, a.epi = g.epilogue, a.rms = g.rms ? 1.f : 0.f;
   a.lda = a.K, a.ldc = g.epilogue == EPI_SWIGLU ? a.N / 2 : g.epilogue == EPI_SWIGLU_BWD ? 2 * a.N : a.N;
   a.ldr = a.N, a.ldp = g.epilogue == EPI_SWIGLU_BWD ? 2 * a.N : a.N;
   const size_t pre_size = m * size_t(a.ldp);

@@ -103,8 +103,8 @@ struct GemmArgs {
   // Unless null, each row's largest |C| is raised into c_max (atomicMax on the bits; the caller zeroed it).
   uint32_t* c_max = nullptr;
   // EPI_PLAIN, EPI_SWIGLU in the formats of several parts: the product of A's rows over their root mean squares (an RMSNorm, its
-  // gain in the weight).
-  bool rms = false;
+  // gain in the weight), unless 0; to the kernel 1 / K.
+  float rms = 0.f;
   float* C = nullptr;        // [M, N] (EPI_SWIGLU: [M,N/2]; EPI_SWIGLU_BWD: [M,2N])
   int ldc = 0;
   int M = 0, N = 0, K = 0;

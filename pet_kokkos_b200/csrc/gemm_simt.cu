@@ -155,7 +155,7 @@ void gemm(Stream& st, Arena& arena, const GemmArgs& a) {
   const GemmTask q{a, weight_of(a)};
   if (gemm_tensor_usable(st, a, q.w)) return gemm_tensor(st, arena, &q, 1);
   if (!a.B) throw Error(3, "gemm: this weight has no fp32 copy for the CUDA cores");
-  if (a.epi != EPI_PLAIN || a.bias || a.res || a.c_max || a.rms) throw Error(3, "gemm: the CUDA cores give the plain product alone");
+  if (a.epi != EPI_PLAIN || a.bias || a.res || a.c_max || a.rms != 0.f) throw Error(3, "gemm: the CUDA cores give the plain product alone");
   const long long tiles = (long long) cdiv(a.M, BM) * cdiv(a.N, BN);
   launch(st, k_gemm_native, (unsigned) tiles, 256, 0, a);
   PETB_LAUNCH_CHECK(st);

@@ -715,10 +715,10 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1) k_gemm_tc(co
         cluster_sync_all();
         if (!ok) return;
       }
-      if (kNorms && p.rms) {
+      if (kNorms && p.rms != 0.f) {
         if (!(ok = mbar_wait_warp(squares_there, norms & 1, abort_flag))) return;
         // (a row's largest value over its root mean square lies in [1, sqrt K]: the product with its scale is a normal number)
-        unscale *= 1.0f / sqrtf((squares[q * 32 + lane] + squares[TBM + q * 32 + lane]) / p.K + kRmsEps);
+        unscale *= reciprocal_root(fmaf(squares[q * 32 + lane] + squares[TBM + q * 32 + lane], p.rms, kRmsEps));
         __syncwarp();
         if (lane == 0) mbar_arrive(squares_read);
         ++norms;
@@ -757,7 +757,7 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1) k_gemm_tc(co
               scale_pair(v[j + 2 * i], v[j + 2 * i + 1], two[i] << 16, two[i] & 0xFFFF0000u, unscale);
           }
           if (kAhead) ask_scales(c + CS);
-        } else if (kNorms && p.rms) {
+        } else if (kNorms && p.rms != 0.f) {
 #pragma unroll
           for (int j = 0; j < AC; ++j) v[j] *= unscale;
         }
@@ -843,7 +843,7 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1) k_gemm_tc(co
           for (int c = 0; c < 8; ++c) v[c] = *reinterpret_cast<const float4*>(slab + swizzled<128>(r, c));
 #pragma unroll
           for (int c = 0; c < 8; ++c) {
-            if (kNorms && p.rms) add_squares(sq[0], v[c]);
+            if (kNorms && p.rms != 0.f) add_squares(sq[0], v[c]);
             split2<FMT>(v[c].x, v[c].y, s, part[0][2 * c], part[1][2 * c], part[2][2 * c]);
             split2<FMT>(v[c].z, v[c].w, s, part[0][2 * c + 1], part[1][2 * c + 1], part[2][2 * c + 1]);
           }
@@ -862,7 +862,7 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1) k_gemm_tc(co
         __syncwarp();
         if (lane == 0) mbar_arrive(ready + sp);
       }
-      if (ok && kNorms && p.rms) ok = hand_over(norms++, group, r, 0, sq, 1);
+      if (ok && kNorms && p.rms != 0.f) ok = hand_over(norms++, group, r, 0, sq, 1);
     }
   } else if (!L::T1) {
     if (L::kMoveRegs) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(L::kRegsConv));
@@ -907,7 +907,7 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1) k_gemm_tc(co
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
               const float4 v = *reinterpret_cast<const float4*>(slab + swizzled<64>(r, c));
-              if (kNorms && p.rms) add_squares(sq[j], v);
+              if (kNorms && p.rms != 0.f) add_squares(sq[j], v);
               *reinterpret_cast<float4*>(slab + L::kSlab + swizzled<64>(r, c)) =
                   make_float4(tf32_low(v.x), tf32_low(v.y), tf32_low(v.z), tf32_low(v.w));
             }
@@ -921,7 +921,7 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1) k_gemm_tc(co
           for (int c = 0; c < 4; ++c) {
             uint4 h, m, l;
             const float4 a = v[2 * c], b = v[2 * c + 1];
-            if (kNorms && p.rms) add_squares(sq[j], a), add_squares(sq[j], b);
+            if (kNorms && p.rms != 0.f) add_squares(sq[j], a), add_squares(sq[j], b);
             split2<FMT>(a.x, a.y, s, h.x, m.x, l.x), split2<FMT>(a.z, a.w, s, h.y, m.y, l.y);
             split2<FMT>(b.x, b.y, s, h.z, m.z, l.z), split2<FMT>(b.z, b.w, s, h.w, m.w, l.w);
             *reinterpret_cast<uint4*>(slab + swizzled<128>(r, c)) = h;
@@ -936,7 +936,7 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1) k_gemm_tc(co
           else mbar_arrive(ready + sa);
         }
       }
-      if (ok && kNorms && p.rms) ok = hand_over(norms++, group, first * 32 + lane, 32 * WPG, sq, 4 / WPG);
+      if (ok && kNorms && p.rms != 0.f) ok = hand_over(norms++, group, first * 32 + lane, 32 * WPG, sq, 4 / WPG);
     }
   }
   if (SPLIT && (warp < kEpiWarp0 || warp >= kConvWarp0)) {
@@ -991,6 +991,7 @@ Side make_side(const GemmTask& q) {
   const PackedB& w = q.w;
   Side s;
   s.p = a, s.b_unscale = w.unscale;
+  if (a.rms != 0.f) s.p.rms = 1.0f / a.K;
   s.map_a = map_2d(CU_TENSOR_MAP_DATA_TYPE_FLOAT32, a.A, a.K, a.M, size_t(a.lda) * 4, L::BK, box_rows(a.M),
                    L::T2 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B);
   const auto half = w.fmt == FMT_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
@@ -1098,7 +1099,7 @@ Plan plan_split(const GemmArgs& a, int bn_whole, int sms) {
   constexpr bool X3 = three_parts(FMT);
   const int steps = (a.K + 31) / 32, rows = cdiv(a.M, TBM);
   Plan best;
-  if (a.K < 1024 || a.K % 32 || a.N % 64 || a.rms) return best;
+  if (a.K < 1024 || a.K % 32 || a.N % 64 || a.rms != 0.f) return best;
   if (rows * cdiv(a.N, bn_whole) > sms) return best;
   best.clocks = (long long) steps * step_clocks<FMT>(width_index(bn_whole));
   for (int i = 0; i < 3; ++i)
@@ -1188,7 +1189,7 @@ Plan plan_two(const GemmArgs& a, const GemmArgs& b, int sms) {
       if (X3 && (EPI == EPI_SWIGLU || EPI == EPI_SWIGLU_BWD)) most += most / 4;
       if (most < best.clocks) best.bn = bn, best.pair = pair, best.parts = 1, best.rounds = rounds, best.clocks = most;
     }
-    if (EPI != EPI_PLAIN || bn != 64 || a.K < 1024 || a.K % 32 || a.rms || b.rms || (X3 && b.K > 1024)) continue;
+    if (EPI != EPI_PLAIN || bn != 64 || a.K < 1024 || a.K % 32 || a.rms != 0.f || b.rms != 0.f || (X3 && b.K > 1024)) continue;
     for (int parts = 2; parts <= 8; parts *= 2) {  // side 0's tiles shared as plan_split would (few rows: narrow tiles)
       if (bn / parts < (X3 ? 16 : 32) || sa % parts || sa / parts < 4) continue;
       if (X3 && parts != (a.K <= 1024 ? 1 : a.K <= 4096 ? 4 : cdiv(a.K, 1024))) continue;
@@ -1240,7 +1241,7 @@ extern template void run_format<EPI_PLAIN, FMT_F16X3_FULL>(Stream&, const GemmTa
 template <int EPI>
 void run_tensor(Stream& st, const GemmTask* q, int n) {
   for (int i = 0; i < n; ++i)
-    if (q[i].a.rms && ((EPI != EPI_PLAIN && EPI != EPI_SWIGLU) || (!three_parts(q[i].w.fmt) && q[i].w.fmt != FMT_F16X2 && q[i].w.fmt != FMT_TF32X2)))
+    if (q[i].a.rms != 0.f && ((EPI != EPI_PLAIN && EPI != EPI_SWIGLU) || (!three_parts(q[i].w.fmt) && q[i].w.fmt != FMT_F16X2 && q[i].w.fmt != FMT_TF32X2)))
       throw Error(3, "gemm: no kernel for this operand format and epilogue after a norm");
   switch (q[0].w.fmt) {
     case FMT_F16X3: return run_format<EPI, FMT_F16X3>(st, q, n);

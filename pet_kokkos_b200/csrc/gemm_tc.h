@@ -29,5 +29,11 @@ struct GemmTask {
 // One or two GEMMs of one epilogue and operand format; two go as one launch where that is expected to end first.
 template <int EPI>
 void run_tensor(Stream& st, const GemmTask* q, int n);
+extern template void run_tensor<EPI_PLAIN>(Stream&, const GemmTask*, int);
+extern template void run_tensor<EPI_SILU>(Stream&, const GemmTask*, int);
+extern template void run_tensor<EPI_SWIGLU>(Stream&, const GemmTask*, int);
+extern template void run_tensor<EPI_SILU_BWD>(Stream&, const GemmTask*, int);
+extern template void run_tensor<EPI_SWIGLU_BWD>(Stream&, const GemmTask*, int);
+extern template void run_tensor<EPI_COMPRESS>(Stream&, const GemmTask*, int);
 
 }  // namespace petb

@@ -596,7 +596,7 @@ PassOut Model::run_feedforward(Stream& st, Arena& save, Arena& tmp, const Packed
   };
   const auto gain_of = [&](const std::string& name) { return fold ? nullptr : vec(name + ".weight"); };
   const auto normed = [&](GemmArgs a) {
-    a.rms = fold;
+    a.rms = fold ? 1.f : 0.f;
     return a;
   };
   // qkv = W_in . norm(tokens) + b
