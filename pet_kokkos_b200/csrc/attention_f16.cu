@@ -23,9 +23,8 @@
 // dV = P^T dO and each key's column sum of dS is a row sum. Nothing S x S is stored and the warps never wait on each other
 // once the tile is staged. Every sum has one owner and a fixed order. Exponents are taken to base 2.
 //
-// What bounds it: latency (dependent products of three or six instructions, 20 warps an SM by registers), then the issue
-// slots: of about 400 instructions for 16 queries x 16 keys, 84 are products. Hence small CTAs, four of them on an SM at the
-// usual 80 rows: one stages its tile while the others multiply.
+// What bounds it: latency (a tile's loads; dependent products of three or six instructions; 15 to 20 warps an SM by registers and shared
+// memory). Hence small CTAs, three or four of them on an SM at the usual 80 rows: one stages its tile while the others multiply.
 #include <cuda_fp16.h>
 
 #include "attention.h"
@@ -250,11 +249,11 @@ __device__ __forceinline__ float max_abs(float m, const float4& x) {
 
 // A thread's 16 bytes of row r (a token row of the atom) of a tensor, in parts.
 template <int HD, int P>
-__device__ __forceinline__ void put(uint8_t* dst, int r, int c, const float4& x) {  // (x scaled)
+__device__ __forceinline__ void put(uint8_t* dst, int r, int c, const float4& x, int row_bytes = pitch<HD, P>()) {  // (x scaled)
   uint32_t lo[P], hi[P];
   split2<P>(x.x, x.y, lo), split2<P>(x.z, x.w, hi);
 #pragma unroll
-  for (int j = 0; j < P; ++j) *reinterpret_cast<uint2*>(dst + r * pitch<HD, P>() + j * HD * 2 + c * 2) = make_uint2(lo[j], hi[j]);
+  for (int j = 0; j < P; ++j) *reinterpret_cast<uint2*>(dst + r * row_bytes + j * HD * 2 + c * 2) = make_uint2(lo[j], hi[j]);
 }
 __device__ __forceinline__ float4 get(const float* src, size_t at, bool live) {
   return live ? __ldg(reinterpret_cast<const float4*>(src + at)) : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -409,7 +408,20 @@ __global__ void __launch_bounds__(32 * MAXB, MAXB <= 5 ? resident<HD, P, 3>(16 *
   }
 }
 
-template <int HD, int P, int MAXT, int BLOCKS>
+// Bytes of a row of V's tile where dS takes its place (ONCE): P parts of as many queries as the tile has rows.
+template <int HD, int P>
+__host__ __device__ constexpr int shared_pitch(int rows) {
+  return pitch<HD, P>() > P * rows * 2 + 16 ? pitch<HD, P>() : P * rows * 2 + 16;
+}
+
+// ONCE: a warp per block of 16 keys, no more. Scores and score adjoints are made once, transposed, by the warp that has the keys:
+// it sums dK and dV and leaves dS^T, in parts, in the rows of V's tile that are its keys' (nobody else reads those, and it has them
+// in registers); then, all warps' dS there, it takes the queries of the same rows for dQ = sc dS K. Per 16 x 16 block 60 products
+// instead of 84 (P = 2), 22 ldmatrix instead of 44, half the exponentials and splits; V's rows are longer, so fewer CTAs share an SM.
+// That alone gave 5 % (P = 1, 2; P = 3 lost 5): the warps waited for the tile's loads (two of eight stalled cycles) and for one another
+// behind them. With all of a thread's rows asked for at once (U) instead of in three trips: diamond1728 P = 2 2.16 ms -> 1.87, P = 3 3.64 ->
+// 3.57, 16-thousand-atom batch 9.25 -> 8.6, water1791 P = 1 0.737 -> 0.705 (U alone: 2.22, 3.65, 9.85, 0.705).
+template <int HD, int P, int MAXT, int BLOCKS, bool ONCE>
 __global__ void __launch_bounds__(MAXT, BLOCKS) k_attn_bwd_f16(AttnArgs p) {
   after_previous();
   constexpr int KS = HD / 16;
@@ -422,11 +434,12 @@ __global__ void __launch_bounds__(MAXT, BLOCKS) k_attn_bwd_f16(AttnArgs p) {
   const int e0 = p.off[n], cnt = p.off[n + 1] - e0 + 1;
   const int S16 = round16(cnt), SM = round16(p.S);
   constexpr int PB = pitch<HD, P>();
-  uint8_t *sq = smem, *sk = sq + SM * PB, *sv = sk + SM * PB, *sg = sv + SM * PB;
-  float *slc = reinterpret_cast<float*>(sg + SM * PB), *sm = slc + SM, *sl = sm + SM, *sd = sl + SM, *sn = sd + SM;
-  // Staging: a thread's loads of U rows' pieces are all under way before it looks for the tile's scales or splits any. The
+  const int PV = ONCE ? shared_pitch<HD, P>(SM) : PB;
+  uint8_t *sq = smem, *sk = sq + SM * PB, *sg = sk + SM * PB, *sv = sg + SM * PB;
+  float *slc = reinterpret_cast<float*>(sv + SM * PV), *sm = slc + SM, *sl = sm + SM, *sd = sl + SM, *sn = sd + SM, *su = sn + SM;  // (su: ONCE, P = 3)
+  // Staging: a thread's loads of U rows' pieces (of all its rows, up to five blocks) are all under way before it looks for the tile's scales or splits any. The
   // HD / 4 lanes that hold a row of dO, V and O add up its Dq = dO . O and its norms on the way.
-  constexpr int Q = HD / 4, U = 2;
+  constexpr int Q = HD / 4, U = MAXT <= 160 && HD <= 32 ? 4 : 2;
   float4 x0[U], x1[U], x2[U], x3[U], x4[U];
   auto fetch = [&](int t0) {
 #pragma unroll
@@ -476,7 +489,7 @@ __global__ void __launch_bounds__(MAXT, BLOCKS) k_attn_bwd_f16(AttnArgs p) {
       const int t = t0 + u * blockDim.x, r = t / Q, c = (t % Q) * 4;
       if (t >= S16 * Q) break;  // whole warps: a row block of 16 is 16 Q threads
       const float4 v = x2[u] * scv, go = x3[u] * scg;
-      put<HD, P>(sq, r, c, x0[u] * scq), put<HD, P>(sk, r, c, x1[u] * sck), put<HD, P>(sv, r, c, v), put<HD, P>(sg, r, c, go);
+      put<HD, P>(sq, r, c, x0[u] * scq), put<HD, P>(sk, r, c, x1[u] * sck), put<HD, P>(sv, r, c, v, PV), put<HD, P>(sg, r, c, go);
       float d = dot4(go, x4[u]), gg = dot4(go, go), vv = dot4(v, v);
 #pragma unroll
       for (int o = Q / 2; o > 0; o >>= 1) {
@@ -494,6 +507,96 @@ __global__ void __launch_bounds__(MAXT, BLOCKS) k_attn_bwd_f16(AttnArgs p) {
   const float f = usq * usk * p.sc * kLog2e;  // a scaled score product to a score, base 2
   const float vmax = sqrtf(__uint_as_float(s_vnorm)), gmax = sqrtf(__uint_as_float(s_gnorm));
   const int nb = S16 / 16;
+  if constexpr (ONCE) {
+    if (P == 3) {  // a query's own scale over the common one, and what undoes its own
+      const uint32_t all = __float_as_uint(fmaxf(2.1f * gmax * vmax, 1e-9f));
+      for (int r = threadIdx.x; r < S16; r += blockDim.x) {
+        const uint32_t own = __float_as_uint(fmaxf(2.1f * sn[r] * vmax, 1e-9f));
+        sn[r] = scale_of(own) * unscale_of(all), su[r] = unscale_of(own);
+      }
+      __syncthreads();
+    }
+    const int r0 = 16 * warp, i0 = r0 + g, i1 = r0 + g + 8;  // this lane's two rows: keys, then queries
+    const size_t g0 = i0 == 0 ? size_t(n) : size_t(p.N) + e0 + i0 - 1, g1 = size_t(p.N) + e0 + i1 - 1;
+    const uint32_t bound = __float_as_uint(fmaxf(2.1f * gmax * vmax, 1e-9f));  // |dP - D| at most: brings dS to 2^15 (see below)
+    if (warp < nb) {
+      uint32_t kf[KS][P][4], vf[KS][P][4];
+#pragma unroll
+      for (int ks = 0; ks < KS; ++ks)
+#pragma unroll
+        for (int j = 0; j < P; ++j) {
+          load_a<HD, P>(kf[ks][j], ak, r0, ks, j, lane);
+          ldsm4(vf[ks][j], av + (r0 + (lane & 15)) * PV + j * HD * 2 + ks * 32 + (lane >> 4) * 16);
+        }
+      __syncwarp();
+      const float lc0 = slc[i0], lc1 = slc[i1];
+      const float ds = scale_of(bound) * (1.f / 32768.f), fds = usv * unscale_of(bound) * usg;
+      float dk[HD / 8][4], dv[HD / 8][4];
+      clear<HD>(dk), clear<HD>(dv);
+      float cf0 = 0.f, cf1 = 0.f;
+      for (int b = 0; b < S16; b += 16) {
+        Acc<P, 2> c, w;
+        two_products<HD, P, true, true>(c, w, kf, vf, ak, av, r0, aq, ag, b, lane);
+        float x[2][4], y[2][4];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const int q = b + 8 * i + 2 * t;  // this lane's two queries of the block
+          const float2 m = *reinterpret_cast<const float2*>(sm + q), il = *reinterpret_cast<const float2*>(sl + q),
+                       d = *reinterpret_cast<const float2*>(sd + q);
+          // probabilities by 2^15, score adjoints by ds
+          x[i][0] = exp2_fast(fmaf(c.get(i, 0), f, lc0) - m.x) * il.x, x[i][1] = exp2_fast(fmaf(c.get(i, 1), f, lc0) - m.y) * il.y;
+          x[i][2] = exp2_fast(fmaf(c.get(i, 2), f, lc1) - m.x) * il.x, x[i][3] = exp2_fast(fmaf(c.get(i, 3), f, lc1) - m.y) * il.y;
+          y[i][0] = x[i][0] * ((w.get(i, 0) - d.x) * ds), y[i][1] = x[i][1] * ((w.get(i, 1) - d.y) * ds);
+          y[i][2] = x[i][2] * ((w.get(i, 2) - d.x) * ds), y[i][3] = x[i][3] * ((w.get(i, 3) - d.y) * ds);
+          cf0 += y[i][0] + y[i][1], cf1 += y[i][2] + y[i][3];
+        }
+        uint32_t a[with_sum<P>()][4];
+        make_a<P>(a, y);
+        product_rows<HD, P>(dk, a, aq, b, lane);
+        if (P == 3) {  // the leading part of a query's row of dS, as dQ wants it, is that of the row's own largest value
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            const float2 o = *reinterpret_cast<const float2*>(sn + b + 8 * i + 2 * t);
+            y[i][0] *= o.x, y[i][1] *= o.y, y[i][2] *= o.x, y[i][3] *= o.y;
+          }
+          make_a<P>(a, y);
+        }
+#pragma unroll
+        for (int j = 0; j < P; ++j)
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            uint8_t* at = sv + size_t(i0) * PV + j * SM * 2 + (b + 8 * i + 2 * t) * 2;
+            *reinterpret_cast<uint32_t*>(at) = a[j][2 * i], *reinterpret_cast<uint32_t*>(at + 8 * PV) = a[j][2 * i + 1];
+          }
+        make_a<P>(a, x);
+        product_rows<HD, P>(dv, a, ag, b, lane);
+      }
+      cf0 += __shfl_xor_sync(0xffffffffu, cf0, 1), cf0 += __shfl_xor_sync(0xffffffffu, cf0, 2);
+      cf1 += __shfl_xor_sync(0xffffffffu, cf1, 1), cf1 += __shfl_xor_sync(0xffffffffu, cf1, 2);
+      write_rows<HD>(p.qkv_adj, 3 * D, D + h * HD, g0, g1, i0 < cnt, i1 < cnt, dk, fds * usq * p.sc, fds * usq * p.sc, p.qkv_adj_max, t);
+      write_rows<HD>(p.qkv_adj, 3 * D, 2 * D + h * HD, g0, g1, i0 < cnt, i1 < cnt, dv, usg * (1.f / 32768.f), usg * (1.f / 32768.f),
+                     p.qkv_adj_max, t);
+      if (t == 0) {  // each key's dS summed over its queries: the cutoff factor's share from this head
+        if (i0 < cnt) p.cfh[g0 * p.H + h] = cf0 * fds;
+        if (i1 < cnt) p.cfh[g1 * p.H + h] = cf1 * fds;
+      }
+    }
+    __syncthreads();
+    if (warp >= nb) return;
+    float dq[HD / 8][4];
+    clear<HD>(dq);
+    for (int b = 0; b < S16; b += 16) {
+      uint32_t a[with_sum<P>()][4];
+#pragma unroll
+      for (int j = 0; j < P; ++j)  // 8 x 8 blocks of dS^T, keys down, turned: rows of 16 queries, 16 keys of the contraction
+        ldsm4_t(a[j], av + (b + (lane >> 4) * 8 + (lane & 7)) * PV + j * SM * 2 + (r0 + ((lane >> 3) & 1) * 8) * 2);
+      add_sum<P>(a);
+      product_rows<HD, P>(dq, a, ak, b, lane);
+    }
+    const float f0 = usv * usk * usg * p.sc * (P == 3 ? su[i0] : unscale_of(bound)), f1 = usv * usk * usg * p.sc * (P == 3 ? su[i1] : unscale_of(bound));
+    write_rows<HD>(p.qkv_adj, 3 * D, h * HD, g0, g1, i0 < cnt, i1 < cnt, dq, f0, f1, p.qkv_adj_max, t);
+    return;
+  }
   for (int task = warp; task < 2 * nb; task += nw) {
     const bool keys = task >= nb;
     const int r0 = 16 * (keys ? task - nb : task);
@@ -602,15 +705,23 @@ bool fwd_hd(Stream& st, const AttnArgs& p) {
 }
 template <int HD, int P>
 bool bwd_hd(Stream& st, const AttnArgs& p) {
-  const int blocks = round16(p.S) / 16;
-  const size_t bytes = size_t(round16(p.S)) * (4 * pitch<HD, P>() + 5 * sizeof(float));
+  const int rows = round16(p.S), blocks = rows / 16;
+  const size_t bytes = size_t(rows) * (4 * pitch<HD, P>() + 5 * sizeof(float));
   if (bytes > kMaxBytes) return false;
-  static SmemOptIn o160, o320, o640;
+  static SmemOptIn o128, o160, o320, o640;
+  // Up to five blocks of 16 rows, heads of at most 32: scores once (a head size of 64 has no registers for two tensors' operands).
+  if constexpr (HD <= 32)
+    if (blocks <= 5) {
+      const size_t once = size_t(rows) * (3 * pitch<HD, P>() + shared_pitch<HD, P>(rows) + 6 * sizeof(float));
+      if (blocks <= 4) launch(st, k_attn_bwd_f16<HD, P, 128, P == 3 ? 3 : P == 2 ? 4 : 5, true>, p, once, 32 * blocks, o128);
+      else launch(st, k_attn_bwd_f16<HD, P, 160, P == 3 ? 2 : P == 2 ? 3 : 4, true>, p, once, 32 * blocks, o160);
+      return true;
+    }
   // A warp per 16 rows, which takes queries and then keys, where several CTAs share an SM; where one tile fills it, a warp
   // per 16 queries and one per 16 keys, up to 20: then blocks in turn.
-  if (blocks <= 5) launch(st, k_attn_bwd_f16<HD, P, 160, resident<HD, P, 4>(80)>, p, bytes, 32 * blocks, o160);
-  else if (bytes <= 110 * 1024) launch(st, k_attn_bwd_f16<HD, P, 320, 2>, p, bytes, 32 * (blocks < 10 ? blocks : 10), o320);
-  else launch(st, k_attn_bwd_f16<HD, P, 640, 1>, p, bytes, 64 * (blocks < 10 ? blocks : 10), o640);
+  if (HD > 32 && blocks <= 5) launch(st, k_attn_bwd_f16<HD, P, 160, resident<HD, P, 4>(80), false>, p, bytes, 32 * blocks, o160);
+  else if (bytes <= 110 * 1024) launch(st, k_attn_bwd_f16<HD, P, 320, 2, false>, p, bytes, 32 * (blocks < 10 ? blocks : 10), o320);
+  else launch(st, k_attn_bwd_f16<HD, P, 640, 1, false>, p, bytes, 64 * (blocks < 10 ? blocks : 10), o640);
   return true;
 }
 template <int P>
