@@ -464,15 +464,17 @@ PassOut Model::finish(Stream& st, Arena& save, const PackedEdges& pk, bool grad,
   PassOut out;
   out.per_atom = per_atom;
   out.f.energy = save.alloc<double>(pk.B);
-  structure_energy(st, out.f.energy, per_atom, pk.soff, pk.B);
-  if (!grad) return out;
+  if (!grad) {
+    const ProfScope ps(st, PC_FORCES, 0.0, 8.0 * pk.B);
+    structure_sums(st, out.f.energy, nullptr, per_atom, nullptr, pk.soff, pk.B);
+    return out;
+  }
   out.has_forces = true;
   out.f.edge_grad = save.alloc<double>(3 * size_t(pk.E > 0 ? pk.E : 1));
   out.f.forces = save.alloc<double>(3 * size_t(pk.n_atoms));
   out.f.vir_atom = save.alloc<double>(9 * size_t(pk.n_atoms));
-  out.f.vir9 = save.alloc<double>(9 * size_t(pk.B));
   out.f.vir6 = save.alloc<double>(6 * size_t(pk.B));
-  forces_and_virial(st, save, out.f, pk, x4_adj, cutoff_adj, cf_adj, cutoff_spec(), scale_);
+  forces_and_virial(st, save, out.f, pk, x4_adj, cutoff_adj, cf_adj, cutoff_spec(), scale_, out.f.energy, per_atom);
   return out;
 }
 
@@ -517,10 +519,10 @@ MemoryNeed Model::memory_need(int tier, int N, int E, int n_live) const {
   const double layer = (A + 1) * T * D + e * 3 * D + A * block + (relayer ? n * Dn : 0.0);
   save += (relayer ? 1.0 : G) * layer;
   save += 2 * n * Dh + 2 * e * Dh + 2 * n + e + 2 * n;              // readout
-  save += 5 * e + n * Dn + e * D + T * D + 6 * e + 30 * n;          // adjoints, edge gradients (doubles), forces, virials
+  save += G * A * T * H + 5 * e + n * Dn + e * D + T * D + 6 * e + 30 * n;          // adjoints, edge gradients (doubles), forces, virials
   save += double(row_maxima_words(N, E)) * (relayer ? 2 : 1);       // (a layer run again takes its own)
   // tmp: the fullest scope
-  const double attention_bwd = T * (5 * D + H) + (keep ? 0.0 : T * 4 * D);
+  const double attention_bwd = T * 5 * D + (keep ? 0.0 : T * 4 * D);
   const double norms = folds_norms() ? 0.0 : 1.0;  // the norms' rows
   const double attention_fwd = norms * T * D + (keep ? 0.0 : T * 3 * D);
   const double edge_mlp = c * (2 * F + D) + (keep ? c * F : c * (2 * F + norms * D)) + n * 5 * Dn;  // (beside the atoms')
@@ -734,8 +736,8 @@ PassOut Model::run_feedforward(Stream& st, Arena& save, Arena& tmp, const Packed
   if (relayer)
     for (int L = 0; L < G; ++L) ie_at[L] = {save.alloc<float>(Ea * D)};  // input_edge as it entered layer L
   node_at[0].mx = maxima.take(Na);
-  gather_rows(st, node_at[0].p, mat("node_embedders.0.weight").w, pk.atom_species, N, Dn, node_at[0].mx);
-  gather_rows(st, input_edge.p, mat("edge_embedder.weight").w, pk.species, E, D);
+  gather_rows_two(st, node_at[0].p, mat("node_embedders.0.weight").w, pk.atom_species, N, Dn, node_at[0].mx, input_edge.p,
+                  mat("edge_embedder.weight").w, pk.species, E, D);
   for (int L = 0; L < G; ++L) {
     if (relayer) {
       ie_at[L].mx = input_edge.mx;
@@ -773,15 +775,17 @@ PassOut Model::run_feedforward(Stream& st, Arena& save, Arena& tmp, const Packed
   }
   tap(taps, "node_pred", node_pred, N);
   tap(taps, "edge_pred", edge_pred, E);
-  PETB_CUDA(cudaMemsetAsync(per_atom, 0, sizeof(double) * size_t(pk.n_atoms > 0 ? pk.n_atoms : 1), st.s));
+  if (pk.n_atoms != N)  // (the readout writes those of the centres)
+    PETB_CUDA(cudaMemsetAsync(per_atom, 0, sizeof(double) * size_t(pk.n_atoms > 0 ? pk.n_atoms : 1), st.s));
   readout_energy(st, net, per_atom, node_pred, edge_pred, pk, comp_, scale_, false, true);
   if (!grad) return finish(st, save, pk, false, nullptr, nullptr, nullptr, per_atom);
 
   // ---- backward (src/model.cpp:749-778, src/feedforward.cpp:199-336) ----
   float* x4_adj = save.alloc<float>(Ea * 4);
   float* cf_adj = save.alloc<float>(Ea);
-  PETB_CUDA(cudaMemsetAsync(x4_adj, 0, sizeof(float) * Ea * 4, st.s));
-  PETB_CUDA(cudaMemsetAsync(cf_adj, 0, sizeof(float) * Ea, st.s));
+  const size_t head_words = Ta * H;
+  float* heads = save.alloc<float>(size_t(G) * A * head_words);  // each block's share of every head in the edges' cutoff factors,
+  int blocks_done = 0;                                           // in the order of the backward
   Rows node_adj = maxima.fresh(save.alloc<float>(Na * Dn), Na), ie_adj = maxima.fresh(save.alloc<float>(Ea * D), Ea);
   Rows tok_adj = {save.alloc<float>(Ta * D)};
   {
@@ -879,7 +883,7 @@ PassOut Model::run_feedforward(Stream& st, Arena& save, Arena& tmp, const Packed
         Scope s10(tmp);
         const Rows dmerged = Rows{tmp.alloc<float>(Ta * D)};
         const Rows qkv_adj = maxima.fresh(tmp.alloc<float>(Ta * 3 * D), Ta);
-        float* cfh = tmp.alloc<float>(Ta * H);
+        float* cfh = heads + size_t(blocks_done++) * head_words;
         float* attn_in_adj = tmp.alloc<float>(Ta * D);
         Rows qkv = b.qkv;
         if (!qkv.p) {
@@ -891,7 +895,6 @@ PassOut Model::run_feedforward(Stream& st, Arena& save, Arena& tmp, const Packed
         AttnArgs at = attention_args(b, qkv);
         at.dmerged = dmerged.p, at.qkv_adj = qkv_adj.p, at.qkv_adj_max = qkv_adj.mx, at.cfh = cfh;
         attention_backward(st, at);
-        cutoff_share(st, cf_adj, cfh, pk.cut, N, E, H);
         gm.linear_bwd({attn_in_adj}, qkv_adj, mat(tl + ".attention.input_linear.weight"), T, false);
         // through the norm, back to where the tokens came from: atom rows to the contraction's
         // output adjoint (written), edge rows onto the edge residual (accumulated)
@@ -905,11 +908,12 @@ PassOut Model::run_feedforward(Stream& st, Arena& save, Arena& tmp, const Packed
       Scope s11(tmp);
       const Rows gz = maxima.fresh(tmp.alloc<float>(Ea * D), Ea);
       gm.linear_silu_bwd(gz, tok_adj.from(N, D), mat(g + ".compress.2.weight"), sl.cpre, E);
-      compress_geometry_bwd(st, x4_adj, gz.p, mat(c0 + "@x4").w, E, D);
+      compress_geometry_bwd(st, x4_adj, gz.p, mat(c0 + "@x4").w, E, D, L + 1 < G);
       ie_adj.mx = maxima.take(Ea);
       if (L > 0) gm.linear_bwd(ie_adj, gz, mat(c0 + "@in"), E, true);
     }
   }
+  cutoff_share(st, cf_adj, heads, head_words, blocks_done, pk.cut, N, E, H);
   tap(taps, "x4_adj", x4_adj, size_t(E) * 4);
   tap(taps, "cf_adj", cf_adj, E);
   return finish(st, save, pk, true, x4_adj, edge_pred, cf_adj, per_atom);
@@ -946,7 +950,8 @@ PassOut Model::run_residual(Stream& st, Arena& save, Arena& tmp, const PackedEdg
   float* net = save.alloc<float>(Na);
   float* node_pred = save.alloc<float>(Na);
   double* per_atom = save.alloc<double>(pk.n_atoms > 0 ? pk.n_atoms : 1);
-  PETB_CUDA(cudaMemsetAsync(per_atom, 0, sizeof(double) * size_t(pk.n_atoms > 0 ? pk.n_atoms : 1), st.s));
+  if (pk.n_atoms != N)  // (the readout writes those of the centres)
+    PETB_CUDA(cudaMemsetAsync(per_atom, 0, sizeof(double) * size_t(pk.n_atoms > 0 ? pk.n_atoms : 1), st.s));
 
   for (int L = 0; L < G; ++L) {
     const std::string g = "gnn_layers." + std::to_string(L), ls = std::to_string(L), c0 = g + ".compress.0";
@@ -1038,8 +1043,9 @@ PassOut Model::run_residual(Stream& st, Arena& save, Arena& tmp, const PackedEdg
   float* x4_adj = save.alloc<float>(Ea * 4);
   float* cf_adj = save.alloc<float>(Ea);
   float* cutoff_adj = save.alloc<float>(Ea);  // sum over layers of the edge predictions
-  PETB_CUDA(cudaMemsetAsync(x4_adj, 0, sizeof(float) * Ea * 4, st.s));
-  PETB_CUDA(cudaMemsetAsync(cf_adj, 0, sizeof(float) * Ea, st.s));
+  const size_t head_words = Ta * H;
+  float* heads = save.alloc<float>(size_t(G) * A * head_words);  // each block's share of every head in the edges' cutoff factors,
+  int blocks_done = 0;                                           // in the order of the backward
   PETB_CUDA(cudaMemcpyAsync(cutoff_adj, sav[0].edge_pred, sizeof(float) * Ea, cudaMemcpyDeviceToDevice, st.s));
   for (int L = 1; L < G; ++L) add_inplace(st, cutoff_adj, sav[L].edge_pred, size_t(E));
   float* ie_a = save.alloc<float>(Ea * D);
@@ -1100,7 +1106,7 @@ PassOut Model::run_residual(Stream& st, Arena& save, Arena& tmp, const PackedEdg
         Scope s6(tmp);
         const Rows dmerged = Rows{tmp.alloc<float>(Ta * D)};
         const Rows qkv_adj = maxima.fresh(tmp.alloc<float>(Ta * 3 * D), Ta);
-        float* cfh = tmp.alloc<float>(Ta * H);
+        float* cfh = heads + size_t(blocks_done++) * head_words;
         gm.linear_bwd(dmerged, s1_adj, mat(tl + ".attention.output_linear.weight"), T, false);
         AttnArgs at;
         at.N = N, at.H = H, at.hd = hd, at.S = S, at.sc = sc, at.off = pk.off, at.cut = pk.cut;
@@ -1110,7 +1116,6 @@ PassOut Model::run_residual(Stream& st, Arena& save, Arena& tmp, const PackedEdg
         at.qkv_adj = qkv_adj.p, at.cfh = cfh;
         at.qkv_adj_max = qkv_adj.mx;
         attention_backward(st, at);
-        cutoff_share(st, cf_adj, cfh, pk.cut, N, E, H);
         s1_adj.mx = maxima.take(Ta);
         gm.linear_bwd(s1_adj, qkv_adj, mat(tl + ".attention.input_linear.weight"), T, true);
       }
@@ -1121,11 +1126,12 @@ PassOut Model::run_residual(Stream& st, Arena& save, Arena& tmp, const PackedEdg
       Scope s7(tmp);
       const Rows gz = maxima.fresh(tmp.alloc<float>(Ea * D), Ea);
       gm.linear_silu_bwd(gz, tokens_adj.from(N, D), mat(g + ".compress.2.weight"), sl.cpre, E);
-      compress_geometry_bwd(st, x4_adj, gz.p, mat(c0 + "@x4").w, E, D);
+      compress_geometry_bwd(st, x4_adj, gz.p, mat(c0 + "@x4").w, E, D, L + 1 < G);
       if (L > 0) gm.linear_bwd({ie_next}, gz, mat(c0 + "@in"), E, true);
     }
     ie_adj = ie_next;
   }
+  cutoff_share(st, cf_adj, heads, head_words, blocks_done, pk.cut, N, E, H);
   return finish(st, save, pk, true, x4_adj, cutoff_adj, cf_adj, per_atom);
 }
 

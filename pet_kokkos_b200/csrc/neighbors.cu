@@ -93,7 +93,7 @@ __device__ inline int warp_inclusive(int v, int lane) {
   return v;
 }
 
-// Exclusive scan of a block's chunk into out, its total into sums[block].
+// Exclusive scan of a block's chunk into out, its total into sums[block] (one chunk: into out[n], and nothing is left to do).
 __global__ void __launch_bounds__(kScanThreads) k_scan_chunks(const int* __restrict__ in, int* __restrict__ out,
                                                               int* __restrict__ sums, int n) {
   after_previous();
@@ -121,7 +121,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_chunks(const int* __restr
     if (base + k < n) out[base + k] = run;
     run += v[k];
   }
-  if (threadIdx.x == kScanThreads - 1) sums[blockIdx.x] = run;
+  if (threadIdx.x == kScanThreads - 1) *(gridDim.x == 1 ? out + n : sums + blockIdx.x) = run;
 }
 
 // One block: exclusive scan of the chunk totals in place, the grand total into *total.
@@ -170,12 +170,11 @@ void exclusive_scan(Stream& st, Arena& arena, const int* in, int* out, int n) {
   int* sums = arena.alloc<int>(nb);
   launch(st, k_scan_chunks, nb, kScanThreads, 0, in, out, sums, n);
   PETB_LAUNCH_CHECK(st);
+  if (nb == 1) return;
   launch(st, k_scan_sums, 1, 1024, 0, sums, nb, out + n);
   PETB_LAUNCH_CHECK(st);
-  if (nb > 1) {
-    launch(st, k_scan_add, nb, kScanThreads, 0, out, sums, n);
-    PETB_LAUNCH_CHECK(st);
-  }
+  launch(st, k_scan_add, nb, kScanThreads, 0, out, sums, n);
+  PETB_LAUNCH_CHECK(st);
 }
 
 // ---- wrap, bins ------------------------------------------------------------------

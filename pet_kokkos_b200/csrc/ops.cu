@@ -39,37 +39,52 @@ __device__ __forceinline__ void raise_row(uint32_t* mx, int r, int D4, float m) 
   atomicMax(mx + r, __float_as_uint(m));
 }
 
-__global__ void k_gather_rows(float* __restrict__ out, const float* __restrict__ table, const int* __restrict__ idx, int R,
-                              int D4, uint32_t* __restrict__ mx) {
+// out(r, :) = table(idx(r), :). Two tables' lookups in one launch: blocks from `blocks0` on do the second's.
+struct Lookup {
+  float* out;
+  const float* table;
+  const int* idx;
+  uint32_t* mx;
+  int R, D4;
+};
+__global__ void k_gather_rows(Lookup first, Lookup second, int blocks0) {
   after_previous();
-  const size_t t = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (t >= size_t(R) * D4) return;
-  const int r = int(t / D4), q = int(t % D4);
-  const float4 v = reinterpret_cast<const float4*>(table)[size_t(idx[r]) * D4 + q];
-  reinterpret_cast<float4*>(out)[t] = v;
-  raise_row(mx, r, D4, max4(v));
+  const bool one = int(blockIdx.x) < blocks0;
+  const Lookup& p = one ? first : second;
+  const size_t t = size_t(blockIdx.x - (one ? 0 : blocks0)) * blockDim.x + threadIdx.x;
+  if (t >= size_t(p.R) * p.D4) return;
+  const int r = int(t / p.D4), q = int(t % p.D4);
+  const float4 v = reinterpret_cast<const float4*>(p.table)[size_t(p.idx[r]) * p.D4 + q];
+  reinterpret_cast<float4*>(p.out)[t] = v;
+  raise_row(p.mx, r, p.D4, max4(v));
 }
 
-__global__ void k_compress0(GemmArgs p) {
+// A thread has four columns of `rows` neighbouring rows: the columns' weights (64 bytes a column, four times what it writes of a
+// row) are read once for all of them. 120314 x 256: 104 us with a row a thread, 56 with eight; 38 at HBM's rate.
+__global__ void __launch_bounds__(256) k_compress0(GemmArgs p, int rows) {
   after_previous();
   const size_t t = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  const int D4 = p.N / 4;
-  if (t >= size_t(p.M) * D4) return;
-  const size_t row = t / D4;
-  const int col = int(t % D4) * 4;
-  const float4 b = ld4(p.bias + col), tt = ld4(p.tab + size_t(p.sp[row]) * p.N + col);
-  const float e0 = (float) p.vec[3 * row], e1 = (float) p.vec[3 * row + 1], e2 = (float) p.vec[3 * row + 2], e3 = (float) p.dist[row];
-  float z[4] = {b.x, b.y, b.z, b.w};
-  const float from_table[4] = {tt.x, tt.y, tt.z, tt.w};
+  const int D4 = p.N / 4, col = int(t % D4) * 4;
+  const size_t first = t / D4 * rows;
+  if (first >= size_t(p.M)) return;
+  const float4 b = ld4(p.bias + col);
+  float4 w[4];
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const float4 w = ld4(p.wx + size_t(col + j) * 4);
-    z[j] = z[j] + from_table[j] + w.x * e0 + w.y * e1 + w.z * e2 + w.w * e3;
+  for (int j = 0; j < 4; ++j) w[j] = ld4(p.wx + size_t(col + j) * 4);
+  const size_t end = first + rows < size_t(p.M) ? first + rows : size_t(p.M);
+#pragma unroll 2
+  for (size_t row = first; row < end; ++row) {
+    const float4 tt = ld4(p.tab + size_t(p.sp[row]) * p.N + col);
+    const float e0 = (float) p.vec[3 * row], e1 = (float) p.vec[3 * row + 1], e2 = (float) p.vec[3 * row + 2], e3 = (float) p.dist[row];
+    float z[4] = {b.x, b.y, b.z, b.w};
+    const float from_table[4] = {tt.x, tt.y, tt.z, tt.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) z[j] = z[j] + from_table[j] + w[j].x * e0 + w[j].y * e1 + w[j].z * e2 + w[j].w * e3;
+    st4(p.pre + row * p.ldp + col, make_float4(z[0], z[1], z[2], z[3]));
+    const float4 o = make_float4(silu_f(z[0]), silu_f(z[1]), silu_f(z[2]), silu_f(z[3]));
+    st4(p.C + row * p.ldc + col, o);
+    raise_row(p.c_max, int(row), D4, max_abs4(o.x, o.y, o.z, o.w));
   }
-  st4(p.pre + row * p.ldp + col, make_float4(z[0], z[1], z[2], z[3]));
-  const float4 o = make_float4(silu_f(z[0]), silu_f(z[1]), silu_f(z[2]), silu_f(z[3]));
-  st4(p.C + row * p.ldc + col, o);
-  raise_row(p.c_max, int(row), D4, max_abs4(o.x, o.y, o.z, o.w));
 }
 
 // One warp per row. x = in (+ add, stored back); out = (x - mu) inv w + b.
@@ -588,7 +603,7 @@ __global__ void __launch_bounds__(256) k_concat_norm_remote_bwd(float* __restric
 }
 
 __global__ void __launch_bounds__(256) k_compress_geometry_bwd(float* __restrict__ x4_adj, const float* __restrict__ g,
-                                                               const float* __restrict__ wx, int E, int D) {
+                                                               const float* __restrict__ wx, int E, int D, bool add) {
   after_previous();
   const int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (k >= E) return;
@@ -600,7 +615,7 @@ __global__ void __launch_bounds__(256) k_compress_geometry_bwd(float* __restrict
   }
   a0 = warp_sum(a0), a1 = warp_sum(a1), a2 = warp_sum(a2), a3 = warp_sum(a3);
   if (lane == 0) {
-    float4 v = ld4(x4_adj + 4 * size_t(k));
+    float4 v = add ? ld4(x4_adj + 4 * size_t(k)) : make_float4(0.f, 0.f, 0.f, 0.f);
     v.x += a0, v.y += a1, v.z += a2, v.w += a3;
     st4(x4_adj + 4 * size_t(k), v);
   }
@@ -639,16 +654,20 @@ __global__ void k_readout_seed_bwd(float* __restrict__ out, const float* __restr
   raise_row(mx, r, Dh4, max4(v));
 }
 
-__global__ void k_cutoff_share(float* __restrict__ cf_adj, const float* __restrict__ cfh, const float* __restrict__ cut, int N,
-                               int E, int H) {
+__global__ void k_cutoff_share(float* __restrict__ cf_adj, const float* __restrict__ cfh, size_t stride, int blocks, const float* __restrict__ cut,
+                               int N, int E, int H) {
   after_previous();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= E) return;
   const float cf = cut[k];
-  if (cf <= 0.f) return;
-  float total = 0.f;
-  for (int h = 0; h < H; ++h) total += cfh[size_t(N + k) * H + h];
-  cf_adj[k] += total / cf;
+  float sum = 0.f;
+  if (cf > 0.f)
+    for (int b = 0; b < blocks; ++b, cfh += stride) {
+      float total = 0.f;
+      for (int h = 0; h < H; ++h) total += cfh[size_t(N + k) * H + h];
+      sum += total / cf;
+    }
+  cf_adj[k] = sum;
 }
 
 __global__ void k_add_inplace(float* __restrict__ a, const float* __restrict__ b, size_t n) {
@@ -751,31 +770,38 @@ __global__ void __launch_bounds__(256) k_fold_forces(ForceOut out, PackedEdges p
   }
 }
 
-// out[b T + t] = the sum over structure b's atoms of x[a T + t]. A block per sum, whose warps' parts are added in order: a
-// warp alone takes 12 us for 1728 atoms, one trip to L2 after another.
-__global__ void __launch_bounds__(256) k_struct_sum(double* __restrict__ out, const double* __restrict__ x, const int* __restrict__ soff, int T) {
+// Structure b's energy and, unless w6 is null, its virial in Voigt's order from the atoms' 3 x 3: the ordered sum over its atoms, of both
+// elements of a symmetric pair where there are two. A block per sum, whose warps' parts are added in order: a warp alone takes 12 us
+// for 1728 atoms, one trip to L2 after another. All of them in one launch (three launches before).
+__global__ void __launch_bounds__(256) k_struct_sums(double* __restrict__ energy, double* __restrict__ w6, const double* __restrict__ per_atom,
+                                                     const double* __restrict__ vir_atom, const int* __restrict__ soff) {
   after_previous();
-  __shared__ double part[8];
-  const int b = blockIdx.x / T, t = blockIdx.x % T, end = soff[b + 1];
-  double s = 0.0;
+  __shared__ double part[2][8];
+  const int T = w6 ? 7 : 1, b = blockIdx.x / T, t = blockIdx.x % T, end = soff[b + 1];
+  const bool is_energy = t + 1 == T;
+  constexpr int first[6] = {0, 4, 8, 1, 2, 5}, second[6] = {0, 4, 8, 3, 6, 7};
+  const double *x = per_atom, *y = per_atom;
+  int ld = 1;
+  if (!is_energy) {
+    ld = 9;
+#pragma unroll
+    for (int i = 0; i < 6; ++i)
+      if (i == t) x = vir_atom + first[i], y = vir_atom + second[i];
+  }
+  const bool pair = x != y;
+  double s = 0.0, r = 0.0;
 #pragma unroll 4
-  for (int a = soff[b] + threadIdx.x; a < end; a += 256) s += x[size_t(a) * T + t];
-  s = warp_sum(s);
-  if (threadIdx.x % 32 == 0) part[threadIdx.x / 32] = s;
+  for (int a = soff[b] + threadIdx.x; a < end; a += 256) {
+    s += x[size_t(a) * ld];
+    if (pair) r += y[size_t(a) * ld];
+  }
+  s = warp_sum(s), r = warp_sum(r);
+  if (threadIdx.x % 32 == 0) part[0][threadIdx.x / 32] = s, part[1][threadIdx.x / 32] = r;
   __syncthreads();
   if (threadIdx.x) return;
-  for (int w = 1; w < 8; ++w) s += part[w];
-  out[blockIdx.x] = s;
-}
-
-__global__ void k_voigt(double* __restrict__ w6, const double* __restrict__ w9, int B) {
-  after_previous();
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= B) return;
-  const double* w = w9 + 9 * b;
-  double* o = w6 + 6 * b;
-  o[0] = w[0], o[1] = w[4], o[2] = w[8];
-  o[3] = 0.5 * (w[1] + w[3]), o[4] = 0.5 * (w[2] + w[6]), o[5] = 0.5 * (w[5] + w[7]);
+  for (int w = 1; w < 8; ++w) s += part[0][w], r += part[1][w];
+  if (is_energy) energy[b] = s;
+  else w6[6 * b + t] = pair ? 0.5 * (s + r) : s;
 }
 
 inline unsigned blocks_for(size_t n, int per) { return (unsigned) ((n + per - 1) / per); }
@@ -783,9 +809,15 @@ inline unsigned blocks_for(size_t n, int per) { return (unsigned) ((n + per - 1)
 }  // namespace
 
 void gather_rows(Stream& st, float* out, const float* table, const int* idx, int R, int D, uint32_t* mx) {
-  if (R == 0) return;
-  const ProfScope ps(st, PC_GATHER, 0.0, 8.0 * double(R) * D);
-  launch(st, k_gather_rows, blocks_for(size_t(R) * (D / 4), 256), 256, 0, out, table, idx, R, D / 4, mx);
+  gather_rows_two(st, out, table, idx, R, D, mx, nullptr, nullptr, nullptr, 0, 4);
+}
+void gather_rows_two(Stream& st, float* out, const float* table, const int* idx, int R, int D, uint32_t* mx, float* out2, const float* table2,
+                     const int* idx2, int R2, int D2) {
+  if (R == 0 && R2 == 0) return;
+  const ProfScope ps(st, PC_GATHER, 0.0, 8.0 * (double(R) * D + double(R2) * D2));
+  const unsigned blocks0 = blocks_for(size_t(R) * (D / 4), 256);
+  launch(st, k_gather_rows, blocks0 + blocks_for(size_t(R2) * (D2 / 4), 256), 256, 0, Lookup{out, table, idx, mx, R, D / 4},
+         Lookup{out2, table2, idx2, nullptr, R2, D2 / 4}, int(blocks0));
   PETB_LAUNCH_CHECK(st);
 }
 
@@ -796,7 +828,8 @@ void compress0(Stream& st, float* out, float* pre, const float* b, const float* 
   GemmArgs p;
   p.M = pk.E, p.N = D, p.C = out, p.ldc = D, p.pre = pre, p.ldp = D, p.bias = b, p.tab = tab, p.wx = wx, p.sp = pk.species;
   p.vec = pk.vec, p.dist = pk.dist, p.c_max = mx, p.epi = EPI_COMPRESS;
-  launch(st, k_compress0, blocks_for(size_t(pk.E) * (D / 4), 256), 256, 0, p);
+  const int rows = pk.E < 16384 ? 1 : 8;  // (few rows: all SMs)
+  launch(st, k_compress0, blocks_for(size_t(cdiv(pk.E, rows)) * (D / 4), 256), 256, 0, p, rows);
   PETB_LAUNCH_CHECK(st);
 }
 
@@ -885,10 +918,10 @@ void concat_norm_remote_bwd(Stream& st, float* send, const float* out_adj, const
   PETB_LAUNCH_CHECK(st);
 }
 
-void compress_geometry_bwd(Stream& st, float* x4_adj, const float* g, const float* wx, int E, int D) {
+void compress_geometry_bwd(Stream& st, float* x4_adj, const float* g, const float* wx, int E, int D, bool add) {
   if (E == 0) return;
   const ProfScope ps(st, PC_ELEMENTWISE, 8.0 * double(E) * D, 4.0 * double(E) * D);
-  launch(st, k_compress_geometry_bwd, blocks_for(size_t(E) * 32, 256), 256, 0, x4_adj, g, wx, E, D);
+  launch(st, k_compress_geometry_bwd, blocks_for(size_t(E) * 32, 256), 256, 0, x4_adj, g, wx, E, D, add);
   PETB_LAUNCH_CHECK(st);
 }
 
@@ -909,10 +942,10 @@ void readout_seed_bwd(Stream& st, float* out, const float* w, const float* pre, 
   PETB_LAUNCH_CHECK(st);
 }
 
-void cutoff_share(Stream& st, float* cf_adj, const float* cfh, const float* cut, int N, int E, int H) {
+void cutoff_share(Stream& st, float* cf_adj, const float* cfh, size_t stride, int blocks, const float* cut, int N, int E, int H) {
   if (E == 0) return;
-  const ProfScope ps(st, PC_ELEMENTWISE, double(E) * H, 4.0 * double(E) * (H + 2));
-  launch(st, k_cutoff_share, blocks_for(E, 256), 256, 0, cf_adj, cfh, cut, N, E, H);
+  const ProfScope ps(st, PC_ELEMENTWISE, double(E) * H * blocks, 4.0 * double(E) * (H * blocks + 2));
+  launch(st, k_cutoff_share, blocks_for(E, 256), 256, 0, cf_adj, cfh, stride, blocks, cut, N, E, H);
   PETB_LAUNCH_CHECK(st);
 }
 
@@ -941,7 +974,7 @@ void message_average_bwd(Stream& st, float* ie_adj_out, float* oe_adj, const flo
 }
 
 void forces_and_virial(Stream& st, Arena& arena, ForceOut& out, const PackedEdges& pk, const float* x4_adj, const float* cutoff_adj,
-                       const float* cf_adj, const CutoffSpec& cs, double scale) {
+                       const float* cf_adj, const CutoffSpec& cs, double scale, double* energy, const double* per_atom) {
   const ProfScope ps(st, PC_FORCES, 40.0 * pk.E, 100.0 * double(pk.E) + 96.0 * pk.n_atoms);
   double* pc_adj = pk.adaptive.acut ? arena.alloc<double>(pk.E > 0 ? pk.E : 1) : nullptr;
   if (pk.E > 0) {
@@ -954,15 +987,11 @@ void forces_and_virial(Stream& st, Arena& arena, ForceOut& out, const PackedEdge
   }
   // the adaptive cutoff's share, folded over the raw list, before the per-structure sums
   if (pc_adj) adaptive_backward(st, arena, pk, cs, pc_adj, scale, out.forces, out.vir_atom, &out.adaptive_gmag);
-  launch(st, k_struct_sum, size_t(pk.B) * 9, 256, 0, out.vir9, out.vir_atom, pk.soff, 9);
-  PETB_LAUNCH_CHECK(st);
-  launch(st, k_voigt, blocks_for(pk.B, 128), 128, 0, out.vir6, out.vir9, pk.B);
-  PETB_LAUNCH_CHECK(st);
+  structure_sums(st, energy, out.vir6, per_atom, out.vir_atom, pk.soff, pk.B);
 }
 
-void structure_energy(Stream& st, double* energy, const double* per_atom, const int* soff, int B) {
-  const ProfScope ps(st, PC_FORCES, 0.0, 8.0 * B);
-  launch(st, k_struct_sum, B, 256, 0, energy, per_atom, soff, 1);
+void structure_sums(Stream& st, double* energy, double* vir6, const double* per_atom, const double* vir_atom, const int* soff, int B) {
+  launch(st, k_struct_sums, size_t(B) * (vir6 ? 7 : 1), 256, 0, energy, vir6, per_atom, vir_atom, soff);
   PETB_LAUNCH_CHECK(st);
 }
 

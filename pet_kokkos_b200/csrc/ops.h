@@ -12,6 +12,9 @@ namespace petb {
 
 // out(r,:) = table(idx(r),:)   (gather, src/ops.cpp:109-114)
 void gather_rows(Stream& st, float* out, const float* table, const int* idx, int R, int D, uint32_t* mx = nullptr);
+// Two lookups in one launch, the second without its rows' maxima.
+void gather_rows_two(Stream& st, float* out, const float* table, const int* idx, int R, int D, uint32_t* mx, float* out2, const float* table2,
+                     const int* idx2, int R2, int D2);
 
 // Layer 0's compress.0: pre = b + tab[species] + wx.(v,|v|); out = silu(pre)  (compress_fwd without a GEMM, src/ops.cpp:326-365)
 void compress0(Stream& st, float* out, float* pre, const float* b, const float* tab, const float* wx, const PackedEdges& pk,
@@ -55,7 +58,7 @@ void concat_norm_remote_bwd(Stream& st, float* send, const float* out_adj, const
                             const int* live_packed, int n_live, int D, RemoteRows remote);
 
 // x4_adj(k,c) += sum_d g(k,d) wx(d,c)  (the reduction of compress_bwd, src/ops.cpp:373-401)
-void compress_geometry_bwd(Stream& st, float* x4_adj, const float* g, const float* wx, int E, int D);
+void compress_geometry_bwd(Stream& st, float* x4_adj, const float* g, const float* wx, int E, int D, bool add);
 
 // net(n) = float(node_pred(n) + sum_k double(cut k) * double(edge_pred k)); per_atom(n) = scale*net + comp[species]
 // (readout_accumulate + assemble_energy, src/ops.cpp:406-425). acc: add onto net first.
@@ -68,7 +71,7 @@ void readout_seed_bwd(Stream& st, float* out, const float* w, const float* pre, 
                       int n_local, int R, int Dh, uint32_t* mx = nullptr);
 
 // cf_adj(k) += (sum_h cfh(N+k,h)) / cut(k)  (attn_bwd_cf, src/attention.cpp:1829-1838; only edge slots carry a gradient)
-void cutoff_share(Stream& st, float* cf_adj, const float* cfh, const float* cut, int N, int E, int H);
+void cutoff_share(Stream& st, float* cf_adj, const float* cfh, size_t stride, int blocks, const float* cut, int N, int E, int H);
 
 // a += b, elementwise
 void add_inplace(Stream& st, float* a, const float* b, size_t n);
@@ -83,7 +86,6 @@ struct ForceOut {
   double* edge_grad = nullptr;  // [E,3]
   double* forces = nullptr;     // [n_atoms,3]
   double* vir_atom = nullptr;   // [n_atoms,9]
-  double* vir9 = nullptr;       // [B,9]
   double* vir6 = nullptr;       // [B,6]
   double* energy = nullptr;     // [B]
   // With an adaptive cutoff: the radial gradient it puts on every raw edge, scale included (dE/dv += gmag v).
@@ -92,11 +94,11 @@ struct ForceOut {
 // dE/dv per edge, the per-atom fold, and each structure's ordered sums
 // (forces_and_virial, fold_edge_gradients, sum_by_structure: src/forces.cpp:50-70,287-302,345-411; Voigt: src/model.cpp:983-993)
 void forces_and_virial(Stream& st, Arena& arena, ForceOut& out, const PackedEdges& pk, const float* x4_adj, const float* cutoff_adj,
-                       const float* cf_adj, const CutoffSpec& cs, double scale);
+                       const float* cf_adj, const CutoffSpec& cs, double scale, double* energy, const double* per_atom);
 // The adaptive cutoff's share of forces and virial (adaptive.cu): pc_adj [E] is each kept edge's pair-cutoff adjoint.
 void adaptive_backward(Stream& st, Arena& arena, const PackedEdges& pk, const CutoffSpec& cs, const double* pc_adj, double scale,
                        double* forces, double* vir_atom, double** gmag_out);
-// energy(b) = ordered sum of per_atom over the structure's atoms
-void structure_energy(Stream& st, double* energy, const double* per_atom, const int* soff, int B);
+// energy(b) = ordered sum of per_atom over the structure's atoms; vir6, unless null, that of vir_atom in Voigt's order
+void structure_sums(Stream& st, double* energy, double* vir6, const double* per_atom, const double* vir_atom, const int* soff, int B);
 
 }  // namespace petb
