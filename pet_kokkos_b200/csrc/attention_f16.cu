@@ -416,11 +416,14 @@ __host__ __device__ constexpr int shared_pitch(int rows) {
 
 // ONCE: a warp per block of 16 keys, no more. Scores and score adjoints are made once, transposed, by the warp that has the keys:
 // it sums dK and dV and leaves dS^T, in parts, in the rows of V's tile that are its keys' (nobody else reads those, and it has them
-// in registers); then, all warps' dS there, it takes the queries of the same rows for dQ = sc dS K. Per 16 x 16 block 60 products
-// instead of 84 (P = 2), 22 ldmatrix instead of 44, half the exponentials and splits; V's rows are longer, so fewer CTAs share an SM.
+// in registers); then, all warps' dS there, it takes the queries of the same rows for dQ = sc dS K. In two and three parts a query's row of
+// dS^T is left on the scale of its own largest value: on the tile's, a row of dO 2^-16 of the largest had 13 bits of dQ left instead of 23
+// (one part keeps its 11 bits down to 2^-18). Per 16 x 16 block 60 products instead of 84 (P = 2), 22 ldmatrix instead of 44, half the
+// exponentials; V's rows are longer, so fewer CTAs share an SM.
 // That alone gave 5 % (P = 1, 2; P = 3 lost 5): the warps waited for the tile's loads (two of eight stalled cycles) and for one another
 // behind them. With all of a thread's rows asked for at once (U) instead of in three trips: diamond1728 P = 2 2.16 ms -> 1.87, P = 3 3.64 ->
-// 3.57, 16-thousand-atom batch 9.25 -> 8.6, water1791 P = 1 0.737 -> 0.705 (U alone: 2.22, 3.65, 9.85, 0.705).
+// 3.57, 16-thousand-atom batch 9.25 -> 8.6, water1791 P = 1 0.737 -> 0.705 (U alone: 2.22, 3.65, 9.85, 0.705). The P = 2 figures are
+// without the queries' own scales: those are 0.06 ms of a 12.1 ms pass, and 0.12 as a second split of dS instead of a multiplication.
 template <int HD, int P, int MAXT, int BLOCKS, bool ONCE>
 __global__ void __launch_bounds__(MAXT, BLOCKS) k_attn_bwd_f16(AttnArgs p) {
   after_previous();
@@ -436,7 +439,7 @@ __global__ void __launch_bounds__(MAXT, BLOCKS) k_attn_bwd_f16(AttnArgs p) {
   constexpr int PB = pitch<HD, P>();
   const int PV = ONCE ? shared_pitch<HD, P>(SM) : PB;
   uint8_t *sq = smem, *sk = sq + SM * PB, *sg = sk + SM * PB, *sv = sg + SM * PB;
-  float *slc = reinterpret_cast<float*>(sv + SM * PV), *sm = slc + SM, *sl = sm + SM, *sd = sl + SM, *sn = sd + SM, *su = sn + SM;  // (su: ONCE, P = 3)
+  float *slc = reinterpret_cast<float*>(sv + SM * PV), *sm = slc + SM, *sl = sm + SM, *sd = sl + SM, *sn = sd + SM, *su = sn + SM;  // (su: ONCE, P > 1)
   // Staging: a thread's loads of U rows' pieces (of all its rows, up to five blocks) are all under way before it looks for the tile's scales or splits any. The
   // HD / 4 lanes that hold a row of dO, V and O add up its Dq = dO . O and its norms on the way.
   constexpr int Q = HD / 4, U = MAXT <= 160 && HD <= 32 ? 4 : 2;
@@ -508,11 +511,11 @@ __global__ void __launch_bounds__(MAXT, BLOCKS) k_attn_bwd_f16(AttnArgs p) {
   const float vmax = sqrtf(__uint_as_float(s_vnorm)), gmax = sqrtf(__uint_as_float(s_gnorm));
   const int nb = S16 / 16;
   if constexpr (ONCE) {
-    if (P == 3) {  // a query's own scale over the common one, and what undoes its own
+    if (P >= 2) {  // a query's own scale (P = 3: over the common one), and what undoes it
       const uint32_t all = __float_as_uint(fmaxf(2.1f * gmax * vmax, 1e-9f));
       for (int r = threadIdx.x; r < S16; r += blockDim.x) {
         const uint32_t own = __float_as_uint(fmaxf(2.1f * sn[r] * vmax, 1e-9f));
-        sn[r] = scale_of(own) * unscale_of(all), su[r] = unscale_of(own);
+        sn[r] = scale_of(own) * (P == 3 ? unscale_of(all) : 1.f / 32768.f), su[r] = unscale_of(own);
       }
       __syncthreads();
     }
@@ -530,7 +533,7 @@ __global__ void __launch_bounds__(MAXT, BLOCKS) k_attn_bwd_f16(AttnArgs p) {
         }
       __syncwarp();
       const float lc0 = slc[i0], lc1 = slc[i1];
-      const float ds = scale_of(bound) * (1.f / 32768.f), fds = usv * unscale_of(bound) * usg;
+      const float common = scale_of(bound), ds = common * (1.f / 32768.f), fds = usv * unscale_of(bound) * usg;
       float dk[HD / 8][4], dv[HD / 8][4];
       clear<HD>(dk), clear<HD>(dv);
       float cf0 = 0.f, cf1 = 0.f;
@@ -538,22 +541,43 @@ __global__ void __launch_bounds__(MAXT, BLOCKS) k_attn_bwd_f16(AttnArgs p) {
         Acc<P, 2> c, w;
         two_products<HD, P, true, true>(c, w, kf, vf, ak, av, r0, aq, ag, b, lane);
         float x[2][4], y[2][4];
+        __half2 to_common[2];
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
           const int q = b + 8 * i + 2 * t;  // this lane's two queries of the block
           const float2 m = *reinterpret_cast<const float2*>(sm + q), il = *reinterpret_cast<const float2*>(sl + q),
                        d = *reinterpret_cast<const float2*>(sd + q);
-          // probabilities by 2^15, score adjoints by ds
+          // probabilities by 2^15, score adjoints by ds (P = 2: by the query's own)
           x[i][0] = exp2_fast(fmaf(c.get(i, 0), f, lc0) - m.x) * il.x, x[i][1] = exp2_fast(fmaf(c.get(i, 1), f, lc0) - m.y) * il.y;
           x[i][2] = exp2_fast(fmaf(c.get(i, 2), f, lc1) - m.x) * il.x, x[i][3] = exp2_fast(fmaf(c.get(i, 3), f, lc1) - m.y) * il.y;
-          y[i][0] = x[i][0] * ((w.get(i, 0) - d.x) * ds), y[i][1] = x[i][1] * ((w.get(i, 1) - d.y) * ds);
-          y[i][2] = x[i][2] * ((w.get(i, 2) - d.x) * ds), y[i][3] = x[i][3] * ((w.get(i, 3) - d.y) * ds);
-          cf0 += y[i][0] + y[i][1], cf1 += y[i][2] + y[i][3];
+          const float2 own = P == 2 ? *reinterpret_cast<const float2*>(sn + q) : make_float2(ds, ds);
+          y[i][0] = x[i][0] * ((w.get(i, 0) - d.x) * own.x), y[i][1] = x[i][1] * ((w.get(i, 1) - d.y) * own.y);
+          y[i][2] = x[i][2] * ((w.get(i, 2) - d.x) * own.x), y[i][3] = x[i][3] * ((w.get(i, 3) - d.y) * own.y);
+          if (P == 2) {
+            const float2 u = *reinterpret_cast<const float2*>(su + q);
+            const float rx = u.x * common, ry = u.y * common;
+            to_common[i] = __floats2half2_rn(rx, ry);
+            cf0 += y[i][0] * rx + y[i][1] * ry, cf1 += y[i][2] * rx + y[i][3] * ry;
+          } else {
+            cf0 += y[i][0] + y[i][1], cf1 += y[i][2] + y[i][3];
+          }
         }
         uint32_t a[with_sum<P>()][4];
         make_a<P>(a, y);
-        product_rows<HD, P>(dk, a, aq, b, lane);
-        if (P == 3) {  // the leading part of a query's row of dS, as dQ wants it, is that of the row's own largest value
+        if (P == 2) {  // dK sums over the queries, so wants them on one scale: the parts times a power of two, at most 1
+          uint32_t k[P][4];
+#pragma unroll
+          for (int j = 0; j < P; ++j)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const __half2 v = __hmul2(*reinterpret_cast<const __half2*>(&a[j][i]), to_common[i / 2]);
+              k[j][i] = *reinterpret_cast<const uint32_t*>(&v);
+            }
+          product_rows<HD, P>(dk, k, aq, b, lane);
+        } else {
+          product_rows<HD, P>(dk, a, aq, b, lane);
+        }
+        if (P == 3) {  // dQ wants a query's row of dS on the scale of the row's own largest value
 #pragma unroll
           for (int i = 0; i < 2; ++i) {
             const float2 o = *reinterpret_cast<const float2*>(sn + b + 8 * i + 2 * t);
@@ -593,7 +617,7 @@ __global__ void __launch_bounds__(MAXT, BLOCKS) k_attn_bwd_f16(AttnArgs p) {
       add_sum<P>(a);
       product_rows<HD, P>(dq, a, ak, b, lane);
     }
-    const float f0 = usv * usk * usg * p.sc * (P == 3 ? su[i0] : unscale_of(bound)), f1 = usv * usk * usg * p.sc * (P == 3 ? su[i1] : unscale_of(bound));
+    const float f0 = usv * usk * usg * p.sc * (P >= 2 ? su[i0] : unscale_of(bound)), f1 = usv * usk * usg * p.sc * (P >= 2 ? su[i1] : unscale_of(bound));
     write_rows<HD>(p.qkv_adj, 3 * D, h * HD, g0, g1, i0 < cnt, i1 < cnt, dq, f0, f1, p.qkv_adj_max, t);
     return;
   }
@@ -710,17 +734,20 @@ bool bwd_hd(Stream& st, const AttnArgs& p) {
   if (bytes > kMaxBytes) return false;
   static SmemOptIn o128, o160, o320, o640;
   // Up to five blocks of 16 rows, heads of at most 32: scores once (a head size of 64 has no registers for two tensors' operands).
-  if constexpr (HD <= 32)
+  if constexpr (HD <= 32) {
     if (blocks <= 5) {
       const size_t once = size_t(rows) * (3 * pitch<HD, P>() + shared_pitch<HD, P>(rows) + 6 * sizeof(float));
       if (blocks <= 4) launch(st, k_attn_bwd_f16<HD, P, 128, P == 3 ? 3 : P == 2 ? 4 : 5, true>, p, once, 32 * blocks, o128);
       else launch(st, k_attn_bwd_f16<HD, P, 160, P == 3 ? 2 : P == 2 ? 3 : 4, true>, p, once, 32 * blocks, o160);
       return true;
     }
+  } else if (blocks <= 5) {
+    launch(st, k_attn_bwd_f16<HD, P, 160, resident<HD, P, 4>(80), false>, p, bytes, 32 * blocks, o160);
+    return true;
+  }
   // A warp per 16 rows, which takes queries and then keys, where several CTAs share an SM; where one tile fills it, a warp
   // per 16 queries and one per 16 keys, up to 20: then blocks in turn.
-  if (HD > 32 && blocks <= 5) launch(st, k_attn_bwd_f16<HD, P, 160, resident<HD, P, 4>(80), false>, p, bytes, 32 * blocks, o160);
-  else if (bytes <= 110 * 1024) launch(st, k_attn_bwd_f16<HD, P, 320, 2, false>, p, bytes, 32 * (blocks < 10 ? blocks : 10), o320);
+  if (bytes <= 110 * 1024) launch(st, k_attn_bwd_f16<HD, P, 320, 2, false>, p, bytes, 32 * (blocks < 10 ? blocks : 10), o320);
   else launch(st, k_attn_bwd_f16<HD, P, 640, 1, false>, p, bytes, 64 * (blocks < 10 ? blocks : 10), o640);
   return true;
 }
