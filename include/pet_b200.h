@@ -360,6 +360,20 @@ int pet_debug_gemm(pet_calc* c, const pet_debug_gemm_args* args);
  * where that is the faster way (testing aid). */
 int pet_debug_gemm_two(pet_calc* c, const pet_debug_gemm_args* args);
 
+/* The attention by itself, forward and then backward, on host arrays (testing aid). Row n < n_atoms is atom n's own token, row
+ * n_atoms + k edge k's; an atom's edges are offsets[n] .. offsets[n + 1]. `mode` is a number of csrc/attention.h's enum. */
+typedef struct pet_debug_attention_args {
+  int mode, n_atoms, heads, head_dim;
+  float scale;             /* of the scores: 1 / (sqrt(head_dim) temperature) */
+  const int* offsets;      /* [n_atoms + 1] */
+  const float* cut;        /* [E] cutoff factors */
+  const float* qkv;        /* [T,3D], columns Q | K | V; T = n_atoms + E, D = heads head_dim */
+  const float* dmerged;    /* [T,D] */
+  float *merged, *qkv_adj; /* [T,D], [T,3D] */
+  float* cfh;              /* [T,heads]: each key's score adjoint summed over its queries */
+} pet_debug_attention_args;
+int pet_debug_attention(pet_calc* c, const pet_debug_attention_args* args);
+
 /* A ready-made pet_exchange over NCCL: what an MD engine's pair style does around pet::Exchange
  * (lammps/ML-PET/pair_pet.cpp:268-360 routing, :396-472 exchange_rows, :479-555 set_live / edges), inside the
  * library. Rows of edges to ghosts are packed by a kernel, cross with ncclSend / ncclRecv on the calculator's own

@@ -23,6 +23,7 @@ GEMM_MODES = {"native": 0, "tf32": 1, "bf16": 2, "3xtf32": 3}
 # operand formats and epilogues of the weight GEMM (csrc/gemm.h), for debug_gemm
 GEMM_FORMATS = {"f16x3": 0, "f16x2": 1, "f16": 2, "bf16": 3, "tf32x2": 4, "tf32": 5, "f16x3_full": 6}
 GEMM_EPILOGUES = {"plain": 0, "silu": 1, "swiglu": 2, "silu_bwd": 3, "swiglu_bwd": 4, "compress": 5}
+ATTENTION_MODES = {"native": 0, "tf32x3": 1, "tf32": 2}
 RECOMPUTE_TIERS = {"auto": 0, "never": 1, "wide": 2, "layers": 3}
 
 
@@ -109,6 +110,11 @@ class PetDebugGemmArgs(C.Structure):
                 ("dist", C.POINTER(C.c_double)), ("C", C.POINTER(C.c_float)), ("row_max", C.POINTER(C.c_float)), ("rms", C.c_int)]
 
 
+class PetDebugAttentionArgs(C.Structure):
+    _fields_ = [(f, C.c_int) for f in ("mode", "n_atoms", "heads", "head_dim")] + [("scale", C.c_float), ("offsets", C.POINTER(C.c_int))] + \
+               [(f, C.POINTER(C.c_float)) for f in ("cut", "qkv", "dmerged", "merged", "qkv_adj", "cfh")]
+
+
 class PetRawEdges(C.Structure):
     _fields_ = [("capacity", C.c_int), ("n_edges", C.c_int), ("i", C.POINTER(C.c_int)), ("j", C.POINTER(C.c_int)),
                 ("shift", C.POINTER(C.c_int)), ("vec", C.POINTER(C.c_double)), ("dist", C.POINTER(C.c_double)),
@@ -173,6 +179,7 @@ SIGNATURES = {
                                        C.c_size_t]),
     "pet_debug_gemm": (C.c_int, [C.c_void_p, _P(PetDebugGemmArgs)]),
     "pet_debug_gemm_two": (C.c_int, [C.c_void_p, _P(PetDebugGemmArgs)]),
+    "pet_debug_attention": (C.c_int, [C.c_void_p, _P(PetDebugAttentionArgs)]),
     "pet_gemm_host": (C.c_int, [C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, _P(C.c_float), _P(C.c_float),
                                 _P(C.c_float)]),
 }
@@ -688,6 +695,20 @@ class Calculator:
         given = [self._debug_gemm_args(**first), self._debug_gemm_args(**second)]
         self._check(self._lib.pet_debug_gemm_two(self._h, (PetDebugGemmArgs * 2)(given[0][0], given[1][0])))
         return given[0][2], given[1][2]
+
+    def debug_attention(self, qkv, dmerged, offsets, cut, heads, mode, scale):
+        """The attention's forward and backward by themselves: (merged, qkv_adj, cfh)."""
+        f32 = lambda x: np.ascontiguousarray(x, dtype=np.float32)
+        qkv, dmerged, cut, offsets = f32(qkv), f32(dmerged), f32(cut), np.ascontiguousarray(offsets, dtype=np.int32)
+        T, D = dmerged.shape
+        if qkv.shape != (T, 3 * D) or T != len(offsets) - 1 + offsets[-1] or len(cut) != offsets[-1] or D % heads:
+            raise ValueError("attention: shapes do not agree")
+        merged, qkv_adj, cfh = np.zeros_like(dmerged), np.zeros_like(qkv), np.zeros((T, heads), np.float32)
+        fp = lambda a: a.ctypes.data_as(C.POINTER(C.c_float))
+        g = PetDebugAttentionArgs(ATTENTION_MODES[mode], len(offsets) - 1, heads, D // heads, scale,
+                                  offsets.ctypes.data_as(C.POINTER(C.c_int)), fp(cut), fp(qkv), fp(dmerged), fp(merged), fp(qkv_adj), fp(cfh))
+        self._check(self._lib.pet_debug_attention(self._h, C.byref(g)))
+        return merged, qkv_adj, cfh
 
     def _debug_gemm_args(self, A, W, fmt, epilogue="plain", w_transposed=True, bias=None, res=None, res_row0=0, pre=None, tab=None,
                          species=None, wx=None, vec=None, dist=None, want_pre=True, rms=False):

@@ -512,9 +512,13 @@ __global__ void __launch_bounds__(MAXT, BLOCKS) k_attn_bwd_f16(AttnArgs p) {
   const int nb = S16 / 16;
   if constexpr (ONCE) {
     if (P >= 2) {  // a query's own scale (P = 3: over the common one), and what undoes it
-      const uint32_t all = __float_as_uint(fmaxf(2.1f * gmax * vmax, 1e-9f));
+      const float all_bound = fmaxf(2.1f * gmax * vmax, 1e-9f);
+      // P = 2: at most 2^24 from the common one. The factor that takes a row's parts there for dK is an fp16 number: 2^-25 would be
+      // zero and the row missing. dQ keeps its 22 bits down to rows of 2^-40, and dO itself is not staged any finer.
+      const float least = P == 2 ? all_bound * 0x1p-24f : 0.f;
+      const uint32_t all = __float_as_uint(all_bound);
       for (int r = threadIdx.x; r < S16; r += blockDim.x) {
-        const uint32_t own = __float_as_uint(fmaxf(2.1f * sn[r] * vmax, 1e-9f));
+        const uint32_t own = __float_as_uint(fmaxf(2.1f * sn[r] * vmax, fmaxf(least, 1e-9f)));
         sn[r] = scale_of(own) * (P == 3 ? unscale_of(all) : 1.f / 32768.f), su[r] = unscale_of(own);
       }
       __syncthreads();

@@ -275,5 +275,11 @@ int pet_debug_gemm_two(pet_calc* c, const pet_debug_gemm_args* args) {
     e.gemm_on_host_arrays(args, 2, args->format, args->format);
   });
 }
+int pet_debug_attention(pet_calc* c, const pet_debug_attention_args* args) {
+  return guarded(c, [&](Engine& e) {
+    if (!args) throw petb::Error(PET_ERR_INVALID, "pet: bad attention arguments");
+    e.attention_on_host_arrays(*args);
+  });
+}
 
 }  // extern "C"

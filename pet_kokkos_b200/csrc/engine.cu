@@ -7,6 +7,7 @@
 #include <cstring>
 #include <type_traits>
 
+#include "attention.h"
 #include "gemm.h"
 
 namespace petb {
@@ -1464,6 +1465,41 @@ GemmArgs Engine::gemm_from_host_arrays(const pet_debug_gemm_args& g, int native_
   };
   a.nat = pack(native_format), a.fast = pack(fast_format);
   return a;
+}
+
+void Engine::attention_on_host_arrays(const pet_debug_attention_args& g) {
+  const auto bad = [](bool is) {
+    if (is) throw Error(2, "pet: bad attention arguments");
+  };
+  bad(g.mode < ATTN_NATIVE || g.mode > ATTN_TF32 || g.n_atoms <= 0 || g.heads <= 0 || g.head_dim <= 0 || !g.offsets || g.offsets[0] != 0);
+  AttnArgs a;
+  a.N = g.n_atoms, a.H = g.heads, a.hd = g.head_dim, a.sc = g.scale, a.mode = g.mode;
+  for (int n = 0; n < g.n_atoms; ++n) {
+    const int tokens = g.offsets[n + 1] - g.offsets[n] + 1;
+    bad(tokens < 1);
+    a.S = std::max(a.S, tokens), a.pairs += double(tokens) * tokens;
+  }
+  const size_t E = g.offsets[g.n_atoms], T = g.n_atoms + E, H = g.heads, D = H * g.head_dim;
+  bad((E && !g.cut) || !g.qkv || !g.dmerged || !g.merged || !g.qkv_adj || !g.cfh);
+  PETB_CUDA(cudaSetDevice(device));
+  PETB_CUDA(cudaStreamSynchronize(st.s));
+  tmp_arena.reset();
+  auto up = [&](const auto* from, size_t count) {
+    using V = std::remove_const_t<std::remove_pointer_t<decltype(from)>>;
+    V* to = tmp_arena.alloc<V>(count ? count : 1);
+    if (count) PETB_CUDA(cudaMemcpyAsync(to, from, sizeof(V) * count, cudaMemcpyHostToDevice, st.s));
+    return to;
+  };
+  a.T = double(T);
+  a.off = up(g.offsets, g.n_atoms + 1), a.cut = up(g.cut, E), a.qkv = up(g.qkv, T * 3 * D), a.dmerged = up(g.dmerged, T * D);
+  a.merged = tmp_arena.alloc<float>(T * D), a.ml = tmp_arena.alloc<float>(T * H * 2);
+  a.qkv_adj = tmp_arena.alloc<float>(T * 3 * D), a.cfh = tmp_arena.alloc<float>(T * H);
+  attention_forward(st, a);
+  attention_backward(st, a);
+  PETB_CUDA(cudaMemcpyAsync(g.merged, a.merged, 4 * T * D, cudaMemcpyDeviceToHost, st.s));
+  PETB_CUDA(cudaMemcpyAsync(g.qkv_adj, a.qkv_adj, 4 * T * 3 * D, cudaMemcpyDeviceToHost, st.s));
+  PETB_CUDA(cudaMemcpyAsync(g.cfh, a.cfh, 4 * T * H, cudaMemcpyDeviceToHost, st.s));
+  PETB_CUDA(cudaStreamSynchronize(st.s));
 }
 
 }  // namespace petb

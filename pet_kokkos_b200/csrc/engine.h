@@ -88,6 +88,7 @@ struct Engine {
   void gemm_host(int mode, bool w_transposed, int m, int n, int k, const float* A, const float* W, float* C);
   void gemm_on_host_arrays(const pet_debug_gemm_args* g, int count, int native_format, int fast_format);
   GemmArgs gemm_from_host_arrays(const pet_debug_gemm_args& g, int native_format, int fast_format);
+  void attention_on_host_arrays(const pet_debug_attention_args& g);
 
   int species_index(int Z) const;
 
