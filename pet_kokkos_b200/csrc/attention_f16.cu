@@ -416,9 +416,9 @@ __host__ __device__ constexpr int shared_pitch(int rows) {
 
 // ONCE: a warp per block of 16 keys, no more. Scores and score adjoints are made once, transposed, by the warp that has the keys:
 // it sums dK and dV and leaves dS^T, in parts, in the rows of V's tile that are its keys' (nobody else reads those, and it has them
-// in registers); then, all warps' dS there, it takes the queries of the same rows for dQ = sc dS K. In two and three parts a query's row of
-// dS^T is left on the scale of its own largest value: on the tile's, a row of dO 2^-16 of the largest had 13 bits of dQ left instead of 23
-// (one part keeps its 11 bits down to 2^-18). Per 16 x 16 block 60 products instead of 84 (P = 2), 22 ldmatrix instead of 44, half the
+// in registers); then, all warps' dS there, it takes the queries of the same rows for dQ = sc dS K. A query's row of dS^T is left on the
+// scale of its own largest value: on the tile's, a row of dO 2^-16 of the largest had 13 bits of dQ left instead of 23
+// (one part: 2^-24, four instead of 11). Per 16 x 16 block 60 products instead of 84 (P = 2), 22 ldmatrix instead of 44, half the
 // exponentials; V's rows are longer, so fewer CTAs share an SM.
 // That alone gave 5 % (P = 1, 2; P = 3 lost 5): the warps waited for the tile's loads (two of eight stalled cycles) and for one another
 // behind them. With all of a thread's rows asked for at once (U) instead of in three trips: diamond1728 P = 2 2.16 ms -> 1.87, P = 3 3.64 ->
@@ -439,7 +439,7 @@ __global__ void __launch_bounds__(MAXT, BLOCKS) k_attn_bwd_f16(AttnArgs p) {
   constexpr int PB = pitch<HD, P>();
   const int PV = ONCE ? shared_pitch<HD, P>(SM) : PB;
   uint8_t *sq = smem, *sk = sq + SM * PB, *sg = sk + SM * PB, *sv = sg + SM * PB;
-  float *slc = reinterpret_cast<float*>(sv + SM * PV), *sm = slc + SM, *sl = sm + SM, *sd = sl + SM, *sn = sd + SM, *su = sn + SM;  // (su: ONCE, P > 1)
+  float *slc = reinterpret_cast<float*>(sv + SM * PV), *sm = slc + SM, *sl = sm + SM, *sd = sl + SM, *sn = sd + SM, *su = sn + SM;  // (su: ONCE)
   // Staging: a thread's loads of U rows' pieces (of all its rows, up to five blocks) are all under way before it looks for the tile's scales or splits any. The
   // HD / 4 lanes that hold a row of dO, V and O add up its Dq = dO . O and its norms on the way.
   constexpr int Q = HD / 4, U = MAXT <= 160 && HD <= 32 ? 4 : 2;
@@ -511,15 +511,15 @@ __global__ void __launch_bounds__(MAXT, BLOCKS) k_attn_bwd_f16(AttnArgs p) {
   const float vmax = sqrtf(__uint_as_float(s_vnorm)), gmax = sqrtf(__uint_as_float(s_gnorm));
   const int nb = S16 / 16;
   if constexpr (ONCE) {
-    if (P >= 2) {  // a query's own scale (P = 3: over the common one), and what undoes it
+    {  // a query's own scale (P = 3: over the common one), and the common one over it
       const float all_bound = fmaxf(2.1f * gmax * vmax, 1e-9f);
-      // P = 2: at most 2^24 from the common one. The factor that takes a row's parts there for dK is an fp16 number: 2^-25 would be
-      // zero and the row missing. dQ keeps its 22 bits down to rows of 2^-40, and dO itself is not staged any finer.
-      const float least = P == 2 ? all_bound * 0x1p-24f : 0.f;
+      // P = 1, 2: at most 2^24 from the common one. The factor that takes a row's parts there for dK is an fp16 number: 2^-25 would be
+      // zero and the row missing. dQ keeps its bits down to rows of 2^-40, and dO itself is not staged any finer.
+      const float least = P <= 2 ? all_bound * 0x1p-24f : 0.f;
       const uint32_t all = __float_as_uint(all_bound);
       for (int r = threadIdx.x; r < S16; r += blockDim.x) {
         const uint32_t own = __float_as_uint(fmaxf(2.1f * sn[r] * vmax, fmaxf(least, 1e-9f)));
-        sn[r] = scale_of(own) * (P == 3 ? unscale_of(all) : 1.f / 32768.f), su[r] = unscale_of(own);
+        sn[r] = scale_of(own) * (P == 3 ? unscale_of(all) : 1.f / 32768.f), su[r] = unscale_of(own) * scale_of(all);
       }
       __syncthreads();
     }
@@ -537,7 +537,7 @@ __global__ void __launch_bounds__(MAXT, BLOCKS) k_attn_bwd_f16(AttnArgs p) {
         }
       __syncwarp();
       const float lc0 = slc[i0], lc1 = slc[i1];
-      const float common = scale_of(bound), ds = common * (1.f / 32768.f), fds = usv * unscale_of(bound) * usg;
+      const float ds = scale_of(bound) * (1.f / 32768.f), fds = usv * unscale_of(bound) * usg;
       float dk[HD / 8][4], dv[HD / 8][4];
       clear<HD>(dk), clear<HD>(dv);
       float cf0 = 0.f, cf1 = 0.f;
@@ -551,24 +551,23 @@ __global__ void __launch_bounds__(MAXT, BLOCKS) k_attn_bwd_f16(AttnArgs p) {
           const int q = b + 8 * i + 2 * t;  // this lane's two queries of the block
           const float2 m = *reinterpret_cast<const float2*>(sm + q), il = *reinterpret_cast<const float2*>(sl + q),
                        d = *reinterpret_cast<const float2*>(sd + q);
-          // probabilities by 2^15, score adjoints by ds (P = 2: by the query's own)
+          // probabilities by 2^15, score adjoints by ds (P = 1, 2: by the query's own)
           x[i][0] = exp2_fast(fmaf(c.get(i, 0), f, lc0) - m.x) * il.x, x[i][1] = exp2_fast(fmaf(c.get(i, 1), f, lc0) - m.y) * il.y;
           x[i][2] = exp2_fast(fmaf(c.get(i, 2), f, lc1) - m.x) * il.x, x[i][3] = exp2_fast(fmaf(c.get(i, 3), f, lc1) - m.y) * il.y;
-          const float2 own = P == 2 ? *reinterpret_cast<const float2*>(sn + q) : make_float2(ds, ds);
+          const float2 own = P <= 2 ? *reinterpret_cast<const float2*>(sn + q) : make_float2(ds, ds);
           y[i][0] = x[i][0] * ((w.get(i, 0) - d.x) * own.x), y[i][1] = x[i][1] * ((w.get(i, 1) - d.y) * own.y);
           y[i][2] = x[i][2] * ((w.get(i, 2) - d.x) * own.x), y[i][3] = x[i][3] * ((w.get(i, 3) - d.y) * own.y);
-          if (P == 2) {
+          if (P <= 2) {
             const float2 u = *reinterpret_cast<const float2*>(su + q);
-            const float rx = u.x * common, ry = u.y * common;
-            to_common[i] = __floats2half2_rn(rx, ry);
-            cf0 += y[i][0] * rx + y[i][1] * ry, cf1 += y[i][2] * rx + y[i][3] * ry;
+            to_common[i] = __floats2half2_rn(u.x, u.y);
+            cf0 += y[i][0] * u.x + y[i][1] * u.y, cf1 += y[i][2] * u.x + y[i][3] * u.y;
           } else {
             cf0 += y[i][0] + y[i][1], cf1 += y[i][2] + y[i][3];
           }
         }
         uint32_t a[with_sum<P>()][4];
         make_a<P>(a, y);
-        if (P == 2) {  // dK sums over the queries, so wants them on one scale: the parts times a power of two, at most 1
+        if (P <= 2) {  // dK sums over the queries, so wants them on one scale: the parts times a power of two, at most 1
           uint32_t k[P][4];
 #pragma unroll
           for (int j = 0; j < P; ++j)
@@ -621,7 +620,7 @@ __global__ void __launch_bounds__(MAXT, BLOCKS) k_attn_bwd_f16(AttnArgs p) {
       add_sum<P>(a);
       product_rows<HD, P>(dq, a, ak, b, lane);
     }
-    const float f0 = usv * usk * usg * p.sc * (P >= 2 ? su[i0] : unscale_of(bound)), f1 = usv * usk * usg * p.sc * (P >= 2 ? su[i1] : unscale_of(bound));
+    const float fdq = usv * usk * usg * p.sc * unscale_of(bound), f0 = fdq * su[i0], f1 = fdq * su[i1];
     write_rows<HD>(p.qkv_adj, 3 * D, h * HD, g0, g1, i0 < cnt, i1 < cnt, dq, f0, f1, p.qkv_adj_max, t);
     return;
   }

@@ -1,7 +1,7 @@
 """The attention's backward by itself, on rows of dO that lie apart: what a query with a small row of dO gives dQ and dK, against fp64.
 
 A query's row of dS reaches dQ on the scale of its own largest value, so dQ keeps the format's bits as long as the staged dO does (fp16 parts
-on the tile's scale: two or three parts down to 2^-17 of the largest and more). dK sums over queries, on the tile's
+on the tile's scale: two or three parts down to 2^-17 of the largest and more, one part to 2^-24 and more). dK sums over queries, on the tile's
 scale: every row counts down to 2^-40 of the tile's bound.
 
 The bands add up errors of their own signs by their squares, six of them wide. r is what a product of two operands loses in the format: 2^-12
@@ -69,11 +69,11 @@ def tokens(n, hd, seed):
 
 
 @pytest.mark.parametrize("size", SIZES)
-@pytest.mark.parametrize("mode", ["native", "tf32x3"])
+@pytest.mark.parametrize("mode", list(MODES))
 def test_a_small_row_keeps_its_bits_in_dq(calc, mode, size):
     n, hd = size
     q, k, v, g, cut = tokens(n, hd, 3)
-    down = {n // 3: 16, n - 1: 17}
+    down = {n // 3: 16, n - 1: 17} if mode != "tf32" else {n // 3: 23, n - 1: 24}
     for r, d in down.items():
         g[r] *= 2.0 ** -d
     dq, dk, cfh = one_atom(calc, mode, q, k, v, g, cut)
