@@ -372,7 +372,9 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1) k_gemm_tc(co
   // RMSNorm before the product (GemmArgs::rms). The converter, which sees every value of a row, adds up its squares; the epilogue
   // scales. 122138 rows, FMT_F16X2, norm and attention's input layer 169 us -> 143; the edges' SwiGLU 254 -> 260 with the atoms' tiles in
   // it; and a launch of 4 us less on a small structure's chain. (Sums of squares left in memory by the GEMM before cost it 10-18 us
-  // and this one, which has to wait for them, 35-45.)
+  // and this one, which has to wait for them, 35-45.) A step's squares are summed by themselves: in one chain over K the sum's error
+  // grew with K (1 / rms of 1024 normal values 1.17 of 2^-24 off, root mean square over the rows, and of 256 0.85; now 0.65 and
+  // 0.58, a warp's norm by itself 0.75 and 0.73).
   constexpr bool kNorms = (EPI == EPI_PLAIN || EPI == EPI_SWIGLU) && !SPLIT && (L::X3 || L::X2 || L::T2);
   static_assert(!kNorms || L::kGroups == 2, "two sums a row");
   // SPLIT: parts divides the steps of K
@@ -402,8 +404,8 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1) k_gemm_tc(co
   const uint32_t tmem = *tmem_slot;
   after_previous();
 
-  // A converter lane's squares of a row's 32 columns, added to what it has of the row; and the sums of a tile's rows handed over
-  // to the epilogue, by a warp for `n` rows a lane, `step` apart.
+  // A converter lane's squares of a step's columns of a row, four at a time; and the sums of a tile's rows handed over to the
+  // epilogue, by a warp for `n` rows a lane, `step` apart.
   const auto add_squares = [](float* sq, const float4& v) {
     asm("{ .reg .b64 s, a, b;\n\tmov.b64 s, {%0, %1};\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\t"
         "fma.rn.f32x2 s, a, a, s;\n\tfma.rn.f32x2 s, b, b, s;\n\tmov.b64 {%0, %1}, s; }"
@@ -836,6 +838,7 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1) k_gemm_tc(co
         const bool free_peek = before < 0 || mbar_test(done + before % L::ND, (before / L::ND) & 1);
         peek = mbar_test(full_a + (gone + 2) % NA, ((gone + 2) / NA) & 1);
         uint32_t part[3][16];
+        float of_step[2] = {0.f, 0.f};
         if (live) {
           const uint8_t* slab = ring_a + sa * L::kA;
           float4 v[8];
@@ -843,10 +846,11 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1) k_gemm_tc(co
           for (int c = 0; c < 8; ++c) v[c] = *reinterpret_cast<const float4*>(slab + swizzled<128>(r, c));
 #pragma unroll
           for (int c = 0; c < 8; ++c) {
-            if (kNorms && p.rms != 0.f) add_squares(sq[0], v[c]);
+            if (kNorms && p.rms != 0.f) add_squares(of_step, v[c]);
             split2<FMT>(v[c].x, v[c].y, s, part[0][2 * c], part[1][2 * c], part[2][2 * c]);
             split2<FMT>(v[c].z, v[c].w, s, part[0][2 * c + 1], part[1][2 * c + 1], part[2][2 * c + 1]);
           }
+          if (kNorms) sq[0][0] += of_step[0], sq[0][1] += of_step[1];
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(empty_a + sa);
@@ -903,14 +907,16 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1) k_gemm_tc(co
         for (int j = 0; j < 4 / WPG; ++j) {
           const int r = (first + j * WPG) * 32 + lane;
           if (m0 + r - lane >= p.M) break;  // rows past the matrix: whatever their products are, nobody reads them
+          float of_step[2] = {0.f, 0.f};
           if (L::T2) {  // the slab is h; l goes beside it at the same place
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
               const float4 v = *reinterpret_cast<const float4*>(slab + swizzled<64>(r, c));
-              if (kNorms && p.rms != 0.f) add_squares(sq[j], v);
+              if (kNorms && p.rms != 0.f) add_squares(of_step, v);
               *reinterpret_cast<float4*>(slab + L::kSlab + swizzled<64>(r, c)) =
                   make_float4(tf32_low(v.x), tf32_low(v.y), tf32_low(v.z), tf32_low(v.w));
             }
+            if (kNorms) sq[j][0] += of_step[0], sq[j][1] += of_step[1];
             continue;
           }
           const float s = scale[j];
@@ -921,13 +927,14 @@ __global__ void __launch_bounds__(Tile<BN, FMT, PAIR>::kThreads, 1) k_gemm_tc(co
           for (int c = 0; c < 4; ++c) {
             uint4 h, m, l;
             const float4 a = v[2 * c], b = v[2 * c + 1];
-            if (kNorms && p.rms != 0.f) add_squares(sq[j], a), add_squares(sq[j], b);
+            if (kNorms && p.rms != 0.f) add_squares(of_step, a), add_squares(of_step, b);
             split2<FMT>(a.x, a.y, s, h.x, m.x, l.x), split2<FMT>(a.z, a.w, s, h.y, m.y, l.y);
             split2<FMT>(b.x, b.y, s, h.z, m.z, l.z), split2<FMT>(b.z, b.w, s, h.w, m.w, l.w);
             *reinterpret_cast<uint4*>(slab + swizzled<128>(r, c)) = h;
             if (L::X3 || L::X2) *reinterpret_cast<uint4*>(slab + swizzled<128>(r, 4 + c)) = m;
             if (L::X3) *reinterpret_cast<uint4*>(slab + L::kSlab + swizzled<64>(r, c)) = l;
           }
+          if (kNorms) sq[j][0] += of_step[0], sq[j][1] += of_step[1];
         }
         fence_async_smem();  // generic-proxy writes visible to the tensor core
         __syncwarp();

@@ -53,6 +53,35 @@ def test_against_fp64(calc, fmt, epi, shape):
         assert np.array_equal(C[:r], calc.debug_gemm(A[:r], W, fmt, epi, bias=bias, rms=True)[0])
 
 
+def warp_norm(A):
+    """1 / rms in fp32 as a norm by itself has it: 32 lanes' sums of squares, added in pairs, a quotient of a root."""
+    k = A.shape[1]
+    x = np.zeros((len(A), -(-k // 32) * 32), np.float32)
+    x[:, :k] = A
+    s = np.zeros((len(A), 32), np.float32)
+    for part in np.moveaxis(x.reshape(len(A), -1, 32), 1, 0):
+        s = (part.astype(np.float64) ** 2 + s).astype(np.float32)  # one rounding: a fused multiply and add
+    for o in (16, 8, 4, 2, 1):
+        s = s + s[:, np.arange(32) ^ o]
+    return np.float32(1) / np.sqrt(s[:, 0] / np.float32(k) + np.float32(EPS))
+
+
+@pytest.mark.parametrize("shape", [(3000, 64, 100), (3000, 64, 128), (19201, 256, 256), (3000, 64, 512), (3000, 128, 1024), (3000, 256, 2048)])
+@pytest.mark.parametrize("fmt", FORMATS)
+def test_the_scale_is_no_further_off_than_a_norm_by_itself(calc, fmt, shape):
+    """A column of ones against a weight that reads it alone: the product is the row's 1 / rms as it stands, no other sum with it."""
+    m, n, k = shape
+    A = np.random.default_rng(11).normal(size=(m, k)).astype(np.float32)
+    A[:, k // 2] = 1.0
+    W = np.zeros((n, k), np.float32)
+    W[3, k // 2] = 1.0
+    got = calc.debug_gemm(A, W, fmt, "plain", rms=True)[0][:, 3].astype(np.float64)
+    true = 1.0 / np.sqrt((A.astype(np.float64) ** 2).mean(1) + EPS)
+    off = lambda x: np.sqrt(np.mean((x / true - 1.0) ** 2)) * 2.0 ** 24
+    print(fmt, shape, "off %.3f of 2^-24, by itself %.3f" % (off(got), off(warp_norm(A))))
+    assert off(got) <= off(warp_norm(A))
+
+
 @pytest.mark.parametrize("fmt", FORMATS)
 def test_two_in_one_launch(calc, fmt):
     """The atoms' rows and the edges', one of them normed or both: the bits of one after the other."""
