@@ -87,8 +87,9 @@ inline size_t packed_halves(int fmt, int rows, int K) {
 // Packs W [rows, K] (element (r, k) at W[r * ld_r + k * ld_k]) into `out`, and writes `unscale` (unscale_halves(rows),
 // 16-byte aligned).
 PackedB pack_weight(cudaStream_t s, Format fmt, const float* W, size_t ld_r, size_t ld_k, int rows, int K, uint16_t* out, uint16_t* unscale);
-// A weight in FMT_F16X3 whose values pack_weight found spread becomes one in FMT_F16X3_FULL. Copies a word from the device: the
-// packing has to have ended.
+// Whether pack_weight found the values of a weight in FMT_F16X3 spread. Copies a word from the device: the packing has to have ended.
+bool values_spread(const PackedB& w, int rows);
+// Such a weight becomes one in FMT_F16X3_FULL.
 void full_if_spread(PackedB& w, int rows);
 
 struct GemmArgs {

@@ -129,11 +129,15 @@ PackedB pack_weight(cudaStream_t s, Format fmt, const float* W, size_t ld_r, siz
   return w;
 }
 
-void full_if_spread(PackedB& w, int rows) {
-  if (w.fmt != FMT_F16X3 || rows <= 0) return;
+bool values_spread(const PackedB& w, int rows) {
+  if (w.fmt != FMT_F16X3 || rows <= 0) return false;
   int spread = 0;
   PETB_CUDA(cudaMemcpy(&spread, w.unscale + unscale_halves(rows) - 8, sizeof(int), cudaMemcpyDeviceToHost));
-  if (spread) w.fmt = FMT_F16X3_FULL;
+  return spread != 0;
+}
+
+void full_if_spread(PackedB& w, int rows) {
+  if (values_spread(w, rows)) w.fmt = FMT_F16X3_FULL;
 }
 
 void row_max(Stream& st, uint32_t* mx, const float* x, int ld, int R, int D) {

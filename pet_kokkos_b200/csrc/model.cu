@@ -153,6 +153,15 @@ std::vector<PlanItem> weight_plan(const Hypers& h, bool gains) {
   return plan;
 }
 
+// Whether a gain damps some features by 2^-12 and more against others (zeros leave nothing to damp). Their values may stand out by as
+// much, and a row's scale is that of its largest: two parts hold 22 bits down to 2^-18 of it.
+bool damps(const Tensor& gain) {
+  double least = INFINITY, most = 0.0;
+  for (double g : gain.data)
+    if (g != 0.0) least = std::min(least, std::fabs(g)), most = std::max(most, std::fabs(g));
+  return least < most / 4096.0;
+}
+
 }  // namespace
 
 void Model::put_mat(const std::string& name, const double* src, int ld, int rows, int cols, bool paired, bool operand, const double* gain) {
@@ -187,6 +196,22 @@ void Model::put_mat(const std::string& name, const double* src, int ld, int rows
     m.fast_t = fmt == FMT_F16X3 ? m.nat_t : pack(fmt, true);
   }
   mat_[name] = m;
+}
+
+// A weight and its norm's gain in one, or false and nothing kept. In the native mode the norm stays by itself where the gain would set the
+// weight's columns so far apart that its format needs eight products instead of six, which also never share a launch. One gain of 2^-6,
+// one way -> the other, each against all gains near one: 21 atoms 1.033 -> 1.01-1.03, water648 1.024 -> 1.01-1.02, diamond1728 both 1.02.
+// 3xTF32 has three products either way, and folds any but gains that damp by more than its parts have to spare.
+bool Model::put_after_norm(const std::string& name, const double* src, int rows, int cols, bool paired, const double* gain, const Tensor& host_gain) {
+  if (mode_ != GEMM_NATIVE && damps(host_gain)) return false;
+  const size_t kept = owned_.size();
+  put_mat(name, src, cols, rows, cols, paired, true, gain);
+  PETB_CUDA(cudaDeviceSynchronize());
+  Mat& m = mat_[name];
+  if (mode_ != GEMM_NATIVE || !values_spread(m.nat, rows)) return m.after_norm = true;
+  for (; owned_.size() > kept; owned_.pop_back()) cudaFree(owned_.back());
+  mat_.erase(name);
+  return false;
 }
 
 void Model::put_vec(const std::string& name, const double* src, int len, bool paired) {
@@ -275,8 +300,12 @@ Model::Model(const Checkpoint& ck, int gemm_mode) : h_(ck.hypers), scale_(ck.ene
     if (!it.gain.empty()) {
       const Staged gain(ck.at(it.gain));
       if (gain.rows * gain.cols != dev.cols) throw Error(1, "model: '" + it.gain + "' does not have the width of the layer after it");
-      put_mat(it.name, dev.p, dev.cols, dev.rows, dev.cols, paired, true, gain.p);
-      PETB_CUDA(cudaDeviceSynchronize());
+      if (!put_after_norm(it.name, dev.p, dev.rows, dev.cols, paired, gain.p, ck.at(it.gain))) {
+        put_mat(it.name, dev.p, dev.cols, dev.rows, dev.cols, paired, true);
+        put_vec(it.gain, gain.p, dev.cols, false);
+        norms_apart_ = true;
+      }
+      PETB_CUDA(cudaDeviceSynchronize());  // before the gain goes
     } else if (matrix) put_mat(it.name, dev.p, dev.cols, dev.rows, dev.cols, paired, it.prep != Prep::Table);
     else put_vec(it.name, dev.p, int(t.numel()), paired);
     PETB_CUDA(cudaDeviceSynchronize());
@@ -523,7 +552,7 @@ MemoryNeed Model::memory_need(int tier, int N, int E, int n_live) const {
   save += double(row_maxima_words(N, E)) * (relayer ? 2 : 1);       // (a layer run again takes its own)
   // tmp: the fullest scope
   const double attention_bwd = T * 5 * D + (keep ? 0.0 : T * 4 * D);
-  const double norms = folds_norms() ? 0.0 : 1.0;  // the norms' rows
+  const double norms = folds_norms() && !norms_apart_ ? 0.0 : 1.0;  // the norms' rows
   const double attention_fwd = norms * T * D + (keep ? 0.0 : T * 3 * D);
   const double edge_mlp = c * (2 * F + D) + (keep ? c * F : c * (2 * F + norms * D)) + n * 5 * Dn;  // (beside the atoms')
   const double combination = e * 4 * D + 2 * live * D;
@@ -587,30 +616,30 @@ PassOut Model::run_feedforward(Stream& st, Arena& save, Arena& tmp, const Packed
     at.qkv = qkv.p, at.merged = b.merged.p, at.ml = b.ml;
     return at;
   };
-  // The RMSNorms of a block: folded into the GEMM that reads them, or by themselves in the modes of one part (folds_norms). norm_of
-  // is the input of that GEMM, normed what makes of it the GEMM of the norm.
-  const bool fold = folds_norms();
-  const auto norm_of = [&](const Rows& x, const std::string& name, int R, int width) {
-    if (fold) return x;
+  // The RMSNorms of a block: in the GEMM that reads them, where the weight has taken the gain (Mat::after_norm), or by themselves. norm_of
+  // is the input of that GEMM, normed what makes of it the GEMM of the norm, gain_of what the norm's backward multiplies by.
+  const auto norm_of = [&](const Rows& x, const Mat& reader, const std::string& name, int R, int width) {
+    if (reader.after_norm) return x;
     const Rows y = maxima.fresh(tmp.alloc<float>(size_t(R > 0 ? R : 1) * width), R);
     norm_fwd(st, y.p, x.p, nullptr, vec(name + ".weight"), nullptr, R, width, y.mx);
     return y;
   };
-  const auto gain_of = [&](const std::string& name) { return fold ? nullptr : vec(name + ".weight"); };
-  const auto normed = [&](GemmArgs a) {
-    a.rms = fold ? 1.f : 0.f;
+  const auto gain_of = [&](const Mat& reader, const std::string& name) { return reader.after_norm ? nullptr : vec(name + ".weight"); };
+  const auto normed = [&](GemmArgs a, const Mat& reader) {
+    a.rms = reader.after_norm ? 1.f : 0.f;
     return a;
   };
+  const auto maxima_for = [&](const Mat& reader, size_t R) { return reader.after_norm ? maxima.take(R) : nullptr; };
   // qkv = W_in . norm(tokens) + b
   auto make_qkv = [&](const Rows& qkv, const std::string& tl, const Block& b) {
     Scope s(tmp);
-    const Rows in = norm_of(b.tok, tl + ".norm_attention", T, D);
-    gm.one(normed(Gemms::linear_args(qkv, in, mat(tl + ".attention.input_linear.weight"), vec(tl + ".attention.input_linear.bias"), T)));
+    const Mat& w = mat(tl + ".attention.input_linear.weight");
+    gm.one(normed(Gemms::linear_args(qkv, norm_of(b.tok, w, tl + ".norm_attention", T, D), w, vec(tl + ".attention.input_linear.bias"), T), w));
   };
   // The edge MLP's first half on rows [r0, r0 + nr): pre = W_in . norm(eps) + b and, with `he`, v * sigmoid(g).
   auto edge_mlp_in = [&](const Rows& he, float* pre, const Block& b, int r0, const std::string& tl, int nr) {
-    const Rows in = norm_of(b.eps.from(r0, D), tl + ".norm_mlp", nr, D);
-    return normed(Gemms::swiglu_args(he, pre, in, mat(tl + ".mlp.w_in.weight"), vec(tl + ".mlp.w_in.bias"), nr));
+    const Mat& w = mat(tl + ".mlp.w_in.weight");
+    return normed(Gemms::swiglu_args(he, pre, norm_of(b.eps.from(r0, D), w, tl + ".norm_mlp", nr, D), w, vec(tl + ".mlp.w_in.bias"), nr), w);
   };
 
   // One message-passing layer forward: node_in [N,Dn] -> node_out, input_edge [E,D] updated in place, saves in `sl`
@@ -623,7 +652,10 @@ PassOut Model::run_feedforward(Stream& st, Arena& save, Arena& tmp, const Packed
     // Token buffers: block a's tokens are [input_node ; edge_cur]; its edge output is written
     // straight into the edge rows of block a+1's, the last one's being the layer's out_edge.
     std::vector<Rows> tokbuf(A + 1);
-    for (int a = 0; a <= A; ++a) tokbuf[a] = {save.alloc<float>(Ta * D), fold && a < A ? maxima.take(Ta) : nullptr};
+    for (int a = 0; a <= A; ++a) {
+      tokbuf[a].p = save.alloc<float>(Ta * D);
+      if (a < A) tokbuf[a].mx = maxima_for(mat(g + ".trans.layers." + std::to_string(a) + ".attention.input_linear.weight"), Ta);
+    }
     sl.cpre = save.alloc<float>(Ea * D);
     const auto contraction = [&](int a, const Rows& node) {  // block a's atom tokens
       const std::string tl = g + ".trans.layers." + std::to_string(a);
@@ -650,8 +682,8 @@ PassOut Model::run_feedforward(Stream& st, Arena& save, Arena& tmp, const Packed
       b.tok = tokbuf[a];
       b.merged = maxima.fresh(save.alloc<float>(Ta * D), Ta);
       b.ml = save.alloc<float>(Ta * H * 2);
-      b.eps = {save.alloc<float>(Ea * D), fold ? maxima.take(Ea) : nullptr};
-      b.node_res = {save.alloc<float>(Na * Dn), fold ? maxima.take(Na) : nullptr};
+      b.eps = {save.alloc<float>(Ea * D), maxima_for(w_ein, Ea)};
+      b.node_res = {save.alloc<float>(Na * Dn), maxima_for(w_cin, Na)};
       b.pre_c = save.alloc<float>(Na * w_cin.rows);
       b.qkv = keep ? Rows{save.alloc<float>(Ta * 3 * D)} : Rows{};
       b.pre_e = keep ? save.alloc<float>(Ea * w_ein.rows) : nullptr;
@@ -674,9 +706,9 @@ PassOut Model::run_feedforward(Stream& st, Arena& save, Arena& tmp, const Packed
       // the atoms' MLP, and the edges' a chunk at a time: the first chunk's GEMMs share their launches with the atoms'
       Scope s2(tmp);
       const Rows hc = maxima.fresh(tmp.alloc<float>(Na * (w_cin.rows / 2)), Na);
-      const Rows node_in_rows = norm_of(b.node_res, tl + ".norm_center_features", N, Dn);
+      const Rows node_in_rows = norm_of(b.node_res, w_cin, tl + ".norm_center_features", N, Dn);
       const GemmArgs node_in_args =
-          normed(Gemms::swiglu_args(hc, b.pre_c, node_in_rows, w_cin, vec(tl + ".center_mlp.w_in.bias"), N));
+          normed(Gemms::swiglu_args(hc, b.pre_c, node_in_rows, w_cin, vec(tl + ".center_mlp.w_in.bias"), N), w_cin);
       const GemmArgs node_out_args =
           Gemms::linear_args(node_next, hc, mat(tl + ".center_mlp.w_out.weight"), vec(tl + ".center_mlp.w_out.bias"), N, b.node_res.p, 0);
       const int rows = keep || chunk <= 0 ? (E > 0 ? E : 1) : chunk;
@@ -869,12 +901,12 @@ PassOut Model::run_feedforward(Stream& st, Arena& save, Arena& tmp, const Packed
             gm.two(node_out_args, edge_out_args);
             gm.two(node_in_args, edge_in_args);
             node_adj.mx = maxima.take(Na);
-            norm_bwd_two(st, node_adj.p, cnorm_adj, b.node_res.p, gain_of(tl + ".norm_center_features"), N, Dn, node_adj.mx, adj_rows.p,
-                         enorm_adj, eps_rows, gain_of(tl + ".norm_mlp"), nr, D, eps_adj.mx);
+            norm_bwd_two(st, node_adj.p, cnorm_adj, b.node_res.p, gain_of(w_cin, tl + ".norm_center_features"), N, Dn, node_adj.mx,
+                         adj_rows.p, enorm_adj, eps_rows, gain_of(w_ein, tl + ".norm_mlp"), nr, D, eps_adj.mx);
           } else {
             gm.one(edge_out_args), gm.one(edge_in_args);
-            norm_bwd_two(st, nullptr, nullptr, nullptr, nullptr, 0, Dn, nullptr, adj_rows.p, enorm_adj, eps_rows, gain_of(tl + ".norm_mlp"), nr, D,
-                         eps_adj.from(r0, D).mx);
+            norm_bwd_two(st, nullptr, nullptr, nullptr, nullptr, 0, Dn, nullptr, adj_rows.p, enorm_adj, eps_rows,
+                         gain_of(w_ein, tl + ".norm_mlp"), nr, D, eps_adj.from(r0, D).mx);
           }
           r0 += rows;
         } while (r0 < E);
@@ -895,11 +927,12 @@ PassOut Model::run_feedforward(Stream& st, Arena& save, Arena& tmp, const Packed
         AttnArgs at = attention_args(b, qkv);
         at.dmerged = dmerged.p, at.qkv_adj = qkv_adj.p, at.qkv_adj_max = qkv_adj.mx, at.cfh = cfh;
         attention_backward(st, at);
-        gm.linear_bwd({attn_in_adj}, qkv_adj, mat(tl + ".attention.input_linear.weight"), T, false);
+        const Mat& w_qkv = mat(tl + ".attention.input_linear.weight");
+        gm.linear_bwd({attn_in_adj}, qkv_adj, w_qkv, T, false);
         // through the norm, back to where the tokens came from: atom rows to the contraction's
         // output adjoint (written), edge rows onto the edge residual (accumulated)
         tok_adj.mx = maxima.take(Ta);
-        norm_bwd(st, tok_adj.p, attn_in_adj, b.tok.p, gain_of(tl + ".norm_attention"), false, T, D, N, nullptr, tok_adj.mx);
+        norm_bwd(st, tok_adj.p, attn_in_adj, b.tok.p, gain_of(w_qkv, tl + ".norm_attention"), false, T, D, N, nullptr, tok_adj.mx);
       }
       node_adj.mx = maxima.take(Na);
       gm.linear_bwd(node_adj, tok_adj, mat(tl + ".center_contraction.weight"), N, true);

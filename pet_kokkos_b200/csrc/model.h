@@ -24,6 +24,7 @@ struct Mat {
   int rows = 0, cols = 0;
   // GEMM operands: w (and its transpose) packed for the native mode and for the mode the model was loaded for
   PackedB nat, nat_t, fast, fast_t;
+  bool after_norm = false;  // the gain of the RMSNorm before it is in it
 };
 
 struct PassOut {
@@ -100,13 +101,15 @@ class Model {
   // `src` are doubles in DEVICE memory; the layouts the kernels read are made from them by kernels.
   void put_mat(const std::string& name, const double* src, int ld, int rows, int cols, bool paired, bool operand,
                const double* gain = nullptr);
+  bool put_after_norm(const std::string& name, const double* src, int rows, int cols, bool paired, const double* gain, const Tensor& host_gain);
   void put_vec(const std::string& name, const double* src, int len, bool paired);
   void fold_compress(const Checkpoint& ck, const std::string& c0, int layer);
   void fold_expansion(const Checkpoint& ck, const std::string& block);
 
   // The feedforward featurizer's RMSNorms go into the GEMMs that read them (gain in the weight, 1 / rms in the epilogue), but for the
   // modes of one part: there what a weight loses to its operand's 8 or 11 bits is most of a mode's error, and W times a gain loses
-  // something else than W (pet-mad-s shape, two sets of random weights: forces off by 0.094 -> 0.117 and 0.044 -> 0.035 meV/A).
+  // something else than W (pet-mad-s shape, two sets of random weights: forces off by 0.094 -> 0.117 and 0.044 -> 0.035 meV/A). And but
+  // for gains that damp some features far below others (put_after_norm).
   bool folds_norms() const { return h_.feedforward && (mode_ == GEMM_NATIVE || mode_ == GEMM_TF32X3); }
   bool wide() const { return h_.d_pet > 256; }  // the tensor-core modes' forward on tf32 instructions (put_mat)
 
@@ -118,6 +121,7 @@ class Model {
   double* comp_ = nullptr;  // [n_species] composition energies
   double* probes_ = nullptr;  // [n_probes_] the grid adaptive cutoff's radii (adaptive_probes, src/neighbors.cpp:23-27)
   int n_probes_ = 0;
+  bool norms_apart_ = false;  // folds_norms, yet some weight has its norm by itself
   std::map<std::string, Mat> mat_;
   std::map<std::string, const float*> vec_;
   std::vector<void*> owned_;
