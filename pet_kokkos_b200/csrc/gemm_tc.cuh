@@ -978,10 +978,9 @@ CUtensorMap map_2d(CUtensorMapDataType type, const void* base, int cols, int row
 }
 
 // As many pairs as the device holds at once (a pair needs two SMs of one GPC: fewer than half the SMs may fit), or the last
-// pairs of a persistent kernel would start when the first ones end.
+// pairs of a persistent kernel would start when the first ones end. `table` is the kernel's own.
 template <class K>
-int resident_pairs(K kernel, cudaLaunchConfig_t cfg) {
-  static PerDevice<int> table;
+int resident_pairs(K kernel, cudaLaunchConfig_t cfg, PerDevice<int>& table) {
   int dev = 0;
   cudaGetDevice(&dev);
   return table.get(dev, [&](int& n) {
@@ -1042,6 +1041,7 @@ void launch_tc(Stream& st, const GemmTask* q, const Plan& plan) {
   using L = Tile<BN, FMT, PAIR>;
   static_assert(L::kTotal <= 227 * 1024, "the tile pipeline does not fit shared memory");
   static SmemOptIn opted;
+  static PerDevice<int> pairs;
   auto kernel = k_gemm_tc<EPI, BN, FMT, PAIR, SPLIT, SIDES>;
   opt_in_shared_memory(kernel, L::kTotal, opted);
   Sides<SIDES> g;
@@ -1062,7 +1062,7 @@ void launch_tc(Stream& st, const GemmTask* q, const Plan& plan) {
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 1;
     cfg.numAttrs = 1;
-    cfg.gridDim = dim3(unsigned(2 * std::min<long long>(tiles[0] + tiles[1], resident_pairs(kernel, cfg))));
+    cfg.gridDim = dim3(unsigned(2 * std::min<long long>(tiles[0] + tiles[1], resident_pairs(kernel, cfg, pairs))));
   } else {
     cfg.gridDim = dim3(unsigned(std::min<long long>(tiles[0] + tiles[1], tensor_state().sms)));
   }
