@@ -82,16 +82,23 @@ def test_the_scale_is_no_further_off_than_a_norm_by_itself(calc, fmt, shape):
     assert off(got) <= off(warp_norm(A))
 
 
+TWO = [((130, 512, 512), (4460, 256, 128)), ((2900, 2048, 256), (19000, 512, 256))]  # a CTA a tile; and pairs of CTAs
+
+
+@pytest.mark.parametrize("shapes", TWO)
 @pytest.mark.parametrize("fmt", FORMATS)
-def test_two_in_one_launch(calc, fmt):
+def test_two_in_one_launch(calc, fmt, shapes):
     """The atoms' rows and the edges', one of them normed or both: the bits of one after the other."""
-    shapes = ((130, 512, 512), (4460, 256, 128))
     for normed in ((True, True), (True, False), (False, True)):
         given = []
         for shape, rms in zip(shapes, normed):
             A, W, bias = problem(*shape, 5)
             given.append(dict(A=A, W=W, fmt=fmt, epilogue="swiglu", bias=bias, rms=rms))
-        for x, g in zip(calc.debug_gemm_two(*given), given):
+        before = calc.kernel_launches
+        results = calc.debug_gemm_two(*given)
+        launches = calc.kernel_launches - before - (2 if fmt.startswith("f16") else 0)  # (the passes that look for A's row maxima)
+        assert launches == (2 if fmt == "f16x3_full" else 1)
+        for x, g in zip(results, given):
             assert np.array_equal(x[0], calc.debug_gemm(**g)[0])
 
 
