@@ -261,7 +261,8 @@ void Model::fold_compress(const Checkpoint& ck, const std::string& c0, int L) {
 void Model::fold_expansion(const Checkpoint& ck, const std::string& block) {
   const Staged A(ck.at(block + ".center_expansion.weight")), y(ck.at(block + ".center_expansion.bias"));
   const Staged B(ck.at(block + ".attention.output_linear.weight")), x(ck.at(block + ".attention.output_linear.bias"));
-  if (A.cols != B.rows) throw Error(1, "model: '" + block + ".center_expansion' does not have the shape of an expansion");
+  if (A.cols != B.rows || x.rows < B.rows || y.rows < A.rows)  // (the fold reads them at these lengths)
+    throw Error(1, "model: '" + block + ".center_expansion' does not have the shape of an expansion");
   const Staged W(size_t(A.rows) * B.cols), b(size_t(A.rows));
   k_fold_layers<<<cdiv((long long) A.rows * (B.cols + 1), 128), 128>>>(A.p, B.p, x.p, y.p, A.rows, A.cols, B.cols, W.p, b.p);
   PETB_CUDA(cudaGetLastError());

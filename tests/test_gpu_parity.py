@@ -297,3 +297,18 @@ def test_a_steady_loop_stops_asking_the_driver_for_free_memory(lib_path, models)
     c.compute(large)  # ... so the next one finds them changed and asks again
     assert c.driver_memory_queries > asked, "the pools grew: the cached answer is stale"
     c.close()
+
+
+def test_a_bias_shorter_than_its_fold_is_refused(lib_path, models, tmp_path):
+    """The atoms' expansion is made with the layer before it when a model is loaded, from weights and biases of matching lengths."""
+    from pet_kokkos_b200 import Calculator
+    jp, sp = models("tiny")
+    meta, tens = ck.load_checkpoint(jp, sp)
+    for which in (".center_expansion.bias", ".attention.output_linear.bias"):
+        there = {k: np.array(v, np.float32) for k, v in tens.items()}
+        for n in there:
+            if n.endswith(which):
+                there[n] = there[n][:4]
+        ck.write_safetensors(tmp_path / "short.safetensors", there)
+        with pytest.raises(RuntimeError, match="shape of an expansion"):
+            Calculator(jp, str(tmp_path / "short.safetensors"))
