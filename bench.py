@@ -51,11 +51,11 @@ os.environ.setdefault("OMP_WAIT_POLICY", "passive")
 
 METRIC = "atom_evals_per_s"
 UNIT = "atom-evals/s"
-# DRAM traffic of one weight-GEMM launch per token row (atoms + kept edges), from one ncu capture:
-# dram__bytes_read.sum + dram__bytes_write.sum averaged over the 86 k_gemm_tc launches of one evaluation of the water648
-# workload in the 3xTF32 mode, token-row and atom-row GEMMs as they come (47.6 MB at 25 320 rows;
-# summarised under profiles/). A GEMM reads A once and writes C once, so it grows with the rows.
-GEMM_DRAM_BYTES_PER_TOKEN_ROW = 47.6e6 / 25320
+# DRAM traffic of the weight GEMMs of one evaluation per token row (atoms + kept edges), from one ncu capture:
+# dram__bytes_read.sum + dram__bytes_write.sum over the 56 k_gemm_tc launches of an evaluation of the water648 workload in
+# the 3xTF32 mode, caches flushed before each (4265 MB at 25 320 rows; summarised under profiles/). A GEMM reads A once and
+# writes C once, so it grows with the rows.
+GEMM_DRAM_BYTES_PER_TOKEN_ROW = 4265e6 / 25320
 # products of 16-bit parts that one product of the mode takes on the tensor cores
 PRODUCTS_OF = {"native": 6, "3xtf32": 3, "tf32": 1, "bf16": 1}
 DTYPE_OF = {"native": "f32", "tf32": "tf32", "bf16": "bf16", "3xtf32": "f32 (3xTF32)"}
@@ -580,9 +580,9 @@ def run_ours(args):
                 roof = {"kernel": "weight GEMMs with fused epilogues", "bound": "tensor", "achieved": ach,
                         "peak": peaks["bf16_tflops_sustained"], "unit": "TFLOP/s", "frac": ach / peaks["bf16_tflops_sustained"],
                         "peak_source": f"{peaks['source']} cuBLAS bf16, sustained",
-                        "traffic": GEMM_DRAM_BYTES_PER_TOKEN_ROW * (n_act + n_edges),
-                        "traffic_source": "ncu dram bytes per launch on water648 (summarised under profiles/), "
-                                          "scaled by token rows",
+                        "traffic": GEMM_DRAM_BYTES_PER_TOKEN_ROW * (n_act + n_edges) * 2 / p["launches"],  # (two steps profiled)
+                        "traffic_source": "ncu dram bytes of an evaluation's weight GEMMs on water648 (summarised under "
+                                          "profiles/), scaled by token rows, a launch",
                         "launches": p["launches"], "avg_launch_ms": per_launch_ms}
                 # what the mode asks of the tensor cores: so many products of 16-bit parts for one of its own, at the bf16 rate
                 # (the forward of a model wider than 256 runs in the 3xTF32 and tf32 modes on tf32 instructions, at half of it)

@@ -163,7 +163,7 @@ struct Tile {
   // Steps whose products go into one accumulator. FMT_F16X3's h.h products sum exactly over 1024 columns of K; up to 4096 a
   // longer K goes in four pieces, one for each of four CTAs that share a tile (SPLIT).
   static __device__ int drain(int K) { return !X3 ? 1 << 30 : K > 1024 && K <= 4096 ? (K + 127) / 128 : 1024 / BK; }
-  // 24 + 2 x 200 + 88 registers a thread over the warp groups are the 4 x 128 of the launch, 40 + 2 x 136 + 2 x 80 within the 5 x 96
+  // 40 + 2 x 192 + 88 registers a thread over the warp groups are the 4 x 128 of the launch; 48 + 2 x 136 + 2 x 80 the 5 x 96
   static constexpr bool kMoveRegs = TA || (X3 && BN >= 128);
   static constexpr int kRegsProd = TA ? 48 : 40, kRegsEpi = TA ? 136 : 192, kRegsConv = TA ? 80 : 88;
   static_assert(!T1 || !PAIR, "FMT_TF32 has no converter to tell the other CTA's issuer that a slab has landed");

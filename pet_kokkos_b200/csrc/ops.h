@@ -57,7 +57,7 @@ void concat_norm_bwd(Stream& st, float* edge_adj, const float* out_adj, const fl
 void concat_norm_remote_bwd(Stream& st, float* send, const float* out_adj, const float* oe, const float* w,
                             const int* live_packed, int n_live, int D, RemoteRows remote);
 
-// x4_adj(k,c) += sum_d g(k,d) wx(d,c)  (the reduction of compress_bwd, src/ops.cpp:373-401)
+// x4_adj(k,c) = sum_d g(k,d) wx(d,c), with `add` on top of what is there  (the reduction of compress_bwd, src/ops.cpp:373-401)
 void compress_geometry_bwd(Stream& st, float* x4_adj, const float* g, const float* wx, int E, int D, bool add);
 
 // net(n) = float(node_pred(n) + sum_k double(cut k) * double(edge_pred k)); per_atom(n) = scale*net + comp[species]
@@ -70,7 +70,8 @@ void readout_energy(Stream& st, float* net, double* per_atom, const float* node_
 void readout_seed_bwd(Stream& st, float* out, const float* w, const float* pre, const float* cut, const int* center,
                       int n_local, int R, int Dh, uint32_t* mx = nullptr);
 
-// cf_adj(k) += (sum_h cfh(N+k,h)) / cut(k)  (attn_bwd_cf, src/attention.cpp:1829-1838; only edge slots carry a gradient)
+// cf_adj(k) = sum over the attention blocks, `stride` apart, of (sum_h cfh(N+k,h)) / cut(k); 0 where cut(k) is
+// (attn_bwd_cf, src/attention.cpp:1829-1838; only edge slots carry a gradient)
 void cutoff_share(Stream& st, float* cf_adj, const float* cfh, size_t stride, int blocks, const float* cut, int N, int E, int H);
 
 // a += b, elementwise
