@@ -115,22 +115,26 @@ def test_outliers_that_a_gain_damps(lib_path, tmp_path, init, binades, gemm):
     assert dF <= f_band and dE <= e_band
 
 
+def one_feature_damped(tmp_path, gain):
+    jp, sp = ck.write_random_checkpoint(tmp_path / "plain", dict(d_pet=64, num_heads=2, d_feedforward=64, cutoff=4.5), seed=5, init="n002")
+    meta, tens = ck.load_checkpoint(jp, sp)
+    there = {k: np.array(v, np.float32) for k, v in tens.items()}
+    for n in there:
+        if n.endswith((".norm_attention.weight", ".norm_mlp.weight", ".norm_center_features.weight")):
+            there[n][5] = gain
+    ck.write_safetensors(tmp_path / "damped.safetensors", there)
+    return meta, jp, sp, str(tmp_path / "damped.safetensors")
+
+
 @pytest.mark.parametrize("gemm,damped,apart", [("native", 2.0 ** -6, True), ("native", 0.9, False), ("3xtf32", 2.0 ** -6, False),
                                                ("3xtf32", 2.0 ** -13, True), ("3xtf32", 0.0, False), ("bf16", 2.0 ** -13, False)])
 def test_a_gain_that_spreads_a_weight_stays_out_of_it(lib_path, tmp_path, gemm, damped, apart):
     """Three norms a block run by themselves then, and nothing else changes: the GEMMs keep the format in which two of them share a launch
     (64 atoms: all do that can)."""
     from pet_kokkos_b200 import Calculator
-    shape = dict(d_pet=64, num_heads=2, d_feedforward=64, cutoff=4.5)
-    jp, sp = ck.write_random_checkpoint(tmp_path / "plain", shape, seed=5, init="n002")
-    meta, tens = ck.load_checkpoint(jp, sp)
-    there = {k: np.array(v, np.float32) for k, v in tens.items()}
-    for n in there:
-        if n.endswith((".norm_attention.weight", ".norm_mlp.weight", ".norm_center_features.weight")):
-            there[n][5] = damped
-    ck.write_safetensors(tmp_path / "damped.safetensors", there)
+    meta, jp, sp, damped_sp = one_feature_damped(tmp_path, damped)
     launches = []
-    for weights in (sp, str(tmp_path / "damped.safetensors")):
+    for weights in (sp, damped_sp):
         c = Calculator(jp, weights, gemm=gemm)
         c.compute([st.diamond(2, jitter=0.05, seed=0)])
         before = c.kernel_launches
@@ -139,3 +143,19 @@ def test_a_gain_that_spreads_a_weight_stays_out_of_it(lib_path, tmp_path, gemm, 
         c.close()
     h = meta["hypers"]
     assert launches[1] - launches[0] == (3 * h["num_gnn_layers"] * h["num_attention_layers"] if apart else 0), launches
+
+
+def test_norms_apart_under_every_tier(lib_path, tmp_path, monkeypatch):
+    """The rows and row maxima of norms by themselves in passes that make them again, edges in chunks: the same bits."""
+    from pet_kokkos_b200 import Calculator
+    monkeypatch.setenv("PET_EDGE_CHUNK", "900")
+    _, jp, _, sp = one_feature_damped(tmp_path, 2.0 ** -6)
+    results = []
+    for tier in ("never", "wide", "layers"):
+        c = Calculator(jp, sp, recompute=tier)
+        r = c.compute([st.diamond(2, jitter=0.05, seed=0)])
+        results.append((r.energy, r.forces, r.virial))
+        c.close()
+    for other in results[1:]:
+        for x, y in zip(results[0], other):
+            assert np.array_equal(x, y)
